@@ -2,8 +2,8 @@
 //
 // EFLA, per (batch, head), state S [d, d] fp32 (row = key index i, column = value index j):
 //   lam = |k|^2, c = (1 - exp(-beta lam)) / lam, p = S^T k, e = v - p, S += c k e^T, o = p + c lam e
-// (o equals S_new^T k). Forward: one CTA of four warps per (batch, head, 32 value columns); its threads keep the
-// state in registers for the whole sequence so it never leaves the chip and is never rounded to bf16 - the
+// (o equals S_new^T k). Forward for a few tokens (longer blocks: efla_chunk.cu): one CTA of four warps per (batch, head, 32 value
+// columns); its threads keep the state in registers for all tokens so it never leaves the chip and is never rounded to bf16 - the
 // reference rounds the bf16 state in global memory on every token and launches once per chunk
 // (reference: kernels/cuda/efla.cu:121-197 forward, :199-271 state history, :273-401 backward
 // without the beta gradient; fp32 variant kernels/cuda/efla_scan.cu:99-260 with grad_beta via
@@ -18,26 +18,14 @@
 // kernels/cuda/convolution.cu:4-57,126-189; src/model/prism.zig:948-973). The weight gradient is one
 // pass over the rows per (32 channels, 4 taps) without atomics.
 #include "common.cuh"
+#include "efla_math.cuh"
 #include "elfa_native.h"
 
 namespace elfa {
 namespace {
 
-__device__ __forceinline__ void efla_coeff(float beta, float lam, float& c, float& dc_dbeta, float& dc_dlam) {
-  if (lam < 1e-6f) {
-    c = beta - 0.5f * beta * beta * lam + beta * beta * beta * lam * lam / 6.f;
-    dc_dbeta = 1.f - beta * lam + 0.5f * beta * beta * lam * lam;
-    dc_dlam = -0.5f * beta * beta + beta * beta * beta * lam / 3.f;
-  } else {
-    const float ex = __expf(-beta * lam);
-    c = (1.f - ex) / lam;
-    dc_dbeta = ex;
-    dc_dlam = (beta * lam * ex - (1.f - ex)) / (lam * lam);
-  }
-}
-
-// k, v, o: [B, T, H, D] bf16. state0 / state_out: [B, H, D, D] fp32. ckpt: [B, H, nchunks, D, D] holds the
-// state at the START of every chunk.
+// Token by token, for a few tokens without a gradient (generation): one launch, nothing else to prepare.
+// k, v, o: [B, T, H, D] bf16. state0 / state_out: [B, H, D, D] fp32.
 // The columns of S evolve independently (column j needs k_t, c_t and v_t[j] only), so a CTA owns 32 value columns:
 // grid (B*H, D/32). Its four warps split the D key rows: warp w keeps rows [w D/4, (w+1) D/4) of the 32 columns in
 // registers (lane = column), so the dependent instruction chain of a step is a quarter as long and the four
@@ -122,8 +110,7 @@ __device__ __forceinline__ float efla_step(float (&S)[R], const float* __restric
 template <int D>
 __global__ void __launch_bounds__(32 * EFLA_W) efla_scan_fwd_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
                                                                     const float* __restrict__ beta_ptr, const float* __restrict__ state0,
-                                                                    __nv_bfloat16* __restrict__ o, float* __restrict__ state_out,
-                                                                    float* __restrict__ ckpt, int T, int H, int chunk) {
+                                                                    __nv_bfloat16* __restrict__ o, float* __restrict__ state_out, int T, int H) {
   constexpr int R = D / EFLA_W;
   __shared__ __align__(16) float sk[EFLA_TT][D];
   __shared__ float sv[EFLA_TT][32];
@@ -135,18 +122,12 @@ __global__ void __launch_bounds__(32 * EFLA_W) efla_scan_fwd_kernel(const __nv_b
   float S[R];
 #pragma unroll
   for (int i = 0; i < R; ++i) S[i] = state0 ? state0[((long long)bh * D + i0 + i) * D + col] : 0.f;
-  const int nchunks = (T + chunk - 1) / chunk;
   for (int t0 = 0; t0 < T; t0 += EFLA_TT) {
     const int n = min(EFLA_TT, T - t0);
     efla_load_tile<D>(k, v, nullptr, sk, sv, nullptr, sc, slam, beta, (((long long)b * T + t0) * H + h) * D, (long long)H * D, col, n,
                       warp, lane);
     for (int r = 0; r < n; ++r) {
       const int t = t0 + r;
-      if (ckpt && t % chunk == 0) {
-        float* dst = ckpt + ((long long)bh * nchunks + t / chunk) * D * D;
-#pragma unroll
-        for (int i = 0; i < R; ++i) dst[(i0 + i) * D + col] = S[i];
-      }
       const float c_ = sc[r], vj = sv[r][lane];
       const float p = efla_step<R>(S, sk[r] + i0, c_, vj, spart[r & 1], warp, lane);
       if (warp == 0) o[(((long long)b * T + t) * H + h) * D + col] = __float2bfloat16(p + c_ * slam[r] * (vj - p));
@@ -419,10 +400,10 @@ __global__ void __launch_bounds__(1024) shortconv_bwd_dw_kernel(const __nv_bfloa
 }
 
 template <int D>
-int launch_efla_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out, float* ckpt, int B,
-                    int T, int H, int chunk, cudaStream_t s) {
+int launch_efla_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out, int B,
+                    int T, int H, cudaStream_t s) {
   efla_scan_fwd_kernel<D><<<dim3(B * H, D / 32), 32 * EFLA_W, 0, s>>>(static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), beta, state0,
-                                              static_cast<__nv_bfloat16*>(o), state_out, ckpt, T, H, chunk);
+                                              static_cast<__nv_bfloat16*>(o), state_out, T, H);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;
@@ -449,17 +430,16 @@ int launch_efla_bwd(const void* k, const void* v, const float* beta, const float
 
 using namespace elfa;
 
-// k, v, o: [B, T, H, d] bf16; beta: 1 float; state0 (optional) / state_out: [B, H, d, d] fp32;
-// ckpt: [B, H, ceil(T/chunk), d, d] fp32 (chunk-start states, needed by backward) or null.
+// k, v, o: [B, T, H, d] bf16; beta: 1 float; state0 (optional) / state_out: [B, H, d, d] fp32.
 ELFA_API int elfa_efla_scan_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
-                                float* ckpt, int B, int T, int H, int d, int chunk, void* stream) {
-  ELFA_REQUIRE(k && v && beta && o && B > 0 && T > 0 && H > 0 && chunk > 0, "efla_scan_fwd: bad arguments");
+                                int B, int T, int H, int d, void* stream) {
+  ELFA_REQUIRE(k && v && beta && o && B > 0 && T > 0 && H > 0, "efla_scan_fwd: bad arguments");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (d) {
-    case 32: return launch_efla_fwd<32>(k, v, beta, state0, o, state_out, ckpt, B, T, H, chunk, s);
-    case 64: return launch_efla_fwd<64>(k, v, beta, state0, o, state_out, ckpt, B, T, H, chunk, s);
-    case 96: return launch_efla_fwd<96>(k, v, beta, state0, o, state_out, ckpt, B, T, H, chunk, s);
-    case 128: return launch_efla_fwd<128>(k, v, beta, state0, o, state_out, ckpt, B, T, H, chunk, s);
+    case 32: return launch_efla_fwd<32>(k, v, beta, state0, o, state_out, B, T, H, s);
+    case 64: return launch_efla_fwd<64>(k, v, beta, state0, o, state_out, B, T, H, s);
+    case 96: return launch_efla_fwd<96>(k, v, beta, state0, o, state_out, B, T, H, s);
+    case 128: return launch_efla_fwd<128>(k, v, beta, state0, o, state_out, B, T, H, s);
     default: set_last_error("efla_scan_fwd: head dimension must be 32, 64, 96 or 128"); return ELFA_ERR_UNSUPPORTED;
   }
 }

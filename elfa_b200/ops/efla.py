@@ -23,7 +23,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from ..native import lib, stream_ptr
+from ..native import NativeError, lib, stream_ptr
 from .gemm import gelu_tanh_ref
 
 
@@ -90,30 +90,49 @@ def efla_scan_chunked_ref(k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, 
     return o[:, :T], S
 
 
+_EFLA_CHUNK = 32           # tokens of a chunk of the tensor-core kernels
+# Up to this many tokens without a gradient, one token after the other in one launch beats the two launches of the chunked form
+# (B 8, H 16, d 64, per call on the device: T 1 2.8 us against 8.2, T 16 6.1 against 9.1, T 24 7.7 against 9.4, T 32 9.2 against 9.5;
+# the line lies below the crossing because more heads move it down).
+_EFLA_STEP_TOKENS = 16
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t``, contiguous and on a 16-byte boundary (the kernels copy 16 bytes at a time)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _EflaScan(torch.autograd.Function):
-    """CUDA path: sequential-in-time kernels, one warp per (batch, head, 32 value columns) with its columns
-    of the fp32 state in registers; backward recomputes the states inside each chunk from the
-    chunk-boundary states saved by forward."""
+    """CUDA path. Forward: chunks of 32 tokens on the tensor cores with the fp32 state in registers. Backward recomputes the states
+    inside each chunk from the chunk-boundary states saved by forward (only when a gradient is wanted)."""
 
     @staticmethod
-    def forward(ctx, k, v, beta, state, chunk):
+    def forward(ctx, k, v, beta, state, want_grad):
         B, T, H, d = k.shape
-        kc, vc = k.contiguous(), v.contiguous()
+        kc, vc = _aligned(k), _aligned(v)
         o = torch.empty_like(kc)
-        nchunks = (T + chunk - 1) // chunk
-        ckpt = torch.empty((B, H, nchunks, d, d), dtype=torch.float32, device=k.device)
         s_out = torch.empty((B, H, d, d), dtype=torch.float32, device=k.device)
         bt = beta.detach().float().reshape(1).contiguous()
         st0 = state.float().contiguous() if state is not None else None
-        lib.call("elfa_efla_scan_fwd", kc, vc, bt, st0, o, s_out, ckpt, B, T, H, d, chunk, stream_ptr(kc))
-        ctx.save_for_backward(kc, vc, bt, ckpt)
-        ctx.cfg = (B, T, H, d, chunk, state is not None)
+        if T <= _EFLA_STEP_TOKENS and not want_grad:
+            lib.call("elfa_efla_scan_fwd", kc, vc, bt, st0, o, s_out, B, T, H, d, stream_ptr(kc))
+            return o, s_out
+        nchunks = (T + _EFLA_CHUNK - 1) // _EFLA_CHUNK
+        ckpt = torch.empty((B, H, nchunks, d, d), dtype=torch.float32, device=k.device) if want_grad else None
+        nmat = torch.empty((B, H, nchunks, 3, _EFLA_CHUNK, _EFLA_CHUNK), dtype=torch.bfloat16, device=k.device)
+        coef = torch.empty((B, H, nchunks, 2, _EFLA_CHUNK), dtype=torch.float32, device=k.device)
+        lib.call("elfa_efla_chunk_fwd", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, B, T, H, d, stream_ptr(kc))
+        if want_grad:
+            ctx.save_for_backward(kc, vc, bt, ckpt)
+            ctx.cfg = (B, T, H, d, state is not None)
         return o, s_out
 
     @staticmethod
     def backward(ctx, do, ds_out):
         kc, vc, bt, ckpt = ctx.saved_tensors
-        B, T, H, d, chunk, has_state = ctx.cfg
+        B, T, H, d, has_state = ctx.cfg
+        chunk = _EFLA_CHUNK
         dk = torch.empty_like(kc)
         dv = torch.empty_like(vc)
         rows = B * T * H
@@ -131,10 +150,14 @@ class _EflaScan(torch.autograd.Function):
 def efla_scan(k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, state: Optional[torch.Tensor] = None, chunk: int = 16
               ) -> Tuple[torch.Tensor, torch.Tensor]:
     """EFLA recurrence. CPU tensors use the differentiable reference loop; CUDA bf16 tensors use the
-    native kernels when the head dimension is supported (multiple of 32, at most 128)."""
+    native kernels when the head dimension is supported (multiple of 32, at most 128). ``chunk`` (a positive number) is a hint on
+    how often a state is kept for backward and never changes the result; the native kernels keep one every 32 tokens."""
     d = k.shape[-1]
     if k.is_cuda and k.dtype == torch.bfloat16 and d % 32 == 0 and d <= 128:
-        o, s = _EflaScan.apply(k, v, beta.reshape(1), state, chunk)
+        if chunk <= 0:
+            raise NativeError("efla_scan: chunk must be positive")
+        want = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (k, v, beta, state))
+        o, s = _EflaScan.apply(k, v, beta.reshape(1), state, want)
         return o, s
     # CPU / unsupported shapes: the chunk-parallel form for long sequences (same values up to fp32 rounding, a fraction of
     # the Python-loop time), the token-by-token oracle otherwise

@@ -1,0 +1,62 @@
+"""Chunked EFLA kernels at the edges of a chunk (32 tokens) and of the one-launch form (16 tokens), against the fp32 token loop.
+
+Bounds: outputs and k / v gradients are rounded to bf16 once (2^-9 of the value; 2^-8 of the largest allows for the fp32 noise of both
+sides), states and their gradients stay in fp32 on both sides, where each of the T updates rounds at 2^-24: 1e-5 of the largest covers
+T <= 130 updates of each side.
+"""
+import pytest
+import torch
+
+from elfa_b200 import native
+from elfa_b200.ops import efla as eops
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(dev, B, T, H, d, with_state, seed=0):
+    g = torch.Generator(device=dev).manual_seed(seed)
+    k = (torch.randn(B, T, H, d, generator=g, device=dev) * 0.4).bfloat16()
+    v = torch.randn(B, T, H, d, generator=g, device=dev).bfloat16()
+    s0 = 0.3 * torch.randn(B, H, d, d, generator=g, device=dev) if with_state else None
+    return k, v, torch.tensor([0.3], device=dev), s0
+
+
+def _close(a, b, rel):
+    assert (a.float() - b.float()).abs().max() <= rel * b.float().abs().max()
+
+
+@pytest.mark.parametrize("T", [1, 16, 17, 31, 32, 33, 65, 130])
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+def test_forward_at_chunk_edges(cuda_device, T, d):
+    k, v, beta, s0 = _inputs(cuda_device, 2, T, 3, d, T % 2 == 1, seed=T + d)
+    o, s = eops.efla_scan(k, v, beta, s0)
+    o_ref, s_ref = eops.efla_scan_ref(k, v, beta, s0)
+    assert native.status() == 0
+    _close(o, o_ref, 2 ** -8)
+    _close(s, s_ref, 1e-5)
+
+
+def test_forward_takes_any_layout_and_offset(cuda_device):
+    k, v, beta, _ = _inputs(cuda_device, 2, 40, 2, 64, False)
+    want = eops.efla_scan(k, v, beta)
+    odd = torch.empty(k.numel() + 1, dtype=k.dtype, device=cuda_device)[1:].view(k.shape)     # 2-byte aligned only
+    odd.copy_(k)
+    wide = torch.empty(2, 40, 2, 128, dtype=v.dtype, device=cuda_device)[..., :64]
+    wide.copy_(v)
+    got = eops.efla_scan(odd, wide, beta)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_bad_token_leaves_the_earlier_ones_alone(cuda_device, bad):
+    k, v, beta, _ = _inputs(cuda_device, 1, 64, 1, 64, False)
+    o0, _ = eops.efla_scan(k, v, beta)
+    for which in (0, 1):
+        kv = [k.clone(), v.clone()]
+        kv[which][0, 40, 0, 5] = bad
+        o, _ = eops.efla_scan(*kv, beta)
+        assert torch.equal(o[0, :40], o0[0, :40])
+        assert not torch.isfinite(o[0, 40, 0]).all()
+        if which == 1:                      # a value touches its own column only
+            keep = [j for j in range(64) if j != 5]
+            assert torch.equal(o[0, :, 0, keep], o0[0, :, 0, keep])
