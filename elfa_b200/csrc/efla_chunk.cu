@@ -17,7 +17,6 @@
 // reference: kernels/cuda/efla.cu:121-271,534-552 (chunks are scanned one after the other, the bf16 state in global memory).
 #include "common.cuh"
 #include "elfa_native.h"
-#include "efla_math.cuh"
 #include "mma_sync.cuh"
 
 namespace elfa {
@@ -26,11 +25,14 @@ namespace {
 constexpr int EC = 32;                     // tokens of a chunk
 constexpr int EN_LD = 40;                  // row pitch of N in shared memory (bf16)
 constexpr int EN_ELEMS = 3 * EC * EC;      // one chunk's N: [split][t][s] bf16 in global memory
+constexpr int EC_COEF = 4 * EC;            // one chunk's coefficients in global memory
 
 // ------------------------------------------------------------------------------------------------ state-independent part
 // One warp per (batch, head, chunk): Gram matrix by mma.sync (exact bf16 products), then lane s eliminates column s of the unit
 // lower triangular matrix by forward substitution in fp32 registers (496 multiply-adds, rows broadcast from shared memory).
-// coef: [.., 0][t] = c, [.., 1][t] = ex. Tokens past the end have k = 0: they change neither the state nor another token.
+// coef: [.., 0][t] = c, [1] = ex, [2] = lam, [3] = dc / dlam, evaluated in fp64 and rounded once (one exponential per token; the gradient of
+// beta is a long sum of terms dc_t ex_t in which an error of lam or ex common to all tokens would not average out). Tokens past the
+// end have k = 0: they change neither the state nor another token.
 template <int D>
 __global__ void __launch_bounds__(64) efla_prep_kernel(const __nv_bfloat16* __restrict__ k, const float* __restrict__ beta_ptr,
                                                        __nv_bfloat16* __restrict__ nmat, float* __restrict__ coef, int T, int H,
@@ -79,12 +81,34 @@ __global__ void __launch_bounds__(64) efla_prep_kernel(const __nv_bfloat16* __re
     }
   }
   __syncwarp();
-  float c_, d1, d2;
-  const float lam = sg[lane][lane], beta = *beta_ptr;
-  efla_coeff(beta, lam, c_, d1, d2);
-  const float ex = lam < 1e-6f ? 1.f - c_ * lam : d1;
-  coef[id * 2 * EC + lane] = c_;
-  coef[id * 2 * EC + EC + lane] = ex;
+  double lam = 0.;
+#pragma unroll
+  for (int i = 0; i < D / 8; ++i) {
+    const uint4 v = *reinterpret_cast<const uint4*>(sk + lane * LD + i * 8);
+    const uint32_t* pv = reinterpret_cast<const uint32_t*>(&v);
+    float p[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = bf16_lo(pv[j]) * bf16_lo(pv[j]) + bf16_hi(pv[j]) * bf16_hi(pv[j]);
+    lam += (double)((p[0] + p[1]) + (p[2] + p[3]));
+  }
+  const double beta = *beta_ptr, x_ = beta * lam;
+  double c, ex, dl;
+  if (fabs(x_) < 1e-3) {                   // series: 1 - ex would cancel
+    c = beta * (1. - x_ * (0.5 - x_ * (1. / 6. - x_ / 24.)));
+    ex = 1. - c * lam;
+    dl = beta * beta * (x_ * (1. / 3. - x_ / 8.) - 0.5);
+  } else {
+    const double inv = 1. / lam;
+    ex = exp(-x_);
+    c = (1. - ex) * inv;
+    dl = (beta * ex - c) * inv;
+  }
+  const float c_ = (float)c;
+  float* cf = coef + id * EC_COEF;
+  cf[lane] = c_;
+  cf[EC + lane] = (float)ex;
+  cf[2 * EC + lane] = (float)lam;
+  cf[3 * EC + lane] = (float)dl;
   __syncwarp();
   for (int t = 0; t < EC; ++t)
     if (lane < t) sg[t][lane] *= c_;       // A[t][r] = G[t][r] c_r
@@ -107,18 +131,19 @@ __global__ void __launch_bounds__(64) efla_prep_kernel(const __nv_bfloat16* __re
     const float s = (s0 + s1) + (s2 + s3);
     x[t] = t < lane ? 0.f : (t == lane ? 1.f : -s);
   }
-  __nv_bfloat16* out = nmat + id * EN_ELEMS;
+  // neighbouring lanes trade halves so that a store carries two columns: even lanes write row t, odd lanes row t + 1
+  uint32_t* out = reinterpret_cast<uint32_t*>(nmat + id * EN_ELEMS) + (lane & 1) * (EC / 2) + (lane >> 1);
+  auto put = [&](int split, int t, uint32_t v) {
+    const uint32_t w = __shfl_xor_sync(0xffffffffu, v, 1);
+    out[(split * EC + t) * (EC / 2)] = (lane & 1) ? __byte_perm(w, v, 0x7632) : __byte_perm(v, w, 0x5410);
+  };
 #pragma unroll
   for (int t = 0; t < EC; t += 2) {
     uint32_t hi, mid, lo;
     split3(t > lane ? x[t] : 0.f, t + 1 > lane ? x[t + 1] : 0.f, hi, mid, lo);
-    uint16_t* o16 = reinterpret_cast<uint16_t*>(out);
-    o16[t * EC + lane] = (uint16_t)hi;
-    o16[(t + 1) * EC + lane] = (uint16_t)(hi >> 16);
-    o16[EC * EC + t * EC + lane] = (uint16_t)mid;
-    o16[EC * EC + (t + 1) * EC + lane] = (uint16_t)(mid >> 16);
-    o16[2 * EC * EC + t * EC + lane] = (uint16_t)lo;
-    o16[2 * EC * EC + (t + 1) * EC + lane] = (uint16_t)(lo >> 16);
+    put(0, t, hi);
+    put(1, t, mid);
+    put(2, t, lo);
   }
 }
 
@@ -249,8 +274,14 @@ __device__ __forceinline__ void efla_state_update(float (&S)[D / 8][4], const fl
   }
 }
 
+// Chunk-boundary states are stored as the warps hold them: [B, H, chunk][d / 16 value blocks][d / 8 tiles][lane] float4.
+template <int D>
+__device__ __forceinline__ long long efla_state_slot(long long chunk_id, int vblock, int lane) {
+  return ((chunk_id * (D / 16) + vblock) * (D / 8)) * 32 + lane;      // float4 units; tile n at + 32 n
+}
+
 // Grid (B * H, d / columns of a CTA). k, v, o: [B, T, H, d] bf16. state0 / state_out: [B, H, d, d] fp32 or null. ckpt (or null):
-// [B, H, nchunks, d, d] fp32, the state at the start of every chunk.
+// the state at the start of every chunk.
 // Bound by the dependent chain of a chunk (about 130 mma.sync and 700 instructions of one warp per scheduler), not by memory. With the
 // preparation, B 1, T 8192, 16 heads of 64, no gradient: 397 us, token by token (with its checkpoints) 2364 us; in the training step of
 // B 8, T 2048 the forward went from about 0.75 to 0.13 ms.
@@ -258,7 +289,7 @@ template <int D>
 __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ nmat,
     const float* __restrict__ coef, const float* __restrict__ state0, __nv_bfloat16* __restrict__ o, float* __restrict__ state_out,
-    float* __restrict__ ckpt, int T, int H, int nchunks) {
+    float4* __restrict__ ckpt, int T, int H, int nchunks) {
   using L = EflaStage<D>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
@@ -269,7 +300,7 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
   const long long row0 = ((long long)b * T * H + h) * D, rs = (long long)H * D;
   const __nv_bfloat16 *kb = k + row0, *vb = v + row0 + ccol;
   const __nv_bfloat16* nb = nmat + (long long)bh * nchunks * EN_ELEMS;
-  const float* cb = coef + (long long)bh * nchunks * 2 * EC;
+  const float* cb = coef + (long long)bh * nchunks * EC_COEF;
 
   float S[D / 8][4];                       // S^T: value column g (+ 8), key row 8 n + 2q (+ 1)
 #pragma unroll
@@ -281,7 +312,7 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
   auto fetch = [&](int ch) {
     if (ch < nchunks)
       efla_stage_load<D>(ring + (ch % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, vb + (long long)ch * EC * rs,
-                         nb + (long long)ch * EN_ELEMS, cb + (long long)ch * 2 * EC, rs, min(EC, T - ch * EC));
+                         nb + (long long)ch * EN_ELEMS, cb + (long long)ch * EC_COEF, rs, min(EC, T - ch * EC));
     cp_async_commit();
   };
 #pragma unroll
@@ -293,11 +324,9 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
     const uint32_t st = ring + (ch % EC_STAGES) * L::BYTES;
     const float* cf = reinterpret_cast<const float*>(smem + (ch % EC_STAGES) * L::BYTES + L::C);
     if (ckpt) {
-      float* dst = ckpt + ((long long)bh * nchunks + ch) * D * D + wcol + g;
+      float4* dst = ckpt + efla_state_slot<D>((long long)bh * nchunks + ch, wcol / 16, lane);
 #pragma unroll
-      for (int n = 0; n < D / 8; ++n)
-#pragma unroll
-        for (int x = 0; x < 4; ++x) dst[(n * 8 + 2 * q + (x & 1)) * D + (x >> 1) * 8] = S[n][x];
+      for (int n = 0; n < D / 8; ++n) dst[n * 32] = make_float4(S[n][0], S[n][1], S[n][2], S[n][3]);
     }
     float e[4][4];
     efla_state_times_k<D>(e, S, st + L::K, lane);
@@ -389,7 +418,461 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
   ELFA_CUDA(cudaFuncSetAttribute(efla_chunk_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   efla_chunk_fwd_kernel<D><<<dim3(B * H, D / L::VC), 32 * ec_warps<D>(), bytes, s>>>(
       static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), static_cast<const __nv_bfloat16*>(nmat), coef, state0,
-      static_cast<__nv_bfloat16*>(o), state_out, ckpt, T, H, nchunks);
+      static_cast<__nv_bfloat16*>(o), state_out, reinterpret_cast<float4*>(ckpt), T, H, nchunks);
+  ELFA_CUDA(cudaGetLastError());
+  ::elfa::count_launches(2);
+  return ELFA_OK;
+}
+
+// ------------------------------------------------------------------------------------------------ backward
+// With dS1 the gradient of the state behind a chunk, Y = K dS1 and U = diag(c) E:
+//   dE  = -diag(ex) dO + diag(c) Y        dE0 = dE + N^T dE        dV = dO + dE0        dS0 = dS1 - K^T dE0
+//   dK  = U dS1^T - dE0 S0^T + (dG + dG^T + 2 diag(dlam)) K       dG_ts = -(dE0 E^T)_ts c_s  (t > s)
+//   dc_t = sum_j (Y E)_tj + lam_t sum_j (dO E)_tj - sum_{r > t} (dE0 E^T)_rt (K K^T)_rt
+//   dlam_t = c_t sum_j (dO E)_tj + dc_t dc/dlam,   dbeta = sum_t dc_t ex_t
+// Only dS is sequential: efla_chunk_bwd_state_kernel walks the chunks backwards with dS in registers and writes the dS1 of every chunk;
+// efla_chunk_bwd_kernel then handles all chunks in parallel from the two chunk-boundary states.
+// B 8, T 2048, 16 heads of 64: 95 us and 255 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
+// finish). The parallel kernel issues about 400 mma.sync per warp and chunk (94 us of tensor time at 8.3 cycles each) and reads 370 MB
+// (55 us); a third CTA per SM, at 168 registers, did not make it faster.
+template <int D>
+__global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_bwd_state_kernel(
+    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ nmat,
+    const float* __restrict__ coef, const float* __restrict__ dstate_out, float4* __restrict__ dckpt, float* __restrict__ dstate0, int T,
+    int H, int nchunks) {
+  using L = EflaStage<D>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int bh = blockIdx.x, b = bh / H, h = bh % H;
+  const int ccol = blockIdx.y * L::VC, wcol = ccol + warp * 16;
+  const uint32_t ring = smem_u32(smem);
+  const long long row0 = ((long long)b * T * H + h) * D, rs = (long long)H * D;
+  const __nv_bfloat16 *kb = k + row0, *ob = dout + row0 + ccol;
+  const __nv_bfloat16* nb = nmat + (long long)bh * nchunks * EN_ELEMS;
+  const float* cb = coef + (long long)bh * nchunks * EC_COEF;
+
+  float S[D / 8][4];                       // dS^T, laid out as the state of the forward kernel
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      S[n][x] = dstate_out ? dstate_out[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] : 0.f;
+
+  auto fetch = [&](int i) {                // i-th chunk from the end
+    const int ch = nchunks - 1 - i;
+    if (ch >= 0)
+      efla_stage_load<D>(ring + (i % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, ob + (long long)ch * EC * rs,
+                         nb + (long long)ch * EN_ELEMS, cb + (long long)ch * EC_COEF, rs, min(EC, T - ch * EC));
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < EC_STAGES - 1; ++i) fetch(i);
+  for (int i = 0; i < nchunks; ++i) {
+    cp_async_wait<EC_STAGES - 2>();
+    __syncthreads();
+    fetch(i + EC_STAGES - 1);
+    const uint32_t st = ring + (i % EC_STAGES) * L::BYTES;
+    const float* cf = reinterpret_cast<const float*>(smem + (i % EC_STAGES) * L::BYTES + L::C);
+    float4* dst = dckpt + efla_state_slot<D>((long long)bh * nchunks + nchunks - 1 - i, wcol / 16, lane);
+#pragma unroll
+    for (int n = 0; n < D / 8; ++n) dst[n * 32] = make_float4(S[n][0], S[n][1], S[n][2], S[n][3]);
+    float e[4][4];
+    efla_state_times_k<D>(e, S, st + L::K, lane);
+    uint32_t oq[2][4];
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) ldsm4_t(oq[hf], st + L::V + (lane * L::VLD + warp * 16 + hf * 8) * 2);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
+      const float2 ex = *reinterpret_cast<const float2*>(cf + EC + nt * 8 + 2 * q);
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        e[nt][2 * hf] = cc.x * e[nt][2 * hf] - ex.x * bf16_lo(oq[hf][nt]);
+        e[nt][2 * hf + 1] = cc.y * e[nt][2 * hf + 1] - ex.y * bf16_hi(oq[hf][nt]);
+      }
+    }
+    efla_apply_n<true>(e, st + L::N, lane);
+    efla_state_update<D, true>(S, e, st + L::K, lane);
+  }
+  cp_async_wait<0>();
+  if (dstate0) {
+#pragma unroll
+    for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        dstate0[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] = S[n][x];
+  }
+}
+
+// One CTA per chunk, d / 16 warps; warp w owns value columns 16 w .. 16 w + 15 and all key rows. E, Y, dE0 are recomputed from the
+// chunk-boundary states with the products of the sequential kernels; the contractions over the value columns (dK, dE0 E^T) are
+// partial per warp and added up in warp order through shared memory. A warp's scratch holds transposed splits first, its dK partial
+// last.
+template <int D>
+struct EflaBwdSmem {
+  static constexpr int W = D / 16;
+  static constexpr int LD = D + 8;                                       // K, V, dO tiles and the split state tile (bf16)
+  static constexpr int TILE = EC * LD * 2;
+  static constexpr int SCR_E = 3 * 16 * EN_LD * 2, SCR_S = 3 * 16 * LD * 2, RED_LD = D + 4;
+  static constexpr int SCR = SCR_E + SCR_S > EC * RED_LD * 4 ? SCR_E + SCR_S : EC * RED_LD * 4;
+  static constexpr int GLD = 36;
+  static constexpr int K = 0, V = K + TILE, O = V + TILE, N = O + TILE, C = N + 3 * EC * EN_LD * 2, G = C + EC_COEF * 4,
+                       DA = G + EC * GLD * 4, SUM = DA + W * EC * GLD * 4, DC = SUM + W * 2 * EC * 4, SCRATCH = DC + W * EC * 4,
+                       BYTES = SCRATCH + W * SCR;
+};
+
+__device__ __forceinline__ void stsm4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
+
+// Three splits of a 16 x 32 tile (rows = value columns j, columns = tokens) into scratch [3][16][EN_LD].
+__device__ __forceinline__ void efla_put_tokens(uint32_t scr, const float (&e)[4][4], int lane) {
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+    uint32_t s[3][4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) split3(e[nt][2 * hf], e[nt][2 * hf + 1], s[0][nt], s[1][nt], s[2][nt]);
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      stsm4(scr + (p * 16 * EN_LD + (hf * 8 + (lane & 7)) * EN_LD + (lane >> 3) * 8) * 2, s[p][0], s[p][1], s[p][2], s[p][3]);
+  }
+}
+// ... read back as the A operand (rows = tokens 16 mi .., k = value columns)
+__device__ __forceinline__ void efla_get_a(uint32_t (&a)[3][4], uint32_t scr, int mi, int lane) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+    ldsm4_t(a[p], scr + (p * 16 * EN_LD + ((lane & 7) + (lane >> 4) * 8) * EN_LD + mi * 16 + ((lane >> 3) & 1) * 8) * 2);
+}
+// ... or as the B operand of two tiles (k = value columns, columns = x 16 np .. 16 np + 15), from a scratch of row pitch LD
+template <int LD>
+__device__ __forceinline__ void efla_get_b(uint32_t (&b)[3][4], uint32_t scr, int np, int lane) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) ldsm4_t(b[p], scr + (p * 16 * LD + (lane & 15) * LD + np * 16 + (lane >> 4) * 8) * 2);
+}
+// the i-th of the six products of two split operands, small ones first
+__device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int o, int i) {
+  const int ai = i == 0 || i == 3 ? 1 : (i == 1 ? 2 : 0), bi = i == 0 || i == 4 ? 1 : (i == 2 ? 2 : 0);
+  mma_bf16(acc, a[ai], b[bi][o], b[bi][o + 1]);
+}
+
+template <int D>
+__global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
+    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ dout,
+    const __nv_bfloat16* __restrict__ nmat, const float* __restrict__ coef, const float4* __restrict__ ckpt,
+    const float4* __restrict__ dckpt, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
+    float* __restrict__ dbeta_tok, int T, int H, int nchunks) {
+  using L = EflaBwdSmem<D>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const long long id = blockIdx.x;
+  const int bh = (int)(id / nchunks), ch = (int)(id % nchunks), b = bh / H, h = bh % H;
+  const int t0 = ch * EC, n = min(EC, T - t0);
+  const uint32_t base = smem_u32(smem);
+  const long long rs = (long long)H * D, off = (((long long)b * T + t0) * H + h) * D;
+  const float* cf = reinterpret_cast<const float*>(smem + L::C);
+
+  for (int i = tid; i < EC * (D / 8); i += 2 * D) {
+    const int r = i / (D / 8), c = i % (D / 8);
+    const long long src = off + (r < n ? r : 0) * rs + c * 8;
+    const uint32_t dst = (r * L::LD + c * 8) * 2;
+    cp_async16(base + L::K + dst, k + src, r < n);
+    cp_async16(base + L::V + dst, v + src, r < n);
+    cp_async16(base + L::O + dst, dout + src, r < n);
+  }
+  for (int i = tid; i < 3 * EC * 4; i += 2 * D) cp_async16(base + L::N + ((i / 4) * EN_LD + (i % 4) * 8) * 2, nmat + id * EN_ELEMS + i * 8, true);
+  if (tid < EC_COEF / 4) cp_async16(base + L::C + tid * 16, coef + id * EC_COEF + tid * 4, true);
+  cp_async_commit();
+  const float4* sp = ckpt + efla_state_slot<D>(id, warp, lane);
+  const float4* dp = dckpt + efla_state_slot<D>(id, warp, lane);
+  float S[D / 8][4];
+#pragma unroll
+  for (int i = 0; i < D / 8; ++i) {
+    const float4 f = sp[i * 32];
+    S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+
+  float* sG = reinterpret_cast<float*>(smem + L::G);
+  if (warp < 2) {                          // rows 16 warp .. of the Gram matrix, lower tiles
+    float acc[4][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      uint32_t a[4];
+      ldsm4(a, base + L::K + ((warp * 16 + (lane & 15)) * L::LD + kk * 16 + (lane >> 4) * 8) * 2);
+#pragma unroll
+      for (int np = 0; np < 2; ++np) {
+        uint32_t bq[4];
+        ldsm4(bq, base + L::K + ((np * 16 + (lane & 7) + (lane >> 4) * 8) * L::LD + kk * 16 + ((lane >> 3) & 1) * 8) * 2);
+        mma_bf16(acc[2 * np], a, bq[0], bq[1]);
+        mma_bf16(acc[2 * np + 1], a, bq[2], bq[3]);
+      }
+    }
+#pragma unroll
+    for (int nj = 0; nj < 4; ++nj) {
+      *reinterpret_cast<float2*>(&sG[(warp * 16 + g) * L::GLD + nj * 8 + 2 * q]) = make_float2(acc[nj][0], acc[nj][1]);
+      *reinterpret_cast<float2*>(&sG[(warp * 16 + g + 8) * L::GLD + nj * 8 + 2 * q]) = make_float2(acc[nj][2], acc[nj][3]);
+    }
+  }
+
+  // E and dE0, and the per-token sums over this warp's value columns
+  float e[4][4], de[4][4];
+  efla_state_times_k<D>(e, S, base + L::K, lane);
+  uint32_t vq[2][4], oq[2][4];
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+    ldsm4_t(vq[hf], base + L::V + (lane * L::LD + warp * 16 + hf * 8) * 2);
+    ldsm4_t(oq[hf], base + L::O + (lane * L::LD + warp * 16 + hf * 8) * 2);
+  }
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) e[nt][x] = ((x & 1) ? bf16_hi(vq[x >> 1][nt]) : bf16_lo(vq[x >> 1][nt])) - e[nt][x];
+  efla_apply_n<false>(e, base + L::N, lane);
+#pragma unroll
+  for (int i = 0; i < D / 8; ++i) {
+    const float4 f = dp[i * 32];
+    S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
+  }
+  efla_state_times_k<D>(de, S, base + L::K, lane);
+  float* ssum = reinterpret_cast<float*>(smem + L::SUM) + warp * 2 * EC;
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
+    const float2 ex = *reinterpret_cast<const float2*>(cf + EC + nt * 8 + 2 * q);
+    float ye[2] = {0.f, 0.f}, oe[2] = {0.f, 0.f};
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const float o0 = bf16_lo(oq[hf][nt]), o1 = bf16_hi(oq[hf][nt]);
+      ye[0] += de[nt][2 * hf] * e[nt][2 * hf];
+      ye[1] += de[nt][2 * hf + 1] * e[nt][2 * hf + 1];
+      oe[0] += o0 * e[nt][2 * hf];
+      oe[1] += o1 * e[nt][2 * hf + 1];
+      de[nt][2 * hf] = cc.x * de[nt][2 * hf] - ex.x * o0;
+      de[nt][2 * hf + 1] = cc.y * de[nt][2 * hf + 1] - ex.y * o1;
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int m = 4; m < 32; m <<= 1) {
+        ye[x] += __shfl_xor_sync(0xffffffffu, ye[x], m);
+        oe[x] += __shfl_xor_sync(0xffffffffu, oe[x], m);
+      }
+    if (g == 0) {
+      *reinterpret_cast<float2*>(ssum + nt * 8 + 2 * q) = make_float2(ye[0], ye[1]);
+      *reinterpret_cast<float2*>(ssum + EC + nt * 8 + 2 * q) = make_float2(oe[0], oe[1]);
+    }
+  }
+  efla_apply_n<true>(de, base + L::N, lane);
+
+  const uint32_t scr_e = base + L::SCRATCH + warp * L::SCR, scr_s = scr_e + L::SCR_E;
+  {                                        // dV = dO + dE0, transposed through the scratch
+    uint32_t d2[2][4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf)
+        d2[hf][nt] = pack_bf16(bf16_lo(oq[hf][nt]) + de[nt][2 * hf], bf16_hi(oq[hf][nt]) + de[nt][2 * hf + 1]);
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) stsm4_t(scr_e + (lane * 24 + hf * 8) * 2, d2[hf][0], d2[hf][1], d2[hf][2], d2[hf][3]);
+    __syncwarp();
+    const unsigned char* sc = smem + L::SCRATCH + warp * L::SCR;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = u * 16 + (lane >> 1), hf = lane & 1;
+      if (t < n) *reinterpret_cast<uint4*>(dv + off + t * rs + warp * 16 + hf * 8) = *reinterpret_cast<const uint4*>(sc + (t * 24 + hf * 8) * 2);
+    }
+    __syncwarp();
+  }
+  // dK partial (2 x d / 8 tiles) = U dS1^T - dE0 S0^T
+  float acc[2][D / 8][4];
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) acc[mi][i][x] = 0.f;
+  uint32_t a[2][3][4];
+#pragma unroll
+  for (int term = 0; term < 2; ++term) {
+    float w[4][4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) w[nt][x] = term == 0 ? e[nt][x] * ((x & 1) ? cc.y : cc.x) : -de[nt][x];
+    }
+    if (term == 1) {
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i) {
+        const float4 f = sp[i * 32];
+        S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
+      }
+    }
+    efla_put_tokens(scr_e, w, lane);
+#pragma unroll
+    for (int i4 = 0; i4 < D / 32; ++i4)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t s[3][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) split3(S[4 * i4 + u][2 * hf], S[4 * i4 + u][2 * hf + 1], s[0][u], s[1][u], s[2][u]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+          stsm4(scr_s + (p * 16 * L::LD + (hf * 8 + (lane & 7)) * L::LD + i4 * 32 + (lane >> 3) * 8) * 2, s[p][0], s[p][1], s[p][2], s[p][3]);
+      }
+    __syncwarp();
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi) efla_get_a(a[mi], scr_e, mi, lane);
+#pragma unroll
+    for (int np = 0; np < D / 16; ++np) {
+      uint32_t bq[3][4];
+      efla_get_b<L::LD>(bq, scr_s, np, lane);
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int mi = 0; mi < 2; ++mi) {
+          mma_split(acc[mi][2 * np], a[mi], bq, 0, i);
+          mma_split(acc[mi][2 * np + 1], a[mi], bq, 2, i);
+        }
+    }
+    __syncwarp();
+  }
+  // -dE0 E^T (a still holds -dE0), lower tiles
+  float* sda = reinterpret_cast<float*>(smem + L::DA) + warp * EC * L::GLD;
+  efla_put_tokens(scr_e, e, lane);
+  __syncwarp();
+#pragma unroll
+  for (int np = 0; np < 2; ++np) {
+    uint32_t bq[3][4];
+    efla_get_b<EN_LD>(bq, scr_e, np, lane);
+#pragma unroll
+    for (int mi = np; mi < 2; ++mi)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float da[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 6; ++i) mma_split(da, a[mi], bq, 2 * u, i);
+        *reinterpret_cast<float2*>(&sda[(mi * 16 + g) * L::GLD + np * 16 + u * 8 + 2 * q]) = make_float2(da[0], da[1]);
+        *reinterpret_cast<float2*>(&sda[(mi * 16 + g + 8) * L::GLD + np * 16 + u * 8 + 2 * q]) = make_float2(da[2], da[3]);
+      }
+  }
+  __syncwarp();
+  float* red = reinterpret_cast<float*>(smem + L::SCRATCH + warp * L::SCR);
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) {
+      *reinterpret_cast<float2*>(&red[(mi * 16 + g) * L::RED_LD + i * 8 + 2 * q]) = make_float2(acc[mi][i][0], acc[mi][i][1]);
+      *reinterpret_cast<float2*>(&red[(mi * 16 + g + 8) * L::RED_LD + i * 8 + 2 * q]) = make_float2(acc[mi][i][2], acc[mi][i][3]);
+    }
+  __syncthreads();
+  // dA = sum over the warps; the symmetric matrix dG + dG^T replaces the first slice of sda, column sums of dA G go to sdc
+  float* sym = reinterpret_cast<float*>(smem + L::DA);
+  float* sdc = reinterpret_cast<float*>(smem + L::DC);
+  {
+    float part = 0.f;
+    const float c_s = cf[lane];
+    for (int t = warp; t < EC; t += L::W) {
+      float da = 0.f;
+      if (t > lane) {
+#pragma unroll
+        for (int w = 0; w < L::W; ++w) da += sym[(w * EC + t) * L::GLD + lane];
+        part += da * sG[t * L::GLD + lane];
+        sym[t * L::GLD + lane] = da * c_s;
+      }
+    }
+    sdc[warp * EC + lane] = part;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float ye = 0.f, oe = 0.f, dc = 0.f;
+#pragma unroll
+    for (int w = 0; w < L::W; ++w) {
+      const float* ss = reinterpret_cast<const float*>(smem + L::SUM) + w * 2 * EC;
+      ye += ss[lane];
+      oe += ss[EC + lane];
+      dc += sdc[w * EC + lane];
+    }
+    dc += ye + cf[2 * EC + lane] * oe;
+    sym[lane * L::GLD + lane] = 2.f * (cf[lane] * oe + dc * cf[3 * EC + lane]);
+    if (lane < n) dbeta_tok[((long long)b * T + t0 + lane) * H + h] = dc * cf[EC + lane];
+  } else {
+    for (int t = warp - 1; t < EC; t += L::W - 1)
+      if (t < lane) sym[t * L::GLD + lane] = sym[lane * L::GLD + t];
+  }
+  __syncthreads();
+  // key rows 16 warp ..: dK = sum of the partials + sym K
+  float dkt[2][2][4];
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) dkt[mi][u][x] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks) {
+    uint32_t b0[4];
+    ldsm4_t(b0, base + L::K + ((ks * 16 + (lane & 15)) * L::LD + warp * 16 + (lane >> 4) * 8) * 2);
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi) {
+      float2 f[4];
+      f[0] = *reinterpret_cast<const float2*>(&sym[(mi * 16 + g) * L::GLD + ks * 16 + 2 * q]);
+      f[1] = *reinterpret_cast<const float2*>(&sym[(mi * 16 + g + 8) * L::GLD + ks * 16 + 2 * q]);
+      f[2] = *reinterpret_cast<const float2*>(&sym[(mi * 16 + g) * L::GLD + ks * 16 + 8 + 2 * q]);
+      f[3] = *reinterpret_cast<const float2*>(&sym[(mi * 16 + g + 8) * L::GLD + ks * 16 + 8 + 2 * q]);
+      uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) split3(f[x].x, f[x].y, hi[x], mid[x], lo[x]);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        mma_bf16(dkt[mi][u], lo, b0[2 * u], b0[2 * u + 1]);
+        mma_bf16(dkt[mi][u], mid, b0[2 * u], b0[2 * u + 1]);
+        mma_bf16(dkt[mi][u], hi, b0[2 * u], b0[2 * u + 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int t = mi * 16 + hf * 8 + g;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float2 s = make_float2(dkt[mi][u][2 * hf], dkt[mi][u][2 * hf + 1]);
+#pragma unroll
+        for (int w = 0; w < L::W; ++w) {
+          const float2 r = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(smem + L::SCRATCH + w * L::SCR) + t * L::RED_LD +
+                                                            warp * 16 + u * 8 + 2 * q);
+          s.x += r.x;
+          s.y += r.y;
+        }
+        if (t < n) *reinterpret_cast<uint32_t*>(dk + off + t * rs + warp * 16 + u * 8 + 2 * q) = pack_bf16(s.x, s.y);
+      }
+    }
+}
+
+template <int D>
+int launch_chunk_bwd(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt,
+                     const void* dout, const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0, float* dckpt, int B,
+                     int T, int H, cudaStream_t s) {
+  using L = EflaStage<D>;
+  using M = EflaBwdSmem<D>;
+  const int nchunks = (T + EC - 1) / EC;
+  const long long total = (long long)B * H * nchunks;
+  ELFA_REQUIRE(total < (1ll << 31), "efla_chunk_bwd: too many chunks");
+  constexpr int bytes1 = EC_STAGES * L::BYTES;
+  const auto* K = static_cast<const __nv_bfloat16*>(k);
+  const auto* O = static_cast<const __nv_bfloat16*>(dout);
+  const auto* N = static_cast<const __nv_bfloat16*>(nmat);
+  ELFA_CUDA(cudaFuncSetAttribute(efla_chunk_bwd_state_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes1));
+  ELFA_CUDA(cudaFuncSetAttribute(efla_chunk_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::BYTES));
+  efla_chunk_bwd_state_kernel<D><<<dim3(B * H, D / L::VC), 32 * ec_warps<D>(), bytes1, s>>>(
+      K, O, N, coef, dstate_out, reinterpret_cast<float4*>(dckpt), dstate0, T, H, nchunks);
+  ELFA_CUDA(cudaGetLastError());
+  efla_chunk_bwd_kernel<D><<<(unsigned)total, 2 * D, M::BYTES, s>>>(
+      K, static_cast<const __nv_bfloat16*>(v), O, N, coef, reinterpret_cast<const float4*>(ckpt),
+      reinterpret_cast<const float4*>(dckpt), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), dbeta_tok, T, H, nchunks);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(2);
   return ELFA_OK;
@@ -403,8 +886,8 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 using namespace elfa;
 
 // k, v, o: [B, T, H, d] bf16, 16-byte aligned; beta: 1 float; state0 (optional) / state_out: [B, H, d, d] fp32; ckpt: null or
-// [B, H, ceil(T / 32), d, d] fp32 (chunk-start states, needed by backward). nmat: [B * H * ceil(T / 32), 3, 32, 32] bf16 and
-// coef: [B * H * ceil(T / 32), 2, 32] fp32, 16-byte aligned, are written here.
+// B * H * ceil(T / 32) * d * d floats (chunk-start states in the kernels' own order, needed by backward). nmat: [B * H * ceil(T / 32), 3, 32, 32] bf16 and
+// coef: [B * H * ceil(T / 32), 4, 32] fp32, 16-byte aligned, are written here.
 ELFA_API int elfa_efla_chunk_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
                                  float* ckpt, void* nmat, float* coef, int B, int T, int H, int d, void* stream) {
   ELFA_REQUIRE(k && v && beta && o && nmat && coef && B > 0 && T > 0 && H > 0, "efla_chunk_fwd: bad arguments");
@@ -416,5 +899,26 @@ ELFA_API int elfa_efla_chunk_fwd(const void* k, const void* v, const float* beta
     case 96: return launch_chunk_fwd<96>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, B, T, H, s);
     case 128: return launch_chunk_fwd<128>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, B, T, H, s);
     default: set_last_error("efla_chunk_fwd: head dimension must be 32, 64, 96 or 128"); return ELFA_ERR_UNSUPPORTED;
+  }
+}
+
+// Gradients of elfa_efla_chunk_fwd from what it left in nmat, coef and ckpt. dout: [B, T, H, d] bf16; dstate_out: null or [B, H, d, d]
+// fp32; dk, dv: [B, T, H, d] bf16; dbeta_tok: [B, T, H] per-token terms (add them up); dstate0: null or [B, H, d, d] fp32; dckpt: scratch
+// of ckpt's size.
+ELFA_API int elfa_efla_chunk_bwd(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
+                                 const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0,
+                                 float* dckpt, int B, int T, int H, int d, void* stream) {
+  ELFA_REQUIRE(k && v && nmat && coef && ckpt && dout && dk && dv && dbeta_tok && dckpt && B > 0 && T > 0 && H > 0,
+               "efla_chunk_bwd: bad arguments");
+  ELFA_REQUIRE(aligned16(k) && aligned16(v) && aligned16(nmat) && aligned16(coef) && aligned16(ckpt) && aligned16(dout) && aligned16(dk) &&
+                   aligned16(dv) && aligned16(dckpt),
+               "efla_chunk_bwd: operands must be 16-byte aligned");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (d) {
+    case 32: return launch_chunk_bwd<32>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
+    case 64: return launch_chunk_bwd<64>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
+    case 96: return launch_chunk_bwd<96>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
+    case 128: return launch_chunk_bwd<128>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
+    default: set_last_error("efla_chunk_bwd: head dimension must be 32, 64, 96 or 128"); return ELFA_ERR_UNSUPPORTED;
   }
 }

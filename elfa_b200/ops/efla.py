@@ -104,8 +104,9 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
 
 
 class _EflaScan(torch.autograd.Function):
-    """CUDA path. Forward: chunks of 32 tokens on the tensor cores with the fp32 state in registers. Backward recomputes the states
-    inside each chunk from the chunk-boundary states saved by forward (only when a gradient is wanted)."""
+    """CUDA path. Forward: chunks of 32 tokens on the tensor cores with the fp32 state in registers. Backward: the gradient of
+    the state walks the chunks the same way, everything else is parallel over the chunks, from the chunk-boundary states that forward
+    keeps when a gradient is wanted."""
 
     @staticmethod
     def forward(ctx, k, v, beta, state, want_grad):
@@ -119,32 +120,28 @@ class _EflaScan(torch.autograd.Function):
             lib.call("elfa_efla_scan_fwd", kc, vc, bt, st0, o, s_out, B, T, H, d, stream_ptr(kc))
             return o, s_out
         nchunks = (T + _EFLA_CHUNK - 1) // _EFLA_CHUNK
-        ckpt = torch.empty((B, H, nchunks, d, d), dtype=torch.float32, device=k.device) if want_grad else None
+        ckpt = torch.empty(B * H * nchunks * d * d, dtype=torch.float32, device=k.device) if want_grad else None
         nmat = torch.empty((B, H, nchunks, 3, _EFLA_CHUNK, _EFLA_CHUNK), dtype=torch.bfloat16, device=k.device)
-        coef = torch.empty((B, H, nchunks, 2, _EFLA_CHUNK), dtype=torch.float32, device=k.device)
+        coef = torch.empty((B, H, nchunks, 4, _EFLA_CHUNK), dtype=torch.float32, device=k.device)
         lib.call("elfa_efla_chunk_fwd", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, B, T, H, d, stream_ptr(kc))
         if want_grad:
-            ctx.save_for_backward(kc, vc, bt, ckpt)
+            ctx.save_for_backward(kc, vc, ckpt, nmat, coef)
             ctx.cfg = (B, T, H, d, state is not None)
         return o, s_out
 
     @staticmethod
     def backward(ctx, do, ds_out):
-        kc, vc, bt, ckpt = ctx.saved_tensors
+        kc, vc, ckpt, nmat, coef = ctx.saved_tensors
         B, T, H, d, has_state = ctx.cfg
-        chunk = _EFLA_CHUNK
         dk = torch.empty_like(kc)
         dv = torch.empty_like(vc)
-        rows = B * T * H
-        dbeta = torch.empty(rows, dtype=torch.float32, device=kc.device)                 # per-token terms, summed below
-        ds0 = torch.empty((B, H, d, d), dtype=torch.float32, device=kc.device)
-        work = torch.empty((B * H, chunk, d, d), dtype=torch.float32, device=kc.device)
-        dk_part = torch.empty((d // 32, rows, d), dtype=torch.float32, device=kc.device)  # one slice per block of 32 value columns
-        dc_part = torch.empty((d // 32, rows), dtype=torch.float32, device=kc.device)
+        dbeta = torch.empty(B * T * H, dtype=torch.float32, device=kc.device)            # per-token terms, summed below
+        ds0 = torch.empty((B, H, d, d), dtype=torch.float32, device=kc.device) if has_state else None
+        dckpt = torch.empty_like(ckpt)
         dso = ds_out.float().contiguous() if ds_out is not None else None
-        lib.call("elfa_efla_scan_bwd", kc, vc, bt, ckpt, do.contiguous(), dso, dk, dv, dbeta, ds0, work, dk_part, dc_part,
-                 B, T, H, d, chunk, stream_ptr(kc))
-        return dk, dv, dbeta.sum().reshape(1), (ds0 if has_state else None), None
+        lib.call("elfa_efla_chunk_bwd", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt, B, T, H, d,
+                 stream_ptr(kc))
+        return dk, dv, dbeta.sum().reshape(1), ds0, None
 
 
 def efla_scan(k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, state: Optional[torch.Tensor] = None, chunk: int = 16

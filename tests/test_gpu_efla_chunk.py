@@ -60,3 +60,33 @@ def test_a_bad_token_leaves_the_earlier_ones_alone(cuda_device, bad):
         if which == 1:                      # a value touches its own column only
             keep = [j for j in range(64) if j != 5]
             assert torch.equal(o[0, :, 0, keep], o0[0, :, 0, keep])
+
+
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 65, 130])
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+def test_backward_at_chunk_edges(cuda_device, T, d):
+    with_state = T % 2 == 1
+    k, v, beta, s0 = _inputs(cuda_device, 2, T, 3, d, with_state, seed=T + d)
+    go, gs = torch.randn_like(v), 0.1 * torch.randn(2, 3, d, d, device=cuda_device)
+    grads = []
+    for fn, cast in ((eops.efla_scan, lambda t: t), (eops.efla_scan_ref, lambda t: t.float())):
+        ins = [t.detach().clone().requires_grad_(True) for t in (cast(k), cast(v), beta, s0) if t is not None]
+        o, s = fn(*ins)
+        grads.append(torch.autograd.grad([o, s], ins, [go.to(o.dtype), gs]))
+    assert native.status() == 0
+    got, ref = grads
+    _close(got[0], ref[0], 2 ** -8)
+    _close(got[1], ref[1], 2 ** -8)
+    # beta: a sum over all tokens whose terms cancel; each term is off by at most 2^-20 of its size (about d products)
+    assert abs(got[2] - ref[2]).item() <= 2e-5 * max(1.0, ref[2].abs().item()) + 1e-6 * T * d
+    if with_state:
+        _close(got[3], ref[3], 1e-5)
+
+
+def test_backward_of_one_output_only(cuda_device):
+    k, v, beta, _ = _inputs(cuda_device, 1, 50, 2, 64, False)
+    k.requires_grad_(True)
+    kr = k.detach().float().requires_grad_(True)
+    eops.efla_scan(k, v, beta)[1].square().sum().backward()
+    eops.efla_scan_ref(kr, v, beta)[1].square().sum().backward()
+    _close(k.grad, kr.grad, 2 ** -8)
