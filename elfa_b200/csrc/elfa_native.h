@@ -184,6 +184,11 @@ int elfa_prism_fwd(const void* u, const void* v, const unsigned long long* p, vo
 int elfa_prism_bwd(const void* u, const void* v, const unsigned long long* p, const void* dy, void* du, void* dv,
                    const unsigned long long* dp, long long tokens, int G, int d, int L, void* stream);
 
+int elfa_prism_gated_fwd(const void* u, const void* v, const void* z, long long ldz, void* y, long long tokens, int G, int d, int L,
+                         void* stream);
+int elfa_prism_gated_bwd(const void* u, const void* v, const void* z, long long ldz, const void* dy, void* du, void* dv, void* dz,
+                         long long tokens, int G, int d, int L, void* stream);
+
 // ---- efla.cu -----------------------------------------------------------------------------------
 int elfa_efla_scan_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
                        int B, int T, int H, int d, void* stream);

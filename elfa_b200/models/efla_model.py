@@ -106,13 +106,13 @@ class PrismLayer(nn.Module):
         if conv_tail is not None:
             u = u[:, conv_tail.shape[1]:]
         new_tail = xin[:, -(W - 1):].detach() if W > 1 else None
-        ps = [torch.sigmoid(ops.linear(u, self.w_p[l]).float()) for l in range(self.L)]
-        y = eops.prism_refine(u, v, ps, self.d)
+        y = eops.prism_gated_refine(u, v, list(self.w_p), self.d)
         new_state = None
         if carry_state is not None:
             with torch.no_grad():
                 B, T, D = u.shape
                 G = D // self.d
+                ps = [torch.sigmoid(ops.linear(u, self.w_p[l]).float()) for l in range(self.L)]
                 r = (v.float() - u.float()).view(B, T, G, self.d)
                 deltas, betas, ks = [], [], []
                 for l in range(self.L):

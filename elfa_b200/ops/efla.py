@@ -24,7 +24,7 @@ from typing import Optional, Tuple
 import torch
 
 from ..native import NativeError, lib, stream_ptr
-from .gemm import gelu_tanh_ref
+from .gemm import _accumulate_main_grad, gelu_tanh_ref, gemm, linear
 
 
 def stable_coefficient(beta: torch.Tensor, lam: torch.Tensor) -> torch.Tensor:
@@ -256,6 +256,61 @@ class _PrismRefine(torch.autograd.Function):
         lib.call("elfa_prism_bwd", uc, vc, ctypes.addressof(parr), dyc, du, dv, ctypes.addressof(darr), B * T, D // d, d, len(pcs),
                  stream_ptr(uc))
         return (du, dv, None) + tuple(g.to(p.dtype) for g, p in zip(dps, pcs))
+
+
+class _PrismGated(torch.autograd.Function):
+    """The whole gate of the layer: the ``L`` logit products as one GEMM over the concatenated weights, gates and refinement in one
+    kernel; backward is one kernel, one input-gradient GEMM that adds into ``du`` and the weight gradients."""
+
+    @staticmethod
+    def forward(ctx, u, v, group_dim, *ws):
+        B, T, D = u.shape
+        uc, vc = _aligned(u).view(-1, D), _aligned(v).view(-1, D)
+        wc = torch.cat(ws, 1) if len(ws) > 1 else _aligned(ws[0])
+        z = gemm(uc, wc, b_mn=True)
+        y = torch.empty_like(uc)
+        lib.call("elfa_prism_gated_fwd", uc, vc, z, z.stride(0), y, B * T, D // group_dim, group_dim, len(ws), stream_ptr(uc))
+        ctx.save_for_backward(uc, vc, wc, z)
+        ctx.w_refs, ctx.group_dim, ctx.shape = ws, group_dim, u.shape
+        return y.view(u.shape)
+
+    @staticmethod
+    def backward(ctx, dy):
+        uc, vc, wc, z = ctx.saved_tensors
+        rows, D = uc.shape
+        d, L = ctx.group_dim, len(ctx.w_refs)
+        dyc = _aligned(dy)
+        du, dv, dz = torch.empty_like(uc), torch.empty_like(vc), torch.empty_like(z)
+        lib.call("elfa_prism_gated_bwd", uc, vc, z, z.stride(0), dyc, du, dv, dz, rows, D // d, d, L, stream_ptr(uc))
+        if ctx.needs_input_grad[0]:
+            # two launches: the GEMM's own addition (add_aux) reads a lane's row at a time and takes longer than both for a contraction this
+            # short (16384 x 1024 x 128: 76 us)
+            g = gemm(dz, wc)
+            lib.call("elfa_elementwise", 2, du, g, du, du.numel(), 1.0, stream_ptr(du))
+        dws = [None] * L
+        rest = [l for l, w in enumerate(ctx.w_refs)
+                if ctx.needs_input_grad[3 + l] and not _accumulate_main_grad(w, uc, dz[:, l * d:(l + 1) * d])]
+        if rest:
+            # all of them as one product into fp32, which the GEMM splits along the tokens (D x L d is a handful of tiles, and a bf16
+            # output would walk all tokens in one CTA per tile: B 8, T 2048, D 1024, d 64, L 2: 135 us)
+            dw = gemm(uc, dz, a_mn=True, b_mn=True, out=torch.zeros((D, L * d), dtype=torch.float32, device=dz.device), accumulate=True)
+            for l in rest:
+                dws[l] = dw[:, l * d:(l + 1) * d].to(wc.dtype, memory_format=torch.contiguous_format)
+        return (du.view(ctx.shape), dv.view(ctx.shape), None, *dws)
+
+
+def prism_gated_native(u: torch.Tensor, v: torch.Tensor, ws, group_dim: int) -> bool:
+    """What the fused gate handles: CUDA bf16, at most eight iterations, groups and rows of whole 16-byte vectors."""
+    D = u.shape[-1]
+    return (u.is_cuda and v.shape == u.shape and all(t.dtype == torch.bfloat16 for t in (u, v, *ws)) and 1 <= len(ws) <= 8 and u.numel() > 0
+            and group_dim % 8 == 0 and D % group_dim == 0 and all(w.shape == (D, group_dim) for w in ws))
+
+
+def prism_gated_refine(u: torch.Tensor, v: torch.Tensor, ws, group_dim: int) -> torch.Tensor:
+    """``prism_refine`` with the gates given by their weights: ``p_l = sigmoid(u @ ws[l])``, formed in fp32."""
+    if prism_gated_native(u, v, ws, group_dim):
+        return _PrismGated.apply(u, v, group_dim, *ws)
+    return prism_refine(u, v, [torch.sigmoid(linear(u, w).float()) for w in ws], group_dim)
 
 
 def prism_refine(u: torch.Tensor, v: torch.Tensor, p_list, group_dim: int) -> torch.Tensor:

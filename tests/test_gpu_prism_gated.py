@@ -1,0 +1,45 @@
+"""PRISM gate from its weights (one GEMM, one kernel per direction) against the plain PyTorch form.
+
+The oracle is fp32 throughout except for the logits, which both sides round to bf16. The kernels round results to bf16, and the input
+gradient twice more on its way (its two addends): at most three roundings of 2^-9, 2^-7 of the largest.
+"""
+import pytest
+import torch
+
+from elfa_b200 import native
+from elfa_b200.ops import efla as eops, linear
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,G,d,L", [(1, 1, 8, 1), (33, 3, 32, 2), (64, 16, 64, 3), (7, 5, 64, 4), (20, 2, 128, 8), (19, 4, 24, 5)])
+def test_gated_refine(cuda_device, T, G, d, L):
+    torch.manual_seed(T)
+    D = G * d
+    u = torch.randn(2, T, D, device=cuda_device).bfloat16().requires_grad_(True)
+    v = torch.randn(2, T, D, device=cuda_device).bfloat16().requires_grad_(True)
+    ws = [(torch.randn(D, d, device=cuda_device) * D ** -0.5).bfloat16().requires_grad_(True) for _ in range(L)]
+    assert eops.prism_gated_native(u, v, ws, d)
+    dy = torch.randn(2, T, D, device=cuda_device).bfloat16()
+    y = eops.prism_gated_refine(u, v, ws, d)
+    got = torch.autograd.grad(y, [u, v, *ws], dy)
+    uf, vf, *wf = (t.detach().float().requires_grad_(True) for t in (u, v, *ws))
+    zs = [uf @ w for w in wf]
+    zs = [z + (linear(u, w).detach().float() - z).detach() for z, w in zip(zs, ws)]       # the value of the bf16 logits
+    ref_y = eops.prism_refine_ref(uf, vf, [torch.sigmoid(z) for z in zs], d)
+    ref = torch.autograd.grad(ref_y, [uf, vf, *wf], dy.float())
+    assert native.status() == 0
+    for a, b in zip([y, *got], [ref_y, *ref]):
+        assert a.shape == b.shape and a.dtype == torch.bfloat16
+        assert (a.float() - b).abs().max() <= 2 ** -7 * b.abs().max()
+
+
+def test_other_calls_keep_the_general_path(cuda_device):
+    u = torch.randn(1, 4, 12, device=cuda_device).bfloat16()                       # groups of 12 channels
+    w = torch.randn(12, 12, device=cuda_device).bfloat16()
+    assert not eops.prism_gated_native(u, u, [w], 12)
+    cpu = torch.randn(1, 4, 16)
+    wc = torch.randn(16, 8)
+    assert not eops.prism_gated_native(cpu, cpu, [wc], 8)
+    want = eops.prism_refine_ref(cpu, cpu + 1, [torch.sigmoid(cpu @ wc)], 8)
+    assert torch.allclose(eops.prism_gated_refine(cpu, cpu + 1, [wc], 8), want, atol=1e-6)
