@@ -133,6 +133,152 @@ __global__ void __launch_bounds__(32 * EFLA_W) efla_scan_fwd_kernel(const __nv_b
 }
 
 // ------------------------------------------------------------------------------------ ShortConv
+// Windows of 4, 8 and 16 taps: a warp owns 64 channels (a pair per lane) of one sequence and walks over `span` consecutive time steps with
+// the last W inputs and the W weights in registers (the loop is unrolled W steps, so the window is a ring with fixed register names);
+// every input element is loaded once per span plus the W - 1 steps of the seam, the next W rows are in flight while the current
+// ones are summed, and the sums run on packed fp32 pairs. Other windows (larger rings do not fit the registers) take
+// shortconv_apply_kernel / shortconv_bwd_dw_kernel below.
+// Backward is one walk from late to early: with dy[t .. t + W - 1] as the window, dx[t] = sum_j w[j] dy[t + j] and
+// dw[j] += x[t] dy[t + j]; every warp writes its dw / db sums as one slice of part [slices][W + 1][C], added up in order afterwards.
+// B 8, T 2048, C 1024, W 16: 32 us forward (67 MB; bound by the packed multiply-adds and the latency of 192- and 124-register warps), 58 + 6 us
+// backward; the layer that contains them went from 789 to 454 us when they replaced the general kernels below.
+template <int W>
+__device__ __forceinline__ void shortconv_weights(uint64_t (&wf)[W], const __nv_bfloat16* __restrict__ w, int c) {
+#pragma unroll
+  for (int j = 0; j < W; ++j)
+    wf[j] = pack_f32x2(__bfloat162float(w[(long long)c * W + j]), __bfloat162float(w[(long long)(c + 1) * W + j]));
+}
+__device__ __forceinline__ uint32_t ld_pair(const __nv_bfloat16* base, long long row, long long C, bool ok) {
+  return ok ? *reinterpret_cast<const uint32_t*>(base + row * C) : 0u;
+}
+__device__ __forceinline__ uint64_t pair_f32x2(uint32_t v) { return pack_f32x2(bf16_lo(v), bf16_hi(v)); }
+
+// grid (ceil(B * spans / 4), ceil(C / 64)), block (32, 4)
+template <int W>
+__global__ void __launch_bounds__(128) shortconv_ring_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                 const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y,
+                                                                 int B, int T, int C, int span, int spans) {
+  const int c = blockIdx.y * 64 + 2 * threadIdx.x;
+  const int unit = blockIdx.x * 4 + threadIdx.y;
+  if (c >= C || unit >= B * spans) return;
+  const int b = unit / spans, t0 = (unit % spans) * span, t1 = min(T, t0 + span);
+  const __nv_bfloat16* xb = x + (long long)b * T * C + c;
+  __nv_bfloat16* yb = y + (long long)b * T * C + c;
+  uint64_t wf[W], win[W];
+  shortconv_weights<W>(wf, w, c);
+  const uint64_t b2 = bias ? pack_f32x2(__bfloat162float(bias[c]), __bfloat162float(bias[c + 1])) : 0ull;
+#pragma unroll
+  for (int j = 1; j < W; ++j) win[W - j] = pair_f32x2(ld_pair(xb, t0 - j, C, t0 - j >= 0));
+  win[0] = 0ull;
+  uint32_t nx[W];
+#pragma unroll
+  for (int r = 0; r < W; ++r) nx[r] = ld_pair(xb, t0 + r, C, t0 + r < t1);
+  for (int t = t0; t < t1; t += W) {
+    uint32_t cur[W];
+#pragma unroll
+    for (int r = 0; r < W; ++r) {
+      cur[r] = nx[r];
+      nx[r] = ld_pair(xb, t + W + r, C, t + W + r < t1);
+    }
+#pragma unroll
+    for (int r = 0; r < W; ++r) {
+      win[r] = pair_f32x2(cur[r]);
+      uint64_t s0 = b2, s1 = 0ull;
+#pragma unroll
+      for (int j = 0; j < W; j += 2) {
+        s0 = fma_f32x2(win[(r - j + W) % W], wf[j], s0);
+        s1 = fma_f32x2(win[(r - j - 1 + W) % W], wf[j + 1], s1);
+      }
+      float lo, hi;
+      unpack_f32x2(add_f32x2(s0, s1), lo, hi);
+      if (t + r < t1) *reinterpret_cast<uint32_t*>(yb + (long long)(t + r) * C) = pack_bf16(lo, hi);
+    }
+  }
+}
+
+template <int W>
+__global__ void __launch_bounds__(128) shortconv_ring_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                 const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx,
+                                                                 float* __restrict__ part, int B, int T, int C, int span, int spans) {
+  const int c = blockIdx.y * 64 + 2 * threadIdx.x;
+  const int unit = blockIdx.x * 4 + threadIdx.y;
+  if (c >= C || unit >= B * spans) return;
+  const int b = unit / spans, t0 = (unit % spans) * span, t1 = min(T, t0 + span);
+  const long long off = (long long)b * T * C + c;
+  const __nv_bfloat16 *xb = x + off, *gb = dy + off;
+  __nv_bfloat16* ob = dx + off;
+  uint64_t wf[W], win[W], acc[W], accb = 0ull;
+  shortconv_weights<W>(wf, w, c);
+#pragma unroll
+  for (int j = 0; j < W; ++j) acc[j] = 0ull;
+  // step p of the walk is time t1 - 1 - p; slot r of the ring holds the step with p % W == r
+#pragma unroll
+  for (int j = 1; j < W; ++j) win[W - j] = pair_f32x2(ld_pair(gb, t1 - 1 + j, C, t1 - 1 + j < T));
+  win[0] = 0ull;
+  uint32_t ng[W], nx[W];
+#pragma unroll
+  for (int r = 0; r < W; ++r) {
+    ng[r] = ld_pair(gb, t1 - 1 - r, C, t1 - 1 - r >= t0);
+    nx[r] = ld_pair(xb, t1 - 1 - r, C, t1 - 1 - r >= t0);
+  }
+  for (int t = t1 - 1; t >= t0; t -= W) {
+    uint32_t cg[W], cx[W];
+#pragma unroll
+    for (int r = 0; r < W; ++r) {
+      cg[r] = ng[r];
+      cx[r] = nx[r];
+      ng[r] = ld_pair(gb, t - W - r, C, t - W - r >= t0);
+      nx[r] = ld_pair(xb, t - W - r, C, t - W - r >= t0);
+    }
+#pragma unroll
+    for (int r = 0; r < W; ++r) {
+      win[r] = pair_f32x2(cg[r]);
+      const uint64_t xv = pair_f32x2(cx[r]);            // zero before t0: those steps add nothing
+      accb = add_f32x2(accb, win[r]);
+      uint64_t s0 = 0ull, s1 = 0ull;
+#pragma unroll
+      for (int j = 0; j < W; j += 2) {
+        const uint64_t g0 = win[(r - j + W) % W], g1 = win[(r - j - 1 + W) % W];
+        s0 = fma_f32x2(g0, wf[j], s0);
+        s1 = fma_f32x2(g1, wf[j + 1], s1);
+        acc[j] = fma_f32x2(xv, g0, acc[j]);
+        acc[j + 1] = fma_f32x2(xv, g1, acc[j + 1]);
+      }
+      float lo, hi;
+      unpack_f32x2(add_f32x2(s0, s1), lo, hi);
+      if (t - r >= t0) *reinterpret_cast<uint32_t*>(ob + (long long)(t - r) * C) = pack_bf16(lo, hi);
+    }
+  }
+  float* pb = part + (long long)unit * (W + 1) * C + c;
+#pragma unroll
+  for (int j = 0; j <= W; ++j) {
+    float lo, hi;
+    unpack_f32x2(j < W ? acc[j < W ? j : 0] : accb, lo, hi);
+    *reinterpret_cast<float2*>(pb + (long long)j * C) = make_float2(lo, hi);
+  }
+}
+
+// dw[c, j] = sum over the slices of part[slice][j][c], db[c] from row `taps`. grid (ceil(C / 32), taps + 1), block (32, 16)
+__global__ void __launch_bounds__(512) shortconv_sum_kernel(const float* __restrict__ part, float* __restrict__ dw, float* __restrict__ db,
+                                                            int slices, int C, int taps) {
+  __shared__ float red[16][33];
+  const int c = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y;
+  float s = 0.f;
+  if (c < C) {
+#pragma unroll 4
+    for (int i = threadIdx.y; i < slices; i += 16) s += part[((long long)i * (taps + 1) + j) * C + c];
+  }
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < C) {
+    float tot = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) tot += red[k][threadIdx.x];
+    if (j < taps) dw[(long long)c * taps + j] = tot;
+    else if (db) db[c] = tot;
+  }
+}
+
 // Forward and input gradient share one kernel (DX = false: y[t] = bias + sum_j x[t - j] w[j]; DX = true:
 // dx[t] = sum_j dy[t + j] w[j]). A lane owns a PAIR of adjacent channels (4-byte loads, 128 bytes per warp); the
 // CTA's 64 channels x W weights sit transposed in shared memory (the [C, W] layout read directly would touch a
@@ -252,9 +398,36 @@ ELFA_API int elfa_efla_scan_fwd(const void* k, const void* v, const float* beta,
   }
 }
 
+// Time steps a warp of the register-ring kernels walks: long spans amortise the seam, short ones keep the SMs busy on small inputs.
+static int shortconv_span(int B, int T, int C) {
+  const long long warps64 = (long long)B * ((T + 63) / 64) * ((C + 63) / 64);
+  return warps64 >= 148 * 8 ? 64 : (warps64 >= 148 * 4 ? 32 : 16);
+}
+static bool shortconv_ring(int W) { return W == 4 || W == 8 || W == 16; }
+
+// Slices of the weight-gradient scratch of elfa_shortconv_bwd (slices * (W + 1) * C floats), 0 when it needs none.
+ELFA_API int elfa_shortconv_bwd_slices(int B, int T, int C, int W) {
+  if (!shortconv_ring(W) || B <= 0 || T <= 0 || C <= 0) return 0;
+  const int span = shortconv_span(B, T, C);
+  return B * ((T + span - 1) / span);
+}
+
 ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, int W, void* stream) {
   ELFA_REQUIRE(x && w && y && B > 0 && T > 0 && C > 0 && W > 0, "shortconv_fwd: bad arguments");
   ELFA_REQUIRE(C % 2 == 0 && W <= 128, "shortconv_fwd: the channel count must be even and the window at most 128");
+  if (shortconv_ring(W)) {
+    const auto *X = static_cast<const __nv_bfloat16*>(x), *Wt = static_cast<const __nv_bfloat16*>(w), *Bi = static_cast<const __nv_bfloat16*>(bias);
+    auto* Y = static_cast<__nv_bfloat16*>(y);
+    const int span = shortconv_span(B, T, C), spans = (T + span - 1) / span;
+    const dim3 g((unsigned)(((long long)B * spans + 3) / 4), (C + 63) / 64), blk(32, 4);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (W == 4) shortconv_ring_fwd_kernel<4><<<g, blk, 0, s>>>(X, Wt, Bi, Y, B, T, C, span, spans);
+    else if (W == 8) shortconv_ring_fwd_kernel<8><<<g, blk, 0, s>>>(X, Wt, Bi, Y, B, T, C, span, spans);
+    else shortconv_ring_fwd_kernel<16><<<g, blk, 0, s>>>(X, Wt, Bi, Y, B, T, C, span, spans);
+    ELFA_CUDA(cudaGetLastError());
+    ::elfa::count_launches(1);
+    return ELFA_OK;
+  }
   const long long rows = (long long)B * T;
   dim3 grid((unsigned)((rows + SC_ROWS - 1) / SC_ROWS), (C + 63) / 64), block(32, 8);
   shortconv_apply_kernel<false><<<grid, block, (size_t)W * 64 * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
@@ -265,12 +438,27 @@ ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, 
   return ELFA_OK;
 }
 
-// dx bf16 [B,T,C]; dw fp32 [C,W]; db fp32 [C] or null.
-ELFA_API int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, int B, int T, int C, int W,
-                                void* stream) {
+// dx bf16 [B,T,C]; dw fp32 [C,W]; db fp32 [C] or null; part: scratch of elfa_shortconv_bwd_slices() * (W + 1) * C floats (null when 0).
+ELFA_API int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, float* part, int B, int T,
+                                int C, int W, void* stream) {
   ELFA_REQUIRE(x && w && dy && dx && dw && B > 0 && T > 0 && C > 0 && W > 0, "shortconv_bwd: bad arguments");
   ELFA_REQUIRE(C % 2 == 0 && W <= 128, "shortconv_bwd: the channel count must be even and the window at most 128");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (shortconv_ring(W)) {
+    ELFA_REQUIRE(part, "shortconv_bwd: this window needs the scratch buffer");
+    const auto *X = static_cast<const __nv_bfloat16*>(x), *Wt = static_cast<const __nv_bfloat16*>(w), *G = static_cast<const __nv_bfloat16*>(dy);
+    auto* DX = static_cast<__nv_bfloat16*>(dx);
+    const int span = shortconv_span(B, T, C), spans = (T + span - 1) / span;
+    const dim3 g((unsigned)(((long long)B * spans + 3) / 4), (C + 63) / 64), blk(32, 4);
+    if (W == 4) shortconv_ring_bwd_kernel<4><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
+    else if (W == 8) shortconv_ring_bwd_kernel<8><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
+    else shortconv_ring_bwd_kernel<16><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
+    ELFA_CUDA(cudaGetLastError());
+    shortconv_sum_kernel<<<dim3((C + 31) / 32, W + 1), dim3(32, 16), 0, s>>>(part, dw, db, B * spans, C, W);
+    ELFA_CUDA(cudaGetLastError());
+    ::elfa::count_launches(2);
+    return ELFA_OK;
+  }
   const long long rows = (long long)B * T;
   dim3 grid((unsigned)((rows + SC_ROWS - 1) / SC_ROWS), (C + 63) / 64), block(32, 8);
   shortconv_apply_kernel<true><<<grid, block, (size_t)W * 64 * sizeof(float), s>>>(

@@ -199,8 +199,9 @@ int elfa_efla_chunk_bwd(const void* k, const void* v, const void* nmat, const fl
                         const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0,
                         float* dckpt, int B, int T, int H, int d, void* stream);
 int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, int W, void* stream);
-int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, int B, int T, int C, int W,
-                       void* stream);
+int elfa_shortconv_bwd_slices(int B, int T, int C, int W);
+int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, float* part, int B, int T, int C,
+                       int W, void* stream);
 
 #ifdef __cplusplus
 }

@@ -214,7 +214,9 @@ class _ShortConv(torch.autograd.Function):
         dx = torch.empty_like(xc)
         dw = torch.empty((C, W), dtype=torch.float32, device=xc.device)
         db = torch.empty(C, dtype=torch.float32, device=xc.device) if ctx.has_bias else None
-        lib.call("elfa_shortconv_bwd", xc, weight, dyc, dx, dw, db, B, T, C, W, stream_ptr(xc))
+        slices = lib.raw("elfa_shortconv_bwd_slices")(B, T, C, W)
+        part = torch.empty((slices, W + 1, C), dtype=torch.float32, device=xc.device) if slices else None
+        lib.call("elfa_shortconv_bwd", xc, weight, dyc, dx, dw, db, part, B, T, C, W, stream_ptr(xc))
         return dx, dw.to(weight.dtype), (db.to(weight.dtype) if db is not None else None)
 
 
