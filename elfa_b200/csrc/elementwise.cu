@@ -229,6 +229,87 @@ ELFA_API int elfa_cast(const void* src, int src_type, void* dst, int dst_type, l
   return ELFA_OK;
 }
 
+// ---- gated activation ---------------------------------------------------------------------------------
+// h [rows, 2 F] = [gate | up] -> a [rows, F] = silu(gate) * up, and its gradient in one pass each, straight from the projection's output:
+// no copies of the halves, no intermediate in bf16. Memory bound (3 F and 5 F bf16 per row); two vectors per operand in flight:
+// 4096 rows, F 8192: 45 and 65 us (4.5 and 5.2 TB/s), as separate copies, activation, product and their gradients about 370.
+namespace elfa {
+namespace {
+
+template <bool BWD>
+__global__ void __launch_bounds__(256) swiglu_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ da,
+                                                     __nv_bfloat16* __restrict__ out, long long rows, int F) {
+  constexpr int U = 2;
+  const int per = F / 8;
+  const long long n = rows * per, stride = (long long)gridDim.x * blockDim.x;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += U * stride) {
+    uint4 gq[U], uq[U], dq[U];
+    long long at[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const long long i = i0 + k * stride, r = i / per, c = i - r * per;
+      at[k] = r * 2 * per + c;                       // vector index in h: gate half; the other half is `per` further
+      if (i < n) {
+        gq[k] = reinterpret_cast<const uint4*>(h)[at[k]];
+        uq[k] = reinterpret_cast<const uint4*>(h)[at[k] + per];
+        if (BWD) dq[k] = reinterpret_cast<const uint4*>(da)[i];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const long long i = i0 + k * stride;
+      if (i >= n) continue;
+      const uint32_t *pg = reinterpret_cast<const uint32_t*>(&gq[k]), *pu = reinterpret_cast<const uint32_t*>(&uq[k]),
+                     *pd = reinterpret_cast<const uint32_t*>(&dq[k]);
+      uint4 o0, o1;
+      uint32_t *p0 = reinterpret_cast<uint32_t*>(&o0), *p1 = reinterpret_cast<uint32_t*>(&o1);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float a[2], b[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float g = x ? bf16_hi(pg[j]) : bf16_lo(pg[j]), u = x ? bf16_hi(pu[j]) : bf16_lo(pu[j]);
+          if (!BWD) {
+            a[x] = apply<OP_SILU>(g, 0.f, 1.f) * u;
+          } else {
+            const float d = x ? bf16_hi(pd[j]) : bf16_lo(pd[j]);
+            a[x] = apply<OP_SILU_BWD>(g, d * u, 1.f);
+            b[x] = d * apply<OP_SILU>(g, 0.f, 1.f);
+          }
+        }
+        p0[j] = pack_bf16(a[0], a[1]);
+        if (BWD) p1[j] = pack_bf16(b[0], b[1]);
+      }
+      if (!BWD) {
+        reinterpret_cast<uint4*>(out)[i] = o0;
+      } else {
+        reinterpret_cast<uint4*>(out)[at[k]] = o0;
+        reinterpret_cast<uint4*>(out)[at[k] + per] = o1;
+      }
+    }
+  }
+}
+
+}  // namespace
+}  // namespace elfa
+
+// h: [rows, 2 F] bf16; da: null (forward, out = a [rows, F]) or [rows, F] bf16 (backward, out = dh [rows, 2 F]). F a multiple of 8,
+// pointers 16-byte aligned.
+ELFA_API int elfa_swiglu(const void* h, const void* da, void* out, long long rows, int F, void* stream) {
+  ELFA_REQUIRE(h && out && rows > 0 && F > 0 && F % 8 == 0, "swiglu: bad arguments");
+  ELFA_REQUIRE(((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(da) | reinterpret_cast<uintptr_t>(out)) & 15) == 0,
+               "swiglu: pointers must be 16-byte aligned");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const auto *H = static_cast<const __nv_bfloat16*>(h), *D = static_cast<const __nv_bfloat16*>(da);
+  auto* O = static_cast<__nv_bfloat16*>(out);
+  const int g = ew_grid(rows * F);
+  if (da) elfa::swiglu_kernel<true><<<g, 256, 0, s>>>(H, D, O, rows, F);
+  else elfa::swiglu_kernel<false><<<g, 256, 0, s>>>(H, D, O, rows, F);
+  ELFA_CUDA(cudaGetLastError());
+  ::elfa::count_launches(1);
+  return ELFA_OK;
+}
+
 // ---- row softmax ------------------------------------------------------------------------------------
 // reference: kernels/cuda/layernorm.cu softmax kernel and src/nn/nn_kernels.zig:226-267 (host loop).
 // One warp per row, two passes over the row held in registers when it fits (<= 4096 columns), else

@@ -50,6 +50,7 @@ int elfa_norm_bwd(const void* dy, const void* x, const void* w, const float* mea
 
 // ---- elementwise.cu ----------------------------------------------------------------------------
 int elfa_elementwise(int op, const void* a, const void* b, void* out, long long n, float alpha, void* stream);
+int elfa_swiglu(const void* h, const void* da, void* out, long long rows, int F, void* stream);
 int elfa_embedding_fwd(const long long* ids, const void* tok, const void* pos, void* out, int tokens, int D, int seq, int pos_div, int pos0,
                        int vocab_lo, int vocab_hi, int vocab_total, void* stream);
 int elfa_embedding_bwd(const long long* ids, const void* dy, void* dtok, void* dpos, int tokens, int D, int seq, int pos_div, int pos0,

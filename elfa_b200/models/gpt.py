@@ -135,8 +135,7 @@ class MLP(nn.Module):
     def forward(self, x):
         if self.gated:
             h = tpl.column_parallel_linear(x, self.up, self.pc, quant=self.quant)
-            g, u = h.chunk(2, dim=-1)
-            a = ops.activation(g.contiguous(), "silu") * u
+            a = ops.swiglu(h)
         elif self.act == "gelu":
             a = tpl.column_parallel_linear(x, self.up, self.pc, act="gelu", quant=self.quant)
         else:

@@ -212,6 +212,38 @@ def gelu(x):
     return _Act.apply(x, "gelu")
 
 
+class _SwiGLU(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, h):
+        F = h.shape[-1] // 2
+        hc = h.contiguous()
+        if hc.data_ptr() % 16:
+            hc = hc.clone()
+        ctx.save_for_backward(hc)
+        a = torch.empty((*h.shape[:-1], F), dtype=h.dtype, device=h.device)
+        lib.call("elfa_swiglu", hc, None, a, hc.numel() // (2 * F), F, stream_ptr(hc))
+        return a
+
+    @staticmethod
+    def backward(ctx, da):
+        (hc,) = ctx.saved_tensors
+        F = hc.shape[-1] // 2
+        dac = da.contiguous()
+        if dac.data_ptr() % 16:
+            dac = dac.clone()
+        dh = torch.empty_like(hc)
+        lib.call("elfa_swiglu", hc, dac, dh, hc.numel() // (2 * F), F, stream_ptr(hc))
+        return dh
+
+
+def swiglu(h: torch.Tensor) -> torch.Tensor:
+    """``silu(gate) * up`` of ``h [..., 2 F] = [gate | up]``. CUDA bf16 tensors with F a multiple of 8 take one kernel per direction."""
+    if h.is_cuda and h.dtype == torch.bfloat16 and h.shape[-1] % 16 == 0 and h.numel() > 0:
+        return _SwiGLU.apply(h)
+    g, u = h.chunk(2, dim=-1)
+    return activation(g.contiguous(), "silu") * u
+
+
 # ---------------------------------------------------------------------------------------- embedding
 class _Embedding(torch.autograd.Function):
     @staticmethod
