@@ -369,12 +369,15 @@ class _CrossEntropy(torch.autograd.Function):
             return per.sum() / denom
         assert l2.is_contiguous() and l2.dtype == torch.bfloat16
         rows = l2.shape[0]
-        stats = torch.empty((rows, 4), dtype=torch.float32, device=l2.device)
         per = torch.empty(rows, dtype=torch.float32, device=l2.device)
         st = stream_ptr(l2)
-        lib.call("elfa_xent_stats", l2, l2.stride(0), t1, stats, rows, V, 0, V, st)
-        lib.call("elfa_xent_grad", l2, l2.stride(0), l2, l2.stride(0), t1, stats, 1, per, rows, V, 0, V, float(smoothing), None,
-                 grad_scale / denom, st)
+        if V % 8 == 0 and V <= lib.raw("elfa_xent_row_max")() and l2.data_ptr() % 16 == 0:
+            lib.call("elfa_xent_row", l2, l2.stride(0), t1, per, rows, V, float(smoothing), grad_scale / denom, st)
+        else:        # rows too wide for shared memory, or not whole vectors: statistics, then gradient
+            stats = torch.empty((rows, 4), dtype=torch.float32, device=l2.device)
+            lib.call("elfa_xent_stats", l2, l2.stride(0), t1, stats, rows, V, 0, V, st)
+            lib.call("elfa_xent_grad", l2, l2.stride(0), l2, l2.stride(0), t1, stats, 1, per, rows, V, 0, V, float(smoothing), None,
+                     grad_scale / denom, st)
         ctx.cpu = False
         ctx.save_for_backward(l2)
         ctx.shape = logits.shape

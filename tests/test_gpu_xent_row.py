@@ -1,0 +1,36 @@
+"""One-pass cross-entropy (rows in shared memory) at the edges of its thread tiling and past its widest row, against fp32 PyTorch.
+
+The gradient is rounded to bf16 once (2^-8 of the largest); the loss is an fp32 sum over the rows.
+"""
+import pytest
+import torch
+
+from elfa_b200 import native, ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("V", [8, 4096, 4104, 8000, 16392, 32000, 32768, 32776])
+@pytest.mark.parametrize("smoothing", [0.0, 0.1])
+def test_cross_entropy_widths(cuda_device, V, smoothing):
+    torch.manual_seed(V)
+    rows = 5
+    x = (torch.randn(rows, V, device=cuda_device) * 3).bfloat16()
+    t = torch.randint(3, V, (rows,), device=cuda_device)
+    t[2], t[3] = -100, V - 1
+    x[1, :3] = -200.0                               # far below the maximum: exp underflows
+    xr = x.float().requires_grad_(True)
+    ref = ops.cross_entropy_ref(xr, t, smoothing).sum() / rows if smoothing else torch.nn.functional.cross_entropy(xr, t, reduction="sum", ignore_index=-100) / rows
+    ref.backward()
+    logits = x.clone().requires_grad_(True)
+    loss = ops.cross_entropy(logits * 1, t, smoothing)
+    (g,) = torch.autograd.grad(loss, logits)
+    assert native.status() == 0
+    assert abs(loss.item() - ref.item()) <= 1e-5 * max(1.0, abs(ref.item()))
+    assert (g.float() - xr.grad).abs().max() <= 2 ** -8 * xr.grad.abs().max()
+
+
+def test_bad_target_is_reported(cuda_device):
+    x = torch.randn(2, 64, device=cuda_device).bfloat16()
+    ops.cross_entropy(x, torch.tensor([3, 64], device=cuda_device))
+    assert native.status() == native.ST_BAD_TARGET
