@@ -192,6 +192,8 @@ int elfa_prism_gated_fwd(const void* u, const void* v, const void* z, long long 
                          void* stream);
 int elfa_prism_gated_bwd(const void* u, const void* v, const void* z, long long ldz, const void* dy, void* du, void* dv, void* dz,
                          long long tokens, int G, int d, int L, void* stream);
+int elfa_prism_state(const void* u, const void* v, const void* z, long long ldz, int off_b, int off_k, const float* state, float* out,
+                     int B, int T, int G, int d, int L, float forget, void* stream);
 
 // ---- efla.cu -----------------------------------------------------------------------------------
 int elfa_efla_scan_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,

@@ -106,7 +106,14 @@ class PrismLayer(nn.Module):
         if conv_tail is not None:
             u = u[:, conv_tail.shape[1]:]
         new_tail = xin[:, -(W - 1):].detach() if W > 1 else None
-        y = eops.prism_gated_refine(u, v, list(self.w_p), self.d)
+        wp, wb, wk = list(self.w_p), list(self.w_beta), list(self.w_k)
+        native = carry_state is not None and eops.prism_stream_native(u, v, wp, wb, wk, carry_state, self.d)
+        if native and not torch.is_grad_enabled():
+            y, new_state = eops.prism_stream(u, v, wp, wb, wk, carry_state, self.forget, self.d)
+            return y, new_state, new_tail
+        y = eops.prism_gated_refine(u, v, wp, self.d)
+        if native:
+            return y, eops.prism_stream(u, v, wp, wb, wk, carry_state, self.forget, self.d)[1], new_tail
         new_state = None
         if carry_state is not None:
             with torch.no_grad():

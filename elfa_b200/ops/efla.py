@@ -336,6 +336,31 @@ def prism_refine_ref(u: torch.Tensor, v: torch.Tensor, p_list, group_dim: int) -
 
 
 @torch.no_grad()
+def prism_stream(u: torch.Tensor, v: torch.Tensor, w_p, w_beta, w_k, state: torch.Tensor, forget: float, group_dim: int
+                 ) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Refinement and state carry of a block of tokens without a gradient: ``(u + refined, new state)``. All ``3 L`` projections are one
+    GEMM over the concatenated weights, the refinement and the state carry one kernel each. For what
+    :func:`prism_stream_native` accepts; :func:`prism_state_update` is the same update token by token."""
+    B, T, D = u.shape
+    L, d = len(w_p), group_dim
+    uc, vc = _aligned(u), _aligned(v)
+    z = gemm(uc.view(-1, D), torch.cat((*w_p, *w_beta, *w_k), 1), b_mn=True)
+    y = torch.empty_like(uc)
+    lib.call("elfa_prism_gated_fwd", uc, vc, z, z.stride(0), y, B * T, D // d, d, L, stream_ptr(uc))
+    out = torch.empty_like(state)
+    lib.call("elfa_prism_state", uc, vc, z, z.stride(0), L * d, 2 * L * d, state.contiguous(), out, B, T, D // d, d, L, float(forget),
+             stream_ptr(uc))
+    return y, out
+
+
+def prism_stream_native(u: torch.Tensor, v: torch.Tensor, w_p, w_beta, w_k, state: torch.Tensor, group_dim: int) -> bool:
+    d = group_dim
+    return (prism_gated_native(u, v, w_p, d) and len(w_beta) == len(w_k) == len(w_p) and d in (32, 64, 96, 128)
+            and all(w.dtype == torch.bfloat16 and w.shape == w_p[0].shape for w in (*w_beta, *w_k))
+            and state.is_cuda and state.dtype == torch.float32 and state.shape == (u.shape[0], u.shape[-1] // d, d, d))
+
+
+@torch.no_grad()
 def prism_state_update(state: torch.Tensor, deltas, betas, ks, forget: float) -> torch.Tensor:
     """Carries the PRISM fast-weight state ``[B, G, d, d]`` over a block of tokens.
     ``deltas[l]`` ``[B, T, G, d]``, ``betas[l]`` ``[B, T]``, ``ks[l]`` ``[B, T, d]`` (unit norm).
