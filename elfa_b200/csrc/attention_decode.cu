@@ -1,0 +1,235 @@
+// Attention of a few new positions against a key / value cache (incremental decoding), with the cache's growth in the same pass.
+//
+// q [s, B, H, hd], the new keys / values [s, B, Hkv, hd] (slices of the fused projection output) and the cache [t, B, Hkv, hd] give
+// out [s, B, H * hd] and the cache of t + s rows. Scores, softmax and the sum over the values are fp32. A CTA owns one (batch, key
+// head) and a slice of the positions: it copies its rows into the new cache while they pass through, scores them against all
+// rep * s query rows that share the key head (H / Hkv = rep heads read a key once) and leaves an unnormalised partial result; a second
+// small launch combines the slices (fixed order). Bound by latency at small t and by the
+// read and write of the cache at large t. B 4, 16 heads of 64 on 4 key heads, t 512: 7 + 4.5 us; concatenation, head repetition and fp32 einsum
+// in PyTorch: about 15 launches.
+//
+// reference: src/eval/evaluator.zig:419-470 (generation runs the whole context again for every token).
+#include "common.cuh"
+#include "elfa_native.h"
+
+namespace elfa {
+namespace {
+
+constexpr int DEC_MAX_SLICE = 256;
+
+struct DecodeParams {
+  const __nv_bfloat16 *q, *knew, *vnew, *kold, *vold;
+  __nv_bfloat16 *kout, *vout, *out;
+  float *part, *stat;                  // [slices][B * Hkv * R][hd], [slices][B * Hkv * R][2] (max, sum)
+  long long ss, sb;                    // strides of q / knew / vnew over positions and batch
+  int t, s, B, H, Hkv, slice, slices;
+  float scale;
+};
+
+// R >= s * rep query rows per key head (the surplus rows repeat the last one and are not written)
+template <int HD, int R>
+__global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeParams p) {
+  constexpr int LPK = HD / 8, KPW = 32 / LPK, UN = 4;       // lanes per key, keys per warp and pass, passes in flight
+  constexpr int CP = HD / 2, NG = 128 / CP;                 // value columns are taken in pairs; key groups of the second pass
+  __shared__ float sc[R][DEC_MAX_SLICE];
+  __shared__ float red[NG][R][HD];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b = blockIdx.x / p.Hkv, hk = blockIdx.x % p.Hkv, rep = p.H / p.Hkv, rows = p.s * rep, total = p.t + p.s;
+  const int k0 = blockIdx.y * p.slice, n = min(p.slice, total - k0);
+  const long long crow = (long long)p.B * p.Hkv * HD, coff = ((long long)b * p.Hkv + hk) * HD;
+  const __nv_bfloat16* kn = p.knew + b * p.sb + (long long)hk * HD;
+  const __nv_bfloat16* vn = p.vnew + b * p.sb + (long long)hk * HD;
+
+  float qr[R][8];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int rr = min(r, rows - 1), qi = rr / rep, h = hk * rep + rr % rep;
+    const uint4 v = *reinterpret_cast<const uint4*>(p.q + qi * p.ss + b * p.sb + (long long)h * HD + (lane % LPK) * 8);
+    const uint32_t* pv = reinterpret_cast<const uint32_t*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      qr[r][2 * j] = bf16_lo(pv[j]);
+      qr[r][2 * j + 1] = bf16_hi(pv[j]);
+    }
+  }
+  for (int kb = warp * KPW * UN; kb < n; kb += 4 * KPW * UN) {
+    uint4 kq[UN];
+#pragma unroll
+    for (int x = 0; x < UN; ++x) {
+      const int key = kb + x * KPW + lane / LPK, at = k0 + key;
+      kq[x] = make_uint4(0, 0, 0, 0);
+      if (key < n)
+        kq[x] = at < p.t ? *reinterpret_cast<const uint4*>(p.kold + at * crow + coff + (lane % LPK) * 8)
+                         : *reinterpret_cast<const uint4*>(kn + (at - p.t) * p.ss + (lane % LPK) * 8);
+    }
+#pragma unroll
+    for (int x = 0; x < UN; ++x) {
+      const int key = kb + x * KPW + lane / LPK, at = k0 + key;
+      if (key < n) *reinterpret_cast<uint4*>(p.kout + at * crow + coff + (lane % LPK) * 8) = kq[x];
+      const uint32_t* pk = reinterpret_cast<const uint32_t*>(&kq[x]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float a = 0.f, c = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          a += qr[r][2 * j] * bf16_lo(pk[j]);
+          c += qr[r][2 * j + 1] * bf16_hi(pk[j]);
+        }
+        a += c;
+#pragma unroll
+        for (int o = LPK / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        // query row r stands at position t + r / rep and sees the keys up to its own
+        if (key < n && lane % LPK == 0) sc[r][key] = at <= p.t + r / rep ? a * p.scale : -INFINITY;
+      }
+    }
+  }
+  __syncthreads();
+  for (int r = warp; r < R; r += 4) {
+    float mx = -INFINITY;
+    for (int i = lane; i < n; i += 32) mx = fmaxf(mx, sc[r][i]);
+    mx = warp_max(mx);
+    float sum = 0.f;
+    for (int i = lane; i < n; i += 32) {
+      const float e = mx == -INFINITY ? 0.f : expf(sc[r][i] - mx);
+      sc[r][i] = e;
+      sum += e;
+    }
+    sum = warp_sum(sum);
+    if (lane == 0 && r < rows) {
+      float* st = p.stat + (((long long)blockIdx.y * gridDim.x + blockIdx.x) * rows + r) * 2;
+      st[0] = mx;
+      st[1] = sum;
+    }
+  }
+  __syncthreads();
+  const int grp = threadIdx.x / CP, cp = threadIdx.x % CP;
+  float acc[R][2];
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0.f;
+  constexpr int UV = 8;
+  for (int kb = grp; kb < n; kb += NG * UV) {
+    uint32_t vq[UV];
+#pragma unroll
+    for (int x = 0; x < UV; ++x) {
+      const int key = kb + x * NG, at = k0 + key;
+      vq[x] = 0u;
+      if (key < n)
+        vq[x] = at < p.t ? *reinterpret_cast<const uint32_t*>(p.vold + at * crow + coff + cp * 2)
+                         : *reinterpret_cast<const uint32_t*>(vn + (at - p.t) * p.ss + cp * 2);
+    }
+#pragma unroll
+    for (int x = 0; x < UV; ++x) {
+      const int key = kb + x * NG;
+      if (key >= n) continue;
+      *reinterpret_cast<uint32_t*>(p.vout + (k0 + key) * crow + coff + cp * 2) = vq[x];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        // a hidden key has weight 0 and must not reach the sum even when its value is not finite
+        const float w = sc[r][key];
+        if (w != 0.f) {
+          acc[r][0] += w * bf16_lo(vq[x]);
+          acc[r][1] += w * bf16_hi(vq[x]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) *reinterpret_cast<float2*>(&red[grp][r][cp * 2]) = make_float2(acc[r][0], acc[r][1]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < rows * HD; i += 128) {
+    const int r = i / HD, c = i % HD;
+    float a = 0.f;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) a += red[g][r][c];
+    p.part[(((long long)blockIdx.y * gridDim.x + blockIdx.x) * rows + r) * HD + c] = a;
+  }
+}
+
+// grid B * Hkv * rows, block hd: out = sum_i part_i exp(m_i - M) / sum_i l_i exp(m_i - M)
+__global__ void attn_decode_combine_kernel(const DecodeParams p, int hd) {
+  const int rep = p.H / p.Hkv, rows = p.s * rep, bhk = blockIdx.x / rows, r = blockIdx.x % rows, c = threadIdx.x;
+  const long long step = (long long)p.B * p.Hkv * rows;
+  float M = -INFINITY;
+  for (int i = 0; i < p.slices; ++i) M = fmaxf(M, p.stat[(i * step + blockIdx.x) * 2]);
+  float num = 0.f, den = 0.f;
+  for (int i = 0; i < p.slices; ++i) {
+    const float* st = p.stat + (i * step + blockIdx.x) * 2;
+    const float w = st[0] == -INFINITY ? 0.f : expf(st[0] - M);
+    num += w * p.part[(i * step + blockIdx.x) * hd + c];
+    den += w * st[1];
+  }
+  const int b = bhk / p.Hkv, h = (bhk % p.Hkv) * rep + r % rep;
+  p.out[(((long long)(r / rep) * p.B + b) * p.H + h) * hd + c] = __float2bfloat16(num / den);
+}
+
+template <int HD>
+int launch_decode(const DecodeParams& p, cudaStream_t st) {
+  const int rows = p.s * (p.H / p.Hkv);
+  const dim3 grid(p.B * p.Hkv, p.slices);
+  if (rows <= 1) attn_decode_kernel<HD, 1><<<grid, 128, 0, st>>>(p);
+  else if (rows <= 2) attn_decode_kernel<HD, 2><<<grid, 128, 0, st>>>(p);
+  else if (rows <= 4) attn_decode_kernel<HD, 4><<<grid, 128, 0, st>>>(p);
+  else attn_decode_kernel<HD, 8><<<grid, 128, 0, st>>>(p);
+  ELFA_CUDA(cudaGetLastError());
+  attn_decode_combine_kernel<<<p.B * p.Hkv * rows, HD, 0, st>>>(p, HD);
+  ELFA_CUDA(cudaGetLastError());
+  ::elfa::count_launches(2);
+  return ELFA_OK;
+}
+
+// Positions per CTA: about two CTAs per SM, 32 to DEC_MAX_SLICE positions each.
+int decode_slice(int total, int heads) {
+  const int want = (2 * 148 + heads - 1) / heads;
+  int slice = ((total + want - 1) / want + 31) / 32 * 32;
+  return slice < 32 ? 32 : (slice > DEC_MAX_SLICE ? DEC_MAX_SLICE : slice);
+}
+
+}  // namespace
+}  // namespace elfa
+
+using namespace elfa;
+
+// Slices the positions are split into (sizes the scratch of elfa_attention_decode: slices * B * s * H * (hd + 2) floats).
+ELFA_API int elfa_attention_decode_slices(int total, int B, int Hkv) {
+  if (total <= 0 || B <= 0 || Hkv <= 0) return 0;
+  const int slice = decode_slice(total, B * Hkv);
+  return (total + slice - 1) / slice;
+}
+
+// q / knew / vnew: bf16, element (position i, batch b, head h, column c) at i * ss + b * sb + h * hd + c, 16-byte aligned rows; kold / vold:
+// [t, B, Hkv, hd] and kout / vout: [t + s, B, Hkv, hd] contiguous; out: [s, B, H * hd]. hd 32, 64, 128 or 256, s * H / Hkv <= 8.
+ELFA_API int elfa_attention_decode(const void* q, const void* knew, const void* vnew, long long ss, long long sb, const void* kold,
+                                   const void* vold, void* kout, void* vout, void* out, float* scratch, int t, int s, int B, int H, int Hkv,
+                                   int hd, float scale, void* stream) {
+  ELFA_REQUIRE(q && knew && vnew && kold && vold && kout && vout && out && scratch, "attention_decode: null pointer");
+  ELFA_REQUIRE(t > 0 && s > 0 && B > 0 && Hkv > 0 && H > 0 && H % Hkv == 0 && s * (H / Hkv) <= 8, "attention_decode: bad sizes");
+  ELFA_REQUIRE(ss % 8 == 0 && sb % 8 == 0, "attention_decode: row strides must be multiples of 8");
+  uintptr_t bits = 0;
+  for (const void* ptr : {q, knew, vnew, kold, vold, static_cast<const void*>(kout), static_cast<const void*>(vout)}) bits |= reinterpret_cast<uintptr_t>(ptr);
+  ELFA_REQUIRE((bits & 15) == 0, "attention_decode: operands must be 16-byte aligned");
+  DecodeParams p{};
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.knew = static_cast<const __nv_bfloat16*>(knew);
+  p.vnew = static_cast<const __nv_bfloat16*>(vnew);
+  p.kold = static_cast<const __nv_bfloat16*>(kold);
+  p.vold = static_cast<const __nv_bfloat16*>(vold);
+  p.kout = static_cast<__nv_bfloat16*>(kout);
+  p.vout = static_cast<__nv_bfloat16*>(vout);
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.ss = ss; p.sb = sb;
+  p.t = t; p.s = s; p.B = B; p.H = H; p.Hkv = Hkv;
+  p.slice = decode_slice(t + s, B * Hkv);
+  p.slices = (t + s + p.slice - 1) / p.slice;
+  ELFA_REQUIRE(p.slices <= 65535, "attention_decode: the cache is too long");
+  p.scale = scale;
+  p.part = scratch;
+  p.stat = scratch + (long long)p.slices * B * s * H * hd;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (hd) {
+    case 32: return launch_decode<32>(p, st);
+    case 64: return launch_decode<64>(p, st);
+    case 128: return launch_decode<128>(p, st);
+    case 256: return launch_decode<256>(p, st);
+    default: set_last_error("attention_decode: head dimension must be 32, 64, 128 or 256"); return ELFA_ERR_UNSUPPORTED;
+  }
+}

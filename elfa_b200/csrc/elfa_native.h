@@ -182,6 +182,12 @@ int elfa_p2p_wait(const void* counter, unsigned int target, int wait_ms, void* s
 int elfa_p2p_probe(const void* src, unsigned long long dst, long long bytes, int mode, int ctas, int warps, int piece, int depth,
                    void* stream);
 
+// ---- attention_decode.cu -----------------------------------------------------------------------
+int elfa_attention_decode_slices(int total, int B, int Hkv);
+int elfa_attention_decode(const void* q, const void* knew, const void* vnew, long long ss, long long sb, const void* kold,
+                          const void* vold, void* kout, void* vout, void* out, float* scratch, int t, int s, int B, int H, int Hkv,
+                          int hd, float scale, void* stream);
+
 // ---- prism.cu ----------------------------------------------------------------------------------
 int elfa_prism_fwd(const void* u, const void* v, const unsigned long long* p, void* y, long long tokens, int G, int d, int L,
                    void* stream);

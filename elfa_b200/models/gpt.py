@@ -96,6 +96,9 @@ class Attention(nn.Module):
             q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
         if cache is not None and cache.get("k") is not None:
             # incremental decoding: the new rows attend to the cached keys / values and, causally, to each other
+            if ops.attention_decode_native(q, k, v, cache["k"], cache["v"]):
+                o, cache["k"], cache["v"] = ops.attention_decode(q, k, v, cache["k"], cache["v"])
+                return tpl.row_parallel_linear(o, self.w_o, self.pc, quant=self.quant)
             k_all = torch.cat((cache["k"], k), 0)
             v_all = torch.cat((cache["v"], v), 0)
             cache["k"], cache["v"] = k_all, v_all

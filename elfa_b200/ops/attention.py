@@ -118,3 +118,34 @@ def attention(qkv: torch.Tensor, causal: bool = True, seq_first: bool = True, sc
     if doc_start is not None:
         assert causal and doc_start.dtype == torch.int32 and doc_start.is_contiguous() and doc_start.is_cuda
     return _Attention.apply(qkv, causal, seq_first, sc, num_heads, doc_start)
+
+
+def attention_decode_native(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
+    """What :func:`attention_decode` handles: CUDA bf16, no gradient wanted, at most eight query rows per key head, rows of ``q`` / ``k`` /
+    ``v`` packed and on 16-byte boundaries."""
+    s, B, H, hd = q.shape
+    Hkv = k.shape[2]
+    ts = (q, k, v, k_cache, v_cache)
+    return (q.is_cuda and all(t.dtype == torch.bfloat16 and t.device == q.device for t in ts) and hd in (32, 64, 128, 256)
+            and H % Hkv == 0 and 0 < s * (H // Hkv) <= 8 and k_cache.shape == v_cache.shape and k_cache.shape[0] > 0
+            and k_cache.shape[1:] == (B, Hkv, hd) and k.shape == v.shape == (s, B, Hkv, hd)
+            and q.stride()[:2] == k.stride()[:2] == v.stride()[:2]
+            and all(t.stride(3) == 1 and t.stride(2) == hd and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
+                    for t in (q, k, v))
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)))
+
+
+def attention_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor):
+    """The last ``s`` positions ``q [s, B, H, hd]``, ``k, v [s, B, Hkv, hd]`` against the cache ``[t, B, Hkv, hd]`` and, causally, each other.
+    Returns ``(out [s, B, H * hd], keys [t + s, ...], values [t + s, ...])``: the kernel writes the grown cache as it reads the old one."""
+    s, B, H, hd = q.shape
+    Hkv = k.shape[2]
+    kc, vc = (t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.contiguous().clone() for t in (k_cache, v_cache))
+    t = kc.shape[0]
+    ko, vo = (torch.empty((t + s, B, Hkv, hd), dtype=q.dtype, device=q.device) for _ in range(2))
+    out = torch.empty((s, B, H * hd), dtype=q.dtype, device=q.device)
+    slices = lib.raw("elfa_attention_decode_slices")(t + s, B, Hkv)
+    scratch = torch.empty(slices * B * s * H * (hd + 2), dtype=torch.float32, device=q.device)
+    lib.call("elfa_attention_decode", q, k, v, q.stride(0), q.stride(1), kc, vc, ko, vo, out, scratch, t, s, B, H, Hkv, hd,
+             1.0 / math.sqrt(hd), stream_ptr(q))
+    return out, ko, vo
