@@ -129,16 +129,8 @@ class _Lib:
         return (self.load().elfa_last_error() or b"").decode()
 
     def call(self, name: str, *args) -> None:
-        dll = self.load()
-        conv = []
-        for a in args:
-            if isinstance(a, torch.Tensor):
-                conv.append(a.data_ptr())
-            elif a is None:
-                conv.append(None)
-            else:
-                conv.append(a)
-        rc = getattr(dll, name)(*conv)
+        dll = self._dll or self.load()
+        rc = getattr(dll, name)(*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args])
         if rc != 0:
             raise NativeError(f"{name} failed (code {rc}): {self.last_error()}")
 
@@ -150,7 +142,8 @@ lib = _Lib()
 
 
 def stream_ptr(t: Optional[torch.Tensor] = None) -> int:
-    return torch.cuda.current_stream(t.device if t is not None else None).cuda_stream
+    """The calling thread's current stream on ``t``'s device, as the raw handle (no Stream object in between)."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device() if t is not None else torch.cuda.current_device())
 
 
 def status() -> int:
