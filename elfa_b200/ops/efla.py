@@ -61,8 +61,8 @@ def efla_scan_chunked_ref(k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, 
     ``(I + diag(c) tril(K K^T, -1)) U = diag(c) (V - K S0)``, so with ``Tm = (I + diag(c) tril(K K^T, -1))^{-1} diag(c)``
     (a unit-lower-triangular solve, independent of the state and hence parallel over all chunks):
     ``U = Tm V - (Tm K) S0``, ``O = K S0 + tril(K K^T) U``, ``S_end = S0 + K^T U``.
-    fp32, differentiable; equal to :func:`efla_scan_ref` up to rounding. It is the oracle for a tensor-core kernel of this
-    form (the CUDA kernels here are sequential in time) and a faster CPU path for long sequences."""
+    fp32, differentiable; equal to :func:`efla_scan_ref` up to rounding. The CUDA kernels take this form
+    with 32 tokens per chunk; here it is their oracle and a faster CPU path for long sequences."""
     B, T, H, d = k.shape
     C = min(chunk, T)
     pad = (-T) % C
