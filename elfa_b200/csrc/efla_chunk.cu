@@ -48,10 +48,17 @@ __global__ void __launch_bounds__(64) efla_prep_kernel(const __nv_bfloat16* __re
   __nv_bfloat16* sk = sk_all[warp];
   float(*sg)[36] = sg_all[warp];
   const __nv_bfloat16* kb = k + (((long long)b * T + t0) * H + h) * D;
-  for (int i = lane; i < EC * (D / 8); i += 32) {
-    const int r = i / (D / 8), c = i % (D / 8);
-    const uint4 z = make_uint4(0, 0, 0, 0);
-    *reinterpret_cast<uint4*>(sk + r * LD + c * 8) = r < n ? *reinterpret_cast<const uint4*>(kb + (long long)r * H * D + c * 8) : z;
+  uint4 kq[D / 8];                         // every load of the chunk in flight before the first store
+#pragma unroll
+  for (int u = 0; u < D / 8; ++u) {
+    const int i = u * 32 + lane, r = i / (D / 8), c = i % (D / 8);
+    kq[u] = make_uint4(0, 0, 0, 0);
+    if (r < n) kq[u] = *reinterpret_cast<const uint4*>(kb + (long long)r * H * D + c * 8);
+  }
+#pragma unroll
+  for (int u = 0; u < D / 8; ++u) {
+    const int i = u * 32 + lane, r = i / (D / 8), c = i % (D / 8);
+    *reinterpret_cast<uint4*>(sk + r * LD + c * 8) = kq[u];
   }
   __syncwarp();
   const uint32_t ks = smem_u32(sk);
@@ -432,7 +439,7 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
 //   dlam_t = c_t sum_j (dO E)_tj + dc_t dc/dlam,   dbeta = sum_t dc_t ex_t
 // Only dS is sequential: efla_chunk_bwd_state_kernel walks the chunks backwards with dS in registers and writes the dS1 of every chunk;
 // efla_chunk_bwd_kernel then handles all chunks in parallel from the two chunk-boundary states.
-// B 8, T 2048, 16 heads of 64: 95 us and 255 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
+// B 8, T 2048, 16 heads of 64: 94 us and 259 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
 // finish). The parallel kernel issues about 400 mma.sync per warp and chunk (94 us of tensor time at 8.3 cycles each) and reads 370 MB
 // (55 us); a third CTA per SM, at 168 registers, did not make it faster.
 template <int D>
@@ -581,9 +588,14 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
   }
   for (int i = tid; i < 3 * EC * 4; i += 2 * D) cp_async16(base + L::N + ((i / 4) * EN_LD + (i % 4) * 8) * 2, nmat + id * EN_ELEMS + i * 8, true);
   if (tid < EC_COEF / 4) cp_async16(base + L::C + tid * 16, coef + id * EC_COEF + tid * 4, true);
-  cp_async_commit();
   const float4* sp = ckpt + efla_state_slot<D>(id, warp, lane);
-  const float4* dp = dckpt + efla_state_slot<D>(id, warp, lane);
+  const uint32_t scr_e = base + L::SCRATCH + warp * L::SCR, scr_s = scr_e + L::SCR_E;
+  {                                        // dS1 waits in the scratch (every lane reads back its own vectors) until E is done
+    const float4* dp = dckpt + efla_state_slot<D>(id, warp, lane);
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) cp_async16(scr_s + (i * 32 + lane) * 16, dp + i * 32, true);
+  }
+  cp_async_commit();
   float S[D / 8][4];
 #pragma unroll
   for (int i = 0; i < D / 8; ++i) {
@@ -631,7 +643,7 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
   efla_apply_n<false>(e, base + L::N, lane);
 #pragma unroll
   for (int i = 0; i < D / 8; ++i) {
-    const float4 f = dp[i * 32];
+    const float4 f = reinterpret_cast<const float4*>(smem + L::SCRATCH + warp * L::SCR + L::SCR_E)[i * 32 + lane];
     S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
   }
   efla_state_times_k<D>(de, S, base + L::K, lane);
@@ -665,7 +677,6 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
   }
   efla_apply_n<true>(de, base + L::N, lane);
 
-  const uint32_t scr_e = base + L::SCRATCH + warp * L::SCR, scr_s = scr_e + L::SCR_E;
   {                                        // dV = dO + dE0, transposed through the scratch
     uint32_t d2[2][4];
 #pragma unroll
