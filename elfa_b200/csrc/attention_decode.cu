@@ -78,19 +78,22 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeParams p) 
         a += c;
 #pragma unroll
         for (int o = LPK / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        // query row r stands at position t + r / rep and sees the keys up to its own
-        if (key < n && lane % LPK == 0) sc[r][key] = at <= p.t + r / rep ? a * p.scale : -INFINITY;
+        if (key < n && lane % LPK == 0) sc[r][key] = a * p.scale;
       }
     }
   }
   __syncthreads();
   for (int r = warp; r < R; r += 4) {
+    // which keys are hidden follows from positions, never from the scores: fmaxf passes over NaN, so a slice whose visible scores are all
+    // NaN keeps -inf as its maximum and must still hand its NaN on
+    const int seen = min(n, p.t + r / rep + 1 - k0);
     float mx = -INFINITY;
-    for (int i = lane; i < n; i += 32) mx = fmaxf(mx, sc[r][i]);
+    for (int i = lane; i < seen; i += 32) mx = fmaxf(mx, sc[r][i]);
     mx = warp_max(mx);
+    const float ref = mx == -INFINITY ? 0.f : mx;
     float sum = 0.f;
-    for (int i = lane; i < n; i += 32) {
-      const float e = mx == -INFINITY ? 0.f : expf(sc[r][i] - mx);
+    for (int i = lane; i < seen; i += 32) {
+      const float e = expf(sc[r][i] - ref);
       sc[r][i] = e;
       sum += e;
     }
@@ -124,9 +127,9 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeParams p) 
       *reinterpret_cast<uint32_t*>(p.vout + (k0 + key) * crow + coff + cp * 2) = vq[x];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        // a hidden key has weight 0 and must not reach the sum even when its value is not finite
-        const float w = sc[r][key];
-        if (w != 0.f) {
+        // query row r stands at position t + r / rep; a later key must not reach the sum even when its value is not finite
+        if (k0 + key <= p.t + r / rep) {
+          const float w = sc[r][key];
           acc[r][0] += w * bf16_lo(vq[x]);
           acc[r][1] += w * bf16_hi(vq[x]);
         }
@@ -149,12 +152,13 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeParams p) 
 __global__ void attn_decode_combine_kernel(const DecodeParams p, int hd) {
   const int rep = p.H / p.Hkv, rows = p.s * rep, bhk = blockIdx.x / rows, r = blockIdx.x % rows, c = threadIdx.x;
   const long long step = (long long)p.B * p.Hkv * rows;
+  const int slices = (p.t + r / rep) / p.slice + 1;       // the slices that hold a key this row sees
   float M = -INFINITY;
-  for (int i = 0; i < p.slices; ++i) M = fmaxf(M, p.stat[(i * step + blockIdx.x) * 2]);
+  for (int i = 0; i < slices; ++i) M = fmaxf(M, p.stat[(i * step + blockIdx.x) * 2]);
   float num = 0.f, den = 0.f;
-  for (int i = 0; i < p.slices; ++i) {
+  for (int i = 0; i < slices; ++i) {
     const float* st = p.stat + (i * step + blockIdx.x) * 2;
-    const float w = st[0] == -INFINITY ? 0.f : expf(st[0] - M);
+    const float w = expf(st[0] - M);       // M = -inf: no score above -inf, NaN as in a softmax over such a row
     num += w * p.part[(i * step + blockIdx.x) * hd + c];
     den += w * st[1];
   }

@@ -34,3 +34,19 @@ def test_gradients_and_wide_blocks_keep_the_general_path(cuda_device):
     q, k, v = h[:, :, :8], h[:, :, 8:10], h[:, :, 10:]
     assert not ops.attention_decode_native(q, k, v, kc, kc)                        # 3 x 4 query rows per key head
     assert not ops.attention_decode_native(q[:1].detach().requires_grad_(True), k[:1], v[:1], kc, kc)
+
+
+@pytest.mark.parametrize("t,s", [(31, 1), (32, 1), (33, 1), (64, 2), (95, 2), (600, 1)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_non_finite_key_is_not_dropped(cuda_device, t, s, bad):
+    """At t = 32 and 95 the newest key is the first of its slice: its NaN scores are the only ones there."""
+    torch.manual_seed(t)
+    h = torch.randn(s, 1, 4, 64, device=cuda_device).bfloat16()
+    h[-1, 0, 2, 5], h[-1, 0, 2, 6] = bad, -bad                                     # inf - inf in the score of every query
+    h[:, :, :2, 5:7] = 1.0
+    q, k, v = h[:, :, :2], h[:, :, 2:3], h[:, :, 3:]
+    kc, vc = (torch.randn(t, 1, 1, 64, device=cuda_device).bfloat16() for _ in range(2))
+    o = ops.attention_decode(q, k, v, kc, vc)[0]
+    ref = _attend_cached(q.float(), torch.cat((kc, k)).repeat_interleave(2, 2).float(), torch.cat((vc, v)).repeat_interleave(2, 2).float())
+    assert ref[-1].isnan().all() and (s == 1 or ref[0].isfinite().all())           # the row before the key does not see it
+    assert torch.equal(o.isnan(), ref.isnan())
