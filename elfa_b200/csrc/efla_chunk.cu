@@ -14,6 +14,13 @@
 // updated by one fp32 addition per chunk, so the error of the state is that of the token-by-token fp32 recurrence or smaller
 // (64-bit comparison at T 2048, 16 heads of 64: 2.2e-7 relative; token by token 2.4e-7).
 //
+// Values that are not finite: as in the recurrence, one in K or V reaches its own token and later ones, one in dO its own token and earlier
+// ones, and V and dO their own columns only (for dV; a row of dK adds up all columns). Inside a chunk the products of the chunked form
+// would carry 0 x NaN to the other tokens, so every kernel asks at its end whether a state or a key gradient came out not finite and, if so,
+// runs once more in a checked form that walks the chunks concerned token by token (efla_walk) and overwrites its results. On finite data
+// that costs one barrier. (Asked for inside the walk over the chunks it stood in the chain of dependent products: forward 105 us against 94
+// now, state gradient 98 against 92 at B 8, T 2048, 16 heads of 64.) Gradients of such tokens are not finite; whether infinity or NaN is not kept.
+//
 // reference: kernels/cuda/efla.cu:121-271,534-552 (chunks are scanned one after the other, the bf16 state in global memory).
 #include "common.cuh"
 #include "elfa_native.h"
@@ -281,6 +288,171 @@ __device__ __forceinline__ void efla_state_update(float (&S)[D / 8][4], const fl
   }
 }
 
+// One chunk token by token, for the columns in which a product of the chunked form is not finite: there 0 x NaN inside a product would reach
+// tokens that the recurrence keeps apart. first[hf] is the token from which on value column g + 8 hf takes these results (EC: the column is
+// left alone); its state rows walk all n tokens. Plain fp32 multiply-adds and a quad's shuffles: only the checked forms come here.
+// sp: the state [D / 8][4] in local memory, read and written. OUT: outputs o_t = p + (1 - ex) e go to so [token][24]; otherwise the errors go
+// to ep [4][4] in local memory.
+template <int D, int KLD, int VLD, bool OUT>
+__device__ __noinline__ void efla_walk(float* sp, float* ep, const __nv_bfloat16* sk, const __nv_bfloat16* sv, const float* cf,
+                                       __nv_bfloat16* so, int first0, int first1, int n) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  float S[D / 8][4];
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) S[i / 4][i % 4] = sp[i];
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    float p0 = 0.f, p1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) {
+      const float2 kk = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sk + t * KLD + i * 8 + 2 * q));
+      p0 += kk.x * S[i][0] + kk.y * S[i][1];
+      p1 += kk.x * S[i][2] + kk.y * S[i][3];
+    }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+      p0 += __shfl_xor_sync(0xffffffffu, p0, m);
+      p1 += __shfl_xor_sync(0xffffffffu, p1, m);
+    }
+    const float c = cf[t], w = 1.f - cf[EC + t];
+    const float e0 = __bfloat162float(sv[t * VLD + g]) - p0, e1 = __bfloat162float(sv[t * VLD + g + 8]) - p1;
+    const bool put = OUT ? q == 0 : q == (t & 7) >> 1;
+    if (put && t >= first0) {
+      if (OUT) so[t * 24 + g] = __float2bfloat16(p0 + w * e0);
+      else ep[(t >> 3) * 4 + (t & 1)] = e0;
+    }
+    if (put && t >= first1) {
+      if (OUT) so[t * 24 + g + 8] = __float2bfloat16(p1 + w * e1);
+      else ep[(t >> 3) * 4 + 2 + (t & 1)] = e1;
+    }
+    const float u0 = c * e0, u1 = c * e1;
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) {
+      const float2 kk = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sk + t * KLD + i * 8 + 2 * q));
+      if (first0 < EC) {
+        S[i][0] += kk.x * u0;
+        S[i][1] += kk.y * u0;
+      }
+      if (first1 < EC) {
+        S[i][2] += kk.x * u1;
+        S[i][3] += kk.y * u1;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) sp[i] = S[i / 4][i % 4];
+}
+
+// The same for the gradient of the state, from the last token to the first: de_t = c y - ex dO with y = dS^T k, dS -= k de. All columns; the
+// de go to ep.
+template <int D, int KLD, int VLD>
+__device__ __noinline__ void efla_walk_back(float* sp, float* ep, const __nv_bfloat16* sk, const __nv_bfloat16* so, const float* cf, int n) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  float S[D / 8][4];
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) S[i / 4][i % 4] = sp[i];
+#pragma unroll 1
+  for (int t = n - 1; t >= 0; --t) {
+    float y0 = 0.f, y1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) {
+      const float2 kk = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sk + t * KLD + i * 8 + 2 * q));
+      y0 += kk.x * S[i][0] + kk.y * S[i][1];
+      y1 += kk.x * S[i][2] + kk.y * S[i][3];
+    }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+      y0 += __shfl_xor_sync(0xffffffffu, y0, m);
+      y1 += __shfl_xor_sync(0xffffffffu, y1, m);
+    }
+    const float d0 = cf[t] * y0 - cf[EC + t] * __bfloat162float(so[t * VLD + g]);
+    const float d1 = cf[t] * y1 - cf[EC + t] * __bfloat162float(so[t * VLD + g + 8]);
+    if (q == (t & 7) >> 1) {
+      ep[(t >> 3) * 4 + (t & 1)] = d0;
+      ep[(t >> 3) * 4 + 2 + (t & 1)] = d1;
+    }
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) {
+      const float2 kk = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sk + t * KLD + i * 8 + 2 * q));
+      S[i][0] -= kk.x * d0;
+      S[i][1] -= kk.y * d0;
+      S[i][2] -= kk.x * d1;
+      S[i][3] -= kk.y * d1;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < D / 2; ++i) sp[i] = S[i / 4][i % 4];
+}
+
+// y_t = dS^T k_t of every token, put where the errors are put
+template <int D, int KLD>
+__device__ __noinline__ void efla_rows(const float* sp, float* ep, const __nv_bfloat16* sk, int n) {
+  const int lane = threadIdx.x & 31, q = lane & 3;
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    float y0 = 0.f, y1 = 0.f;
+#pragma unroll 4
+    for (int i = 0; i < D / 8; ++i) {
+      const float2 kk = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sk + t * KLD + i * 8 + 2 * q));
+      y0 += kk.x * sp[i * 4] + kk.y * sp[i * 4 + 1];
+      y1 += kk.x * sp[i * 4 + 2] + kk.y * sp[i * 4 + 3];
+    }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+      y0 += __shfl_xor_sync(0xffffffffu, y0, m);
+      y1 += __shfl_xor_sync(0xffffffffu, y1, m);
+    }
+    if (q == (t & 7) >> 1) {
+      ep[(t >> 3) * 4 + (t & 1)] = y0;
+      ep[(t >> 3) * 4 + 2 + (t & 1)] = y1;
+    }
+  }
+}
+
+// a state tile holds a value that is not finite
+template <int D>
+__device__ __forceinline__ bool efla_not_finite(const float (&S)[D / 8][4]) {
+  float chk = 0.f;
+#pragma unroll
+  for (int i = 0; i < D / 8; ++i)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) chk = fmaf(S[i][x], 0.f, chk);
+  return chk != 0.f;
+}
+// any lane of the warp holds a value that is not finite
+__device__ __forceinline__ bool efla_any_bad(const float (&e)[4][4]) {
+  float chk = 0.f;
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) chk = fmaf(e[nt][x], 0.f, chk);
+  return __any_sync(0xffffffffu, chk != 0.f);
+}
+// first[hf] = the earliest token at which column g + 8 hf is not finite, at most what it was; those entries become 0
+__device__ __forceinline__ void efla_take_bad(float (&e)[4][4], int (&first)[2], int q) {
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (!(fabsf(e[nt][x]) <= 3.402823466e38f)) {
+        first[x >> 1] = min(first[x >> 1], nt * 8 + 2 * q + (x & 1));
+        e[nt][x] = 0.f;
+      }
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+    first[hf] = min(first[hf], __shfl_xor_sync(0xffffffffu, first[hf], 1));
+    first[hf] = min(first[hf], __shfl_xor_sync(0xffffffffu, first[hf], 2));
+  }
+}
+
+// e = V - e for a warp's tile, V^T as read by ldmatrix
+__device__ __forceinline__ void efla_errors(float (&e)[4][4], const uint32_t (&vq)[2][4]) {
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) e[nt][x] = ((x & 1) ? bf16_hi(vq[x >> 1][nt]) : bf16_lo(vq[x >> 1][nt])) - e[nt][x];
+}
+
 // Chunk-boundary states are stored as the warps hold them: [B, H, chunk][d / 16 value blocks][d / 8 tiles][lane] float4.
 template <int D>
 __device__ __forceinline__ long long efla_state_slot(long long chunk_id, int vblock, int lane) {
@@ -289,11 +461,11 @@ __device__ __forceinline__ long long efla_state_slot(long long chunk_id, int vbl
 
 // Grid (B * H, d / columns of a CTA). k, v, o: [B, T, H, d] bf16. state0 / state_out: [B, H, d, d] fp32 or null. ckpt (or null):
 // the state at the start of every chunk.
-// Bound by the dependent chain of a chunk (about 130 mma.sync and 700 instructions of one warp per scheduler), not by memory. With the
-// preparation, B 1, T 8192, 16 heads of 64, no gradient: 397 us, token by token (with its checkpoints) 2364 us; in the training step of
-// B 8, T 2048 the forward went from about 0.75 to 0.13 ms.
-template <int D>
-__global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
+// Bound by the dependent chain of a chunk (132 mma.sync and about 900 instructions of one warp per scheduler), not by memory. With the
+// preparation, B 1, T 8192, 16 heads of 64, no gradient: 354 us, token by token (with its checkpoints) 2364 us; in the training step of
+// B 8, T 2048 the forward went from about 750 to 94 us and 28 us for the preparation.
+template <int D, bool CHECKED>
+__device__ __forceinline__ bool efla_fwd_walk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ nmat,
     const float* __restrict__ coef, const float* __restrict__ state0, __nv_bfloat16* __restrict__ o, float* __restrict__ state_out,
     float4* __restrict__ ckpt, int T, int H, int nchunks) {
@@ -340,42 +512,17 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
     uint32_t vq[2][4];                     // V^T tiles: [value half][token tile], tokens 2q, 2q + 1 of column g
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) ldsm4_t(vq[hf], st + L::V + (lane * L::VLD + warp * 16 + hf * 8) * 2);
-    float chk = 0.f;
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const float vv = (x & 1) ? bf16_hi(vq[x >> 1][nt]) : bf16_lo(vq[x >> 1][nt]);
-        e[nt][x] = vv - e[nt][x];
-        chk = fmaf(e[nt][x], 0.f, chk);
-      }
-    // a non-finite error stays with its token and the later ones: it is taken out of the product (0 x NaN would reach the earlier
-    // tokens of the chunk) and put back behind it
-    const bool bad = __any_sync(0xffffffffu, chk != 0.f);
-    int first[2] = {EC, EC};
-    if (bad) {
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int x = 0; x < 4; ++x)
-          if (!(fabsf(e[nt][x]) <= 3.402823466e38f)) {
-            first[x >> 1] = min(first[x >> 1], nt * 8 + 2 * q + (x & 1));
-            e[nt][x] = 0.f;
-          }
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        first[hf] = min(first[hf], __shfl_xor_sync(0xffffffffu, first[hf], 1));
-        first[hf] = min(first[hf], __shfl_xor_sync(0xffffffffu, first[hf], 2));
-      }
-    }
+    efla_errors(e, vq);
     efla_apply_n<false>(e, st + L::N, lane);
-    if (bad) {
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int x = 0; x < 4; ++x)
-          if (nt * 8 + 2 * q + (x & 1) >= first[x >> 1]) e[nt][x] = __int_as_float(0x7fffffff);
+    int first[2] = {EC, EC};
+    if (CHECKED && efla_any_bad(e)) {      // once more, without the entries at fault: the other columns and the tokens before keep their bits
+      efla_state_times_k<D>(e, S, st + L::K, lane);
+      efla_errors(e, vq);
+      efla_take_bad(e, first, q);
+      efla_apply_n<false>(e, st + L::N, lane);
+      efla_take_bad(e, first, q);
     }
+    const bool bad = CHECKED && __any_sync(0xffffffffu, first[0] < EC || first[1] < EC);
     uint32_t oq[2][4];
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
@@ -388,12 +535,31 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
         e[nt][2 * hf + 1] *= cc.y;
       }
     }
+    if (bad) {
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (first[x >> 1] < EC) e[nt][x] = 0.f;                     // the walk below moves these columns
+    }
     efla_state_update<D, false>(S, e, st + L::K, lane);
     const uint32_t so = smem_u32(stage_o);
     __syncwarp();
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) stsm4_t(so + (lane * 24 + hf * 8) * 2, oq[hf][0], oq[hf][1], oq[hf][2], oq[hf][3]);
     __syncwarp();
+    if (bad) {
+      const unsigned char* sst = smem + (ch % EC_STAGES) * L::BYTES;
+      float sl[D / 2];
+#pragma unroll
+      for (int n = 0; n < D / 2; ++n) sl[n] = S[n / 4][n % 4];
+      efla_walk<D, L::KLD, L::VLD, true>(sl, nullptr, reinterpret_cast<const __nv_bfloat16*>(sst + L::K),
+                                         reinterpret_cast<const __nv_bfloat16*>(sst + L::V) + warp * 16, cf, stage_o, first[0], first[1],
+                                         min(EC, T - ch * EC));
+#pragma unroll
+      for (int n = 0; n < D / 2; ++n) S[n / 4][n % 4] = sl[n];
+      __syncwarp();
+    }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int t = u * 16 + (lane >> 1), hf = lane & 1;
@@ -409,6 +575,24 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
       for (int x = 0; x < 4; ++x)
         state_out[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] = S[n][x];
   }
+  // an error that was not finite anywhere has left its state column not finite (mma.sync: also 0 x NaN)
+  return efla_not_finite<D>(S);
+}
+
+template <int D>
+__device__ __noinline__ void efla_fwd_again(
+    const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* nmat, const float* coef, const float* state0, __nv_bfloat16* o,
+    float* state_out, float4* ckpt, int T, int H, int nchunks) {
+  efla_fwd_walk<D, true>(k, v, nmat, coef, state0, o, state_out, ckpt, T, H, nchunks);
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
+    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ nmat,
+    const float* __restrict__ coef, const float* __restrict__ state0, __nv_bfloat16* __restrict__ o, float* __restrict__ state_out,
+    float4* __restrict__ ckpt, int T, int H, int nchunks) {
+  if (__syncthreads_or(efla_fwd_walk<D, false>(k, v, nmat, coef, state0, o, state_out, ckpt, T, H, nchunks)))
+    efla_fwd_again<D>(k, v, nmat, coef, state0, o, state_out, ckpt, T, H, nchunks);
 }
 
 template <int D>
@@ -442,8 +626,8 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
 // B 8, T 2048, 16 heads of 64: 94 us and 259 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
 // finish). The parallel kernel issues about 400 mma.sync per warp and chunk (94 us of tensor time at 8.3 cycles each) and reads 370 MB
 // (55 us); a third CTA per SM, at 168 registers, did not make it faster.
-template <int D>
-__global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_bwd_state_kernel(
+template <int D, bool CHECKED>
+__device__ __forceinline__ bool efla_bwd_walk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ nmat,
     const float* __restrict__ coef, const float* __restrict__ dstate_out, float4* __restrict__ dckpt, float* __restrict__ dstate0, int T,
     int H, int nchunks) {
@@ -499,7 +683,19 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_bwd_state_kerne
       }
     }
     efla_apply_n<true>(e, st + L::N, lane);
-    efla_state_update<D, true>(S, e, st + L::K, lane);
+    if (!(CHECKED && efla_any_bad(e))) {
+      efla_state_update<D, true>(S, e, st + L::K, lane);
+    } else {                               // e.g. a NaN in dO: it reaches its own and the earlier tokens only
+      float sl[D / 2], unused[16];
+#pragma unroll
+      for (int n = 0; n < D / 2; ++n) sl[n] = S[n / 4][n % 4];
+      const unsigned char* sst = smem + (i % EC_STAGES) * L::BYTES;
+      efla_walk_back<D, L::KLD, L::VLD>(sl, unused, reinterpret_cast<const __nv_bfloat16*>(sst + L::K),
+                                        reinterpret_cast<const __nv_bfloat16*>(sst + L::V) + warp * 16, cf,
+                                        min(EC, T - (nchunks - 1 - i) * EC));
+#pragma unroll
+      for (int n = 0; n < D / 2; ++n) S[n / 4][n % 4] = sl[n];
+    }
   }
   cp_async_wait<0>();
   if (dstate0) {
@@ -509,6 +705,22 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_bwd_state_kerne
       for (int x = 0; x < 4; ++x)
         dstate0[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] = S[n][x];
   }
+  return efla_not_finite<D>(S);
+}
+
+template <int D>
+__device__ __noinline__ void efla_bwd_again(const __nv_bfloat16* k, const __nv_bfloat16* dout, const __nv_bfloat16* nmat, const float* coef,
+                                            const float* dstate_out, float4* dckpt, float* dstate0, int T, int H, int nchunks) {
+  efla_bwd_walk<D, true>(k, dout, nmat, coef, dstate_out, dckpt, dstate0, T, H, nchunks);
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_bwd_state_kernel(
+    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ nmat,
+    const float* __restrict__ coef, const float* __restrict__ dstate_out, float4* __restrict__ dckpt, float* __restrict__ dstate0, int T,
+    int H, int nchunks) {
+  if (__syncthreads_or(efla_bwd_walk<D, false>(k, dout, nmat, coef, dstate_out, dckpt, dstate0, T, H, nchunks)))
+    efla_bwd_again<D>(k, dout, nmat, coef, dstate_out, dckpt, dstate0, T, H, nchunks);
 }
 
 // One CTA per chunk, d / 16 warps; warp w owns value columns 16 w .. 16 w + 15 and all key rows. E, Y, dE0 are recomputed from the
@@ -562,8 +774,8 @@ __device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[3
   mma_bf16(acc, a[ai], b[bi][o], b[bi][o + 1]);
 }
 
-template <int D>
-__global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
+template <int D, bool CHECKED>
+__device__ __forceinline__ bool efla_bwd_chunk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ dout,
     const __nv_bfloat16* __restrict__ nmat, const float* __restrict__ coef, const float4* __restrict__ ckpt,
     const float4* __restrict__ dckpt, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
@@ -636,46 +848,80 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
     ldsm4_t(vq[hf], base + L::V + (lane * L::LD + warp * 16 + hf * 8) * 2);
     ldsm4_t(oq[hf], base + L::O + (lane * L::LD + warp * 16 + hf * 8) * 2);
   }
-#pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) e[nt][x] = ((x & 1) ? bf16_hi(vq[x >> 1][nt]) : bf16_lo(vq[x >> 1][nt])) - e[nt][x];
+  efla_errors(e, vq);
   efla_apply_n<false>(e, base + L::N, lane);
+  const float4* ds1 = reinterpret_cast<const float4*>(smem + L::SCRATCH + warp * L::SCR + L::SCR_E) + lane;
 #pragma unroll
   for (int i = 0; i < D / 8; ++i) {
-    const float4 f = reinterpret_cast<const float4*>(smem + L::SCRATCH + warp * L::SCR + L::SCR_E)[i * 32 + lane];
+    const float4 f = ds1[i * 32];
     S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
   }
   efla_state_times_k<D>(de, S, base + L::K, lane);
   float* ssum = reinterpret_cast<float*>(smem + L::SUM) + warp * 2 * EC;
+  auto sums_and_de = [&]() {               // the sums of Y E and dO E over the warp's columns; de: from Y to dE
 #pragma unroll
-  for (int nt = 0; nt < 4; ++nt) {
-    const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
-    const float2 ex = *reinterpret_cast<const float2*>(cf + EC + nt * 8 + 2 * q);
-    float ye[2] = {0.f, 0.f}, oe[2] = {0.f, 0.f};
+    for (int nt = 0; nt < 4; ++nt) {
+      const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
+      const float2 ex = *reinterpret_cast<const float2*>(cf + EC + nt * 8 + 2 * q);
+      float ye[2] = {0.f, 0.f}, oe[2] = {0.f, 0.f};
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      const float o0 = bf16_lo(oq[hf][nt]), o1 = bf16_hi(oq[hf][nt]);
-      ye[0] += de[nt][2 * hf] * e[nt][2 * hf];
-      ye[1] += de[nt][2 * hf + 1] * e[nt][2 * hf + 1];
-      oe[0] += o0 * e[nt][2 * hf];
-      oe[1] += o1 * e[nt][2 * hf + 1];
-      de[nt][2 * hf] = cc.x * de[nt][2 * hf] - ex.x * o0;
-      de[nt][2 * hf + 1] = cc.y * de[nt][2 * hf + 1] - ex.y * o1;
-    }
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-      for (int m = 4; m < 32; m <<= 1) {
-        ye[x] += __shfl_xor_sync(0xffffffffu, ye[x], m);
-        oe[x] += __shfl_xor_sync(0xffffffffu, oe[x], m);
+      for (int hf = 0; hf < 2; ++hf) {
+        const float o0 = bf16_lo(oq[hf][nt]), o1 = bf16_hi(oq[hf][nt]);
+        ye[0] += de[nt][2 * hf] * e[nt][2 * hf];
+        ye[1] += de[nt][2 * hf + 1] * e[nt][2 * hf + 1];
+        oe[0] += o0 * e[nt][2 * hf];
+        oe[1] += o1 * e[nt][2 * hf + 1];
+        de[nt][2 * hf] = cc.x * de[nt][2 * hf] - ex.x * o0;
+        de[nt][2 * hf + 1] = cc.y * de[nt][2 * hf + 1] - ex.y * o1;
       }
-    if (g == 0) {
-      *reinterpret_cast<float2*>(ssum + nt * 8 + 2 * q) = make_float2(ye[0], ye[1]);
-      *reinterpret_cast<float2*>(ssum + EC + nt * 8 + 2 * q) = make_float2(oe[0], oe[1]);
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) {
+          ye[x] += __shfl_xor_sync(0xffffffffu, ye[x], m);
+          oe[x] += __shfl_xor_sync(0xffffffffu, oe[x], m);
+        }
+      if (g == 0) {
+        *reinterpret_cast<float2*>(ssum + nt * 8 + 2 * q) = make_float2(ye[0], ye[1]);
+        *reinterpret_cast<float2*>(ssum + EC + nt * 8 + 2 * q) = make_float2(oe[0], oe[1]);
+      }
     }
-  }
+  };
+  sums_and_de();
   efla_apply_n<true>(de, base + L::N, lane);
+  if (CHECKED && (efla_any_bad(e) || efla_any_bad(de))) {             // token by token: see efla_walk
+    const __nv_bfloat16* tile = reinterpret_cast<const __nv_bfloat16*>(smem);
+    float sl[D / 2], el[16], dl[16];
+    auto fill = [&](const float4* from) {
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i) {
+        const float4 f = from[i * 32];
+        sl[4 * i] = f.x; sl[4 * i + 1] = f.y; sl[4 * i + 2] = f.z; sl[4 * i + 3] = f.w;
+      }
+    };
+    const bool bad_e = efla_any_bad(e), bad_de = efla_any_bad(de);
+    float keep[16];
+#pragma unroll
+    for (int x = 0; x < 16; ++x) {
+      keep[x] = de[x / 4][x % 4];
+      el[x] = dl[x] = 0.f;                 // tokens past the end
+    }
+    if (bad_e) {
+      fill(sp);
+      efla_walk<D, L::LD, L::LD, false>(sl, el, tile + L::K / 2, tile + L::V / 2 + warp * 16, cf, nullptr, 0, 0, n);
+#pragma unroll
+      for (int x = 0; x < 16; ++x) e[x / 4][x % 4] = el[x];
+    }
+    fill(ds1);
+    efla_rows<D, L::LD>(sl, dl, tile + L::K / 2, n);
+#pragma unroll
+    for (int x = 0; x < 16; ++x) de[x / 4][x % 4] = dl[x];
+    __syncwarp();                          // the sums are written anew
+    sums_and_de();
+    if (bad_de) efla_walk_back<D, L::LD, L::LD>(sl, dl, tile + L::K / 2, tile + L::O / 2 + warp * 16, cf, n);
+#pragma unroll
+    for (int x = 0; x < 16; ++x) de[x / 4][x % 4] = bad_de ? dl[x] : keep[x];
+  }
 
   {                                        // dV = dO + dE0, transposed through the scratch
     uint32_t d2[2][4];
@@ -843,6 +1089,7 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
       }
     }
   }
+  float chk = 0.f;
 #pragma unroll
   for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
@@ -859,8 +1106,27 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
           s.y += r.y;
         }
         if (t < n) *reinterpret_cast<uint32_t*>(dk + off + t * rs + warp * 16 + u * 8 + 2 * q) = pack_bf16(s.x, s.y);
+        chk = fmaf(s.x, 0.f, fmaf(s.y, 0.f, chk));
       }
     }
+  return chk != 0.f;                       // an error or gradient that was not finite is in the key gradient of its token
+}
+
+template <int D>
+__device__ __noinline__ void efla_bwd_chunk_again(const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* dout,
+                                                  const __nv_bfloat16* nmat, const float* coef, const float4* ckpt, const float4* dckpt,
+                                                  __nv_bfloat16* dk, __nv_bfloat16* dv, float* dbeta_tok, int T, int H, int nchunks) {
+  efla_bwd_chunk<D, true>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks);
+}
+
+template <int D>
+__global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
+    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ dout,
+    const __nv_bfloat16* __restrict__ nmat, const float* __restrict__ coef, const float4* __restrict__ ckpt,
+    const float4* __restrict__ dckpt, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
+    float* __restrict__ dbeta_tok, int T, int H, int nchunks) {
+  if (__syncthreads_or(efla_bwd_chunk<D, false>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks)))
+    efla_bwd_chunk_again<D>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks);
 }
 
 template <int D>

@@ -90,3 +90,56 @@ def test_backward_of_one_output_only(cuda_device):
     eops.efla_scan(k, v, beta)[1].square().sum().backward()
     eops.efla_scan_ref(kr, v, beta)[1].square().sum().backward()
     _close(k.grad, kr.grad, 2 ** -8)
+
+
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+def test_an_infinite_value_gives_an_infinite_output(cuda_device, d):
+    """o = p + c lam (v - p) is infinite for its token, the state gets the sign of the key, later outputs of the column are NaN; a column
+    of a finite chunk keeps its bits. Token 40 is the last one, or one in the middle of its chunk."""
+    for T in (41, 64):
+        k, v, beta, s0 = _inputs(cuda_device, 1, T, 2, d, True)
+        o0, f0 = eops.efla_scan(k, v, beta, s0)
+        v[0, 40, 0, 5] = float("inf")
+        o, s = eops.efla_scan(k, v, beta, s0)
+        assert o[0, 40, 0, 5] == float("inf") and o[0, 41:, 0, 5].isnan().all()
+        o[0, 40:, 0, 5] = o0[0, 40:, 0, 5]
+        assert torch.equal(o, o0)
+        if T == 41:
+            assert torch.equal(s[0, 0, :, 5], torch.copysign(torch.full((d,), float("inf"), device=cuda_device), k[0, 40, 0].float()))
+        s[0, 0, :, 5] = f0[0, 0, :, 5]
+        assert torch.equal(s, f0)
+
+
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_backward_keeps_a_bad_token_to_its_side(cuda_device, d, bad):
+    """A bad value touches the key gradients of its own and later tokens only and no value gradient; a bad output gradient touches its own
+    and earlier tokens only, and its own column of the value gradients. The finite ones are those of the clean call, up to the bf16 rounding
+    of sums taken in another order."""
+    T = 100
+    k, v, beta, s0 = _inputs(cuda_device, 1, T, 2, d, True)
+    torch.manual_seed(d)
+    go, gs = torch.randn_like(v), 0.1 * torch.randn(1, 2, d, d, device=cuda_device)
+
+    def grads(v, go):
+        ins = [t.detach().clone().requires_grad_(True) for t in (k, v, s0)]
+        o, s = eops.efla_scan(ins[0], ins[1], beta, ins[2])
+        return torch.autograd.grad([o, s], ins, [go, gs])
+
+    dk0, dv0, ds0 = grads(v, go)
+    v1 = v.clone()
+    v1[0, 41, 0, 5] = bad
+    dk, dv, ds = grads(v1, go)
+    assert torch.equal(dv, dv0) and torch.equal(ds, ds0) and torch.equal(dk[:, :, 1], dk0[:, :, 1])
+    _close(dk[:, :41, 0], dk0[:, :41, 0], 2 ** -8)
+    assert not dk[0, 41:, 0].isfinite().any()
+    g1 = go.clone()
+    g1[0, 41, 0, 5] = bad
+    dk, dv, ds = grads(v, g1)
+    assert torch.equal(dk[:, :, 1], dk0[:, :, 1])
+    _close(dk[:, 42:, 0], dk0[:, 42:, 0], 2 ** -8)
+    _close(dv[:, 42:, 0], dv0[:, 42:, 0], 2 ** -8)
+    assert not dk[0, :42, 0].isfinite().any() and not dv[0, :42, 0, 5].isfinite().any()
+    keep = [j for j in range(d) if j != 5]
+    _close(dv[:, :, 0, keep], dv0[:, :, 0, keep], 2 ** -8)
+    _close(ds[:, :, :, keep], ds0[:, :, :, keep], 1e-5)
