@@ -347,9 +347,9 @@ def prism_stream(u: torch.Tensor, v: torch.Tensor, w_p, w_beta, w_k, state: torc
     z = gemm(uc.view(-1, D), torch.cat((*w_p, *w_beta, *w_k), 1), b_mn=True)
     y = torch.empty_like(uc)
     lib.call("elfa_prism_gated_fwd", uc, vc, z, z.stride(0), y, B * T, D // d, d, L, stream_ptr(uc))
-    out = torch.empty_like(state)
-    lib.call("elfa_prism_state", uc, vc, z, z.stride(0), L * d, 2 * L * d, state.contiguous(), out, B, T, D // d, d, L, float(forget),
-             stream_ptr(uc))
+    st = state.contiguous()
+    out = torch.empty_like(st)               # of the contiguous state: a strided one would hand its strides on
+    lib.call("elfa_prism_state", uc, vc, z, z.stride(0), L * d, 2 * L * d, st, out, B, T, D // d, d, L, float(forget), stream_ptr(uc))
     return y, out
 
 

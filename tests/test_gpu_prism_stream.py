@@ -30,3 +30,17 @@ def test_state_carry(cuda_device, T, G, d, L):
     assert (s - want).abs().max() <= 1e-5 * want.abs().max()
     ref = u.float() + sum(deltas).view(B, T, D)
     assert (y.float() - ref).abs().max() <= 2 ** -8 * ref.abs().max()
+
+
+@pytest.mark.parametrize("order", [(1, 0, 2, 3), (0, 2, 1, 3), (0, 1, 3, 2)])
+def test_state_of_any_stride(cuda_device, order):
+    torch.manual_seed(0)
+    B, T, G, d, L = 2, 5, 32, 32, 2
+    u, v = (torch.randn(B, T, G * d, device=cuda_device).bfloat16() for _ in range(2))
+    wp, wb, wk = ([(torch.randn(G * d, d, device=cuda_device) * (G * d) ** -0.5).bfloat16() for _ in range(L)] for _ in range(3))
+    s0 = torch.randn(B, G, d, d, device=cuda_device)
+    view = s0.permute(order).contiguous().permute(order)          # the same values, dense in another order (each order is its own inverse)
+    assert not view.is_contiguous() and torch.equal(view, s0)
+    want = eops.prism_stream(u, v, wp, wb, wk, s0, 0.97, d)
+    got = eops.prism_stream(u, v, wp, wb, wk, view, 0.97, d)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
