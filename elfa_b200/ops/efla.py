@@ -302,10 +302,11 @@ class _PrismGated(torch.autograd.Function):
 
 
 def prism_gated_native(u: torch.Tensor, v: torch.Tensor, ws, group_dim: int) -> bool:
-    """What the fused gate handles: CUDA bf16, at most eight iterations, groups and rows of whole 16-byte vectors."""
-    D = u.shape[-1]
-    return (u.is_cuda and v.shape == u.shape and all(t.dtype == torch.bfloat16 for t in (u, v, *ws)) and 1 <= len(ws) <= 8 and u.numel() > 0
-            and group_dim % 8 == 0 and D % group_dim == 0 and all(w.shape == (D, group_dim) for w in ws))
+    """What the fused gate handles: CUDA bf16 on one device, at most eight iterations, groups and rows of whole 16-byte vectors."""
+    D, dev = u.shape[-1], u.device
+    return (u.is_cuda and v.shape == u.shape and all(t.dtype == torch.bfloat16 and t.device == dev for t in (u, v, *ws))
+            and 1 <= len(ws) <= 8 and u.numel() > 0 and group_dim % 8 == 0 and D % group_dim == 0
+            and all(w.shape == (D, group_dim) for w in ws))
 
 
 def prism_gated_refine(u: torch.Tensor, v: torch.Tensor, ws, group_dim: int) -> torch.Tensor:
@@ -354,10 +355,10 @@ def prism_stream(u: torch.Tensor, v: torch.Tensor, w_p, w_beta, w_k, state: torc
 
 
 def prism_stream_native(u: torch.Tensor, v: torch.Tensor, w_p, w_beta, w_k, state: torch.Tensor, group_dim: int) -> bool:
-    d = group_dim
+    d, dev = group_dim, u.device
     return (prism_gated_native(u, v, w_p, d) and len(w_beta) == len(w_k) == len(w_p) and d in (32, 64, 96, 128)
-            and all(w.dtype == torch.bfloat16 and w.shape == w_p[0].shape for w in (*w_beta, *w_k))
-            and state.is_cuda and state.dtype == torch.float32 and state.shape == (u.shape[0], u.shape[-1] // d, d, d))
+            and all(w.dtype == torch.bfloat16 and w.shape == w_p[0].shape and w.device == dev for w in (*w_beta, *w_k))
+            and state.device == dev and state.dtype == torch.float32 and state.shape == (u.shape[0], u.shape[-1] // d, d, d))
 
 
 @torch.no_grad()

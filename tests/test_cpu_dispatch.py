@@ -1,0 +1,27 @@
+"""Which calls the native paths take, asked with stand-ins for CUDA tensors: nothing here touches a device."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from elfa_b200.ops import efla as eops
+
+
+def _fake(*shape, device="cuda:0", dtype=torch.bfloat16):
+    return SimpleNamespace(shape=torch.Size(shape), device=torch.device(device), dtype=dtype, is_cuda=device.startswith("cuda"),
+                           numel=lambda: torch.Size(shape).numel())
+
+
+@pytest.mark.parametrize("other", ["cpu", "cuda:1"])
+def test_prism_kernels_want_one_device(other):
+    """A kernel given a host pointer, or one of another GPU, would fault: those calls belong to the general path, which refuses them."""
+    d, D = 32, 64
+    u, v, s = _fake(2, 3, D), _fake(2, 3, D), _fake(2, 2, d, d, dtype=torch.float32)
+    ws = [[_fake(D, d) for _ in range(2)] for _ in range(3)]
+    assert eops.prism_gated_native(u, v, ws[0], d) and eops.prism_stream_native(u, v, *ws, s, d)
+    assert not eops.prism_gated_native(u, _fake(2, 3, D, device=other), ws[0], d)
+    assert not eops.prism_stream_native(u, v, *ws, _fake(2, 2, d, d, device=other, dtype=torch.float32), d)
+    for i in range(3):
+        moved = [list(w) for w in ws]
+        moved[i][1] = _fake(D, d, device=other)
+        assert not eops.prism_stream_native(u, v, *moved, s, d)
