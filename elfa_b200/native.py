@@ -143,7 +143,10 @@ lib = _Lib()
 
 def stream_ptr(t: Optional[torch.Tensor] = None) -> int:
     """The calling thread's current stream on ``t``'s device, as the raw handle (no Stream object in between)."""
-    return torch._C._cuda_getCurrentRawStream(t.get_device() if t is not None else torch.cuda.current_device())
+    i = t.get_device() if t is not None else torch.cuda.current_device()
+    if i < 0:            # the index of a host tensor, which stands for the current device: no kernel may be given such a tensor
+        raise ValueError(f"Expected a cuda device, but got: {t.device}")
+    return torch._C._cuda_getCurrentRawStream(i)
 
 
 def status() -> int:

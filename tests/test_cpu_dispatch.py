@@ -4,6 +4,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
+from elfa_b200 import native
 from elfa_b200.ops import efla as eops
 
 
@@ -25,3 +26,12 @@ def test_prism_kernels_want_one_device(other):
         moved = [list(w) for w in ws]
         moved[i][1] = _fake(D, d, device=other)
         assert not eops.prism_stream_native(u, v, *moved, s, d)
+
+
+def test_a_host_tensor_has_no_stream(monkeypatch):
+    asked = []
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda i: asked.append(i) or 7, raising=False)
+    assert native.stream_ptr(SimpleNamespace(get_device=lambda: 1)) == 7 and asked == [1]
+    with pytest.raises(ValueError, match="cuda device"):
+        native.stream_ptr(torch.zeros(1))
+    assert asked == [1]
