@@ -159,6 +159,42 @@ __global__ void __launch_bounds__(XENT_THREADS) xent_grad_kernel(__nv_bfloat16* 
 // kernels about 300.
 constexpr int XENT_ROW_MAX = 8 * 8 * XENT_THREADS;
 
+// The row of xent_row_kernel when its maximum leaves base 2 (|x| log2(e) past the largest float: rows of the type's lowest value, for one; or
+// infinite logits): in natural units, everything relative to the maximum.
+__device__ __noinline__ void xent_row_huge(__nv_bfloat16* x, const uint4* xrow, int nvec, int V, bool valid, float tl, int tv, int tj,
+                                           float smoothing, float grad_scale, float* loss, float (*red)[XENT_THREADS / 32]) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float m = -INFINITY;
+  for (int i = threadIdx.x; i < nvec * 8; i += XENT_THREADS) m = fmaxf(m, __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xrow)[i]));
+  m = warp_max(m);
+  __syncthreads();
+  if (lane == 0) red[0][wid] = m;
+  __syncthreads();
+  for (int i = 0; i < XENT_THREADS / 32; ++i) m = fmaxf(m, red[0][i]);
+  float s = 0.f, sx = 0.f;
+  for (int i = threadIdx.x; i < nvec * 8; i += XENT_THREADS) {
+    const float f = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xrow)[i]) - m;
+    s += expf(f);
+    sx += f / (float)V;                    // the plain sum would overflow
+  }
+  s = warp_sum(s);
+  sx = warp_sum(sx);
+  if (lane == 0) { red[1][wid] = s; red[2][wid] = sx; }
+  __syncthreads();
+  s = sx = 0.f;
+  for (int i = 0; i < XENT_THREADS / 32; ++i) { s += red[1][i]; sx += red[2][i]; }
+  if (threadIdx.x == 0) {
+    float l = (1.f - smoothing) * (tl - m - logf(s));
+    if (smoothing != 0.f) l += smoothing * (sx - logf(s));
+    *loss = valid ? -l : 0.f;
+  }
+  const float gs = valid ? grad_scale : 0.f, off = -gs * (smoothing / (float)V), tg = gs * (1.f - smoothing);
+  for (int i = threadIdx.x; i < nvec * 8; i += XENT_THREADS) {
+    const float f = expf(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xrow)[i]) - m) / s * gs + off;
+    x[i] = __float2bfloat16(f - (valid && i == tv * 8 + tj ? tg : 0.f));
+  }
+}
+
 __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16* __restrict__ logits, long long ld,
                                                                    const long long* __restrict__ targets, float* __restrict__ loss_out, int V,
                                                                    float smoothing, float grad_scale, unsigned int* status) {
@@ -207,8 +243,12 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
   for (int i = 1; i < XENT_THREADS / 32; ++i) { online_combine2(M2, S, sm[0][i], sm[1][i]); SX += sm[2][i]; }
   const float lse2 = M2 + log2f(S), lse = lse2 * 0.6931471805599453f;
   const bool valid = t >= 0 && t < V;
+  if (threadIdx.x == 0 && !valid && t != -100) atomicOr(status, (unsigned)ELFA_ST_BAD_TARGET);
+  if (fabsf(M2) == INFINITY) {             // (a thread whose own maximum overflows downwards rightly adds nothing to a larger one)
+    xent_row_huge(x, xrow, nvec, V, valid, tl, valid ? (int)(t >> 3) : -1, (int)(t & 7), smoothing, grad_scale, loss_out + row, sm);
+    return;
+  }
   if (threadIdx.x == 0) {
-    if (!valid && t != -100) atomicOr(status, (unsigned)ELFA_ST_BAD_TARGET);
     float loss = (1.f - smoothing) * (tl - lse);
     if (smoothing != 0.f) loss += (smoothing / (float)V) * (SX - (float)V * lse);
     loss_out[row] = valid ? -loss : 0.f;

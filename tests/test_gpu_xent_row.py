@@ -34,3 +34,31 @@ def test_bad_target_is_reported(cuda_device):
     x = torch.randn(2, 64, device=cuda_device).bfloat16()
     ops.cross_entropy(x, torch.tensor([3, 64], device=cuda_device))
     assert native.status() == native.ST_BAD_TARGET
+
+
+@pytest.mark.parametrize("V", [64, 4104, 32000])
+@pytest.mark.parametrize("smoothing", [0.0, 0.1])
+def test_logits_near_the_largest_float(cuda_device, V, smoothing):
+    """x log2(e) overflows above 2.36e38: a row of the lowest value is a uniform one, two equal maxima share the probability. 64-bit oracle;
+    one rounding of the gradient to bf16 (2^-8 of the largest) and fp32 sums for the loss."""
+    low, rows = torch.finfo(torch.bfloat16).min, 6
+    x = torch.zeros(rows, V, device=cuda_device).bfloat16()
+    x[0] = low
+    x[1], x[1, 7] = low, -2.5e38
+    x[2, 5] = x[2, V - 3] = 3e38
+    x[3, 5], x[3, 6] = 2.5e38, 3e38
+    x[4, :V // 2] = low                                        # an ordinary row with a mask
+    x[5, 8:] = low                                             # all but one thread's elements masked
+    t = torch.tensor([3, 7, 5, 6, V - 1, 2], device=cuda_device)
+    for r in range(rows):
+        if smoothing and r in (4, 5):                          # the sum over such a row's log-probabilities leaves fp32
+            continue
+        xr = x[r:r + 1].double().requires_grad_(True)
+        ref = torch.nn.functional.cross_entropy(xr, t[r:r + 1], label_smoothing=smoothing)
+        (gr,) = torch.autograd.grad(ref, xr)
+        xi = x[r:r + 1].clone().requires_grad_(True)
+        loss = ops.cross_entropy(xi * 1, t[r:r + 1], smoothing)
+        (g,) = torch.autograd.grad(loss, xi)
+        assert native.status() == 0
+        assert abs(loss.item() - ref.item()) <= 1e-5 * max(1.0, abs(ref.item())), r
+        assert (g.double() - gr).abs().max() <= 2 ** -8 * gr.abs().max() + 1e-7, r
