@@ -40,6 +40,8 @@ int elfa_pinned_free(void* p);
 int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                    long long ldc, int a_mn_major, int b_mn_major, const void* bias, const void* aux, long long ldaux,
                    void* preact, long long ldpre, float alpha, unsigned flags, int force_bn, int max_ctas, void* stream);
+int elfa_gemm_bf16_parts_count(int M, int N, int K);
+int elfa_gemm_bf16_parts(const void* A, const void* B, float* parts, int M, int N, int K, long long lda, long long ldb, void* stream);
 
 // ---- norm.cu -----------------------------------------------------------------------------------
 int elfa_norm_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* sum_out, float* mean_out,
@@ -194,6 +196,8 @@ int elfa_prism_fwd(const void* u, const void* v, const unsigned long long* p, vo
 int elfa_prism_bwd(const void* u, const void* v, const unsigned long long* p, const void* dy, void* du, void* dv,
                    const unsigned long long* dp, long long tokens, int G, int d, int L, void* stream);
 
+int elfa_prism_weight_sum(const float* parts, int splits, long long split_stride, int D, int d, int L, const unsigned long long* outs,
+                          void* stream);
 int elfa_prism_gated_fwd(const void* u, const void* v, const void* z, long long ldz, void* y, long long tokens, int G, int d, int L,
                          void* stream);
 int elfa_prism_gated_bwd(const void* u, const void* v, const void* z, long long ldz, const void* dy, void* du, void* dv, void* dz,

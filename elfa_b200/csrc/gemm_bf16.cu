@@ -65,6 +65,7 @@ struct GemmParams {
   int staged;        // epilogue goes through shared memory + TMA store (plain bf16 output)
   int splits;        // split-K factor (fp32 accumulate outputs only; partial tiles are added atomically)
   int kb_per_split;  // K blocks per split
+  int split_rows;    // > 0: split s stores its partial tile this many rows further down C for each s instead of adding to C (splits is given)
   int sfb_atoms;     // MXFP8: row blocks of the B scale tensor
 };
 
@@ -678,7 +679,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int mb, nb, shard;
       tile_coords_comm<COMM>(p, cm, tile, mb, nb, shard, TILE_M);
       const int m0 = mb * TILE_M + (int)cta_rank * BM, n0 = nb * BN;
-      const int dst_row = COMM == COMM_RS ? cm.rank * cm.rows_per_rank + (m0 - shard * cm.rows_per_rank) : m0;
+      const int dst_row = COMM == COMM_RS ? cm.rank * cm.rows_per_rank + (m0 - shard * cm.rows_per_rank) : m0 + (unit - tile * splits) * p.split_rows;
       const int dst_map = COMM == COMM_RS ? shard : 0;
       for (int cc = 0; cc < CPT; ++cc, ++g) {
         named_bar_sync(2 + (g & 1), 160);               // chunk g is staged
@@ -1042,8 +1043,8 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, in
   }
   if (TWO) max_ctas /= 2;    // work slots are CTA pairs
   const int num_kb_host = MX ? (p.K + 127) / 128 : (p.K + BK - 1) / BK;
-  p.splits = 1;
-  if (COMM == COMM_NONE && !deterministic_mode() && (p.flags & (ELFA_EPI_ACCUM | ELFA_EPI_OUT_F32)) == (ELFA_EPI_ACCUM | ELFA_EPI_OUT_F32)) {
+  if (p.split_rows == 0) p.splits = 1;
+  if (COMM == COMM_NONE && p.split_rows == 0 && !deterministic_mode() && (p.flags & (ELFA_EPI_ACCUM | ELFA_EPI_OUT_F32)) == (ELFA_EPI_ACCUM | ELFA_EPI_OUT_F32)) {
     // fp32 accumulate outputs (weight gradients): split K when the tile count fills the SMs badly
     const int t = p.tiles_m * p.tiles_n;
     auto eff = [&](int sp) { const int u = t * sp; return (double)u / (double)(((u + max_ctas - 1) / max_ctas) * max_ctas); };
@@ -1184,6 +1185,52 @@ ELFA_API int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
     case 256: return dispatch_layout<256>(a_mn_major, b_mn_major, tmA, tmB, p, ctas, s, &om);
     case 128: return dispatch_layout<128>(a_mn_major, b_mn_major, tmA, tmB, p, ctas, s, &om);
     default: return dispatch_layout<64>(a_mn_major, b_mn_major, tmA, tmB, p, ctas, s, &om);
+  }
+}
+
+// Partial products of a contraction whose output has fewer tiles than the GPU has SMs, one per slice of the contraction and each in
+// a place of its own, so that they can be added up in a fixed order (the fp32 accumulate form above adds them atomically, as they come).
+// Slices: as many as fill the SMs with at least 8 K blocks (512 rows) each, none empty.
+static int gemm_parts_plan(int M, int N, int K, int* kb_per) {
+  const int BN = pick_bn(M, N, 0), tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), num_kb = (K + BK - 1) / BK;
+  const int splits = std::max(1, std::min(sm_count() / tiles, num_kb / 8));
+  *kb_per = (num_kb + splits - 1) / splits;
+  return (num_kb + *kb_per - 1) / *kb_per;
+}
+
+ELFA_API int elfa_gemm_bf16_parts_count(int M, int N, int K) {
+  int kb = 0;
+  return M > 0 && N > 0 && K > 0 ? gemm_parts_plan(M, N, K, &kb) : 0;
+}
+
+// parts [count][M rounded up to 128][N] fp32 = slices of A^T B with A [K, M], B [K, N] (both with the output index contiguous); rows past M
+// are zero.
+ELFA_API int elfa_gemm_bf16_parts(const void* A, const void* B, float* parts, int M, int N, int K, long long lda, long long ldb,
+                                  void* stream) {
+  ELFA_REQUIRE(A && B && parts && M > 0 && N > 0 && K > 0, "gemm_parts: bad arguments");
+  ELFA_REQUIRE(N % 8 == 0 && lda % 8 == 0 && ldb % 8 == 0, "gemm_parts: N and the row pitches must be multiples of 8");
+  GemmParams p{};
+  p.M = M; p.N = N; p.K = K;
+  p.C = parts; p.ldc = N;
+  p.alpha = 1.f;
+  p.flags = ELFA_EPI_OUT_F32;
+  p.status = status_word();
+  ELFA_REQUIRE(p.status != nullptr, "gemm_parts: no status word");
+  p.splits = gemm_parts_plan(M, N, K, &p.kb_per_split);
+  p.split_rows = (M + BM - 1) / BM * BM;
+  p.staged = 2;
+  const int BN = pick_bn(M, N, 0);
+  CUtensorMap tmA, tmB;
+  OutMaps om{};
+  int rc = cached_tmap_bf16(&tmA, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BK, 64);
+  if (rc == ELFA_OK) rc = cached_tmap_bf16(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, 64);
+  if (rc == ELFA_OK) rc = cached_tmap(&om.m[0], parts, 4, (uint64_t)p.splits * p.split_rows, (uint64_t)N, (uint64_t)N, BM, 32);
+  if (rc != ELFA_OK) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (BN) {
+    case 256: return launch_gemm<256, true, true>(tmA, tmB, p, sm_count(), s, nullptr, nullptr, &om);
+    case 128: return launch_gemm<128, true, true>(tmA, tmB, p, sm_count(), s, nullptr, nullptr, &om);
+    default: return launch_gemm<64, true, true>(tmA, tmB, p, sm_count(), s, nullptr, nullptr, &om);
   }
 }
 

@@ -289,6 +289,37 @@ int dispatch_prism_gated(const void* u, const void* v, const void* z, long long 
   }
 }
 
+// ---- weight gradients of the gates ----------------------------------------------------------------------
+// out_l [D, d] = sum over the slices of parts [slice][row][L d], columns l d .. l d + d - 1, in slice order: the same bits on every call. A
+// thread owns one element. mode: 0 bf16 store, 1 fp32 store, 2 fp32 add, 3 bf16 add, -1 not wanted.
+struct PrismSumOut {
+  void* out[PRISM_MAX_L];
+  long long ld[PRISM_MAX_L];
+  int mode[PRISM_MAX_L];
+};
+
+__global__ void __launch_bounds__(256) prism_weight_sum_kernel(const float* __restrict__ parts, int splits, long long split_stride, int D,
+                                                               int d, int L, const PrismSumOut o) {
+  const int cols = L * d;
+  const long long n = (long long)D * cols;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const int row = (int)(i / cols), col = (int)(i % cols), l = col / d;
+    const int mode = o.mode[l];
+    if (mode < 0) continue;
+    float s = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) s += parts[k * split_stride + i];
+    const long long at = row * o.ld[l] + (col - l * d);
+    if (mode == 1 || mode == 2) {
+      float* p = static_cast<float*>(o.out[l]) + at;
+      *p = mode == 2 ? *p + s : s;
+    } else {
+      __nv_bfloat16* p = static_cast<__nv_bfloat16*>(o.out[l]) + at;
+      *p = __float2bfloat16(mode == 3 ? __bfloat162float(*p) + s : s);
+    }
+  }
+}
+
 // ---- fast-weight state carry ---------------------------------------------------------------------------
 // Per (batch, group), state S [D, D] fp32 over the tokens t and iterations l (reference: src/model/prism.zig:318-421):
 //   k = z_k / |z_k|, b = sigmoid(mean z_b), delta_l as in the refinement
@@ -451,6 +482,26 @@ ELFA_API int elfa_prism_gated_bwd(const void* u, const void* v, const void* z, l
   ELFA_REQUIRE(d % 8 == 0 && ldz % 8 == 0 && prism_aligned(u, v) && prism_aligned(z, dy) && prism_aligned(du, dv) && prism_aligned(dz, dz),
                "prism_gated_bwd: 8-element alignment");
   return dispatch_prism_gated(u, v, z, ldz, dy, du, dv, dz, tokens, G, d, L, static_cast<cudaStream_t>(stream));
+}
+
+// parts: what elfa_gemm_bf16_parts left, split_stride elements from slice to slice. outs: L triples (pointer, row pitch, mode; see
+// prism_weight_sum_kernel), host memory.
+ELFA_API int elfa_prism_weight_sum(const float* parts, int splits, long long split_stride, int D, int d, int L, const unsigned long long* outs,
+                                   void* stream) {
+  ELFA_REQUIRE(parts && outs && splits > 0 && D > 0 && d > 0 && L >= 1 && L <= PRISM_MAX_L, "prism_weight_sum: bad arguments");
+  PrismSumOut o{};
+  for (int l = 0; l < L; ++l) {
+    o.out[l] = reinterpret_cast<void*>(outs[3 * l]);
+    o.ld[l] = (long long)outs[3 * l + 1];
+    o.mode[l] = (int)(long long)outs[3 * l + 2];
+    ELFA_REQUIRE(o.mode[l] >= -1 && o.mode[l] <= 3 && (o.mode[l] < 0 || o.out[l]), "prism_weight_sum: bad output");
+  }
+  const long long blocks = ((long long)D * L * d + 255) / 256;
+  prism_weight_sum_kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(parts, splits, split_stride, D,
+                                                                                                               d, L, o);
+  ELFA_CUDA(cudaGetLastError());
+  count_launches(1);
+  return ELFA_OK;
 }
 
 // Carries the fast-weight state [B, G, d, d] fp32 over T tokens. u, v: [B, T, G * d] bf16; z: [B * T, ..] bf16 with row pitch ldz holding the

@@ -19,12 +19,13 @@ Math restated from the reference (all three are host loops there):
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional, Tuple
 
 import torch
 
 from ..native import NativeError, lib, stream_ptr
-from .gemm import _accumulate_main_grad, gelu_tanh_ref, gemm, linear
+from .gemm import gelu_tanh_ref, gemm, linear
 
 
 def stable_coefficient(beta: torch.Tensor, lam: torch.Tensor) -> torch.Tensor:
@@ -233,7 +234,6 @@ class _PrismRefine(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, u, v, group_dim, *ps):
-        import ctypes
         B, T, D = u.shape
         uc, vc = u.contiguous(), v.contiguous()
         pcs = [p.contiguous() for p in ps]
@@ -246,7 +246,6 @@ class _PrismRefine(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        import ctypes
         uc, vc, *pcs = ctx.saved_tensors
         B, T, D = uc.shape
         d = ctx.group_dim
@@ -260,9 +259,42 @@ class _PrismRefine(torch.autograd.Function):
         return (du, dv, None) + tuple(g.to(p.dtype) for g, p in zip(dps, pcs))
 
 
+def _prism_weight_grads(ws, wanted, u: torch.Tensor, dz: torch.Tensor, d: int):
+    """``u^T dz`` as the gradients of the gates' weights, one per column block of ``d``: returned, or added to a weight's ``main_grad``
+    (overwritten when that is fresh). ``D x L d`` is a handful of tiles, so the product is cut along the tokens and the
+    pieces are added up in order: the same bits on every call, in the deterministic mode and outside it (B 8, T 2048, D 1024, d 64, L 2:
+    17 + 3 us; unsplit, one product per weight, 71 us each)."""
+    L, (rows, D) = len(ws), u.shape
+    outs, triples = [None] * L, []
+    for l, w in enumerate(ws):
+        if not wanted[l]:
+            triples += [0, 0, 2 ** 64 - 1]
+            continue
+        to = getattr(w, "main_grad", None)
+        if to is None:
+            to = outs[l] = torch.empty((D, d), dtype=w.dtype, device=u.device)
+            add = False
+        else:
+            add = not getattr(w, "_grad_fresh", False)
+            w._grad_fresh = False
+        f32 = to.dtype == torch.float32
+        assert to.shape == (D, d) and to.stride(1) == 1 and (f32 or to.dtype == torch.bfloat16)
+        triples += [to.data_ptr(), to.stride(0), (2 if add else 1) if f32 else (3 if add else 0)]
+    if any(wanted):
+        n = lib.raw("elfa_gemm_bf16_parts_count")(D, L * d, rows)
+        parts = torch.empty((n, (D + 127) // 128 * 128, L * d), dtype=torch.float32, device=u.device)
+        lib.call("elfa_gemm_bf16_parts", u, dz, parts, D, L * d, rows, u.stride(0), dz.stride(0), stream_ptr(u))
+        shared = len({id(w) for w in ws}) < L       # one buffer for several iterations: one after the other
+        for l in range(L if shared else 1):
+            some = [x if not shared or i // 3 == l else (2 ** 64 - 1 if i % 3 == 2 else x) for i, x in enumerate(triples)]
+            arr = (ctypes.c_uint64 * (3 * L))(*some)
+            lib.call("elfa_prism_weight_sum", parts, n, parts.stride(0), D, d, L, ctypes.addressof(arr), stream_ptr(u))
+    return outs
+
+
 class _PrismGated(torch.autograd.Function):
     """The whole gate of the layer: the ``L`` logit products as one GEMM over the concatenated weights, gates and refinement in one
-    kernel; backward is one kernel, one input-gradient GEMM that adds into ``du`` and the weight gradients."""
+    kernel; backward is one kernel, one input-gradient GEMM with an addition into ``du``, and one split product for all weight gradients."""
 
     @staticmethod
     def forward(ctx, u, v, group_dim, *ws):
@@ -289,15 +321,7 @@ class _PrismGated(torch.autograd.Function):
             # short (16384 x 1024 x 128: 76 us)
             g = gemm(dz, wc)
             lib.call("elfa_elementwise", 2, du, g, du, du.numel(), 1.0, stream_ptr(du))
-        dws = [None] * L
-        rest = [l for l, w in enumerate(ctx.w_refs)
-                if ctx.needs_input_grad[3 + l] and not _accumulate_main_grad(w, uc, dz[:, l * d:(l + 1) * d])]
-        if rest:
-            # all of them as one product into fp32, which the GEMM splits along the tokens (D x L d is a handful of tiles, and a bf16
-            # output would walk all tokens in one CTA per tile: B 8, T 2048, D 1024, d 64, L 2: 135 us)
-            dw = gemm(uc, dz, a_mn=True, b_mn=True, out=torch.zeros((D, L * d), dtype=torch.float32, device=dz.device), accumulate=True)
-            for l in rest:
-                dws[l] = dw[:, l * d:(l + 1) * d].to(wc.dtype, memory_format=torch.contiguous_format)
+        dws = _prism_weight_grads(ctx.w_refs, ctx.needs_input_grad[3:], uc, dz, d)
         return (du.view(ctx.shape), dv.view(ctx.shape), None, *dws)
 
 

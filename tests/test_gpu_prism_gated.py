@@ -43,3 +43,51 @@ def test_other_calls_keep_the_general_path(cuda_device):
     assert not eops.prism_gated_native(cpu, cpu, [wc], 8)
     want = eops.prism_refine_ref(cpu, cpu + 1, [torch.sigmoid(cpu @ wc)], 8)
     assert torch.allclose(eops.prism_gated_refine(cpu, cpu + 1, [wc], 8), want, atol=1e-6)
+
+
+def _weight_call(cuda_device, T, G, d, L):
+    torch.manual_seed(T)
+    D = G * d
+    u, v, dy = (torch.randn(2, T, D, device=cuda_device).bfloat16() for _ in range(3))
+    ws = [(torch.randn(D, d, device=cuda_device) * D ** -0.5).bfloat16().requires_grad_(True) for _ in range(L)]
+    return u, v, dy, ws
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("T,G,d,L", [(1, 1, 8, 1), (700, 3, 24, 3), (4100, 16, 64, 2), (2048, 5, 128, 8)])
+def test_weight_gradients_have_one_order(cuda_device, T, G, d, L, deterministic):
+    """Every call gives the same bits, with the deterministic mode and without; a main_grad is overwritten when fresh and added to when not,
+    with the fp32 sum whose rounding is the gradient returned otherwise; inputs that want no gradient change nothing for the others."""
+    u, v, dy, ws = _weight_call(cuda_device, T, G, d, L)
+    native.set_deterministic(deterministic)
+    try:
+        def run(*wrt):
+            return torch.autograd.grad(eops.prism_gated_refine(u, v, ws, d), wrt, dy, allow_unused=True)
+
+        first = run(*ws)
+        for _ in range(3):
+            assert all(torch.equal(a, b) for a, b in zip(run(*ws), first))
+        ws[0].requires_grad_(False)
+        assert all(torch.equal(a, b) for a, b in zip(run(*ws[1:]), first[1:])) if L > 1 else True
+        ws[0].requires_grad_(True)
+        for w in ws:
+            w.main_grad = torch.full(w.shape, 7.0, device=cuda_device)
+            w._grad_fresh = True
+        assert all(g is None for g in run(*ws))
+        once = [w.main_grad.clone() for w in ws]
+        assert all(torch.equal(a.bfloat16(), b) for a, b in zip(once, first)) and not any(w._grad_fresh for w in ws)
+        run(*ws)
+        assert all(torch.equal(w.main_grad, a + a) for w, a in zip(ws, once))
+        assert native.status() == 0
+    finally:
+        native.set_deterministic(False)
+
+
+def test_one_weight_for_two_iterations(cuda_device):
+    u, v, dy, (w, _) = _weight_call(cuda_device, 50, 2, 32, 2)
+    copy = w.detach().clone().requires_grad_(True)
+    a, b = torch.autograd.grad(eops.prism_gated_refine(u, v, [w, copy], 32), [w, copy], dy)
+    w.main_grad, w._grad_fresh = torch.zeros(w.shape, device=cuda_device), True
+    torch.autograd.grad(eops.prism_gated_refine(u, v, [w, w], 32), [w], dy, allow_unused=True)
+    want = a.float() + b.float()
+    assert (w.main_grad - want).abs().max() <= 2 ** -8 * want.abs().max()            # the two addends are rounded to bf16
