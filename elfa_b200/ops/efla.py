@@ -92,10 +92,17 @@ def efla_scan_chunked_ref(k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, 
 
 
 _EFLA_CHUNK = 32           # tokens of a chunk of the tensor-core kernels
-# Up to this many tokens without a gradient, one token after the other in one launch beats the two launches of the chunked form
-# (B 8, H 16, d 64, per call on the device: T 1 2.8 us against 8.2, T 16 6.1 against 9.1, T 24 7.7 against 9.4, T 32 9.2 against 9.5;
-# the line lies below the crossing because more heads move it down).
-_EFLA_STEP_TOKENS = 16
+
+
+def _efla_step_tokens(states: int) -> int:
+    """Up to this many tokens a call without a gradient goes token by token, in one launch; the chunked form takes two launches and two
+    workspaces. ``states``: state elements of the call, ``B H d^2``. The line lies where whole calls cross, one after the other with the
+    host's part included (microseconds, token form / chunked form):
+    2^18 (1 x 16 heads of 64): T 64 21 / 31, T 112 27 / 31, T 128 31 / 31; 2^19 (8 x 16 of 64): T 112 30 / 31, T 128 33 / 31;
+    2^20 (16 x 16 of 64): T 96 31 / 31, T 112 37 / 31; 2^21 (8 x 16 of 128): T 64 29 / 31, T 80 35 / 31;
+    2^22 (8 x 32 of 128): T 32 29 / 31, T 48 42 / 31; 2^23 (16 x 32 of 128): T 17 31 / 33, T 24 39 / 35.
+    Past 2^19 the device's time counts: the token form's grows with tokens times states."""
+    return 112 if states <= 1 << 19 else max(16, min(96, (1 << 27) // states))
 
 
 def _aligned(t: torch.Tensor) -> torch.Tensor:
@@ -117,7 +124,7 @@ class _EflaScan(torch.autograd.Function):
         s_out = torch.empty((B, H, d, d), dtype=torch.float32, device=k.device)
         bt = beta.detach().float().reshape(1).contiguous()
         st0 = state.float().contiguous() if state is not None else None
-        if T <= _EFLA_STEP_TOKENS and not want_grad:
+        if not want_grad and (T <= 16 or T <= _efla_step_tokens(B * H * d * d)):
             lib.call("elfa_efla_scan_fwd", kc, vc, bt, st0, o, s_out, B, T, H, d, stream_ptr(kc))
             return o, s_out
         nchunks = (T + _EFLA_CHUNK - 1) // _EFLA_CHUNK

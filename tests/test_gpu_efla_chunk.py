@@ -98,9 +98,10 @@ def test_an_infinite_value_gives_an_infinite_output(cuda_device, d):
     of a finite chunk keeps its bits. Token 40 is the last one, or one in the middle of its chunk."""
     for T in (41, 64):
         k, v, beta, s0 = _inputs(cuda_device, 1, T, 2, d, True)
-        o0, f0 = eops.efla_scan(k, v, beta, s0)
+        run = lambda: [x.detach() for x in eops.efla_scan(k.detach().requires_grad_(True), v, beta, s0)]      # a gradient: the chunked form
+        o0, f0 = run()
         v[0, 40, 0, 5] = float("inf")
-        o, s = eops.efla_scan(k, v, beta, s0)
+        o, s = run()
         assert o[0, 40, 0, 5] == float("inf") and o[0, 41:, 0, 5].isnan().all()
         o[0, 40:, 0, 5] = o0[0, 40:, 0, 5]
         assert torch.equal(o, o0)
@@ -143,3 +144,20 @@ def test_backward_keeps_a_bad_token_to_its_side(cuda_device, d, bad):
     keep = [j for j in range(d) if j != 5]
     _close(dv[:, :, 0, keep], dv0[:, :, 0, keep], 2 ** -8)
     _close(ds[:, :, :, keep], ds0[:, :, :, keep], 1e-5)
+
+
+@pytest.mark.parametrize("T", [1, 16, 17, 31, 32, 33, 65, 112, 113])
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+def test_both_forms_at_the_line(cuda_device, monkeypatch, T, d):
+    """Blocks without a gradient go token by token while whole calls are faster that way (few states: up to 112 tokens), with a gradient never."""
+    k, v, beta, s0 = _inputs(cuda_device, 1, T, 2, d, T % 2 == 1, seed=T + d)
+    names, call = [], eops.lib.call
+    monkeypatch.setattr(eops.lib, "call", lambda name, *a: names.append(name) or call(name, *a))
+    o, s = eops.efla_scan(k, v, beta, s0)
+    o2, s2 = (x.detach() for x in eops.efla_scan(k.detach().requires_grad_(True), v, beta, s0))
+    assert names == ["elfa_efla_scan_fwd" if T <= 112 else "elfa_efla_chunk_fwd", "elfa_efla_chunk_fwd"]
+    o_ref, s_ref = eops.efla_scan_ref(k, v, beta, s0)
+    for a, b in ((o, s), (o2, s2)):
+        _close(a, o_ref, 2 ** -8)
+        _close(b, s_ref, 1e-5)
+    assert [eops._efla_step_tokens(1 << n) for n in range(12, 27, 2)] == [112, 112, 112, 112, 96, 32, 16, 16]
