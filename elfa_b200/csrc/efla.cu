@@ -18,8 +18,8 @@ namespace elfa {
 namespace {
 
 __device__ __forceinline__ float efla_coeff(float beta, float lam) {
-  if (lam < 1e-6f) return beta - 0.5f * beta * beta * lam + beta * beta * beta * lam * lam / 6.f;
-  return (1.f - __expf(-beta * lam)) / lam;
+  // expm1f: 1 - exp would cancel for short keys (at beta lam = 1e-6 one step of fp32 is 6 %, and the chunked form has c in fp64)
+  return lam < 1e-30f ? beta : -expm1f(-beta * lam) / lam;
 }
 
 // Token by token, for a few tokens without a gradient (generation): one launch, nothing else to prepare.

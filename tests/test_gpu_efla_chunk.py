@@ -161,3 +161,22 @@ def test_both_forms_at_the_line(cuda_device, monkeypatch, T, d):
         _close(a, o_ref, 2 ** -8)
         _close(b, s_ref, 1e-5)
     assert [eops._efla_step_tokens(1 << n) for n in range(12, 27, 2)] == [112, 112, 112, 112, 96, 32, 16, 16]
+
+
+@pytest.mark.parametrize("T", [8, 17, 113])
+@pytest.mark.parametrize("std", [0.0, 1e-5, 2e-4, 3e-3, 0.05])
+def test_short_keys_have_the_same_coefficient_in_both_forms(cuda_device, T, std):
+    """c = (1 - exp(-beta lam)) / lam cancels for short keys. 64-bit loop; the state is a sum of T terms that fp32 rounds a handful of times each."""
+    g = torch.Generator(device=cuda_device).manual_seed(T)
+    k = (torch.randn(1, T, 2, 64, generator=g, device=cuda_device) * std).bfloat16()
+    v = torch.randn(1, T, 2, 64, generator=g, device=cuda_device).bfloat16()
+    S = torch.zeros(1, 2, 64, 64, dtype=torch.float64, device=cuda_device)
+    for t in range(T):
+        kt, vt = k[:, t].double(), v[:, t].double()
+        lam = (kt * kt).sum(-1)
+        c = torch.where(lam == 0, torch.full_like(lam, 0.3), -torch.expm1(-0.3 * lam) / lam.clamp_min(1e-300))
+        S = S + c[..., None, None] * kt[..., :, None] * (vt - torch.einsum("bhi,bhij->bhj", kt, S))[..., None, :]
+    beta = torch.tensor([0.3], device=cuda_device)
+    for want in (False, True):
+        s = eops.efla_scan(k.detach().requires_grad_(want), v, beta)[1].detach()
+        assert (s.double() - S).abs().max() <= 2e-6 * S.abs().max()
