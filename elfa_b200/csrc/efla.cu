@@ -11,6 +11,8 @@
 // ShortConv: y[b,t,c] = bias[c] + sum_w x[b,t-w,c] weight[c,w] (reference:
 // kernels/cuda/convolution.cu:4-57,126-189; src/model/prism.zig:948-973). The weight gradient is one
 // pass over the rows per (32 channels, 4 taps) without atomics.
+#include <type_traits>
+
 #include "common.cuh"
 #include "elfa_native.h"
 
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(32 * EFLA_W) efla_scan_fwd_kernel(const __nv_b
 // shortconv_apply_kernel / shortconv_bwd_dw_kernel below.
 // Backward is one walk from late to early: with dy[t .. t + W - 1] as the window, dx[t] = sum_j w[j] dy[t + j] and
 // dw[j] += x[t] dy[t + j]; every warp writes its dw / db sums as one slice of part [slices][W + 1][C], added up in order afterwards.
-// B 8, T 2048, C 1024, W 16: 27 us forward (67 MB; bound by the packed multiply-adds and the latency of 192- and 124-register warps), 55 + 6 us
+// B 8, T 2048, C 1024, W 16: 27 us forward (67 MB; bound by the packed multiply-adds and the latency of 202- and 126-register warps), 45 + 6 us
 // backward; the layer that contains them went from 789 to 454 us when they replaced the general kernels below.
 // A lane's weights are 4 W consecutive bytes; one at a time they would cost 2 W loads that touch 32 lines each, more than the
 // inputs (31.5 against 26.5 us forward).
@@ -169,6 +171,42 @@ __device__ __forceinline__ uint32_t ld_pair(const __nv_bfloat16* base, long long
 }
 __device__ __forceinline__ uint64_t pair_f32x2(uint32_t v) { return pack_f32x2(bf16_lo(v), bf16_hi(v)); }
 
+// The ring stands in zeros for what lies outside the sequence, and 0 x infinity is NaN. Forward leaves those products out of a sequence's first
+// W outputs. Backward looks, where its walk reaches past the end, for values that are not finite (weights; the sums of tap 0 and of the
+// bias, which see every input and output gradient of the walk) and then forms the same sums again, in the same order, without them.
+__device__ __forceinline__ bool not_finite_f32x2(uint64_t v) {
+  float lo, hi;
+  unpack_f32x2(v, lo, hi);
+  return fmaf(lo, 0.f, hi * 0.f) != 0.f;
+}
+template <int W>
+__device__ __forceinline__ bool shortconv_weights_bad(const uint64_t (&wf)[W]) {
+  uint64_t z = 0ull;
+#pragma unroll
+  for (int j = 0; j < W; ++j) z = fma_f32x2(wf[j], 0ull, z);
+  return not_finite_f32x2(z);
+}
+template <int W>
+__device__ __noinline__ void shortconv_bwd_again(const __nv_bfloat16* xb, const __nv_bfloat16* wc, const __nv_bfloat16* gb,
+                                                 __nv_bfloat16* ob, float* pb, int t0, int t1, int T, int C) {
+  for (int ch = 0; ch < 2; ++ch) {
+    float acc[W + 1];
+    for (int j = 0; j <= W; ++j) acc[j] = 0.f;
+    for (int t = t1 - 1; t >= t0; --t) {
+      const float xv = __bfloat162float(xb[(long long)t * C + ch]);
+      float s[2] = {0.f, 0.f};
+      for (int j = 0; j < W && t + j < T; ++j) {
+        const float g = __bfloat162float(gb[(long long)(t + j) * C + ch]);
+        s[j & 1] = fmaf(g, __bfloat162float(wc[ch * W + j]), s[j & 1]);
+        acc[j] = fmaf(xv, g, acc[j]);
+        if (j == 0) acc[W] += g;
+      }
+      ob[(long long)t * C + ch] = __float2bfloat16(s[0] + s[1]);
+    }
+    for (int j = 0; j <= W; ++j) pb[(long long)j * C + ch] = acc[j];
+  }
+}
+
 // grid (ceil(B * spans / 4), ceil(C / 64)), block (32, 4)
 template <int W>
 __global__ void __launch_bounds__(128) shortconv_ring_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
@@ -189,7 +227,7 @@ __global__ void __launch_bounds__(128) shortconv_ring_fwd_kernel(const __nv_bflo
   uint32_t nx[W];
 #pragma unroll
   for (int r = 0; r < W; ++r) nx[r] = ld_pair(xb, t0 + r, C, t0 + r < t1);
-  for (int t = t0; t < t1; t += W) {
+  auto block = [&](auto edge, int t) {
     uint32_t cur[W];
 #pragma unroll
     for (int r = 0; r < W; ++r) {
@@ -202,14 +240,20 @@ __global__ void __launch_bounds__(128) shortconv_ring_fwd_kernel(const __nv_bflo
       uint64_t s0 = b2, s1 = 0ull;
 #pragma unroll
       for (int j = 0; j < W; j += 2) {
-        s0 = fma_f32x2(win[(r - j + W) % W], wf[j], s0);
-        s1 = fma_f32x2(win[(r - j - 1 + W) % W], wf[j + 1], s1);
+        if (!edge.value || j <= r) s0 = fma_f32x2(win[(r - j + W) % W], wf[j], s0);
+        if (!edge.value || j + 1 <= r) s1 = fma_f32x2(win[(r - j - 1 + W) % W], wf[j + 1], s1);
       }
       float lo, hi;
       unpack_f32x2(add_f32x2(s0, s1), lo, hi);
       if (t + r < t1) *reinterpret_cast<uint32_t*>(yb + (long long)(t + r) * C) = pack_bf16(lo, hi);
     }
+  };
+  int t = t0;
+  if (t == 0) {
+    block(std::true_type{}, 0);
+    t = W;
   }
+  for (; t < t1; t += W) block(std::false_type{}, t);
 }
 
 template <int W>
@@ -272,6 +316,8 @@ __global__ void __launch_bounds__(128) shortconv_ring_bwd_kernel(const __nv_bflo
     unpack_f32x2(j < W ? acc[j < W ? j : 0] : accb, lo, hi);
     *reinterpret_cast<float2*>(pb + (long long)j * C) = make_float2(lo, hi);
   }
+  if (t1 + W - 1 > T && (not_finite_f32x2(acc[0]) || not_finite_f32x2(accb) || shortconv_weights_bad<W>(wf)))
+    shortconv_bwd_again<W>(xb, w + (long long)c * W, gb, ob, pb, t0, t1, T, C);
 }
 
 // dw[c, j] = sum over the slices of part[slice][j][c], db[c] from row `taps`. grid (ceil(C / 32), taps + 1), block (32, 16)

@@ -29,3 +29,39 @@ def test_shortconv_edges(cuda_device, B, T, C, W, bias):
     assert native.status() == 0
     for a, r in zip([y, *got], [yr, *ref]):
         assert (a.float() - r).abs().max() <= 2 ** -8 * r.abs().max()
+
+
+@pytest.mark.parametrize("W", [4, 5, 8, 16])
+@pytest.mark.parametrize("T", [1, 3, 16, 17, 40, 65, 130])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nothing_beyond_the_sequence_is_multiplied(cuda_device, T, W, bad):
+    """Terms that reach outside the sequence do not exist; formed with zeros they would make NaN of a value that is not finite."""
+    torch.manual_seed(T + W)
+    C, c = 66, 9
+    other = [i for i in range(C) if i != c]
+    x0, dy0 = (torch.randn(2, T, C, device=cuda_device).bfloat16() for _ in range(2))
+    w0 = torch.randn(C, W, device=cuda_device).bfloat16()
+
+    def run(x, w, dy):
+        ins = [t.clone().requires_grad_(True) for t in (x, w)]
+        y = eops.shortconv(*ins)
+        return [y.detach(), *torch.autograd.grad(y, ins, dy)]
+
+    clean = run(x0, w0, dy0)
+    taps, times = torch.arange(W, device=cuda_device), torch.arange(T, device=cuda_device)
+    for what in range(3):
+        x, w, dy = x0.clone(), w0.clone(), dy0.clone()
+        if what == 0:
+            x[0, T - 1, c] = bad             # the last input meets the last output gradient through tap 0 only
+        elif what == 1:
+            dy[0, 0, c] = bad                # the first output gradient meets the first input through tap 0 only
+        else:
+            w[c, W - 1] = bad                # the last tap: outputs from W - 1 on, input gradients up to T - W
+        y, dx, dw = run(x, w, dy)
+        ok_y = (times < T - 1 if what == 0 else torch.full_like(times, what == 1) > 0) if what < 2 else times < W - 1
+        ok_dx = (torch.full_like(times, 1) > 0 if what == 0 else times > 0) if what < 2 else times > T - W
+        assert torch.equal(y[0, :, c].isfinite(), ok_y) and torch.equal(dx[0, :, c].isfinite(), ok_dx)
+        assert torch.equal(dw[c].isfinite(), taps > 0 if what < 2 else taps >= 0)
+        for got, ref in zip((y, dx), clean):
+            assert torch.equal(got[:, :, other], ref[:, :, other])
+        assert torch.equal(dw[other], clean[2][other])
