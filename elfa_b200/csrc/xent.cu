@@ -241,16 +241,20 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
   float M2 = sm[0][0], S = sm[1][0], SX = sm[2][0];
 #pragma unroll
   for (int i = 1; i < XENT_THREADS / 32; ++i) { online_combine2(M2, S, sm[0][i], sm[1][i]); SX += sm[2][i]; }
-  const float lse2 = M2 + log2f(S), lse = lse2 * 0.6931471805599453f;
+  const float ls = log2f(S), lse2 = M2 + ls;
   const bool valid = t >= 0 && t < V;
   if (threadIdx.x == 0 && !valid && t != -100) atomicOr(status, (unsigned)ELFA_ST_BAD_TARGET);
   if (fabsf(M2) == INFINITY) {             // (a thread whose own maximum overflows downwards rightly adds nothing to a larger one)
     xent_row_huge(x, xrow, nvec, V, valid, tl, valid ? (int)(t >> 3) : -1, (int)(t & 7), smoothing, grad_scale, loss_out + row, sm);
     return;
   }
-  if (threadIdx.x == 0) {
-    float loss = (1.f - smoothing) * (tl - lse);
-    if (smoothing != 0.f) loss += (smoothing / (float)V) * (SX - (float)V * lse);
+  if (threadIdx.x == XENT_THREADS - 1) {     // the thread with the fewest vectors
+    // the loss in natural units, from the maximum as it is: M2 carries the rounding of M log2(e), and a result in base 2 would be rounded at
+    // 1.44 times its size (up to 1.5 times the error against 64 bits). M is a bf16 number, so M2 ln(2) rounds to it.
+    constexpr float LN2 = 0.6931471805599453f;
+    const float M = __bfloat162float(__float2bfloat16(M2 * LN2)), l = (ls - fmaf(M, L2E, -M2)) * LN2;
+    float loss = (1.f - smoothing) * ((tl - M) - l);
+    if (smoothing != 0.f) loss += (smoothing / (float)V) * (SX - (float)V * (M + l));
     loss_out[row] = valid ? -loss : 0.f;
   }
   const float gs = valid ? grad_scale : 0.f, off = -gs * (smoothing / (float)V), tg = gs * (1.f - smoothing);

@@ -62,3 +62,20 @@ def test_logits_near_the_largest_float(cuda_device, V, smoothing):
         assert native.status() == 0
         assert abs(loss.item() - ref.item()) <= 1e-5 * max(1.0, abs(ref.item())), r
         assert (g.double() - gr).abs().max() <= 2 ** -8 * gr.abs().max() + 1e-7, r
+
+
+@pytest.mark.parametrize("V,scale", [(4096, 1.0), (8000, 3.0), (32000, 1.0), (32000, 3.0), (32000, 10.0), (32000, 40.0)])
+def test_loss_is_as_close_to_64_bits_as_in_two_kernels(cuda_device, V, scale):
+    rows = 2048
+    torch.manual_seed(V)
+    x = (torch.randn(rows, V, device=cuda_device) * scale).bfloat16()
+    t = torch.randint(0, V, (rows,), device=cuda_device)
+    st = native.stream_ptr(x)
+    one, two, stats = (torch.empty(rows, *s, device=cuda_device) for s in ((), (), (4,)))
+    a, b = x.clone(), x.clone()
+    native.lib.call("elfa_xent_row", a, V, t, one, rows, V, 0.0, 1.0, st)
+    native.lib.call("elfa_xent_stats", b, V, t, stats, rows, V, 0, V, st)
+    native.lib.call("elfa_xent_grad", b, V, b, V, t, stats, 1, two, rows, V, 0, V, 0.0, None, 1.0, st)
+    ref = torch.cat([torch.nn.functional.cross_entropy(x[i:i + 256].double(), t[i:i + 256], reduction="none") for i in range(0, rows, 256)])
+    err = [(e.double() - ref).norm().item() for e in (one, two)]
+    assert err[0] <= 1.02 * err[1]                     # the same roundings in another order: 2 % for the sample
