@@ -91,3 +91,18 @@ def test_one_weight_for_two_iterations(cuda_device):
     torch.autograd.grad(eops.prism_gated_refine(u, v, [w, w], 32), [w], dy, allow_unused=True)
     want = a.float() + b.float()
     assert (w.main_grad - want).abs().max() <= 2 ** -8 * want.abs().max()            # the two addends are rounded to bf16
+
+
+@pytest.mark.parametrize("M,N,K,pieces", [(8, 8, 1, 1), (128, 64, 512, 1), (136, 24, 700, 1), (1024, 128, 8200, 9), (640, 1024, 1500, 3), (4736, 1024, 256, 1)])
+def test_split_product_adds_up(cuda_device, M, N, K, pieces):
+    """Every tile width of the split product (64, 128, 256 columns), ragged rows, columns and contraction: the pieces add up to the product. fp32
+    sums of exact bf16 products: 2^-20 of the largest for 8200 terms in blocks of 16 and a few pieces."""
+    torch.manual_seed(M)
+    a, b = torch.randn(K, M, device=cuda_device).bfloat16(), torch.randn(K, N, device=cuda_device).bfloat16()
+    n = native.lib.raw("elfa_gemm_bf16_parts_count")(M, N, K)
+    assert n == pieces                               # on 148 SMs
+    parts = torch.full((n, (M + 127) // 128 * 128, N), float("nan"), device=cuda_device)
+    native.lib.call("elfa_gemm_bf16_parts", a, b, parts, M, N, K, M, N, native.stream_ptr(a))
+    want = a.double().t() @ b.double()
+    assert native.status() == 0
+    assert (parts.double().sum(0)[:M] - want).abs().max() <= 2 ** -20 * want.abs().max() * max(1, K / 256) ** 0.5
