@@ -50,11 +50,11 @@ class EflaConfig:
     enabled: bool = True
     num_heads: int = 128
     state_dim: int = 128
-    chunk_size: int = 4096
+    chunk_size: int = 4096          # read, without effect: the kernels take 32 tokens per chunk, results never depended on it
     learned_beta: bool = True
     initial_beta: float = 1.0
     beta_schedule: str = field(default="constant", metadata=_enum(BETA_SCHEDULES))
-    use_chunked_scan: bool = True
+    use_chunked_scan: bool = True   # read, without effect (the form is chosen by length and gradient)
 
 
 @dataclass

@@ -1,4 +1,4 @@
-// EFLA recurrence token by token (a few tokens without a gradient; longer blocks and backward: efla_chunk.cu) and the causal depthwise
+// EFLA recurrence token by token (blocks of up to about a hundred tokens without a gradient; the others and backward: efla_chunk.cu) and the causal depthwise
 // ShortConv (forward and backward).
 //
 // EFLA, per (batch, head), state S [d, d] fp32 (row = key index i, column = value index j):
@@ -24,7 +24,7 @@ __device__ __forceinline__ float efla_coeff(float beta, float lam) {
   return lam < 1e-30f ? beta : -expm1f(-beta * lam) / lam;
 }
 
-// Token by token, for a few tokens without a gradient (generation): one launch, nothing else to prepare.
+// Token by token, for short blocks without a gradient (generation; the line is in ops/efla.py): one launch, nothing else to prepare.
 // k, v, o: [B, T, H, D] bf16. state0 / state_out: [B, H, D, D] fp32.
 // The columns of S evolve independently (column j needs k_t, c_t and v_t[j] only), so a CTA owns 32 value columns:
 // grid (B*H, D/32). Its four warps split the D key rows: warp w keeps rows [w D/4, (w+1) D/4) of the 32 columns in

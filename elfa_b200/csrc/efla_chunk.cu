@@ -461,7 +461,7 @@ __device__ __forceinline__ long long efla_state_slot(long long chunk_id, int vbl
 
 // Grid (B * H, d / columns of a CTA). k, v, o: [B, T, H, d] bf16. state0 / state_out: [B, H, d, d] fp32 or null. ckpt (or null):
 // the state at the start of every chunk.
-// Bound by the dependent chain of a chunk (132 mma.sync and about 900 instructions of one warp per scheduler), not by memory. With the
+// Bound by the dependent chain of a chunk (132 mma.sync and about 880 instructions of one warp per scheduler), not by memory. With the
 // preparation, B 1, T 8192, 16 heads of 64, no gradient: 354 us, token by token (with its checkpoints) 2364 us; in the training step of
 // B 8, T 2048 the forward went from about 750 to 94 us and 28 us for the preparation.
 template <int D, bool CHECKED>
@@ -623,7 +623,7 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
 //   dlam_t = c_t sum_j (dO E)_tj + dc_t dc/dlam,   dbeta = sum_t dc_t ex_t
 // Only dS is sequential: efla_chunk_bwd_state_kernel walks the chunks backwards with dS in registers and writes the dS1 of every chunk;
 // efla_chunk_bwd_kernel then handles all chunks in parallel from the two chunk-boundary states.
-// B 8, T 2048, 16 heads of 64: 94 us and 259 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
+// B 8, T 2048, 16 heads of 64: 92 us and 253 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
 // finish). The parallel kernel issues about 400 mma.sync per warp and chunk (94 us of tensor time at 8.3 cycles each) and reads 370 MB
 // (55 us); a third CTA per SM, at 168 registers, did not make it faster.
 template <int D, bool CHECKED>

@@ -98,7 +98,8 @@ int prism_grid(long long n) {
 // The layer's own form: p_l = sigmoid(z_l) with the bf16 logits z_l [tokens, d] at z + l d (row pitch ldz), formed in fp32 inside the
 // kernel; backward returns the gradient of the logits (bf16). A thread owns VEC channels of a token (16- or 8-byte accesses) and
 // walks over the groups with UG groups' loads in flight. gelu(x) = x sigmoid(2 u) with u the argument of the tanh form: one
-// exponential and one reciprocal at fp32 accuracy (tanh.approx has 2^-11), and the derivative reuses the sigmoid. Bound by the special
+// exponential and one reciprocal (tanh.approx has 2^-11), and the derivative reuses the sigmoid. They are __expf and __fdividef; results, gradients
+// and the carried fp32 state are as far from 64 bits as with PyTorch's functions (state: 5.5e-8 to 8.2e-7 relative against 6.0e-8 to 8.2e-7). Bound by the special
 // functions (two per element and iteration) and memory about equally: 16384 tokens x 1024 channels, two iterations: 40 us forward (100 MB),
 // 47 us backward (168 MB). With fp32 gates the layer ran PyTorch's elementwise kernels before: 2.85 ms forward and backward, 0.79 with these.
 __device__ __forceinline__ float prism_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }

@@ -65,7 +65,7 @@ class EflaLayer(nn.Module):
             self.w_k.tp_shard = self.w_v.tp_shard = ("col", tp)
             self.w_o.tp_shard = ("row", tp)
             self.beta_param.tp_replicated = True
-        self.chunk = max(1, min(m.efla.chunk_size, 16)) if m.efla.use_chunked_scan else 16
+        self.chunk = max(1, min(m.efla.chunk_size, 16)) if m.efla.use_chunked_scan else 16       # no effect on results or memory
 
     def forward(self, x, state=None, sp_group=None):
         B, T, D = x.shape

@@ -155,8 +155,9 @@ class _EflaScan(torch.autograd.Function):
 def efla_scan(k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, state: Optional[torch.Tensor] = None, chunk: int = 16
               ) -> Tuple[torch.Tensor, torch.Tensor]:
     """EFLA recurrence. CPU tensors use the differentiable reference loop; CUDA bf16 tensors use the
-    native kernels when the head dimension is supported (multiple of 32, at most 128). ``chunk`` (a positive number) is a hint on
-    how often a state is kept for backward and never changes the result; the native kernels keep one every 32 tokens."""
+    native kernels when the head dimension is supported (multiple of 32, at most 128). ``chunk`` (a positive number) was the
+    distance of the states kept for backward and has no effect any more: with a gradient wanted the kernels keep ``T / 32`` states (and about
+    6.5 KB per 32 tokens and head), and backward as many again while it runs. A caller that passed more than 64 to save memory holds more."""
     d = k.shape[-1]
     if k.is_cuda and k.dtype == torch.bfloat16 and d % 32 == 0 and d <= 128:
         if chunk <= 0:

@@ -1,4 +1,4 @@
-"""Chunked EFLA kernels at the edges of a chunk (32 tokens) and of the one-launch form (16 tokens), against the fp32 token loop.
+"""Chunked EFLA kernels at the edges of a chunk (32 tokens) and of the one-launch form (112 tokens of few states), against the fp32 token loop.
 
 Bounds: outputs and k / v gradients are rounded to bf16 once (2^-9 of the value; 2^-8 of the largest allows for the fp32 noise of both
 sides), states and their gradients stay in fp32 on both sides, where each of the T updates rounds at 2^-24: 1e-5 of the largest covers
