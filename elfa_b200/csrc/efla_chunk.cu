@@ -1036,7 +1036,7 @@ __device__ __forceinline__ bool efla_bwd_chunk(
 #pragma unroll
         for (int w = 0; w < L::W; ++w) da += sym[(w * EC + t) * L::GLD + lane];
         part += da * sG[t * L::GLD + lane];
-        sym[t * L::GLD + lane] = da * c_s;
+        sym[t * L::GLD + lane] = CHECKED && c_s == 0.f ? 0.f : da * c_s;     // c = 0: a key whose square overflows changes nothing
       }
     }
     sdc[warp * EC + lane] = part;

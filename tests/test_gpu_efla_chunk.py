@@ -180,3 +180,28 @@ def test_short_keys_have_the_same_coefficient_in_both_forms(cuda_device, T, std)
     for want in (False, True):
         s = eops.efla_scan(k.detach().requires_grad_(want), v, beta)[1].detach()
         assert (s.double() - S).abs().max() <= 2e-6 * S.abs().max()
+
+
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+def test_a_key_whose_square_overflows_changes_nothing(cuda_device, d):
+    """|k|^2 past the largest float makes c zero: the state passes by, and later tokens are those of a call in which that key is zero. (5e37: the
+    products of that key with the state stay finite, their sums over the value columns do not.)"""
+    T = 130
+    for seed in range(6):
+        k, v, beta, s0 = _inputs(cuda_device, 1, T, 2, d, True, seed=seed)
+        torch.manual_seed(seed)
+        go, gs = 50 * torch.randn_like(v), 0.1 * torch.randn(1, 2, d, d, device=cuda_device)
+        got = []
+        for low in (True, False):
+            kk = k.clone()
+            kk[0, 41, 0] = 0.0
+            if low:
+                kk[0, 41, 0, 3] = -5e37
+            ins = [t.detach().requires_grad_(True) for t in (kk, v)]
+            o, s = eops.efla_scan(*ins, beta, s0)
+            got.append([o.detach(), s.detach(), *torch.autograd.grad([o, s], ins, [go, gs])])
+        (o, s, dk, dv), (o0, s0_, dk0, dv0) = got
+        _close(o[:, 42:], o0[:, 42:], 2 ** -8)
+        _close(s, s0_, 1e-5)
+        _close(dk[:, 42:], dk0[:, 42:], 2 ** -8)
+        _close(dv[:, 42:], dv0[:, 42:], 2 ** -8)
