@@ -1164,7 +1164,7 @@ using namespace elfa;
 
 // k, v, o: [B, T, H, d] bf16, 16-byte aligned; beta: 1 float; state0 (optional) / state_out: [B, H, d, d] fp32; ckpt: null or
 // B * H * ceil(T / 32) * d * d floats (chunk-start states in the kernels' own order, needed by backward). nmat: [B * H * ceil(T / 32), 3, 32, 32] bf16 and
-// coef: [B * H * ceil(T / 32), 4, 32] fp32, 16-byte aligned, are written here.
+// coef: [B * H * ceil(T / 32), 4, 32] fp32, 16-byte aligned, are written here. No output may share memory with an input (a call may run twice).
 ELFA_API int elfa_efla_chunk_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
                                  float* ckpt, void* nmat, float* coef, int B, int T, int H, int d, void* stream) {
   ELFA_REQUIRE(k && v && beta && o && nmat && coef && B > 0 && T > 0 && H > 0, "efla_chunk_fwd: bad arguments");
