@@ -32,16 +32,22 @@ int make_qkv_tmap(CUtensorMap* tm, const void* qkv, int S, int B, int H, int hd,
 
 namespace {
 
-constexpr int ATTB_THREADS = 320;
 constexpr int SUBB = 128 * 128;
+constexpr int ATTB_CW = 32;                           // columns of a compute warp
+constexpr int ATTB_SPLIT = 128 / ATTB_CW;             // compute warps per tensor-memory lane quarter
+constexpr int ATTB_COMPUTE = 4 * ATTB_SPLIT;          // compute warps
+constexpr int ATTB_THREADS = 32 * (3 + ATTB_COMPUTE);
 
-// Grouped-query attention (Hkv < H): the key-tile pass runs one CTA per key / value head and walks the query tiles of every
-// query head of its group one after the other, so dK / dV are summed in a fixed order; the query-tile pass reads the group's
-// key head. Packed sequences (doc_start, see the forward kernel): masked like the causal diagonal, block pairs without a
-// visible (query, key) pair are skipped.
+// Grouped-query attention (Hkv < H): the key-tile pass runs `nsplit` CTAs (a cluster) per key / value head, each walking the query
+// tiles of its share of the group's query heads one head after the other; the shares are added up in rank order, so dK / dV are summed in a
+// fixed order. The query-tile pass reads the group's key head. Packed sequences (doc_start, see the forward kernel): masked like the causal
+// diagonal, block pairs without a visible (query, key) pair are skipped.
 struct AttnBwdParams {
   int S, B, H, hd;
   int Hkv;
+  int nsplit;             // key-tile pass: CTAs (of one cluster) that share the query heads of a key head
+  const __nv_bfloat16 *qkv, *dout;
+  long long q_stride_s, q_stride_b, o_stride_s, o_stride_b;
   const int* doc_start;   // [B, S] or null
   const float* lse;    // [B, H, S] natural log
   const float* delta;  // [B, H, S]
@@ -53,57 +59,99 @@ struct AttnBwdParams {
   unsigned int* status;
 };
 
-enum { BB_RES = 0, BB_INFULL0, BB_INFULL1, BB_INFREE0, BB_INFREE1, BB_S, BB_DP, BB_P, BB_DS, BB_ACC, BB_COUNT };
+// P and dS are handed over in two halves (the first and second 16 columns of every compute warp): BB_P, BB_DS and the one behind each
+enum { BB_RES0 = 0, BB_RES1, BB_QF0, BB_QE0 = BB_QF0 + 4, BB_OF0 = BB_QE0 + 4, BB_OE0 = BB_OF0 + 3, BB_VF0 = BB_OE0 + 3, BB_S = BB_VF0 + 2,
+       BB_DP, BB_P, BB_DS = BB_P + 2, BB_ACC = BB_DS + 2, BB_COUNT };
 
-template <int HDP>
+template <int HDP, bool DKV>
 struct BwdSmem {
+  // The resident pair is the A operand of S and dP. Where tensor memory has room for it (all but the key-tile pass of 128-wide heads) it is
+  // read from there: from shared memory a 128 x 128 x 16 product reads A and B in exactly the 64 cycles it takes, and the tiles that arrive
+  // and the other products come on top.
+  static constexpr bool RES_TM = !DKV || HDP == 64;
   static constexpr int NSUB = HDP / 64;
+  static constexpr int TILE = NSUB * SUBB;
+  // rings of the inner tiles: one slot more for the operand that two products far apart read (Q, or K in the query-tile pass)
+  static constexpr int NQ = RES_TM ? 4 : 3, NO = NQ - 1;
   static constexpr int RES0 = 0;
-  static constexpr int RES1 = RES0 + NSUB * SUBB;
-  static constexpr int IN0 = RES1 + NSUB * SUBB;           // [2 slots][NSUB]
-  static constexpr int IN1 = IN0 + 2 * NSUB * SUBB;        // [2 slots][NSUB]
-  static constexpr int VEC_OFF = IN1 + 2 * NSUB * SUBB;    // lse2 / delta / document start of the inner query tile: [2 slots][3][128] words
-  static constexpr int BAR_OFF = VEC_OFF + 2 * 3 * 128 * 4;
+  static constexpr int RES1 = RES0 + (RES_TM ? 0 : TILE);
+  static constexpr int INQ = RES1 + (RES_TM ? 0 : TILE);
+  static constexpr int INO = INQ + NQ * TILE;
+  static constexpr int VEC = 2 * 128 * 4 + 128;            // -lse2, -delta * scale (fp32), document start relative to the key tile (bytes)
+  static constexpr int VEC_OFF = INO + NO * TILE;          // [2 slots]
+  static constexpr int BAR_OFF = VEC_OFF + 2 * VEC;
   static constexpr int TOTAL = BAR_OFF + BB_COUNT * 8 + 16;
-  static constexpr int DYN = TOTAL + 1024;
+  static constexpr int RED_LD = 2 * HDP + 4;               // fp32 pitch of the accumulators handed to the cluster, over the rings
+  static_assert(!DKV || 128 * RED_LD * 4 <= (NQ + NO) * TILE, "accumulators fit the rings");
+  static_assert(TOTAL <= 232448, "shared memory of a CTA");
 };
 
-// delta[b,h,s] = sum_d dO[s,b,h,d] * O[s,b,h,d]; one warp per (s,b,h).
+// delta[b,h,s] = sum_d dO[s,b,h,d] * O[s,b,h,d]; LPR lanes per (s, b, h), 16 bytes each, so that every lane has work at hd = 8 LPR, and two rows in
+// flight per lane. Bound by memory: 65536 rows x 2 of 128: see the launch.
+template <int LPR>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                                          long long o_stride_s, long long o_stride_b, float* __restrict__ delta, int S,
                                                          int B, int H, int hd) {
-  const long long gw = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+  constexpr int ROWS = 256 / LPR;            // rows of a block per round
+  const int l = threadIdx.x & (LPR - 1);
   const long long total = (long long)S * B * H;
-  if (gw >= total) return;
-  const int h = (int)(gw % H);
-  const int b = (int)((gw / H) % B);
-  const int s = (int)(gw / ((long long)H * B));
-  const long long off = (long long)s * o_stride_s + (long long)b * o_stride_b + (long long)h * hd;
-  float acc = 0.f;
-  for (int v = lane; v < hd / 8; v += 32) {
-    const uint4 a = *reinterpret_cast<const uint4*>(o + off + v * 8);
-    const uint4 d = *reinterpret_cast<const uint4*>(dout + off + v * 8);
-    const uint32_t* pa = reinterpret_cast<const uint32_t*>(&a);
-    const uint32_t* pd = reinterpret_cast<const uint32_t*>(&d);
+  const long long row0 = (long long)blockIdx.x * (2 * ROWS) + threadIdx.x / LPR;
+  float acc[2] = {0.f, 0.f};
+  long long at[2];
+  uint4 a[2], d[2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc += bf16_lo(pa[j]) * bf16_lo(pd[j]) + bf16_hi(pa[j]) * bf16_hi(pd[j]);
+  for (int u = 0; u < 2; ++u) {
+    const long long row = row0 + u * ROWS;
+    a[u] = d[u] = make_uint4(0, 0, 0, 0);
+    at[u] = -1;
+    if (row < total) {
+      const int h = (int)(row % H);
+      const long long sb = row / H;
+      const int b = (int)(sb % B), s = (int)(sb / B);
+      at[u] = ((long long)b * H + h) * S + s;
+      if (l * 8 < hd) {
+        const long long off = (long long)s * o_stride_s + (long long)b * o_stride_b + (long long)h * hd + l * 8;
+        a[u] = *reinterpret_cast<const uint4*>(o + off);
+        d[u] = *reinterpret_cast<const uint4*>(dout + off);
+      }
+    }
   }
-  acc = warp_sum(acc);
-  if (lane == 0) delta[((long long)b * H + h) * S + s] = acc;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const uint32_t* pa = reinterpret_cast<const uint32_t*>(&a[u]);
+    const uint32_t* pd = reinterpret_cast<const uint32_t*>(&d[u]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[u] += bf16_lo(pa[j]) * bf16_lo(pd[j]) + bf16_hi(pa[j]) * bf16_hi(pd[j]);
+#pragma unroll
+    for (int m = LPR / 2; m > 0; m >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], m);
+    if (l == 0 && at[u] >= 0) delta[at[u]] = acc[u];
+  }
+}
+
+// tcgen05.wait::ld that the 32 loaded registers pass through, so that no use of them can be scheduled ahead of it
+__device__ __forceinline__ void tmem_ld_wait32(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]),
+                 "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]),
+                 "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])::"memory");
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
 template <int HDP, bool DKV>
 __global__ void __launch_bounds__(ATTB_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO, const AttnBwdParams p) {
-  using L = BwdSmem<HDP>;
-  constexpr int NSUB = L::NSUB;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  using L = BwdSmem<HDP, DKV>;
+  constexpr int NSUB = L::NSUB, NQ = L::NQ, NO = L::NO, CW = ATTB_CW;
+  constexpr bool RES_TM = L::RES_TM;
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + BB_COUNT);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
-  float* svec = reinterpret_cast<float*>(smem + L::VEC_OFF);
   const uint32_t sbase = smem_u32(smem);
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) { return bar0 + 8u * i; };
@@ -112,8 +160,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   // one-dimensional grid, heaviest outer tile first over the whole grid: every (batch, head) runs its longest tile before any
   // runs its second longest, so the short CTAs fill the tail of the launch
   const int n_heads = DKV ? p.Hkv : p.H;
-  const int hb = (int)(blockIdx.x % (unsigned)(n_heads * p.B));
-  const int rank = (int)(blockIdx.x / (unsigned)(n_heads * p.B));
+  const int nsplit = DKV ? p.nsplit : 1;
+  const int bid = (int)blockIdx.x / nsplit, share = (int)blockIdx.x % nsplit;
+  const int hb = bid % (n_heads * p.B);
+  const int rank = bid / (n_heads * p.B);
   const int h = hb % n_heads, b = hb / n_heads;     // DKV: key / value head; DQ: query head
   const int group = p.H / p.Hkv;
   const int kvh = DKV ? h : h / group;
@@ -123,21 +173,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   int in_end = DKV ? p.n_tiles : (p.causal ? outer + 1 : p.n_tiles);
   const int* dstart = p.doc_start ? p.doc_start + (long long)b * p.S : nullptr;
   if (dstart) {
-    if (DKV) {      // query tiles whose first row's document starts after this key tile see none of it
+    if (DKV) {      // query tiles whose first row's document starts after this key tile see none of it; 32 tiles asked at once
       int e = in_begin + 1;
-      while (e < in_end && dstart[e * 128] <= outer * 128 + 127) ++e;
-      in_end = e;
+      while (e < in_end) {
+        const int t = e + lane;
+        const unsigned hidden = __ballot_sync(0xffffffffu, t < in_end && dstart[(long long)min(t, in_end - 1) * 128] > outer * 128 + 127);
+        if (hidden) {
+          in_end = e + __ffs(hidden) - 1;
+          break;
+        }
+        e += 32;
+      }
     } else {
       in_begin = dstart[outer * 128] / 128;
     }
   }
   const int n_in = in_end - in_begin;                     // inner tiles per head
-  const int n_iter = DKV ? n_in * group : n_in;           // DKV: every query head of the group in turn
+  const int heads = DKV ? group / nsplit : 1;             // query heads of this CTA
+  const int hq0 = DKV ? kvh * group + share * heads : h;
+  const int n_iter = n_in * heads;                        // DKV: every query head of the share in turn
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmQKV);
     prefetch_tmap(&tmDO);
-    for (int i = 0; i < BB_COUNT; ++i) mbar_init(bar(i), (i == BB_P || i == BB_DS) ? 8 : 1);   // one arrival per compute warp
+    for (int i = 0; i < BB_COUNT; ++i)      // one arrival per compute warp, or one
+      mbar_init(bar(i), (i >= BB_P && i < BB_ACC) || (RES_TM && i <= BB_RES1) ? ATTB_COMPUTE : 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -149,36 +209,44 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  // fp32 S (or S^T) and dP (or dP^T); their bf16 successors P / dS overwrite the first 64 columns
-  const uint32_t TM_S = tmem_base, TM_DP = tmem_base + 128, TM_ACC0 = tmem_base + 256, TM_ACC1 = tmem_base + 256 + HDP;
+  // fp32 S (or S^T) and dP (or dP^T); their bf16 successors P / dS overwrite the first 16 of the warp's 32 columns they come from
+  const uint32_t TM_S = tmem_base, TM_DP = tmem_base + 128, TM_ACC0 = tmem_base + 256, TM_ACC1 = tmem_base + 256 + HDP,
+                 TM_RES0 = tmem_base + 384, TM_RES1 = TM_RES0 + HDP / 2;
 
   // resident pair: (K_j, V_j) in DKV mode, (Q_i, dO_i) in DQ mode; the inner pair is the other one
   const uint32_t sRes0 = sbase + L::RES0, sRes1 = sbase + L::RES1;
-  auto sIn0 = [&](int slot) { return sbase + L::IN0 + slot * NSUB * SUBB; };
-  auto sIn1 = [&](int slot) { return sbase + L::IN1 + slot * NSUB * SUBB; };
+  auto sQ = [&](int slot) { return sbase + L::INQ + slot * L::TILE; };
+  auto sO = [&](int slot) { return sbase + L::INO + slot * L::TILE; };
 
   if (warp == 0) {
     if (lane == 0) {
-      auto load_qdo = [&](uint32_t dq, uint32_t ddo, int hq, int tile, int bar_id) {
-        for (int s = 0; s < NSUB; ++s) {
-          tma_load_4d(dq + s * SUBB, &tmQKV, s * 64, hq, b, tile * 128, bar(bar_id));
-          tma_load_4d(ddo + s * SUBB, &tmDO, s * 64, hq, b, tile * 128, bar(bar_id));
-        }
+      auto load = [&](uint32_t dst, const CUtensorMap* tm, int head, int tile, int bar_id) {
+        mbar_expect_tx(bar(bar_id), L::TILE);
+        for (int s = 0; s < NSUB; ++s) tma_load_4d(dst + s * SUBB, tm, s * 64, head, b, tile * 128, bar(bar_id));
       };
-      auto load_kv = [&](uint32_t dk, uint32_t dv, int tile, int bar_id) {
-        for (int s = 0; s < NSUB; ++s) {
-          tma_load_4d(dk + s * SUBB, &tmQKV, s * 64, p.H + kvh, b, tile * 128, bar(bar_id));
-          tma_load_4d(dv + s * SUBB, &tmQKV, s * 64, p.H + p.Hkv + kvh, b, tile * 128, bar(bar_id));
-        }
+      auto load_q = [&](int it) {                         // Q, or K in the query-tile pass
+        const int hq = hq0 + it / n_in, t = in_begin + it % n_in;
+        load(sQ(it % NQ), &tmQKV, DKV ? hq : p.H + kvh, t, BB_QF0 + it % NQ);
       };
-      mbar_expect_tx(bar(BB_RES), 2 * NSUB * SUBB);
-      if (DKV) load_kv(sRes0, sRes1, outer, BB_RES); else load_qdo(sRes0, sRes1, h, outer, BB_RES);
-      for (int it = 0; it < n_iter; ++it) {
-        const int slot = it & 1;
-        if (it >= 2 && !mbar_wait(bar(BB_INFREE0 + slot), ((it >> 1) - 1) & 1, abort_flag, p.status)) break;
-        mbar_expect_tx(bar(BB_INFULL0 + slot), 2 * NSUB * SUBB);
-        if (DKV) load_qdo(sIn0(slot), sIn1(slot), kvh * group + it / n_in, in_begin + it % n_in, BB_INFULL0 + slot);
-        else load_kv(sIn0(slot), sIn1(slot), in_begin + it, BB_INFULL0 + slot);
+      auto load_o = [&](int it) {                         // dO, or V
+        const int hq = hq0 + it / n_in, t = in_begin + it % n_in;
+        load(sO(it % NO), DKV ? &tmDO : &tmQKV, DKV ? hq : p.H + p.Hkv + kvh, t, BB_OF0 + it % NO);
+      };
+      if (!RES_TM) load(sRes0, &tmQKV, p.H + kvh, outer, BB_RES0);
+      load_q(0);
+      if (!RES_TM) load(sRes1, &tmQKV, p.H + p.Hkv + kvh, outer, BB_RES1);
+      load_o(0);
+      for (int it = 1; it < NQ; ++it) {                   // NO = NQ - 1
+        if (it < n_iter) load_q(it);
+        if (it < NO && it < n_iter) load_o(it);
+      }
+      for (int it = 0; it + NO < n_iter; ++it) {          // slots in the order in which the products give them back
+        if (!mbar_wait(bar(BB_OE0 + it % NO), (it / NO) & 1, abort_flag, p.status)) break;
+        load_o(it + NO);
+        if (it + NQ < n_iter) {
+          if (!mbar_wait(bar(BB_QE0 + it % NQ), (it / NQ) & 1, abort_flag, p.status)) break;
+          load_q(it + NQ);
+        }
       }
     }
   } else if (warp == 1) {
@@ -192,243 +260,280 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       // read, dP after dS was multiplied), so the exponentials of tile it+1 overlap the accumulator MMAs of tile it.
       // DKV: S^T = K Q^T, dP^T = V dO^T (A = resident);  DQ: S = Q K^T, dP = dO V^T (A = resident)
       auto issue_s = [&](int it) {
-        const uint32_t a0 = sRes0, b0 = sIn0(it & 1);
+        const uint32_t a0 = sRes0, b0 = sQ(it % NQ);
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < HDP / 16; ++kk) {
             const uint32_t off = (kk / 4) * SUBB + (kk % 4) * 32;
-            tc_mma_f16(TM_S, make_smem_desc(a0 + off, 16, 1024, 2), make_smem_desc(b0 + off, 16, 1024, 2), idesc_s, kk != 0);
+            if (RES_TM) tc_mma_f16_ts(TM_S, TM_RES0 + kk * 8, make_smem_desc(b0 + off, 16, 1024, 2), idesc_s, kk != 0);
+            else tc_mma_f16(TM_S, make_smem_desc(a0 + off, 16, 1024, 2), make_smem_desc(b0 + off, 16, 1024, 2), idesc_s, kk != 0);
           }
           tc_commit(bar(BB_S));
         }
         __syncwarp();
       };
       auto issue_dp = [&](int it) {
-        const uint32_t a1 = sRes1, b1 = sIn1(it & 1);
+        const uint32_t a1 = sRes1, b1 = sO(it % NO);
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < HDP / 16; ++kk) {
             const uint32_t off = (kk / 4) * SUBB + (kk % 4) * 32;
-            tc_mma_f16(TM_DP, make_smem_desc(a1 + off, 16, 1024, 2), make_smem_desc(b1 + off, 16, 1024, 2), idesc_s, kk != 0);
+            if (RES_TM) tc_mma_f16_ts(TM_DP, TM_RES1 + kk * 8, make_smem_desc(b1 + off, 16, 1024, 2), idesc_s, kk != 0);
+            else tc_mma_f16(TM_DP, make_smem_desc(a1 + off, 16, 1024, 2), make_smem_desc(b1 + off, 16, 1024, 2), idesc_s, kk != 0);
           }
           tc_commit(bar(BB_DP));
+          if (!DKV) tc_commit(bar(BB_OE0 + it % NO));
         }
         __syncwarp();
       };
-      bool ok = wait(BB_RES, 0);
-      if (ok && n_iter > 0) {
-        ok = wait(BB_INFULL0, 0);
-        if (ok) {
-          tc_fence_after();
-          issue_s(0);
-          issue_dp(0);
+      // A (16 columns of P or dS per step, 8 tensor-memory columns) lies in the first half of its compute warp's columns; acc += A B over the
+      // steps that the warps' first (half 0) or second 16 columns make up
+      auto issue_acc = [&](uint32_t acc, uint32_t a, uint32_t b, int half, bool first) {
+        if (elect_one()) {
+#pragma unroll
+          for (int w = 0; w < ATTB_SPLIT; ++w)
+            tc_mma_f16_ts(acc, a + w * CW + half * 8, make_smem_desc(b + (2 * w + half) * 2048, SUBB, 1024, 2), idesc_acc, !(first && half == 0 && w == 0));
         }
+        __syncwarp();
+      };
+      bool ok = wait(BB_RES0, 0) && wait(BB_QF0, 0);
+      if (ok) {
+        tc_fence_after();
+        issue_s(0);
+        ok = wait(BB_RES1, 0) && wait(BB_OF0, 0);
+      }
+      if (ok) {
+        tc_fence_after();
+        issue_dp(0);
       }
       for (int it = 0; it < n_iter && ok; ++it) {
-        const int slot = it & 1;
-        const uint32_t b0 = sIn0(slot), b1 = sIn1(slot);
-        if (!wait(BB_P, it & 1)) { ok = false; break; }      // the S columns have been read (DKV: P is in place)
-        tc_fence_after();
-        if (DKV) {
-          if (elect_one()) {
+        const uint32_t b0 = sQ(it % NQ), b1 = sO(it % NO);
+        if (DKV) {          // dV[key, d] += sum_q P^T[key, q] dO[q, d]
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)   // dV[key, d] += sum_q P^T[key, q] dO[q, d]
-              tc_mma_f16_ts(TM_ACC0, TM_S + kk * 8, make_smem_desc(b1 + kk * 2048, SUBB, 1024, 2), idesc_acc, (it | kk) != 0);
+          for (int half = 0; half < 2 && ok; ++half) {
+            ok = wait(BB_P + half, it & 1);
+            if (!ok) break;
+            tc_fence_after();
+            issue_acc(TM_ACC0, TM_S, b1, half, it == 0);
           }
+          if (!ok) break;
+          if (elect_one()) tc_commit(bar(BB_OE0 + it % NO));
           __syncwarp();
         }
         if (it + 1 < n_iter) {
-          if (!wait(BB_INFULL0 + ((it + 1) & 1), ((it + 1) >> 1) & 1)) { ok = false; break; }
+          if (!wait(BB_QF0 + (it + 1) % NQ, ((it + 1) / NQ) & 1)) { ok = false; break; }
+          if (!DKV && !wait(BB_P, it & 1)) { ok = false; break; }          // the S columns have been read
           tc_fence_after();
           issue_s(it + 1);
         }
-        if (!wait(BB_DS, it & 1)) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          if (DKV) {
+        // dK[key, d] += sum_q dS^T[key, q] Q[q, d], or dQ[q, d] += sum_key dS[q, key] K[key, d]
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)   // dK[key, d] += sum_q dS^T[key, q] Q[q, d]
-              tc_mma_f16_ts(TM_ACC1, TM_DP + kk * 8, make_smem_desc(b0 + kk * 2048, SUBB, 1024, 2), idesc_acc, (it | kk) != 0);
-          } else {
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)   // dQ[q, d] += sum_key dS[q, key] K[key, d]
-              tc_mma_f16_ts(TM_ACC0, TM_DP + kk * 8, make_smem_desc(b0 + kk * 2048, SUBB, 1024, 2), idesc_acc, (it | kk) != 0);
-          }
-          tc_commit(bar(BB_INFREE0 + slot));
+        for (int half = 0; half < 2 && ok; ++half) {
+          ok = wait(BB_DS + half, it & 1);
+          if (!ok) break;
+          tc_fence_after();
+          issue_acc(DKV ? TM_ACC1 : TM_ACC0, TM_DP, b0, half, it == 0);
         }
+        if (!ok) break;
+        if (elect_one()) tc_commit(bar(BB_QE0 + it % NQ));
         __syncwarp();
-        if (it + 1 < n_iter) issue_dp(it + 1);
+        if (it + 1 < n_iter) {
+          if (!wait(BB_OF0 + (it + 1) % NO, ((it + 1) / NO) & 1)) { ok = false; break; }
+          tc_fence_after();
+          issue_dp(it + 1);
+        }
       }
       if (ok) {
         if (elect_one()) tc_commit(bar(BB_ACC));
         __syncwarp();
       }
     }
+  } else if (warp == 2) {
+    // per-query vectors of the inner query tiles, one iteration ahead of the compute warps (loaded by them, each iteration began with the
+    // latency of these loads)
+    if (DKV) {
+      for (int it = 0; it < n_iter; ++it) {
+        const int q_tile = in_begin + it % n_in, hq = hq0 + it / n_in;
+        const long long base = ((long long)b * p.H + hq) * p.S;
+        float lv[4], dv[4];
+        int ds[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int qrow = q_tile * 128 + u * 32 + lane;
+          const bool in = qrow < p.S;
+          // stored negated (and delta pre-multiplied by the softmax scale) so that both uses are one fused multiply-add
+          lv[u] = in ? -p.lse[base + qrow] * 1.4426950408889634f : -INFINITY;   // -inf -> exp2(-inf) = 0 for rows past the end
+          dv[u] = in ? -p.delta[base + qrow] * p.scale : 0.f;
+          ds[u] = dstart ? min(max(dstart[min(qrow, p.S - 1)] - outer * 128, 0), 128) : 0;
+        }
+        if (it >= 2) {        // the slot was last read before the product that gave back the Q tile of it - 2
+          const bool free = mbar_wait(bar(BB_QE0 + (it - 2) % NQ), ((it - 2) / NQ) & 1, abort_flag, p.status);
+          if (!__all_sync(0xffffffffu, free)) break;
+        }
+        uint8_t* vs = smem + L::VEC_OFF + (it & 1) * L::VEC;
+        float* vf = reinterpret_cast<float*>(vs);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          vf[u * 32 + lane] = lv[u];
+          vf[128 + u * 32 + lane] = dv[u];
+          vs[1024 + u * 32 + lane] = (uint8_t)ds[u];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(BB_VF0 + (it & 1)));
+      }
+    }
   } else {
     // ---------------------------------------------------------------- compute warps
-    const int cw = warp - 2;
-    const int ct = threadIdx.x - 64;              // 0..255 inside the compute group
     const int quarter = warp & 3;
-    const int half = cw >> 2;                     // which 64 columns of the block
+    const int part = (warp - 3) >> 2;             // which columns of the block
     const int row_local = quarter * 32 + lane;    // lane of tensor memory: key row (DKV) or query row (DQ)
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const float LOG2E = 1.4426950408889634f;
+    const int colw = part * CW;
     bool ok = true;
     float lse2 = 0.f, dlt = 0.f;
     bool row_ok = true;
     int lower = 0;                                // DQ: first key this query row may see (packed sequences)
+    int doc_last = 0;                             // DQ: document start of the last query row
     if (!DKV) {
       const int row = outer * 128 + row_local;
       row_ok = row < p.S;
       if (row_ok) {   // negated / pre-scaled like the shared-memory vectors of the other mode
-        lse2 = -p.lse[((long long)b * p.H + h) * p.S + row] * LOG2E;
+        lse2 = -p.lse[((long long)b * p.H + h) * p.S + row] * 1.4426950408889634f;
         dlt = -p.delta[((long long)b * p.H + h) * p.S + row] * p.scale;
         if (dstart) lower = dstart[row];
       }
+      if (dstart) doc_last = dstart[min(outer * 128 + 127, p.S - 1)];
     }
-    for (int it = 0; it < n_iter; ++it) {
-      const int q_tile = DKV ? in_begin + it % n_in : outer;
-      const int k_tile = DKV ? outer : in_begin + it;
-      const int hq = DKV ? kvh * group + it / n_in : h;      // query head of this iteration
-      float* vl = svec + (it & 1) * 384;          // [0,128) lse2, [128,256) delta, [256,384) document start of the inner query tile
-      const int* vdoc = reinterpret_cast<const int*>(vl + 256);
-      if (DKV) {
-        const int qi = ct & 127;
-        const int qrow = q_tile * 128 + qi;
-        const long long idx = ((long long)b * p.H + hq) * p.S + qrow;
-        // stored negated (and delta pre-multiplied by the softmax scale) so that both uses are one fused multiply-add
-        if (ct < 128) {
-          vl[qi] = qrow < p.S ? -p.lse[idx] * LOG2E : -INFINITY;   // -inf -> exp2(-inf) = 0 for rows past the end
-          if (dstart) reinterpret_cast<int*>(vl + 256)[qi] = dstart[min(qrow, p.S - 1)];
-        } else {
-          vl[128 + qi] = qrow < p.S ? -p.delta[idx] * p.scale : 0.f;
+    if (RES_TM) {       // the resident pair into tensor memory: HDP / SPLIT columns of this thread's row, zeros past the end
+      constexpr int VN = HDP / ATTB_SPLIT / 8;
+      const int row = outer * 128 + row_local, e0 = part * (HDP / ATTB_SPLIT);
+      const __nv_bfloat16* r0 = p.qkv + (long long)row * p.q_stride_s + (long long)b * p.q_stride_b + (long long)(DKV ? p.H + kvh : h) * p.hd + e0;
+      const __nv_bfloat16* r1 = DKV ? r0 + (long long)p.Hkv * p.hd : p.dout + (long long)row * p.o_stride_s + (long long)b * p.o_stride_b + (long long)h * p.hd + e0;
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        uint32_t v[VN * 4];
+#pragma unroll
+        for (int i = 0; i < VN; ++i) {
+          uint4 q = make_uint4(0, 0, 0, 0);
+          if (row < p.S && e0 + i * 8 < p.hd) q = *reinterpret_cast<const uint4*>((which ? r1 : r0) + i * 8);
+          v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
         }
-        named_bar_sync(1, 256);
+        const uint32_t dst = (which ? TM_RES1 : TM_RES0) + lane_addr + e0 / 2;
+        if constexpr (VN == 4) tmem_st16(dst, v); else tmem_st8(dst, v);
       }
-      // After a timeout the loop keeps running without touching tensor memory so that every warp
-      // still reaches the named barriers below (the waits return immediately once the abort flag is up).
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(bar(BB_RES0));
+        mbar_arrive(bar(BB_RES1));
+      }
+    }
+    const float sc2 = p.scale_log2;
+    const uint64_t sc2x2 = pack_f32x2(sc2, sc2), scx2 = pack_f32x2(p.scale, p.scale);
+    for (int it = 0, in_tile = in_begin; it < n_iter; ++it, in_tile = in_tile + 1 < in_end ? in_tile + 1 : in_begin) {
+      const int k_tile = DKV ? outer : in_tile;
+      const uint8_t* vs = smem + L::VEC_OFF + (it & 1) * L::VEC;
+      const float* vl = reinterpret_cast<const float*>(vs);
+      const uint8_t* vdoc = vs + 1024;
+      if (DKV && ok) ok = mbar_wait(bar(BB_VF0 + (it & 1)), (it >> 1) & 1, abort_flag, p.status);
       if (ok) ok = mbar_wait(bar(BB_S), it & 1, abort_flag, p.status);
       ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
       tc_fence_after();
-      const bool diag = p.causal && q_tile == k_tile;
-      float ev[64];                      // this thread's 64 probabilities (fp32, kept for dS)
-      uint32_t keep[32];                 // ... and as bf16 pairs (P, then dS)
-      // ---- phase 1: P = exp2(S * scale - lse). `diag` (and a ragged last tile) is uniform over the CTA: only
+      const bool diag = p.causal && in_tile == outer;
+      uint32_t rs[32];                   // S, then the probabilities (fp32, kept for dS)
+      tmem_ld32(TM_S + lane_addr + colw, rs);
+      tmem_ld_wait32(rs);
+      if (!DKV) {                        // the S columns have been read: the next S product may overwrite them
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(BB_P));
+      }
+      // ---- phase 1: P = exp2(S * scale - lse), 16 columns at a time. `diag` (and a ragged last tile) is uniform over the CTA: only
       // those tiles pay for the per-element mask test. The per-query vectors come from shared memory four at a time.
-      const float sc2 = p.scale_log2;
-      const uint64_t sc2x2 = pack_f32x2(sc2, sc2), scx2 = pack_f32x2(p.scale, p.scale);
-      auto phase1 = [&](auto masked_tag) {
+      auto phase1 = [&](auto masked_tag, int half) {
         constexpr bool MASK = decltype(masked_tag)::value;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int col0 = half * 64 + c * 32;
-          uint32_t rs[32];
-          tmem_ld32(TM_S + lane_addr + col0, rs);
-          tmem_ld_wait();
+        for (int i = half * 16; i < half * 16 + 16; i += 4) {
+          float l4[4] = {lse2, lse2, lse2, lse2};
+          if (DKV) {
+            const float4 t4 = *reinterpret_cast<const float4*>(vl + colw + i);
+            l4[0] = t4.x; l4[1] = t4.y; l4[2] = t4.z; l4[3] = t4.w;
+          }
+          if (MASK) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            float l4[4] = {lse2, lse2, lse2, lse2};
-            if (DKV) {
-              const float4 t4 = *reinterpret_cast<const float4*>(vl + col0 + i);
-              l4[0] = t4.x; l4[1] = t4.y; l4[2] = t4.z; l4[3] = t4.w;
+            for (int u = 0; u < 4; ++u) {
+              const int col = colw + i + u;
+              float e = fast_exp2(fmaf(__uint_as_float(rs[i + u]), sc2, l4[u]));
+              // DKV: lane = key, column = query -> masked when key > query; DQ: lane = query, column = key
+              bool masked = DKV ? (diag && row_local > col) : (!row_ok || (diag && col > row_local));
+              if (dstart) masked = masked || (DKV ? (row_local < (int)vdoc[col]) : (k_tile * 128 + col < lower));
+              if (masked) e = 0.f;
+              rs[i + u] = __float_as_uint(e);
             }
-            if (MASK) {
+          } else {
 #pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const int col = col0 + i + u;
-                float e = fast_exp2(fmaf(__uint_as_float(rs[i + u]), sc2, l4[u]));
-                // DKV: lane = key, column = query -> masked when key > query; DQ: lane = query, column = key
-                bool masked = DKV ? (diag && row_local > col) : (!row_ok || (diag && col > row_local));
-                if (dstart) masked = masked || (DKV ? (k_tile * 128 + row_local < vdoc[col]) : (k_tile * 128 + col < lower));
-                if (masked) e = 0.f;
-                ev[c * 32 + i + u] = e;
-              }
-            } else {
-#pragma unroll
-              for (int u = 0; u < 4; u += 2) {   // packed pairs: one FFMA instruction per two elements
-                float x0, x1;
-                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i + u]), __uint_as_float(rs[i + u + 1])), sc2x2,
-                                       pack_f32x2(l4[u], l4[u + 1])), x0, x1);
-                ev[c * 32 + i + u] = fast_exp2(x0);
-                ev[c * 32 + i + u + 1] = fast_exp2(x1);
-              }
+            for (int u = 0; u < 4; u += 2) {   // packed pairs: one FFMA instruction per two elements
+              float x0, x1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i + u]), __uint_as_float(rs[i + u + 1])), sc2x2,
+                                     pack_f32x2(l4[u], l4[u + 1])), x0, x1);
+              rs[i + u] = __float_as_uint(fast_exp2(x0));
+              rs[i + u + 1] = __float_as_uint(fast_exp2(x1));
             }
           }
         }
       };
-      if (ok) {
-        // a document boundary inside the block pair: the key tile starts before the query tile's last document does
-        const bool doc_mask = dstart && k_tile * 128 < dstart[min(q_tile * 128 + 127, p.S - 1)];
-        const bool any_mask = diag || doc_mask || (!DKV && (outer + 1) * 128 > p.S);
-        if (any_mask) phase1(std::true_type{}); else phase1(std::false_type{});
-      }
-      if (DKV) {
-        // The bf16 results go back into tensor memory on top of fp32 columns: a row's 128 values take
-        // 64 columns, so the upper half lands on columns the partner warp (other half, same lanes) was
-        // reading. All 256 compute threads therefore finish their loads before anyone stores.
+      // eight registers of bf16 pairs into tensor memory, then this half is handed to the MMA warp
+      auto hand_over = [&](uint32_t at, const uint32_t (&t)[8], int bar_id, int half) {
+        tmem_st8(at + lane_addr + colw + half * 8, t);
+        tmem_st_wait();
         tc_fence_before();
-        named_bar_sync(1, 256);
-        tc_fence_after();
-        if (ok) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(bar_id + half));
+      };
+      // a document boundary inside the block pair: the key tile starts before the query tile's last document does
+      const bool doc_mask = dstart && (DKV ? vdoc[127] > 0 : k_tile * 128 < doc_last);
+      const bool any_mask = diag || doc_mask || (!DKV && (outer + 1) * 128 > p.S);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) keep[i] = pack_bf16(ev[2 * i], ev[2 * i + 1]);
-          uint32_t t0[16], t1[16];
+      for (int half = 0; half < 2; ++half) {
+        if (any_mask) phase1(std::true_type{}, half); else phase1(std::false_type{}, half);
+        if (DKV) {
+          uint32_t t[8];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) { t0[i] = keep[i]; t1[i] = keep[16 + i]; }
-          tmem_st16(TM_S + lane_addr + half * 32, t0);
-          tmem_st16(TM_S + lane_addr + half * 32 + 16, t1);
-          tmem_st_wait();
+          for (int i = 0; i < 8; ++i) t[i] = pack_bf16(__uint_as_float(rs[half * 16 + 2 * i]), __uint_as_float(rs[half * 16 + 2 * i + 1]));
+          hand_over(TM_S, t, BB_P, half);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(BB_P));
-      } else {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(BB_P));            // the S columns have been read: the next S product may overwrite them
       }
       // ---- phase 2: dS = P * (dP - delta) * scale
-      if (ok) ok = mbar_wait(bar(BB_DP), it & 1, abort_flag, p.status);
+      ok = mbar_wait(bar(BB_DP), it & 1, abort_flag, p.status);
       ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
       tc_fence_after();
+      uint32_t rd[32];
+      tmem_ld32(TM_DP + lane_addr + colw, rd);
+      tmem_ld_wait32(rd);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        if (!ok) break;
-        const int col0 = half * 64 + c * 32;
-        uint32_t rd[32];
-        tmem_ld32(TM_DP + lane_addr + col0, rd);
-        tmem_ld_wait();
+      for (int half = 0; half < 2; ++half) {
+        uint32_t t[8];
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
+        for (int i = half * 16; i < half * 16 + 16; i += 4) {
           float d4[4] = {dlt, dlt, dlt, dlt};
           if (DKV) {
-            const float4 t4 = *reinterpret_cast<const float4*>(vl + 128 + col0 + i);
+            const float4 t4 = *reinterpret_cast<const float4*>(vl + 128 + colw + i);
             d4[0] = t4.x; d4[1] = t4.y; d4[2] = t4.z; d4[3] = t4.w;
           }
           // dS = P * (dP * scale - delta * scale): one packed FFMA and one packed FMUL per two elements
           float x0, x1, x2, x3;
           const uint64_t t01 = fma_f32x2(pack_f32x2(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])), scx2, pack_f32x2(d4[0], d4[1]));
           const uint64_t t23 = fma_f32x2(pack_f32x2(__uint_as_float(rd[i + 2]), __uint_as_float(rd[i + 3])), scx2, pack_f32x2(d4[2], d4[3]));
-          unpack_f32x2(fma_f32x2(pack_f32x2(ev[c * 32 + i], ev[c * 32 + i + 1]), t01, 0ull), x0, x1);
-          unpack_f32x2(fma_f32x2(pack_f32x2(ev[c * 32 + i + 2], ev[c * 32 + i + 3]), t23, 0ull), x2, x3);
-          keep[c * 16 + (i >> 1)] = pack_bf16(x0, x1);
-          keep[c * 16 + (i >> 1) + 1] = pack_bf16(x2, x3);
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), t01, 0ull), x0, x1);
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i + 2]), __uint_as_float(rs[i + 3])), t23, 0ull), x2, x3);
+          t[(i - half * 16) >> 1] = pack_bf16(x0, x1);
+          t[((i - half * 16) >> 1) + 1] = pack_bf16(x2, x3);
         }
+        hand_over(TM_DP, t, BB_DS, half);
       }
-      tc_fence_before();
-      named_bar_sync(1, 256);            // every thread has read its dP columns before dS overwrites them
-      tc_fence_after();
-      if (ok) {
-        uint32_t t0[16], t1[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { t0[i] = keep[i]; t1[i] = keep[16 + i]; }
-        tmem_st16(TM_DP + lane_addr + half * 32, t0);
-        tmem_st16(TM_DP + lane_addr + half * 32 + 16, t1);
-        tmem_st_wait();
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(BB_DS));
     }
     // ---------------------------------------------------------------- epilogue
     if (ok) {
@@ -440,12 +545,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       const int row = outer * 128 + row_local;   // key row (DKV) or query row (DQ)
       constexpr int CHUNKS = HDP / 32;           // 32-column chunks per accumulator
       constexpr int NACC = DKV ? 2 : 1;
-      // split the NACC * CHUNKS chunks between the two warps that share this lane quarter
-      for (int idx = half; idx < NACC * CHUNKS; idx += 2) {
+      // split the NACC * CHUNKS chunks between the warps that share this lane quarter
+      for (int idx = part; idx < NACC * CHUNKS; idx += ATTB_SPLIT) {
         const int acc = idx / CHUNKS, c = idx % CHUNKS;
         uint32_t r[32];
         tmem_ld32((acc == 0 ? TM_ACC0 : TM_ACC1) + lane_addr + c * 32, r);
-        tmem_ld_wait();
+        tmem_ld_wait32(r);
+        if (DKV && nsplit > 1) {                 // to the cluster, over the tiles: every product that read them is done
+          float* red = reinterpret_cast<float*>(smem + L::INQ) + row_local * L::RED_LD + idx * 32;
+#pragma unroll
+          for (int g = 0; g < 8; ++g) *reinterpret_cast<uint4*>(red + g * 4) = make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+          continue;
+        }
         // DKV: acc 0 = dV, acc 1 = dK of key head `kvh`; DQ: dQ of query head `h`; heads are [H query | Hkv key | Hkv value]
         const int head = DKV ? (acc == 0 ? p.H + p.Hkv + kvh : p.H + kvh) : h;
         if (row < p.S) {
@@ -468,6 +579,30 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
+  if (DKV && nsplit > 1) {                       // dV | dK of 128 / nsplit rows: the shares of the cluster, added up in rank order
+    cluster_sync_all();
+    const int rows = 128 / nsplit;
+    const uint32_t red = sbase + L::INQ;
+    if (!*abort_flag) {
+      for (int i = threadIdx.x; i < rows * (2 * HDP / 8); i += ATTB_THREADS) {
+        const int rl = share * rows + i / (2 * HDP / 8), c = i % (2 * HDP / 8) * 8, d0 = c % HDP;
+        const int row = outer * 128 + rl;
+        if (row >= p.S || d0 >= p.hd) continue;
+        float s[8] = {};
+        for (int w = 0; w < nsplit; ++w) {
+          const uint32_t src = map_to_cta(red + (uint32_t)(rl * L::RED_LD + c) * 4, w);
+          const float4 x = ld_cluster_f4(src), y = ld_cluster_f4(src + 16);
+          s[0] += x.x; s[1] += x.y; s[2] += x.z; s[3] += x.w;
+          s[4] += y.x; s[5] += y.y; s[6] += y.z; s[7] += y.w;
+        }
+        const int head = c < HDP ? p.H + p.Hkv + kvh : p.H + kvh;
+        *reinterpret_cast<uint4*>(p.dqkv + (long long)row * p.d_stride_s + (long long)b * p.d_stride_b + (long long)head * p.hd + d0) =
+            make_uint4(pack_bf16(s[0], s[1]), pack_bf16(s[2], s[3]), pack_bf16(s[4], s[5]), pack_bf16(s[6], s[7]));
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();                          // nobody leaves while its shared memory is being read
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
@@ -476,16 +611,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 
 template <int HDP, bool DKV>
 int launch_attn_bwd(const CUtensorMap& tmQKV, const CUtensorMap& tmDO, const AttnBwdParams& p, cudaStream_t stream) {
-  using L = BwdSmem<HDP>;
+  using L = BwdSmem<HDP, DKV>;
   auto kern = attn_bwd_kernel<HDP, DKV>;
-  static bool configured = false;
-  if (!configured) {
-    ELFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN));
-    configured = true;
-  }
-  dim3 grid((unsigned)p.n_tiles * (DKV ? p.Hkv : p.H) * p.B);
-  kern<<<grid, ATTB_THREADS, L::DYN, stream>>>(tmQKV, tmDO, p);
-  ELFA_CUDA(cudaGetLastError());
+  ELFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+  const unsigned nsplit = DKV ? p.nsplit : 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)p.n_tiles * (DKV ? p.Hkv : p.H) * p.B * nsplit);
+  cfg.blockDim = dim3(ATTB_THREADS);
+  cfg.dynamicSmemBytes = L::TOTAL;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = nsplit;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = nsplit > 1 ? 1 : 0;
+  ELFA_CUDA(cudaLaunchKernelEx(&cfg, kern, tmQKV, tmDO, p));
   ::elfa::count_launches(1);
   return ELFA_OK;
 }
@@ -512,10 +653,12 @@ ELFA_API int elfa_attention_bwd_ex(const void* qkv, long long stride_s, long lon
   unsigned int* st = status_word();
   ELFA_REQUIRE(st != nullptr, "attention_bwd: no status word");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const long long nwarps = (long long)S * B * H;
-  attn_delta_kernel<<<(unsigned)((nwarps + 7) / 8), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out),
-                                                                 static_cast<const __nv_bfloat16*>(dout), o_stride_s, o_stride_b,
-                                                                 delta, S, B, H, hd);
+  const long long rows = (long long)S * B * H;
+  const int per = hd <= 64 ? 64 : 32;      // rows of a block
+  ELFA_REQUIRE((rows + per - 1) / per < (1ll << 31), "attention_bwd: too many rows");
+  auto delta_kernel = hd <= 64 ? attn_delta_kernel<8> : attn_delta_kernel<16>;
+  delta_kernel<<<(unsigned)((rows + per - 1) / per), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout),
+                                                                  o_stride_s, o_stride_b, delta, S, B, H, hd);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   CUtensorMap tmQKV, tmDO;
@@ -527,6 +670,10 @@ ELFA_API int elfa_attention_bwd_ex(const void* qkv, long long stride_s, long lon
   p.S = S; p.B = B; p.H = H; p.hd = hd;
   p.Hkv = Hkv;
   p.doc_start = doc_start;
+  p.qkv = static_cast<const __nv_bfloat16*>(qkv);
+  p.dout = static_cast<const __nv_bfloat16*>(dout);
+  p.q_stride_s = stride_s; p.q_stride_b = stride_b;
+  p.o_stride_s = o_stride_s; p.o_stride_b = o_stride_b;
   p.lse = lse; p.delta = delta;
   p.dqkv = static_cast<__nv_bfloat16*>(dqkv);
   p.d_stride_s = d_stride_s; p.d_stride_b = d_stride_b;
@@ -534,6 +681,8 @@ ELFA_API int elfa_attention_bwd_ex(const void* qkv, long long stride_s, long lon
   p.scale_log2 = scale * 1.4426950408889634f;
   p.causal = causal;
   p.n_tiles = (S + 127) / 128;
+  p.nsplit = 1;
+  while (p.nsplit < 4 && H / Hkv % (2 * p.nsplit) == 0 && (long long)p.n_tiles * Hkv * B * p.nsplit < 2 * device_sm_count()) p.nsplit *= 2;
   p.status = st;
   if (hd <= 64) {
     rc = launch_attn_bwd<64, true>(tmQKV, tmDO, p, s);
