@@ -83,9 +83,9 @@ struct QParams {
 
 template <int BN, int STAGES, bool TWO, bool FP4 = false>
 struct QSmem {
-  // B scale atoms per tile: a tile starts 0 / 32 / 64 / 96 rows into a 128-row atom depending on BN
-  // (128: always 0 -> 1 atom; 192: 0 or 64 -> 2; 224: 0 / 32 / 64 / 96 -> 3)
-  static constexpr int NATOM = BN <= 128 ? 1 : (BN <= 192 ? 2 : 3);
+  // B scale atoms per tile (128: 1; 192: starts 0 or 64 rows into an atom, 2; 256: 2)
+  static_assert(BN == 128 || BN == 192 || BN == 256, "tile widths");
+  static constexpr int NATOM = BN <= 128 ? 1 : 2;
   static constexpr int KSF = FP4 ? 4 : 1;                 // scale atoms along K per stage: an atom covers 4 blocks of 32 (fp8) or 16 (fp4) elements
   static constexpr int A_BYTES = QBM * QBK;
   static constexpr int B_BYTES = (TWO ? BN / 2 : BN) * QBK;
@@ -154,6 +154,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   auto empty_bar = [&](int s) { return bar0 + 8u * (STAGES + s); };
   auto tfull_bar = [&](int b) { return bar0 + 8u * (2 * STAGES + b); };
   auto tempty_bar = [&](int b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
+  const uint32_t over_bar = bar0 + 8u * (2 * STAGES + 4);      // SHARED; the all-gather variant's push barriers otherwise
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -163,11 +164,16 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   // tensor memory: accumulator b at column 256 * b, one set of scale-factor columns behind each accumulator.
   // K tiles alternate between the two sets, so the copy of the next tile's scales does not have to
   // wait for the MMAs that still read the current ones.
+  // BN = 256: two whole accumulators and the scales are 24 columns too many, so the accumulators share 24 columns: columns 232 .. 255 are the last
+  // ones of the first and the first ones of the second. The epilogue reads the group of 64 that holds them first and raises over_bar, for
+  // which the next tile's first product waits (some 500 cycles per tile; the rest of the epilogue runs under that tile's products).
+  constexpr bool SHARED = BN == 256;
+  static_assert(!SHARED || (TWO && !FP4 && !AG), "the 256-wide tile is for CTA pairs");
   constexpr uint32_t TMEM_COLS = 512;
-  constexpr uint32_t ACC_STRIDE = 256;
-  constexpr uint32_t SFA_COL = BN;                 // 4 columns per atom, KSF atoms
-  constexpr uint32_t SFB_COL = BN + 4 * KSF;       // 4 columns per atom, KSF * NATOM atoms
-  static_assert(BN % 16 == 0 && BN + 4 * KSF * (1 + L::NATOM) <= 256, "tile does not fit the tensor-memory plan");
+  constexpr uint32_t ACC_STRIDE = SHARED ? 232 : 256;
+  constexpr uint32_t SF_COLS = 4 * KSF * (1 + L::NATOM);       // 4 columns per atom: KSF atoms of A, KSF * NATOM of B
+  constexpr uint32_t SF_SET0 = SHARED ? 488 : BN, SF_STRIDE = SHARED ? SF_COLS : ACC_STRIDE;
+  static_assert(SHARED ? 232 + BN <= 488 && 488 + 2 * SF_COLS <= 512 : BN + SF_COLS <= 256, "tile does not fit the tensor-memory plan");
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmA);
@@ -182,7 +188,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       mbar_init(tfull_bar(b), 1);
       mbar_init(tempty_bar(b), TWO ? 8 : 4);
     }
-    for (int b = 0; b < 4; ++b) mbar_init(bar0 + 8u * (2 * STAGES + 4 + b), 1);
+    for (int b = 0; b < 4; ++b) mbar_init(bar0 + 8u * (2 * STAGES + 4 + b), SHARED ? 8 : 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -267,7 +273,9 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         q_tile_coords_ag<AG>(p, cm, tile, TILE_M, mb, nb, shard);
         const uint32_t sfb_shift = (uint32_t)((nb * BN) % 128) / 32;   // tile starts inside an atom: skip its first columns
         const uint32_t buf = tile_iter & 1, bph = (tile_iter >> 1) & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(tempty_bar(buf), bph ^ 1, abort_flag, p.status));
+        ok = mbar_wait(tempty_bar(buf), bph ^ 1, abort_flag, p.status);
+        if (SHARED && ok && tile_iter > 0) ok = mbar_wait(over_bar, (tile_iter - 1) & 1, abort_flag, p.status);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + buf * ACC_STRIDE;
@@ -281,29 +289,29 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           const uint32_t b_base = smem_u32(sB + s * L::B_BYTES);
           const uint32_t sf_base = smem_u32(sSF + s * L::SF_BYTES);
           // scale atoms: 32 rows of 16 bytes, no swizzle, 8-row core matrices 128 bytes apart
-          const uint32_t sf_tmem = tmem_base + (it & 1u) * ACC_STRIDE;
+          const uint32_t sfa_tmem = tmem_base + SF_SET0 + (it & 1u) * SF_STRIDE, sfb_tmem = sfa_tmem + 4 * KSF;
           if (elect_one()) {
 #pragma unroll
           for (int q = 0; q < KSF; ++q) {
-            if (TWO) tc_cp_32x128b_warpx4_pair(sf_tmem + SFA_COL + 4 * q, make_smem_desc(sf_base + q * SF_ATOM, 0, 128, 0));
-            else tc_cp_32x128b_warpx4(sf_tmem + SFA_COL + 4 * q, make_smem_desc(sf_base + q * SF_ATOM, 0, 128, 0));
+            if (TWO) tc_cp_32x128b_warpx4_pair(sfa_tmem + 4 * q, make_smem_desc(sf_base + q * SF_ATOM, 0, 128, 0));
+            else tc_cp_32x128b_warpx4(sfa_tmem + 4 * q, make_smem_desc(sf_base + q * SF_ATOM, 0, 128, 0));
           }
 #pragma unroll
           for (int j = 0; j < KSF * L::NATOM; ++j) {
-            if (TWO) tc_cp_32x128b_warpx4_pair(sf_tmem + SFB_COL + 4 * j, make_smem_desc(sf_base + (KSF + j) * SF_ATOM, 0, 128, 0));
-            else tc_cp_32x128b_warpx4(sf_tmem + SFB_COL + 4 * j, make_smem_desc(sf_base + (KSF + j) * SF_ATOM, 0, 128, 0));
+            if (TWO) tc_cp_32x128b_warpx4_pair(sfb_tmem + 4 * j, make_smem_desc(sf_base + (KSF + j) * SF_ATOM, 0, 128, 0));
+            else tc_cp_32x128b_warpx4(sfb_tmem + 4 * j, make_smem_desc(sf_base + (KSF + j) * SF_ATOM, 0, 128, 0));
           }
 #pragma unroll
           for (int k = 0; k < QBK / QUMMA_K; ++k) {
             const uint64_t da = make_smem_desc(a_base + k * 32, 16, 1024, 2);
             const uint64_t db = make_smem_desc(b_base + k * 32, 16, 1024, 2);
             if (FP4)   // all four scale bytes of a column belong to this instruction's 64 K-elements
-              tc_mma_nvf4(tmem_d, da, db, make_idesc_nvf4(TILE_M, BN), (kb | k) != 0 ? 1u : 0u, sf_tmem + SFA_COL + 4 * k,
-                          sf_tmem + SFB_COL + 4 * L::NATOM * k + sfb_shift);
-            else if (TWO) tc_mma_mxf8_pair(tmem_d, da, db, make_idesc_mxf8(TILE_M, BN, k, k), (kb | k) != 0 ? 1u : 0u, sf_tmem + SFA_COL,
-                                      sf_tmem + SFB_COL + sfb_shift);
-            else tc_mma_mxf8(tmem_d, da, db, make_idesc_mxf8(TILE_M, BN, k, k), (kb | k) != 0 ? 1u : 0u, sf_tmem + SFA_COL,
-                             sf_tmem + SFB_COL + sfb_shift);
+              tc_mma_nvf4(tmem_d, da, db, make_idesc_nvf4(TILE_M, BN), (kb | k) != 0 ? 1u : 0u, sfa_tmem + 4 * k,
+                          sfb_tmem + 4 * L::NATOM * k + sfb_shift);
+            else if (TWO) tc_mma_mxf8_pair(tmem_d, da, db, make_idesc_mxf8(TILE_M, BN, k, k), (kb | k) != 0 ? 1u : 0u, sfa_tmem,
+                                      sfb_tmem + sfb_shift);
+            else tc_mma_mxf8(tmem_d, da, db, make_idesc_mxf8(TILE_M, BN, k, k), (kb | k) != 0 ? 1u : 0u, sfa_tmem,
+                             sfb_tmem + sfb_shift);
           }
           if (TWO) tc_commit_pair(empty_bar(s)); else tc_commit(empty_bar(s));
           }
@@ -336,7 +344,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const int row = m0 + q * 32 + lane;
       const bool row_ok = row < p.M;
       const uint32_t tcol0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * ACC_STRIDE;
-      if (!(fl & ELFA_EPI_BIAS)) {
+      if (SHARED || !(fl & ELFA_EPI_BIAS)) {         // SHARED is not launched with a bias
         // bf16 output (optionally the pre-activation too): 64 accumulator columns at a time through the warp's private 4 KB of shared memory, written as
         // whole 128-byte lines (common.cuh: warp_stage_64cols / warp_flush_64cols)
         const uint32_t stage = smem_u32(smem + L::EPI_OFF) + q * 4096;
@@ -344,11 +352,19 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         __nv_bfloat16* cbase = p.C + (long long)row0 * p.ldc + n0;
         const int rows_valid = p.M - row0;
         uint32_t ra[32], rb[32];
-        tmem_ld32(tcol0, ra);
-        tmem_ld32(tcol0 + 32, rb);
+        // SHARED: from the end that the next tile's accumulator overlaps
+        auto chunk = [&](int c) { return SHARED && buf == 0 ? BN / 32 - 2 - c : c; };
+        tmem_ld32(tcol0 + chunk(0) * 32, ra);
+        tmem_ld32(tcol0 + (chunk(0) + 1) * 32, rb);
 #pragma unroll
-        for (int c = 0; c < BN / 32; c += 2) {
+        for (int i = 0; i < BN / 32; i += 2) {
+          const int c = chunk(i);
           tmem_ld_wait();
+          if (SHARED && i == 0) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(over_bar, 0));
+          }
           if (fl & ELFA_EPI_STORE_PREACT) {
             warp_stage_64cols(stage, ra, rb, alpha, lane);
             __syncwarp();
@@ -357,9 +373,9 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           }
           if (fl & ELFA_EPI_GELU) warp_stage_64cols<true>(stage, ra, rb, alpha, lane);
           else warp_stage_64cols(stage, ra, rb, alpha, lane);
-          if (c + 2 < BN / 32) {
-            tmem_ld32(tcol0 + (c + 2) * 32, ra);
-            tmem_ld32(tcol0 + (c + 3) * 32, rb);
+          if (i + 2 < BN / 32) {
+            tmem_ld32(tcol0 + chunk(i + 2) * 32, ra);
+            tmem_ld32(tcol0 + (chunk(i + 2) + 1) * 32, rb);
           }
           __syncwarp();
           warp_flush_64cols(stage, cbase + c * 32, p.ldc, rows_valid, p.N - n0 - c * 32, lane);
@@ -486,6 +502,13 @@ int launch_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& 
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;
+}
+
+// Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile
+bool wide_pair(int M, int N, int K) {
+  const long long pairs = device_sm_count() / 2, tm = (M + 255) / 256, kt = (K + QBK - 1) / QBK;
+  const long long r256 = (tm * ((N + 255) / 256) + pairs - 1) / pairs, r192 = (tm * ((N + 191) / 192) + pairs - 1) / pairs;
+  return r256 * (632 * kt + 700) < r192 * (566 * kt);
 }
 
 // Tensor map over a scale tensor viewed as [atoms, 128] 32-bit words, box = `box_atoms` rows. Small cache:
@@ -681,12 +704,14 @@ ELFA_API int elfa_gemm_mxfp8(const void* A, const void* sfa, const void* B, cons
                "gemm_mxfp8: scale tensors must be 16-byte aligned");
   unsigned int* st = status_word();
   ELFA_REQUIRE(st != nullptr, "gemm_mxfp8: no status word");
-  // force_bn: 128 / 192 single-CTA tiles, 384 = CTA pairs on 256 x 192 tiles (the default for problems that fill at
+  // force_bn: 128 / 192 single-CTA tiles, 384 / 512 = CTA pairs on 256 x 192 / 256 x 256 tiles (the default for problems that fill at
   // least one wave of pairs). A 256 x 224 pair tile was tried and raised a misaligned-address fault on multi-tile
   // problems; it is not instantiated.
-  const bool pair = force_bn == 384 ||
+  ELFA_REQUIRE(force_bn != 512 || !(flags & ELFA_EPI_BIAS), "gemm_mxfp8: the 256-wide tile takes no bias");
+  const bool pair = force_bn == 384 || force_bn == 512 ||
                     (force_bn == 0 && N > 128 && (long long)((M + 255) / 256) * ((N + 191) / 192) >= device_sm_count() / 2);
-  const int BN = pair ? 192 : ((force_bn == 128 || force_bn == 192) ? force_bn : (N <= 128 ? 128 : 192));
+  const bool wide = force_bn == 512 || (force_bn == 0 && pair && !(flags & ELFA_EPI_BIAS) && wide_pair(M, N, K));
+  const int BN = pair ? (wide ? 256 : 192) : ((force_bn == 128 || force_bn == 192) ? force_bn : (N <= 128 ? 128 : 192));
   CUtensorMap tmA, tmB;
   int rc = shared_tmap(&tmA, A, 1, (uint64_t)M, (uint64_t)K, (uint64_t)K, QBM, QBK);
   if (rc != ELFA_OK) return rc;
@@ -694,7 +719,7 @@ ELFA_API int elfa_gemm_mxfp8(const void* A, const void* sfa, const void* B, cons
   if (rc != ELFA_OK) return rc;
   // scale tensors as [atoms, 128] 32-bit words; one box = the atoms of one tile and K tile
   const int kt = (K + QBK - 1) / QBK;
-  const int natom_b = BN <= 128 ? 1 : (BN <= 192 ? 2 : 3);
+  const int natom_b = BN <= 128 ? 1 : 2;
   CUtensorMap tmSFA, tmSFB;
   rc = sf_tmap(&tmSFA, sfa, (uint64_t)((M + 127) / 128) * kt, 1);
   if (rc != ELFA_OK) return rc;
@@ -714,6 +739,7 @@ ELFA_API int elfa_gemm_mxfp8(const void* A, const void* sfa, const void* B, cons
   p.flags = flags;
   p.status = st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (wide) return launch_q<256, 6, true>(tmA, tmB, tmSFA, tmSFB, p, s);
   if (pair) return launch_q<192, 7, true>(tmA, tmB, tmSFA, tmSFB, p, s);
   if (BN == 192) return launch_q<192, 5, false>(tmA, tmB, tmSFA, tmSFB, p, s);
   return launch_q<128, 6, false>(tmA, tmB, tmSFA, tmSFB, p, s);
