@@ -22,6 +22,8 @@
 // now, state gradient 98 against 92 at B 8, T 2048, 16 heads of 64.) Gradients of such tokens are not finite; whether infinity or NaN is not kept.
 //
 // reference: kernels/cuda/efla.cu:121-271,534-552 (chunks are scanned one after the other, the bf16 state in global memory).
+#include <algorithm>
+
 #include "common.cuh"
 #include "elfa_native.h"
 #include "mma_sync.cuh"
@@ -174,7 +176,7 @@ struct EflaStage {                         // byte offsets inside one stage of t
   static constexpr int K = 0, V = K + EC * KLD * 2, N = V + EC * VLD * 2, C = N + 3 * EC * EN_LD * 2, BYTES = C + 2 * EC * 4;
 };
 
-template <int D>
+template <int D, bool CUT>
 __device__ __forceinline__ void efla_stage_load(uint32_t st, const __nv_bfloat16* __restrict__ kb, const __nv_bfloat16* __restrict__ vb,
                                                 const __nv_bfloat16* __restrict__ nm, const float* __restrict__ cf, long long row_stride,
                                                 int n) {
@@ -184,9 +186,10 @@ __device__ __forceinline__ void efla_stage_load(uint32_t st, const __nv_bfloat16
     const int r = i / (D / 8), c = i % (D / 8);
     cp_async16(st + L::K + (r * L::KLD + c * 8) * 2, kb + (r < n ? r : 0) * row_stride + c * 8, r < n);
   }
-  for (int i = threadIdx.x; i < EC * (L::VC / 8); i += NT) {
+  for (int i = threadIdx.x; i < EC * (L::VC / 8); i += NT) {           // CUT: without values zeros
     const int r = i / (L::VC / 8), c = i % (L::VC / 8);
-    cp_async16(st + L::V + (r * L::VLD + c * 8) * 2, vb + (r < n ? r : 0) * row_stride + c * 8, r < n);
+    const bool has = !CUT || vb;
+    cp_async16(st + L::V + (r * L::VLD + c * 8) * 2, has ? vb + (r < n ? r : 0) * row_stride + c * 8 : kb, has && r < n);
   }
   for (int i = threadIdx.x; i < 3 * EC * 4; i += NT)
     cp_async16(st + L::N + ((i / 4) * EN_LD + (i % 4) * 8) * 2, nm + i * 8, true);
@@ -459,25 +462,33 @@ __device__ __forceinline__ long long efla_state_slot(long long chunk_id, int vbl
   return ((chunk_id * (D / 16) + vblock) * (D / 8)) * 32 + lane;      // float4 units; tile n at + 32 n
 }
 
-// Grid (B * H, d / columns of a CTA). k, v, o: [B, T, H, d] bf16. state0 / state_out: [B, H, d, d] fp32 or null. ckpt (or null):
-// the state at the start of every chunk.
+// A walk over the chunks [c0, c1) of one head. state0: null (zero) or the head's [d, d] start; identity: start from the identity instead.
+// With vals = outs = null and ckpt = null only the state is walked; state_out (or null) gets the last one.
+struct EflaWalk {
+  int c0, c1;
+  bool identity;
+  const float* state0;
+  float* state_out;
+};
+
+// k, v, o: [B, T, H, d] bf16; v and o may be null (see EflaWalk). ckpt (or null): the state at the start of every chunk.
 // Bound by the dependent chain of a chunk (132 mma.sync and about 880 instructions of one warp per scheduler), not by memory. With the
-// preparation, B 1, T 8192, 16 heads of 64, no gradient: 354 us, token by token (with its checkpoints) 2364 us; in the training step of
-// B 8, T 2048 the forward went from about 750 to 94 us and 28 us for the preparation.
-template <int D, bool CHECKED>
+// preparation, B 1, T 8192, 16 heads of 64, no gradient: 354 us in one walk, token by token (with its checkpoints) 2364 us; in the training step
+// of B 8, T 2048 the forward went from about 750 to 94 us and 28 us for the preparation.
+template <int D, bool CHECKED, bool CUT>
 __device__ __forceinline__ bool efla_fwd_walk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ nmat,
-    const float* __restrict__ coef, const float* __restrict__ state0, __nv_bfloat16* __restrict__ o, float* __restrict__ state_out,
-    float4* __restrict__ ckpt, int T, int H, int nchunks) {
+    const float* __restrict__ coef, __nv_bfloat16* __restrict__ o, float4* __restrict__ ckpt, int T, int H, int nchunks, EflaWalk w) {
   using L = EflaStage<D>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int bh = blockIdx.x, b = bh / H, h = bh % H;
   const int ccol = blockIdx.y * L::VC, wcol = ccol + warp * 16;       // first value column of the CTA / of this warp
   const uint32_t ring = smem_u32(smem);
+  const int c0 = CUT ? w.c0 : 0, c1 = CUT ? w.c1 : nchunks;
   __nv_bfloat16* stage_o = reinterpret_cast<__nv_bfloat16*>(smem + EC_STAGES * L::BYTES) + warp * EC * 24;   // [32 tokens][16 + 8]
   const long long row0 = ((long long)b * T * H + h) * D, rs = (long long)H * D;
-  const __nv_bfloat16 *kb = k + row0, *vb = v + row0 + ccol;
+  const __nv_bfloat16 *kb = k + row0, *vb = !CUT || v ? v + row0 + ccol : nullptr;
   const __nv_bfloat16* nb = nmat + (long long)bh * nchunks * EN_ELEMS;
   const float* cb = coef + (long long)bh * nchunks * EC_COEF;
 
@@ -486,17 +497,20 @@ __device__ __forceinline__ bool efla_fwd_walk(
   for (int n = 0; n < D / 8; ++n)
 #pragma unroll
     for (int x = 0; x < 4; ++x)
-      S[n][x] = state0 ? state0[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] : 0.f;
+    {
+      const int row = n * 8 + 2 * q + (x & 1), col = wcol + g + (x >> 1) * 8;
+      S[n][x] = CUT && w.identity ? (row == col ? 1.f : 0.f) : (w.state0 ? w.state0[row * D + col] : 0.f);
+    }
 
   auto fetch = [&](int ch) {
-    if (ch < nchunks)
-      efla_stage_load<D>(ring + (ch % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, vb + (long long)ch * EC * rs,
+    if (ch < c1)
+      efla_stage_load<D, CUT>(ring + (ch % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, !CUT || vb ? vb + (long long)ch * EC * rs : nullptr,
                          nb + (long long)ch * EN_ELEMS, cb + (long long)ch * EC_COEF, rs, min(EC, T - ch * EC));
     cp_async_commit();
   };
 #pragma unroll
-  for (int i = 0; i < EC_STAGES - 1; ++i) fetch(i);
-  for (int ch = 0; ch < nchunks; ++ch) {
+  for (int i = 0; i < EC_STAGES - 1; ++i) fetch(c0 + i);
+  for (int ch = c0; ch < c1; ++ch) {
     cp_async_wait<EC_STAGES - 2>();
     __syncthreads();                       // chunk ch has landed for every thread; the stage of chunk ch - 1 is free
     fetch(ch + EC_STAGES - 1);
@@ -543,11 +557,13 @@ __device__ __forceinline__ bool efla_fwd_walk(
           if (first[x >> 1] < EC) e[nt][x] = 0.f;                     // the walk below moves these columns
     }
     efla_state_update<D, false>(S, e, st + L::K, lane);
-    const uint32_t so = smem_u32(stage_o);
-    __syncwarp();
+    if (!CUT || o) {
+      const uint32_t so = smem_u32(stage_o);
+      __syncwarp();
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf) stsm4_t(so + (lane * 24 + hf * 8) * 2, oq[hf][0], oq[hf][1], oq[hf][2], oq[hf][3]);
-    __syncwarp();
+      for (int hf = 0; hf < 2; ++hf) stsm4_t(so + (lane * 24 + hf * 8) * 2, oq[hf][0], oq[hf][1], oq[hf][2], oq[hf][3]);
+      __syncwarp();
+    }
     if (bad) {
       const unsigned char* sst = smem + (ch % EC_STAGES) * L::BYTES;
       float sl[D / 2];
@@ -563,41 +579,151 @@ __device__ __forceinline__ bool efla_fwd_walk(
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int t = u * 16 + (lane >> 1), hf = lane & 1;
-      if (ch * EC + t < T)
+      if ((!CUT || o) && ch * EC + t < T)
         *reinterpret_cast<uint4*>(o + row0 + ((long long)ch * EC + t) * rs + wcol + hf * 8) = *reinterpret_cast<const uint4*>(stage_o + t * 24 + hf * 8);
     }
   }
   cp_async_wait<0>();
-  if (state_out) {
+  if (w.state_out) {
 #pragma unroll
     for (int n = 0; n < D / 8; ++n)
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-        state_out[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] = S[n][x];
+      for (int x = 0; x < 4; ++x) w.state_out[(n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] = S[n][x];
   }
   // an error that was not finite anywhere has left its state column not finite (mma.sync: also 0 x NaN)
   return efla_not_finite<D>(S);
 }
 
+template <int D, bool CUT>
+__device__ __noinline__ void efla_fwd_again(const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* nmat, const float* coef,
+                                            __nv_bfloat16* o, float4* ckpt, int T, int H, int nchunks, EflaWalk w) {
+  efla_fwd_walk<D, true, CUT>(k, v, nmat, coef, o, ckpt, T, H, nchunks, w);
+}
+
+// Segments. A walk of n chunks is cut into P segments of `seg` chunks, since a chunk's update is affine in the state (S1 = A S0 + B):
+//   FIRST  segment 0 from its known start, with its outputs; segments 1 .. P - 2 from zero (their B) and, without values, from the identity
+//          (their A), states only: 2 P - 3 walks per head side by side
+//   (efla_combine_kernel: start of segment p + 1 = A_p start_p + B_p)
+//   REST   segments 1 .. P - 1 from their starts, with their outputs
+// The walk in one piece is compiled apart (CUT = false): asking for what may be absent in it cost 5 us of 94.
+// Three times the work in 2 / P of the steps: worth it where the heads alone leave the chip idle (see efla_segments). The maps contract (the
+// eigenvalues of a token's factor lie in (0, 1]), so an error of a start dies out along its segment.
+// work: start [P], A [P], B [P], each [B H, d, d] fp32.
+enum { EFLA_FIRST, EFLA_REST };
+
+__device__ __forceinline__ float* efla_work(float* work, int which, int P, int p, int bh, int dd) {
+  return work + (((long long)which * P + p) * gridDim.x + bh) * dd;
+}
+
+// Grid (B * H, d / columns of a CTA, walks). state0 / state_out: [B, H, d, d] fp32 or null.
+template <int D, bool CUT>
+__global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
+    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ nmat,
+    const float* __restrict__ coef, const float* state0, __nv_bfloat16* __restrict__ o, float* state_out,
+    float4* __restrict__ ckpt, float* work, int T, int H, int nchunks, int P, int seg, int phase) {
+  const int bh = blockIdx.x, z = blockIdx.z;
+  EflaWalk w{0, nchunks, false, state0 ? state0 + (long long)bh * D * D : nullptr, state_out ? state_out + (long long)bh * D * D : nullptr};
+  if (CUT) {
+    const bool map = phase == EFLA_FIRST && z > 0;                       // a segment's A or B
+    const int p = phase == EFLA_REST ? z + 1 : (z > P - 2 ? z - (P - 2) : z);
+    w.c0 = p * seg;
+    w.c1 = min(nchunks, w.c0 + seg);
+    if (map) {
+      w.identity = z > P - 2;
+      w.state0 = nullptr;
+      w.state_out = efla_work(work, w.identity ? 1 : 2, P, p, bh, D * D);
+      if (w.identity) v = nullptr;
+      o = nullptr;
+      ckpt = nullptr;
+    } else {
+      if (p > 0) w.state0 = efla_work(work, 0, P, p, bh, D * D);
+      if (p < P - 1) w.state_out = p == 0 ? efla_work(work, 0, P, 1, bh, D * D) : nullptr;
+    }
+  }
+  if (__syncthreads_or(efla_fwd_walk<D, false, CUT>(k, v, nmat, coef, o, ckpt, T, H, nchunks, w)))
+    efla_fwd_again<D, CUT>(k, v, nmat, coef, o, ckpt, T, H, nchunks, w);
+}
+
+// start[p + dir] = A[p] start[p] + B[p] for the P - 2 inner segments, in order; a CTA owns 16 columns of a head, a thread D / 16 rows of one
+// column. The next A is on its way while this one is used. fp32 sums in four parts of D / 4: the errors that this adds to a start stay below
+// those of the walks (64-bit comparison, B 1, T 8192, 16 heads of 64, 10
+// segments: final state as in one walk). Grid (B * H, d / 16).
 template <int D>
-__device__ __noinline__ void efla_fwd_again(
-    const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* nmat, const float* coef, const float* state0, __nv_bfloat16* o,
-    float* state_out, float4* ckpt, int T, int H, int nchunks) {
-  efla_fwd_walk<D, true>(k, v, nmat, coef, state0, o, state_out, ckpt, T, H, nchunks);
+__global__ void __launch_bounds__(256) efla_combine_kernel(float* __restrict__ work, int P, int dir) {
+  constexpr int EPT = D / 16, DD = D * D, LD = D + 4, VPT = DD / 1024;       // 16-byte vectors of A per thread
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* sa = reinterpret_cast<float*>(smem);
+  float(*ss)[17] = reinterpret_cast<float(*)[17]>(smem + D * LD * 4);
+  const int bh = blockIdx.x, col = threadIdx.x & 15, r0 = (threadIdx.x >> 4) * EPT, c = blockIdx.y * 16 + col;
+  int p = dir > 0 ? 1 : P - 2;
+  const float* s0 = efla_work(work, 0, P, p, bh, DD);
+  float4 nxt[VPT];
+  float bn[EPT];
+  auto fetch = [&](int at) {
+    const float4* a = reinterpret_cast<const float4*>(efla_work(work, 1, P, at, bh, DD));
+    const float* bb = efla_work(work, 2, P, at, bh, DD);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) nxt[i] = a[threadIdx.x + i * 256];
+#pragma unroll
+    for (int i = 0; i < EPT; ++i) bn[i] = bb[(r0 + i) * D + c];
+  };
+  fetch(p);
+#pragma unroll
+  for (int i = 0; i < EPT; ++i) ss[r0 + i][col] = s0[(r0 + i) * D + c];
+  for (int n = 0; n < P - 2; ++n, p += dir) {
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int at = (threadIdx.x + i * 256) * 4;
+      *reinterpret_cast<float4*>(sa + at / D * LD + at % D) = nxt[i];
+    }
+    float sum[EPT];
+#pragma unroll
+    for (int i = 0; i < EPT; ++i) sum[i] = bn[i];
+    __syncthreads();
+    if (n + 1 < P - 2) fetch(p + dir);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float acc[EPT];
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) acc[i] = 0.f;
+#pragma unroll 2
+      for (int j = q * (D / 4); j < (q + 1) * (D / 4); j += 4) {
+        float x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = ss[j + u][col];
+#pragma unroll
+        for (int i = 0; i < EPT; ++i) {
+          const float4 a = *reinterpret_cast<const float4*>(sa + (r0 + i) * LD + j);
+          acc[i] += a.x * x[0] + a.y * x[1] + (a.z * x[2] + a.w * x[3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) sum[i] += acc[i];
+    }
+    __syncthreads();
+    float* out = efla_work(work, 0, P, p + dir, bh, DD);
+#pragma unroll
+    for (int i = 0; i < EPT; ++i) {
+      out[(r0 + i) * D + c] = sum[i];
+      ss[r0 + i][col] = sum[i];
+    }
+  }
 }
 
 template <int D>
-__global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
-    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ nmat,
-    const float* __restrict__ coef, const float* __restrict__ state0, __nv_bfloat16* __restrict__ o, float* __restrict__ state_out,
-    float4* __restrict__ ckpt, int T, int H, int nchunks) {
-  if (__syncthreads_or(efla_fwd_walk<D, false>(k, v, nmat, coef, state0, o, state_out, ckpt, T, H, nchunks)))
-    efla_fwd_again<D>(k, v, nmat, coef, state0, o, state_out, ckpt, T, H, nchunks);
+int launch_combine(float* work, int BH, int P, int dir, cudaStream_t s) {
+  if (P < 3) return ELFA_OK;
+  constexpr int bytes = (D * (D + 4) + D * 17) * 4;
+  ELFA_CUDA(cudaFuncSetAttribute(efla_combine_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  efla_combine_kernel<D><<<dim3(BH, D / 16), 256, bytes, s>>>(work, P, dir);
+  ELFA_CUDA(cudaGetLastError());
+  ::elfa::count_launches(1);
+  return ELFA_OK;
 }
 
 template <int D>
 int launch_chunk_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out, float* ckpt,
-                     void* nmat, float* coef, int B, int T, int H, cudaStream_t s) {
+                     void* nmat, float* coef, float* work, int P, int B, int T, int H, cudaStream_t s) {
   using L = EflaStage<D>;
   const int nchunks = (T + EC - 1) / EC;
   const long long total = (long long)B * H * nchunks;
@@ -606,12 +732,30 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
                                                                  coef, T, H, nchunks, total);
   ELFA_CUDA(cudaGetLastError());
   constexpr int bytes = EC_STAGES * L::BYTES + ec_warps<D>() * EC * 24 * 2;
-  ELFA_CUDA(cudaFuncSetAttribute(efla_chunk_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  efla_chunk_fwd_kernel<D><<<dim3(B * H, D / L::VC), 32 * ec_warps<D>(), bytes, s>>>(
-      static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), static_cast<const __nv_bfloat16*>(nmat), coef, state0,
-      static_cast<__nv_bfloat16*>(o), state_out, reinterpret_cast<float4*>(ckpt), T, H, nchunks);
+  int seg = nchunks;
+  if (P > 1) {
+    seg = (nchunks + P - 1) / P;
+    P = (nchunks + seg - 1) / seg;
+  }
+  auto kernel = P > 1 ? efla_chunk_fwd_kernel<D, true> : efla_chunk_fwd_kernel<D, false>;
+  ELFA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  auto walk = [&](int phase, int walks) {
+    kernel<<<dim3(B * H, D / L::VC, walks), 32 * ec_warps<D>(), bytes, s>>>(
+        static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), static_cast<const __nv_bfloat16*>(nmat), coef, state0,
+        static_cast<__nv_bfloat16*>(o), state_out, reinterpret_cast<float4*>(ckpt), work, T, H, nchunks, P, seg, phase);
+    ::elfa::count_launches(1);
+  };
+  ::elfa::count_launches(1);
+  if (P <= 1) {
+    walk(EFLA_FIRST, 1);
+  } else {
+    walk(EFLA_FIRST, 2 * P - 3);
+    ELFA_CUDA(cudaGetLastError());
+    const int rc = launch_combine<D>(work, B * H, P, 1, s);
+    if (rc != ELFA_OK) return rc;
+    walk(EFLA_REST, P - 1);
+  }
   ELFA_CUDA(cudaGetLastError());
-  ::elfa::count_launches(2);
   return ELFA_OK;
 }
 
@@ -626,19 +770,19 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
 // B 8, T 2048, 16 heads of 64: 92 us and 253 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
 // finish). The parallel kernel issues about 400 mma.sync per warp and chunk (94 us of tensor time at 8.3 cycles each) and reads 370 MB
 // (55 us); a third CTA per SM, at 168 registers, did not make it faster.
-template <int D, bool CHECKED>
+template <int D, bool CHECKED, bool CUT>
 __device__ __forceinline__ bool efla_bwd_walk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ nmat,
-    const float* __restrict__ coef, const float* __restrict__ dstate_out, float4* __restrict__ dckpt, float* __restrict__ dstate0, int T,
-    int H, int nchunks) {
+    const float* __restrict__ coef, float4* __restrict__ dckpt, int T, int H, int nchunks, EflaWalk w) {
   using L = EflaStage<D>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int bh = blockIdx.x, b = bh / H, h = bh % H;
   const int ccol = blockIdx.y * L::VC, wcol = ccol + warp * 16;
   const uint32_t ring = smem_u32(smem);
+  const int c0 = CUT ? w.c0 : 0, c1 = CUT ? w.c1 : nchunks;
   const long long row0 = ((long long)b * T * H + h) * D, rs = (long long)H * D;
-  const __nv_bfloat16 *kb = k + row0, *ob = dout + row0 + ccol;
+  const __nv_bfloat16 *kb = k + row0, *ob = !CUT || dout ? dout + row0 + ccol : nullptr;
   const __nv_bfloat16* nb = nmat + (long long)bh * nchunks * EN_ELEMS;
   const float* cb = coef + (long long)bh * nchunks * EC_COEF;
 
@@ -647,26 +791,31 @@ __device__ __forceinline__ bool efla_bwd_walk(
   for (int n = 0; n < D / 8; ++n)
 #pragma unroll
     for (int x = 0; x < 4; ++x)
-      S[n][x] = dstate_out ? dstate_out[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] : 0.f;
+    {
+      const int row = n * 8 + 2 * q + (x & 1), col = wcol + g + (x >> 1) * 8;
+      S[n][x] = CUT && w.identity ? (row == col ? 1.f : 0.f) : (w.state0 ? w.state0[row * D + col] : 0.f);
+    }
 
   auto fetch = [&](int i) {                // i-th chunk from the end
-    const int ch = nchunks - 1 - i;
-    if (ch >= 0)
-      efla_stage_load<D>(ring + (i % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, ob + (long long)ch * EC * rs,
+    const int ch = c1 - 1 - i;
+    if (ch >= c0)
+      efla_stage_load<D, CUT>(ring + (i % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, !CUT || ob ? ob + (long long)ch * EC * rs : nullptr,
                          nb + (long long)ch * EN_ELEMS, cb + (long long)ch * EC_COEF, rs, min(EC, T - ch * EC));
     cp_async_commit();
   };
 #pragma unroll
   for (int i = 0; i < EC_STAGES - 1; ++i) fetch(i);
-  for (int i = 0; i < nchunks; ++i) {
+  for (int i = 0; i < c1 - c0; ++i) {
     cp_async_wait<EC_STAGES - 2>();
     __syncthreads();
     fetch(i + EC_STAGES - 1);
     const uint32_t st = ring + (i % EC_STAGES) * L::BYTES;
     const float* cf = reinterpret_cast<const float*>(smem + (i % EC_STAGES) * L::BYTES + L::C);
-    float4* dst = dckpt + efla_state_slot<D>((long long)bh * nchunks + nchunks - 1 - i, wcol / 16, lane);
+    if (!CUT || dckpt) {
+      float4* dst = dckpt + efla_state_slot<D>((long long)bh * nchunks + c1 - 1 - i, wcol / 16, lane);
 #pragma unroll
-    for (int n = 0; n < D / 8; ++n) dst[n * 32] = make_float4(S[n][0], S[n][1], S[n][2], S[n][3]);
+      for (int n = 0; n < D / 8; ++n) dst[n * 32] = make_float4(S[n][0], S[n][1], S[n][2], S[n][3]);
+    }
     float e[4][4];
     efla_state_times_k<D>(e, S, st + L::K, lane);
     uint32_t oq[2][4];
@@ -692,35 +841,54 @@ __device__ __forceinline__ bool efla_bwd_walk(
       const unsigned char* sst = smem + (i % EC_STAGES) * L::BYTES;
       efla_walk_back<D, L::KLD, L::VLD>(sl, unused, reinterpret_cast<const __nv_bfloat16*>(sst + L::K),
                                         reinterpret_cast<const __nv_bfloat16*>(sst + L::V) + warp * 16, cf,
-                                        min(EC, T - (nchunks - 1 - i) * EC));
+                                        min(EC, T - (c1 - 1 - i) * EC));
 #pragma unroll
       for (int n = 0; n < D / 2; ++n) S[n / 4][n % 4] = sl[n];
     }
   }
   cp_async_wait<0>();
-  if (dstate0) {
+  if (w.state_out) {
 #pragma unroll
     for (int n = 0; n < D / 8; ++n)
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-        dstate0[((long long)bh * D + n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] = S[n][x];
+      for (int x = 0; x < 4; ++x) w.state_out[(n * 8 + 2 * q + (x & 1)) * D + wcol + g + (x >> 1) * 8] = S[n][x];
   }
   return efla_not_finite<D>(S);
 }
 
-template <int D>
+template <int D, bool CUT>
 __device__ __noinline__ void efla_bwd_again(const __nv_bfloat16* k, const __nv_bfloat16* dout, const __nv_bfloat16* nmat, const float* coef,
-                                            const float* dstate_out, float4* dckpt, float* dstate0, int T, int H, int nchunks) {
-  efla_bwd_walk<D, true>(k, dout, nmat, coef, dstate_out, dckpt, dstate0, T, H, nchunks);
+                                            float4* dckpt, int T, int H, int nchunks, EflaWalk w) {
+  efla_bwd_walk<D, true, CUT>(k, dout, nmat, coef, dckpt, T, H, nchunks, w);
 }
 
-template <int D>
+// Segments as in the forward kernel, from the last one to the first: FIRST walks the last segment from dstate_out and the inner ones from zero
+// and (without dO) from the identity, which gives the transposed maps.
+template <int D, bool CUT>
 __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_bwd_state_kernel(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ nmat,
-    const float* __restrict__ coef, const float* __restrict__ dstate_out, float4* __restrict__ dckpt, float* __restrict__ dstate0, int T,
-    int H, int nchunks) {
-  if (__syncthreads_or(efla_bwd_walk<D, false>(k, dout, nmat, coef, dstate_out, dckpt, dstate0, T, H, nchunks)))
-    efla_bwd_again<D>(k, dout, nmat, coef, dstate_out, dckpt, dstate0, T, H, nchunks);
+    const float* __restrict__ coef, const float* dstate_out, float4* __restrict__ dckpt, float* dstate0, float* work, int T, int H,
+    int nchunks, int P, int seg, int phase) {
+  const int bh = blockIdx.x, z = blockIdx.z;
+  EflaWalk w{0, nchunks, false, dstate_out ? dstate_out + (long long)bh * D * D : nullptr, dstate0 ? dstate0 + (long long)bh * D * D : nullptr};
+  if (CUT) {
+    const bool map = phase == EFLA_FIRST && z > 0;
+    const int p = phase == EFLA_REST ? z : (z == 0 ? P - 1 : (z > P - 2 ? z - (P - 2) : z));
+    w.c0 = p * seg;
+    w.c1 = min(nchunks, w.c0 + seg);
+    if (map) {
+      w.identity = z > P - 2;
+      w.state0 = nullptr;
+      w.state_out = efla_work(work, w.identity ? 1 : 2, P, p, bh, D * D);
+      if (w.identity) dout = nullptr;
+      dckpt = nullptr;
+    } else {
+      if (p < P - 1) w.state0 = efla_work(work, 0, P, p, bh, D * D);
+      if (p > 0) w.state_out = p == P - 1 ? efla_work(work, 0, P, P - 2, bh, D * D) : nullptr;
+    }
+  }
+  if (__syncthreads_or(efla_bwd_walk<D, false, CUT>(k, dout, nmat, coef, dckpt, T, H, nchunks, w)))
+    efla_bwd_again<D, CUT>(k, dout, nmat, coef, dckpt, T, H, nchunks, w);
 }
 
 // One CTA per chunk, d / 16 warps; warp w owns value columns 16 w .. 16 w + 15 and all key rows. E, Y, dE0 are recomputed from the
@@ -1131,8 +1299,8 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
 
 template <int D>
 int launch_chunk_bwd(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt,
-                     const void* dout, const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0, float* dckpt, int B,
-                     int T, int H, cudaStream_t s) {
+                     const void* dout, const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0, float* dckpt,
+                     float* work, int P, int B, int T, int H, cudaStream_t s) {
   using L = EflaStage<D>;
   using M = EflaBwdSmem<D>;
   const int nchunks = (T + EC - 1) / EC;
@@ -1142,16 +1310,34 @@ int launch_chunk_bwd(const void* k, const void* v, const void* nmat, const float
   const auto* K = static_cast<const __nv_bfloat16*>(k);
   const auto* O = static_cast<const __nv_bfloat16*>(dout);
   const auto* N = static_cast<const __nv_bfloat16*>(nmat);
-  ELFA_CUDA(cudaFuncSetAttribute(efla_chunk_bwd_state_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes1));
   ELFA_CUDA(cudaFuncSetAttribute(efla_chunk_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::BYTES));
-  efla_chunk_bwd_state_kernel<D><<<dim3(B * H, D / L::VC), 32 * ec_warps<D>(), bytes1, s>>>(
-      K, O, N, coef, dstate_out, reinterpret_cast<float4*>(dckpt), dstate0, T, H, nchunks);
+  int seg = nchunks;
+  if (P > 1) {
+    seg = (nchunks + P - 1) / P;
+    P = (nchunks + seg - 1) / seg;
+  }
+  auto kernel = P > 1 ? efla_chunk_bwd_state_kernel<D, true> : efla_chunk_bwd_state_kernel<D, false>;
+  ELFA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes1));
+  auto walk = [&](int phase, int walks) {
+    kernel<<<dim3(B * H, D / L::VC, walks), 32 * ec_warps<D>(), bytes1, s>>>(
+        K, O, N, coef, dstate_out, reinterpret_cast<float4*>(dckpt), dstate0, work, T, H, nchunks, P, seg, phase);
+    ::elfa::count_launches(1);
+  };
+  if (P <= 1) {
+    walk(EFLA_FIRST, 1);
+  } else {
+    walk(EFLA_FIRST, 2 * P - 3);
+    ELFA_CUDA(cudaGetLastError());
+    const int rc = launch_combine<D>(work, B * H, P, -1, s);
+    if (rc != ELFA_OK) return rc;
+    walk(EFLA_REST, P - 1);
+  }
   ELFA_CUDA(cudaGetLastError());
   efla_chunk_bwd_kernel<D><<<(unsigned)total, 2 * D, M::BYTES, s>>>(
       K, static_cast<const __nv_bfloat16*>(v), O, N, coef, reinterpret_cast<const float4*>(ckpt),
       reinterpret_cast<const float4*>(dckpt), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), dbeta_tok, T, H, nchunks);
   ELFA_CUDA(cudaGetLastError());
-  ::elfa::count_launches(2);
+  ::elfa::count_launches(1);
   return ELFA_OK;
 }
 
@@ -1162,19 +1348,50 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 using namespace elfa;
 
+// How many segments a walk over T tokens is cut into (1: none), and with them how large `work` is: 3 * segments * B * H * d * d floats.
+// One walk takes nchunks steps; cut, FIRST takes nchunks / P steps of (2 P - 3) walks per head and column block and REST as many of P - 1. A step
+// costs the latency of a chunk's chain while an SM has one CTA, 1.25 of it with two (its registers hold no third) and whole rounds beyond.
+ELFA_API int elfa_efla_segments(int B, int T, int H, int d) {
+  const int nchunks = (T + EC - 1) / EC, sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  const long long units = (long long)B * H * (d == 128 || d == 96 ? 2 : 1);
+  const double step = d == 128 ? 2.0 : (d == 96 ? 1.6 : 1.4), combine = d == 128 ? 1.8 : 0.9;      // microseconds
+  auto steps = [&](long long walks) {
+    const long long ctas = units * walks, full = ctas / (2 * sms), rest = ctas % (2 * sms);
+    return step * (1.25 * (double)full + (rest == 0 ? 0. : (rest <= sms ? 1. : 1.25)));
+  };
+  double best = nchunks * steps(1);
+  int at = 1;
+  for (int P = 3; P <= 16 && nchunks / P >= 4; ++P) {
+    const int seg = (nchunks + P - 1) / P;
+    const double t = seg * (steps(2 * P - 3) + steps(P - 1)) + 8 + combine * (P - 2);      // two more launches
+    if (t < 0.95 * best) {
+      best = t;
+      at = P;
+    }
+  }
+  return at;
+}
+
 // k, v, o: [B, T, H, d] bf16, 16-byte aligned; beta: 1 float; state0 (optional) / state_out: [B, H, d, d] fp32; ckpt: null or
 // B * H * ceil(T / 32) * d * d floats (chunk-start states in the kernels' own order, needed by backward). nmat: [B * H * ceil(T / 32), 3, 32, 32] bf16 and
 // coef: [B * H * ceil(T / 32), 4, 32] fp32, 16-byte aligned, are written here. No output may share memory with an input (a call may run twice).
 ELFA_API int elfa_efla_chunk_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
                                  float* ckpt, void* nmat, float* coef, int B, int T, int H, int d, void* stream) {
+  return elfa_efla_chunk_fwd_cut(k, v, beta, state0, o, state_out, ckpt, nmat, coef, nullptr, 1, B, T, H, d, stream);
+}
+
+// The same with the walk in `segments` segments (from elfa_efla_segments, or 1 to T / 128), work: 16-byte aligned scratch of that size.
+ELFA_API int elfa_efla_chunk_fwd_cut(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
+                                     float* ckpt, void* nmat, float* coef, float* work, int segments, int B, int T, int H, int d, void* stream) {
   ELFA_REQUIRE(k && v && beta && o && nmat && coef && B > 0 && T > 0 && H > 0, "efla_chunk_fwd: bad arguments");
+  ELFA_REQUIRE(segments >= 1 && segments <= 16 && (segments == 1 || work), "efla_chunk_fwd: bad segments");
   ELFA_REQUIRE(aligned16(k) && aligned16(v) && aligned16(o) && aligned16(nmat) && aligned16(coef), "efla_chunk_fwd: operands must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (d) {
-    case 32: return launch_chunk_fwd<32>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, B, T, H, s);
-    case 64: return launch_chunk_fwd<64>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, B, T, H, s);
-    case 96: return launch_chunk_fwd<96>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, B, T, H, s);
-    case 128: return launch_chunk_fwd<128>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, B, T, H, s);
+    case 32: return launch_chunk_fwd<32>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, work, segments, B, T, H, s);
+    case 64: return launch_chunk_fwd<64>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, work, segments, B, T, H, s);
+    case 96: return launch_chunk_fwd<96>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, work, segments, B, T, H, s);
+    case 128: return launch_chunk_fwd<128>(k, v, beta, state0, o, state_out, ckpt, nmat, coef, work, segments, B, T, H, s);
     default: set_last_error("efla_chunk_fwd: head dimension must be 32, 64, 96 or 128"); return ELFA_ERR_UNSUPPORTED;
   }
 }
@@ -1185,6 +1402,14 @@ ELFA_API int elfa_efla_chunk_fwd(const void* k, const void* v, const float* beta
 ELFA_API int elfa_efla_chunk_bwd(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
                                  const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0,
                                  float* dckpt, int B, int T, int H, int d, void* stream) {
+  return elfa_efla_chunk_bwd_cut(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, nullptr, 1, B, T, H, d, stream);
+}
+
+// The same in segments, see elfa_efla_chunk_fwd_cut.
+ELFA_API int elfa_efla_chunk_bwd_cut(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
+                                     const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0,
+                                     float* dckpt, float* work, int segments, int B, int T, int H, int d, void* stream) {
+  ELFA_REQUIRE(segments >= 1 && segments <= 16 && (segments == 1 || work), "efla_chunk_bwd: bad segments");
   ELFA_REQUIRE(k && v && nmat && coef && ckpt && dout && dk && dv && dbeta_tok && dckpt && B > 0 && T > 0 && H > 0,
                "efla_chunk_bwd: bad arguments");
   ELFA_REQUIRE(aligned16(k) && aligned16(v) && aligned16(nmat) && aligned16(coef) && aligned16(ckpt) && aligned16(dout) && aligned16(dk) &&
@@ -1192,10 +1417,10 @@ ELFA_API int elfa_efla_chunk_bwd(const void* k, const void* v, const void* nmat,
                "efla_chunk_bwd: operands must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (d) {
-    case 32: return launch_chunk_bwd<32>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
-    case 64: return launch_chunk_bwd<64>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
-    case 96: return launch_chunk_bwd<96>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
-    case 128: return launch_chunk_bwd<128>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, B, T, H, s);
+    case 32: return launch_chunk_bwd<32>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, work, segments, B, T, H, s);
+    case 64: return launch_chunk_bwd<64>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, work, segments, B, T, H, s);
+    case 96: return launch_chunk_bwd<96>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, work, segments, B, T, H, s);
+    case 128: return launch_chunk_bwd<128>(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, work, segments, B, T, H, s);
     default: set_last_error("efla_chunk_bwd: head dimension must be 32, 64, 96 or 128"); return ELFA_ERR_UNSUPPORTED;
   }
 }

@@ -209,11 +209,17 @@ int elfa_prism_state(const void* u, const void* v, const void* z, long long ldz,
 int elfa_efla_scan_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
                        int B, int T, int H, int d, void* stream);
 // ---- efla_chunk.cu -----------------------------------------------------------------------------
+int elfa_efla_segments(int B, int T, int H, int d);
 int elfa_efla_chunk_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
                         float* ckpt, void* nmat, float* coef, int B, int T, int H, int d, void* stream);
 int elfa_efla_chunk_bwd(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
                         const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0,
                         float* dckpt, int B, int T, int H, int d, void* stream);
+int elfa_efla_chunk_fwd_cut(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out, float* ckpt,
+                            void* nmat, float* coef, float* work, int segments, int B, int T, int H, int d, void* stream);
+int elfa_efla_chunk_bwd_cut(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
+                            const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0, float* dckpt, float* work,
+                            int segments, int B, int T, int H, int d, void* stream);
 int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, int W, void* stream);
 int elfa_shortconv_bwd_slices(int B, int T, int C, int W);
 int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, float* part, int B, int T, int C,

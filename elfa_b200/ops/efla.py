@@ -111,6 +111,12 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+def _efla_segments(k: torch.Tensor, B: int, T: int, H: int, d: int):
+    """Into how many segments the kernels cut the walk over the chunks, and the scratch that takes (start, map and offset of each)."""
+    n = lib.raw("elfa_efla_segments")(B, T, H, d)
+    return n, torch.empty(3 * n * B * H * d * d, dtype=torch.float32, device=k.device) if n > 1 else None
+
+
 class _EflaScan(torch.autograd.Function):
     """CUDA path. Forward: chunks of 32 tokens on the tensor cores with the fp32 state in registers. Backward: the gradient of
     the state walks the chunks the same way, everything else is parallel over the chunks, from the chunk-boundary states that forward
@@ -131,7 +137,11 @@ class _EflaScan(torch.autograd.Function):
         ckpt = torch.empty(B * H * nchunks * d * d, dtype=torch.float32, device=k.device) if want_grad else None
         nmat = torch.empty((B, H, nchunks, 3, _EFLA_CHUNK, _EFLA_CHUNK), dtype=torch.bfloat16, device=k.device)
         coef = torch.empty((B, H, nchunks, 4, _EFLA_CHUNK), dtype=torch.float32, device=k.device)
-        lib.call("elfa_efla_chunk_fwd", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, B, T, H, d, stream_ptr(kc))
+        cut, work = _efla_segments(kc, B, T, H, d)
+        if cut > 1:
+            lib.call("elfa_efla_chunk_fwd_cut", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, work, cut, B, T, H, d, stream_ptr(kc))
+        else:
+            lib.call("elfa_efla_chunk_fwd", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, B, T, H, d, stream_ptr(kc))
         if want_grad:
             ctx.save_for_backward(kc, vc, ckpt, nmat, coef)
             ctx.cfg = (B, T, H, d, state is not None)
@@ -147,8 +157,12 @@ class _EflaScan(torch.autograd.Function):
         ds0 = torch.empty((B, H, d, d), dtype=torch.float32, device=kc.device) if has_state else None
         dckpt = torch.empty_like(ckpt)
         dso = ds_out.float().contiguous() if ds_out is not None else None
-        lib.call("elfa_efla_chunk_bwd", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt, B, T, H, d,
-                 stream_ptr(kc))
+        cut, work = _efla_segments(kc, B, T, H, d)
+        if cut > 1:
+            lib.call("elfa_efla_chunk_bwd_cut", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt, work, cut, B, T, H, d,
+                     stream_ptr(kc))
+        else:
+            lib.call("elfa_efla_chunk_bwd", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt, B, T, H, d, stream_ptr(kc))
         return dk, dv, dbeta.sum().reshape(1), ds0, None
 
 

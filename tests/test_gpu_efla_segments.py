@@ -1,0 +1,77 @@
+"""The EFLA walk in segments: joined at every kind of boundary, against the token-by-token recurrence.
+
+Bounds: states are fp32 sums; a segment adds the roundings of its start (2^-24 a term) to the errors of its own walk, and the maps contract, so
+1e-5 of the largest value that the state (or its gradient) had on its way covers both forms. That is what it starts from for the gradient, which
+only shrinks where the outputs' gradient is smaller. Outputs and k / v gradients are rounded to bf16 once (2^-8 of the largest).
+"""
+import pytest
+import torch
+
+from elfa_b200 import native
+from elfa_b200.native import lib, stream_ptr
+from elfa_b200.ops import efla as eops
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(dev, B, T, H, d):
+    g = torch.Generator(device=dev).manual_seed(T + d)
+    r = lambda *s, std=1.0: torch.randn(*s, generator=g, device=dev) * std
+    return (r(B, T, H, d, std=0.4).bfloat16(), r(B, T, H, d).bfloat16(), torch.tensor([0.3], device=dev), r(B, H, d, d, std=0.3),
+            r(B, T, H, d).bfloat16(), r(B, H, d, d, std=0.1))
+
+
+def _run(P, k, v, beta, s0, do, ds):
+    """Forward and backward through the native entry points with the walk in P segments."""
+    B, T, H, d = k.shape
+    n = (T + 31) // 32
+    new = lambda *s, dt=torch.float32: torch.empty(*s, dtype=dt, device=k.device)
+    ckpt, dckpt, coef, nmat = new(B * H * n * d * d), new(B * H * n * d * d), new(B, H, n, 4, 32), new(B, H, n, 3, 32, 32, dt=torch.bfloat16)
+    work = new(3 * P * B * H * d * d) if P > 1 else None
+    o, s, dk, dv, ds0, db = torch.empty_like(k), torch.empty_like(s0), torch.empty_like(k), torch.empty_like(k), torch.empty_like(s0), new(B * T * H)
+    lib.call("elfa_efla_chunk_fwd_cut", k, v, beta, s0, o, s, ckpt, nmat, coef, work, P, B, T, H, d, stream_ptr(k))
+    lib.call("elfa_efla_chunk_bwd_cut", k, v, nmat, coef, ckpt, do, ds, dk, dv, db, ds0, dckpt, work, P, B, T, H, d, stream_ptr(k))
+    assert native.status() == 0
+    return o, s, dk, dv, ds0
+
+
+@pytest.mark.parametrize("d", [32, 64, 96, 128])
+@pytest.mark.parametrize("T,P", [(64, 2), (96, 3), (97, 3), (160, 4), (200, 5), (512, 16), (530, 16), (33, 16)])
+def test_segments(cuda_device, d, T, P):
+    ins = _inputs(cuda_device, 2, T, 3, d)
+    got = _run(P, *ins)
+    want = [t.detach().double().requires_grad_(True) for t in ins[:4]]
+    o, s = eops.efla_scan_ref(*want)                                    # fp32 inside
+    ref = [o, s, *torch.autograd.grad([o, s], [want[0], want[1], want[3]], [ins[4].to(o.dtype), ins[5].to(s.dtype)])]
+    for a, b, rel, top in zip(got, ref, (2 ** -8, 1e-5, 2 ** -8, 2 ** -8, 1e-5), (0, 0, 0, 0, ins[5].abs().max())):
+        assert (a.double() - b).abs().max() <= rel * max(b.abs().max(), top)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [0, 70, 128, 255, 256, 511])
+def test_a_bad_value_stays_behind_its_token_and_in_its_column(cuda_device, bad, at):
+    k, v, beta, s0, do, ds = _inputs(cuda_device, 1, 512, 2, 64)
+    clean = _run(4, k, v, beta, s0, do, ds)
+    v[0, at, 0, 5] = bad
+    o, s, _, dv, _ = _run(4, k, v, beta, s0, do, ds)
+    assert not torch.isfinite(o[0, at:, 0, 5]).any() and not torch.isfinite(s[0, 0, :, 5]).any()
+    o[0, at:, 0, 5] = clean[0][0, at:, 0, 5]
+    s[0, 0, :, 5] = clean[1][0, 0, :, 5]
+    assert torch.equal(o, clean[0]) and torch.equal(s, clean[1]) and torch.equal(dv, clean[3])
+    v[0, at, 0, 5] = 1.0
+    clean = _run(4, k, v, beta, s0, do, ds)
+    do[0, at, 0, 5] = bad                                               # backward: its own and earlier tokens
+    _, _, _, dv, ds0 = _run(4, k, v, beta, s0, do, ds)
+    assert not torch.isfinite(dv[0, :at + 1, 0, 5]).any() and not torch.isfinite(ds0[0, 0, :, 5]).any()
+    dv[0, :at + 1, 0, 5] = clean[3][0, :at + 1, 0, 5]
+    ds0[0, 0, :, 5] = clean[4][0, 0, :, 5]
+    # the chunk with the bad value is walked token by token in all columns: other fp32 roundings
+    for a, b, rel in ((dv, clean[3], 2 ** -8), (ds0, clean[4], 1e-5)):
+        assert (a.float() - b.float()).abs().max() <= rel * b.float().abs().max()
+
+
+def test_the_rule_gives_segments_that_fit(cuda_device):
+    for B, T, H, d in ((1, 8192, 16, 64), (2, 1531, 8, 128), (8, 2048, 16, 64), (1, 113, 4, 32), (1, 1, 1, 64), (64, 4096, 16, 64)):
+        n = lib.raw("elfa_efla_segments")(B, T, H, d)
+        assert 1 <= n <= 16 and (n == 1 or (T + 31) // 32 >= 4 * n)
+    assert lib.raw("elfa_efla_segments")(1, 8192, 16, 64) > 1 and lib.raw("elfa_efla_segments")(64, 4096, 16, 64) == 1
