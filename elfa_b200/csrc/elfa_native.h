@@ -225,6 +225,12 @@ int elfa_shortconv_bwd_slices(int B, int T, int C, int W);
 int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, float* part, int B, int T, int C,
                        int W, void* stream);
 
+// ---- stream.cu ---------------------------------------------------------------------------------
+int elfa_gpt_stream_work(const long long* dims);
+int elfa_gpt_stream(const unsigned long long* p, const long long* dims, float eps, void* stream);
+int elfa_efla_stream_work(const long long* dims, int step_tokens);
+int elfa_efla_stream(const unsigned long long* p, const long long* dims, const float* forget, float eps, int step_tokens, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

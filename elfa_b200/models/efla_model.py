@@ -31,6 +31,7 @@ from ..config import Config
 from ..ops import efla as eops
 from ..parallel import tp as tpl
 from ..parallel.mesh import ParallelContext
+from . import streaming
 from .gpt import Norm, _dtype
 
 
@@ -320,6 +321,9 @@ class EflaModel(nn.Module):
         """ids ``[B, T]`` → (logits ``[B, T, V]``, per-layer states) for streaming / generation."""
         if states is None:
             states = self.init_states(ids.shape[0])
+        native = streaming.efla_stream(self, ids, states)
+        if native is not None:
+            return native
         n, states = self.hidden_states(ids, states)
         return self._logits(n, gather=True), states
 

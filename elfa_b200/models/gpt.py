@@ -30,6 +30,7 @@ from ..config import Config
 from ..parallel.mesh import ParallelContext
 from ..parallel import tp as tpl
 from ..quant.qat import QuantSpec
+from . import streaming
 
 
 def _dtype(name: str) -> torch.dtype:
@@ -337,6 +338,9 @@ class GPTModel(nn.Module):
             states = {"pos": 0, "layers": [{"k": None, "v": None} for _ in self.blocks]}
         if states["pos"] + ids.shape[1] > self.max_positions:
             raise ValueError(f"position {states['pos'] + ids.shape[1]} is past the model's {self.max_positions} learned positions")
+        native = streaming.gpt_stream(self, ids, states)
+        if native is not None:
+            return native
         n = self.hidden_states(ids, states["pos"], states["layers"])
         states["pos"] += ids.shape[1]
         head = self.lm_head if self.lm_head is not None else self.embed_tokens

@@ -120,14 +120,17 @@ def attention(qkv: torch.Tensor, causal: bool = True, seq_first: bool = True, sc
     return _Attention.apply(qkv, causal, seq_first, sc, num_heads, doc_start)
 
 
+DECODE_HEAD_DIMS, DECODE_ROWS = (32, 64, 128, 256), 8        # what the kernel is built for: head dimensions, query rows per key head
+
+
 def attention_decode_native(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
     """What :func:`attention_decode` handles: CUDA bf16, no gradient wanted, at most eight query rows per key head, rows of ``q`` / ``k`` /
     ``v`` packed and on 16-byte boundaries."""
     s, B, H, hd = q.shape
     Hkv = k.shape[2]
     ts = (q, k, v, k_cache, v_cache)
-    return (q.is_cuda and all(t.dtype == torch.bfloat16 and t.device == q.device for t in ts) and hd in (32, 64, 128, 256)
-            and H % Hkv == 0 and 0 < s * (H // Hkv) <= 8 and k_cache.shape == v_cache.shape and k_cache.shape[0] > 0
+    return (q.is_cuda and all(t.dtype == torch.bfloat16 and t.device == q.device for t in ts) and hd in DECODE_HEAD_DIMS
+            and H % Hkv == 0 and 0 < s * (H // Hkv) <= DECODE_ROWS and k_cache.shape == v_cache.shape and k_cache.shape[0] > 0
             and k_cache.shape[1:] == (B, Hkv, hd) and k.shape == v.shape == (s, B, Hkv, hd)
             and q.stride()[:2] == k.stride()[:2] == v.stride()[:2]
             and all(t.stride(3) == 1 and t.stride(2) == hd and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
