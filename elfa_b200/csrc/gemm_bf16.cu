@@ -40,6 +40,7 @@
 #include "comm.cuh"
 #include "common.cuh"
 #include "elfa_native.h"
+#include "gemm_skinny.cuh"
 
 namespace elfa {
 namespace {
@@ -1138,6 +1139,16 @@ ELFA_API int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
   ELFA_REQUIRE(!(flags & ELFA_EPI_STORE_PREACT) || (preact && ldpre % 8 == 0), "gemm: preact flag without pointer");
   unsigned int* st = status_word();
   ELFA_REQUIRE(st != nullptr, "gemm: no status word");
+
+  // a few rows: the matrix is read once by plain loads
+  auto whole16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (M <= SKINNY_ROWS && !a_mn_major && K % 8 == 0 && force_bn == 0 && max_ctas <= 0 &&
+      !(flags & ~(ELFA_EPI_BIAS | ELFA_EPI_GELU | ELFA_EPI_STORE_PREACT)) && whole16(A) && whole16(B) && whole16(C) &&
+      (!(flags & ELFA_EPI_STORE_PREACT) || whole16(preact))) {
+    const SkinnyParams q{static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(B), static_cast<const __nv_bfloat16*>(bias),
+                         static_cast<__nv_bfloat16*>(C), static_cast<__nv_bfloat16*>(preact), lda, ldb, ldc, ldpre, M, N, K, alpha, flags};
+    return launch_gemm_skinny(q, b_mn_major != 0, static_cast<cudaStream_t>(stream));
+  }
 
   // force_bn 512 selects the CTA-pair kernel (256 x 256 tiles per pair); by default it is used when the
   // problem fills at least one wave of pairs with such tiles

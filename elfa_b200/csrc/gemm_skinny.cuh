@@ -1,0 +1,20 @@
+// Products of a few rows (gemm_skinny.cu), reached through elfa_gemm_bf16.
+#pragma once
+#include "common.cuh"
+
+namespace elfa {
+
+constexpr int SKINNY_ROWS = 8;
+
+struct SkinnyParams {
+  const __nv_bfloat16 *A, *B, *bias;
+  __nv_bfloat16 *C, *preact;
+  long long lda, ldb, ldc, ldpre;
+  int M, N, K;
+  float alpha;
+  unsigned flags;                          // ELFA_EPI_BIAS, ELFA_EPI_GELU, ELFA_EPI_STORE_PREACT
+};
+
+int launch_gemm_skinny(const SkinnyParams& p, bool b_mn, cudaStream_t s);
+
+}  // namespace elfa

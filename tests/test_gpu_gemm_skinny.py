@@ -1,0 +1,67 @@
+"""Products of one to eight rows (plain loads, no tensor-core tile) against fp64 and against the tensor-core form.
+
+Bound: bf16 operands, fp32 sums of K terms in any order (K 2^-24 of the sum of magnitudes at worst; 2^-12 of the largest output covers K <= 11008 of
+random signs) and one rounding of the output to bf16 (2^-9 of itself): 2^-8 of the largest.
+"""
+import pytest
+import torch
+
+from elfa_b200 import native, ops
+from elfa_b200.ops.gemm import gelu_tanh_ref, gemm
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(dev, M, N, K, bmn):
+    g = torch.Generator(device=dev).manual_seed(M * 7 + N + K)
+    r = lambda *s: torch.randn(*s, generator=g, device=dev)
+    return r(M, K).bfloat16(), (r(K, N) if bmn else r(N, K)).mul(K ** -0.5).bfloat16()
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9])                    # 9: the tensor-core form
+@pytest.mark.parametrize("N,K", [(8, 8), (64, 256), (72, 264), (1000, 1104), (1536, 1024), (256, 11008), (32000, 128)])
+@pytest.mark.parametrize("bmn", [True, False])
+def test_matches_the_product(cuda_device, M, N, K, bmn):
+    a, b = _operands(cuda_device, M, N, K, bmn)
+    want = a.double() @ (b.double() if bmn else b.double().t())
+    y = gemm(a, b, b_mn=bmn)
+    assert native.status() == 0
+    assert (y.double() - want).abs().max() <= 2 ** -8 * want.abs().max()
+    assert torch.equal(y, gemm(a, b, b_mn=bmn))
+
+
+@pytest.mark.parametrize("bmn", [True, False])
+def test_epilogue_and_pitches(cuda_device, bmn):
+    a, b = _operands(cuda_device, 5, 136, 320, bmn)
+    wide = torch.randn(5, 400, device=cuda_device).bfloat16()
+    wide[:, 8:328] = a
+    bias = torch.randn(136, device=cuda_device).bfloat16()
+    out = torch.full((5, 200), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    pre = torch.full((5, 144), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    gemm(wide[:, 8:328], b, b_mn=bmn, bias=bias, gelu=True, preact=pre[:, :136], out=out[:, 64:], alpha=0.5)
+    want = 0.5 * (a.double() @ (b.double() if bmn else b.double().t())) + bias.double()
+    assert (pre[:, :136].double() - want).abs().max() <= 2 ** -8 * want.abs().max()
+    # the activation uses the hardware tanh: 2^-11 of its own besides the rounding
+    assert (out[:, 64:].double() - gelu_tanh_ref(want)).abs().max() <= 2 ** -7 * want.abs().max()
+    assert (out[:, :64] == 7).all() and (pre[:, 136:] == 7).all()
+
+
+def test_not_finite_values_stay_in_their_row_and_column(cuda_device):
+    for bmn in (True, False):
+        a, b = _operands(cuda_device, 3, 64, 256, bmn)
+        y = gemm(a, b, b_mn=bmn)
+        a[1, 200] = float("nan")
+        (b if bmn else b.t())[17, 40] = float("inf")
+        z = gemm(a, b, b_mn=bmn)
+        assert z[1].isnan().all() and not torch.isfinite(z[:, 40]).any()
+        keep = [j for j in range(64) if j != 40]
+        assert torch.equal(z[::2, keep], y[::2, keep])
+
+
+def test_linear_backward_of_a_few_rows(cuda_device):
+    x = torch.randn(4, 256, device=cuda_device).bfloat16().requires_grad_(True)
+    w = (torch.randn(256, 512, device=cuda_device) / 16).bfloat16().requires_grad_(True)
+    dy = torch.randn(4, 512, device=cuda_device).bfloat16()
+    dx, dw = torch.autograd.grad(ops.linear(x, w), [x, w], dy)
+    for got, want in ((dx, dy.double() @ w.double().t()), (dw, x.double().t() @ dy.double())):
+        assert (got.double() - want).abs().max() <= 2 ** -8 * want.abs().max()
