@@ -15,10 +15,10 @@
 // is one 32-lane x 128-bit tcgen05.cp into 4 tensor-memory columns (replicated to the 4 lane quarters);
 // the k-th MMA of a 128-wide K tile selects byte k of those columns through the instruction descriptor.
 //
-// Roles per CTA (192 threads, persistent, one CTA per SM):
+// Roles per CTA (persistent, one CTA per SM):
 //   warp 0   : producer - TMA loads of the A / B tiles (128-byte swizzle) and bulk copies of the scale atoms
 //   warp 1   : tensor-memory owner; one lane copies scales to tensor memory and issues the MMAs
-//   warps 2-5: epilogue (one 32-lane quarter each): tcgen05.ld -> bias / GELU -> bf16 -> global
+//   then four or eight epilogue warps (one or two per 32-lane quarter, taking groups of 64 columns in turn): tcgen05.ld -> bias / GELU -> bf16 -> global
 // Every wait is bounded (status word + abort flag), like the bf16 kernel.
 //
 // TWO = true: the two CTAs of a cluster form a pair (tcgen05 cta_group::2) on a 256 x BN tile. Each CTA
@@ -44,8 +44,7 @@ namespace {
 constexpr int QBM = 128;       // tile rows
 constexpr int QBK = 128;       // K elements (= bytes) per stage: one 128-byte swizzle row
 constexpr int QUMMA_K = 32;    // K per instruction for 8-bit operands
-constexpr int Q_THREADS = 192;
-constexpr int Q_THREADS_AG = 256;   // + two push warps (all-gather variant)
+constexpr int q_threads(int epi, bool ag) { return 64 + 32 * epi + (ag ? 64 : 0); }     // + epilogue warps, + two push warps (all-gather variant)
 constexpr int SF_ATOM = 512;   // bytes of one scale atom (128 rows x 4 K-blocks)
 
 // All-gather variant (AG = true): A = all_gather_rows of the ranks' quantised rows. Every rank has quantised its rows into
@@ -81,7 +80,7 @@ struct QParams {
   int tiles_m, tiles_n, group_m;
 };
 
-template <int BN, int STAGES, bool TWO, bool FP4 = false>
+template <int BN, int STAGES, bool TWO, bool FP4 = false, int EPI = 4>
 struct QSmem {
   // B scale atoms per tile (128: 1; 192: starts 0 or 64 rows into an atom, 2; 256: 2)
   static_assert(BN == 128 || BN == 192 || BN == 256, "tile widths");
@@ -94,8 +93,8 @@ struct QSmem {
   static constexpr int BAR_OFF = SF_OFF + STAGES * SF_BYTES;
   static constexpr int NUM_BARS = 2 * STAGES + 4 + 4;   // ring full / empty, accumulator full / empty, push buffers (all-gather variant)
   static constexpr int TOTAL0 = BAR_OFF + NUM_BARS * 8 + 16;
-  static constexpr int EPI_OFF = (TOTAL0 + 127) / 128 * 128;      // epilogue staging: 4 warps x 4 KB (whole-line stores)
-  static constexpr int TOTAL = EPI_OFF + 4 * 4096;
+  static constexpr int EPI_OFF = (TOTAL0 + 127) / 128 * 128;      // epilogue staging: 4 KB per warp (whole-line stores)
+  static constexpr int TOTAL = EPI_OFF + EPI * 4096;
   static constexpr int DYN = TOTAL + 1024;
   static constexpr int PUSH_OFF = (TOTAL + 127) / 128 * 128;      // all-gather variant: 2 warps x 2 buffers of PUSH_PIECE bytes
   static constexpr int DYN_AG = PUSH_OFF + 4 * PUSH_PIECE + 1024;
@@ -130,15 +129,16 @@ __device__ __forceinline__ void q_tile_coords_ag(const QParams& p, const QComm& 
   nb = lt / tm_shard;
 }
 
-template <int BN, int STAGES, bool TWO, bool FP4 = false, bool AG = false>
-__global__ void __launch_bounds__(AG ? Q_THREADS_AG : Q_THREADS, 1)
+// EPI: epilogue warps, 4 or 8 (one or two per lane quarter)
+template <int BN, int STAGES, bool TWO, bool FP4 = false, bool AG = false, int EPI = 4>
+__global__ void __launch_bounds__(q_threads(EPI, AG), 1)
 gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmSFA, const __grid_constant__ CUtensorMap tmSFB, const QParams p,
                   const QComm cm) {
-  using L = QSmem<BN, STAGES, TWO, FP4>;
+  using L = QSmem<BN, STAGES, TWO, FP4, EPI>;
   static_assert(!(FP4 && TWO), "the NVFP4 variant is single-CTA");
   static_assert(!(FP4 && AG), "the all-gather variant is MXFP8 only");
-  constexpr int KSF = L::KSF;
+  constexpr int KSF = L::KSF, PARTS = EPI / 4;
   constexpr int TILE_M = TWO ? 2 * QBM : QBM;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -186,7 +186,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), TWO ? 8 : 4);
+      mbar_init(tempty_bar(b), TWO ? 2 * EPI : EPI);
     }
     for (int b = 0; b < 4; ++b) mbar_init(bar0 + 8u * (2 * STAGES + 4 + b), SHARED ? 8 : 1);
     *abort_flag = 0;
@@ -322,9 +322,9 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
       }
     }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
-    const int q = warp & 3;
+  } else if (warp < 2 + EPI) {
+    // ------------------------------------------------------------------ epilogue
+    const int q = warp & 3, part = (warp - 2) >> 2;
     uint32_t tile_iter = 0;
     const unsigned fl = p.flags;
     float alpha = 1.f;
@@ -347,18 +347,22 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (SHARED || !(fl & ELFA_EPI_BIAS)) {         // SHARED is not launched with a bias
         // bf16 output (optionally the pre-activation too): 64 accumulator columns at a time through the warp's private 4 KB of shared memory, written as
         // whole 128-byte lines (common.cuh: warp_stage_64cols / warp_flush_64cols)
-        const uint32_t stage = smem_u32(smem + L::EPI_OFF) + q * 4096;
+        const uint32_t stage = smem_u32(smem + L::EPI_OFF) + (warp - 2) * 4096;
         const int row0 = m0 + q * 32;
         __nv_bfloat16* cbase = p.C + (long long)row0 * p.ldc + n0;
         const int rows_valid = p.M - row0;
         uint32_t ra[32], rb[32];
-        // SHARED: from the end that the next tile's accumulator overlaps
-        auto chunk = [&](int c) { return SHARED && buf == 0 ? BN / 32 - 2 - c : c; };
-        tmem_ld32(tcol0 + chunk(0) * 32, ra);
-        tmem_ld32(tcol0 + (chunk(0) + 1) * 32, rb);
+        // this warp's groups of 64 columns; SHARED: from the end that the next tile's accumulator overlaps
+        constexpr int NG = BN / 64;
+        auto group = [&](int i) { return SHARED && buf == 0 ? NG - 1 - i : i; };
+        if (part < NG) {
+          tmem_ld32(tcol0 + group(part) * 64, ra);
+          tmem_ld32(tcol0 + group(part) * 64 + 32, rb);
+        }
 #pragma unroll
-        for (int i = 0; i < BN / 32; i += 2) {
-          const int c = chunk(i);
+        for (int i0 = 0; i0 < NG; i0 += PARTS) {
+          const int i = i0 + part, c = group(i) * 2;
+          if (i >= NG) break;
           tmem_ld_wait();
           if (SHARED && i == 0) {
             tc_fence_before();
@@ -373,9 +377,9 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           }
           if (fl & ELFA_EPI_GELU) warp_stage_64cols<true>(stage, ra, rb, alpha, lane);
           else warp_stage_64cols(stage, ra, rb, alpha, lane);
-          if (i + 2 < BN / 32) {
-            tmem_ld32(tcol0 + chunk(i + 2) * 32, ra);
-            tmem_ld32(tcol0 + (chunk(i + 2) + 1) * 32, rb);
+          if (i + PARTS < NG) {
+            tmem_ld32(tcol0 + group(i + PARTS) * 64, ra);
+            tmem_ld32(tcol0 + group(i + PARTS) * 64 + 32, rb);
           }
           __syncwarp();
           warp_flush_64cols(stage, cbase + c * 32, p.ldc, rows_valid, p.N - n0 - c * 32, lane);
@@ -389,14 +393,14 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         continue;
       }
       uint32_t rnext[32];
-      tmem_ld32(tcol0, rnext);
+      tmem_ld32(tcol0 + part * 32, rnext);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = part; c < BN / 32; c += PARTS) {
         uint32_t r[32];
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) r[j] = rnext[j];
-        if (c + 1 < BN / 32) tmem_ld32(tcol0 + (c + 1) * 32, rnext);
+        if (c + PARTS < BN / 32) tmem_ld32(tcol0 + (c + PARTS) * 32, rnext);
         const int col0 = n0 + c * 32;
         if (col0 >= p.N) continue;   // uniform across the warp
         float v[32];
@@ -433,8 +437,8 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
   } else if (AG) {
-    // ------------------------------------------------------------------ push warps (6, 7)
-    const int w = warp - 6;
+    // ------------------------------------------------------------------ push warps
+    const int w = warp - 2 - EPI;
     push_ranges(reinterpret_cast<const char*>(cm.peer_buf[cm.rank]), cm.peer_buf, cm.peer_flags, cm.rank, cm.world, cm.plan,
                 smem_u32(smem + L::PUSH_OFF) + w * 2 * PUSH_PIECE, bar0 + 8u * (2 * STAGES + 4 + w * 2),
                 bar0 + 8u * (2 * STAGES + 4 + w * 2 + 1), 1, w, lane, abort_flag, p.status);
@@ -458,15 +462,15 @@ int q_grid_ctas(int M, int N) {
   return (TWO ? 2 : 1) * (tiles < slots ? tiles : slots);
 }
 
-template <int BN, int STAGES, bool TWO, bool FP4 = false, bool AG = false>
+template <int BN, int STAGES, bool TWO, bool FP4 = false, bool AG = false, int EPI = 4>
 int launch_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmSFA, const CUtensorMap& tmSFB, QParams p,
              cudaStream_t stream, const QComm* comm = nullptr) {
-  using L = QSmem<BN, STAGES, TWO, FP4>;
+  using L = QSmem<BN, STAGES, TWO, FP4, EPI>;
   constexpr int TILE_M = TWO ? 2 * QBM : QBM;
   constexpr int DYN = AG ? L::DYN_AG : L::DYN;
-  constexpr int NT = AG ? Q_THREADS_AG : Q_THREADS;
+  constexpr int NT = q_threads(EPI, AG);
   static_assert(DYN <= 227 * 1024, "shared memory plan exceeds the per-CTA limit");
-  auto kern = gemm_mxfp8_kernel<BN, STAGES, TWO, FP4, AG>;
+  auto kern = gemm_mxfp8_kernel<BN, STAGES, TWO, FP4, AG, EPI>;
   static bool configured = false;
   if (!configured) {
     ELFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN));
@@ -504,7 +508,8 @@ int launch_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& 
   return ELFA_OK;
 }
 
-// Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile
+// Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile. Measured (us, 192 / 256 wide): 4096 x 11008 x 4096
+// 155 / 138, 2048 x 4096 x 4096 38 / 31, 1500 x 4096 x 4096 28 / 30 (both one round: the narrow one).
 bool wide_pair(int M, int N, int K) {
   const long long pairs = device_sm_count() / 2, tm = (M + 255) / 256, kt = (K + QBK - 1) / QBK;
   const long long r256 = (tm * ((N + 255) / 256) + pairs - 1) / pairs, r192 = (tm * ((N + 191) / 192) + pairs - 1) / pairs;
@@ -739,7 +744,10 @@ ELFA_API int elfa_gemm_mxfp8(const void* A, const void* sfa, const void* B, cons
   p.flags = flags;
   p.status = st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (wide) return launch_q<256, 6, true>(tmA, tmB, tmSFA, tmSFB, p, s);
+  // Eight epilogue warps where a tile's products take less time than four need to write it (with GELU about 5 us for 192 columns, 7 for 256; a K block
+  // 0.34 us); their staging costs a stage of the ring. 4096 x 11008 x 1024: 192 wide 65 -> 57 us, 256 wide 73 -> 57; x 4096: 192 wide 155 -> 158.
+  if (wide) return launch_q<256, 5, true, false, false, 8>(tmA, tmB, tmSFA, tmSFB, p, s);
+  if (pair && kt <= 12) return launch_q<192, 6, true, false, false, 8>(tmA, tmB, tmSFA, tmSFB, p, s);
   if (pair) return launch_q<192, 7, true>(tmA, tmB, tmSFA, tmSFB, p, s);
   if (BN == 192) return launch_q<192, 5, false>(tmA, tmB, tmSFA, tmSFB, p, s);
   return launch_q<128, 6, false>(tmA, tmB, tmSFA, tmSFB, p, s);
