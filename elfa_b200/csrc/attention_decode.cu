@@ -42,6 +42,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeParams p) 
   const __nv_bfloat16* kn = p.knew + b * p.sb + (long long)hk * HD;
   const __nv_bfloat16* vn = p.vnew + b * p.sb + (long long)hk * HD;
 
+  pdl_wait();
+  pdl_next();
   float qr[R][8];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -157,6 +159,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeParams p) 
 // one per thread, and the partial results are fetched eight at a time: one slice after the other they took 9.7 us at B 1, t 4096
 // (129 slices), 9.1 this way; with 17 slices (B 4, t 512) 4.5 and 4.1.
 __global__ void attn_decode_combine_kernel(const DecodeParams p, int hd) {
+  pdl_wait();
+  pdl_next();
   __shared__ float sw[256], red[2][8];
   const int rep = p.H / p.Hkv, rows = p.s * rep, bhk = blockIdx.x / rows, r = blockIdx.x % rows, c = threadIdx.x;
   const int warp = c >> 5, warps = hd >> 5;
@@ -215,12 +219,10 @@ template <int HD>
 int launch_decode(const DecodeParams& p, cudaStream_t st) {
   const int rows = p.s * (p.H / p.Hkv);
   const dim3 grid(p.B * p.Hkv, p.slices);
-  if (rows <= 1) attn_decode_kernel<HD, 1><<<grid, 128, 0, st>>>(p);
-  else if (rows <= 2) attn_decode_kernel<HD, 2><<<grid, 128, 0, st>>>(p);
-  else if (rows <= 4) attn_decode_kernel<HD, 4><<<grid, 128, 0, st>>>(p);
-  else attn_decode_kernel<HD, 8><<<grid, 128, 0, st>>>(p);
+  auto kernel = rows <= 1 ? attn_decode_kernel<HD, 1> : (rows <= 2 ? attn_decode_kernel<HD, 2> : (rows <= 4 ? attn_decode_kernel<HD, 4> : attn_decode_kernel<HD, 8>));
+  ELFA_CUDA(launch_chain(kernel, grid, dim3(128), 0, st, 1, p));
   ELFA_CUDA(cudaGetLastError());
-  attn_decode_combine_kernel<<<p.B * p.Hkv * rows, HD, 0, st>>>(p, HD);
+  ELFA_CUDA(launch_chain(attn_decode_combine_kernel, dim3(p.B * p.Hkv * rows), dim3(HD), 0, st, 1, p, HD));
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(2);
   return ELFA_OK;

@@ -65,12 +65,47 @@ int make_tmap_nd_bf16(CUtensorMap* out, const void* base, int ndim, const uint64
 int shared_tmap(CUtensorMap* out, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t ld_elems,
                 uint32_t box_rows, uint32_t box_cols);
 int device_sm_count();
+// While a scope is open on this thread, the kernels that ask for it are launched with programmatic stream serialisation: their blocks may start
+// before the launch ahead of them has finished and wait inside (pdl_wait). Only for a chain in which nothing that a kernel reads before its
+// pdl_wait is written by the chain, and whose first launch is an ordinary one.
+bool pdl_open();
+struct PdlScope {
+  explicit PdlScope(bool on);
+  ~PdlScope();
+  bool was;
+};
 
 
 #ifdef __CUDACC__
 // ----------------------------------------------------------------------------------------------
 // device helpers
 // ----------------------------------------------------------------------------------------------
+// Returns once the launches ahead in the stream are complete and visible (at once in an ordinary launch). Every kernel that may be launched early
+// calls it in every thread before it reads what they wrote or writes anything, and lets the next launch start only then (pdl_next): so at most
+// the launch directly ahead is still running when a kernel starts.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... K, typename... A>
+inline cudaError_t launch_chain(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_y, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  cfg.attrs = at;
+  if (cluster_y > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = at[cfg.numAttrs].val.clusterDim.z = 1;
+    at[cfg.numAttrs++].val.clusterDim.y = cluster_y;
+  }
+  if (pdl_open()) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

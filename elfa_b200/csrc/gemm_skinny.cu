@@ -43,23 +43,25 @@ __device__ __forceinline__ void skinny_store(const SkinnyParams& p, int m, int n
   put(p.C + m * p.ldc + n);
 }
 
-// B [K, N], output index contiguous. A CTA owns 128 columns and a slice of the contraction, its eight warps 16 rows of B in turn: thread (g, q) of a
+// B [K, N], output index contiguous. A CTA owns 64 HALVES columns and a slice of the contraction, its eight warps 16 rows of B in turn: thread (g, q) of a
 // warp loads 16 bytes (columns 8 g .. and 64 + 8 g ..) of rows 2 q, 2 q + 1, 2 q + 8 and 2 q + 9, pairs the rows by byte permutation, and product
 // j of eight takes column 8 g + j (fragment row g) and 64 + 8 g + j (row g + 8). The slices of a column block are the CTAs of one cluster; warps
 // and slices add up in a fixed order.
+template <int HALVES>
 __global__ void __launch_bounds__(256) skinny_nn_kernel(const SkinnyParams p, int ks) {
   __shared__ __align__(16) float part[8][8][132];      // [warp][row of A][column]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const int n0 = blockIdx.x * 128, k1 = min(p.K, (int)(blockIdx.y + 1) * ks);
+  const int n0 = blockIdx.x * (64 * HALVES), k1 = min(p.K, (int)(blockIdx.y + 1) * ks);
   const int na = n0 + 8 * g, nb = na + 64;
-  const bool ina = na < p.N, inb = nb < p.N;           // N is a multiple of 8
+  const bool ina = na < p.N, inb = HALVES > 1 && nb < p.N;           // N is a multiple of 8
   float acc[8][4];
 #pragma unroll
   for (int j = 0; j < 8; ++j)
 #pragma unroll
     for (int x = 0; x < 4; ++x) acc[j][x] = 0.f;
-  for (int k = blockIdx.y * ks + warp * 16; k < k1; k += 128) {
-    uint4 w[4][2];                                     // rows 2 q, 2 q + 1, 2 q + 8, 2 q + 9 of both column halves
+  // the rows 2 q, 2 q + 1, 2 q + 8, 2 q + 9 of both column halves; the first ones before the launches ahead are waited for
+  uint4 w[4][2];
+  auto load = [&](int k) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int kr = k + 2 * q + (r & 1) + (r >> 1) * 8;
@@ -68,6 +70,19 @@ __global__ void __launch_bounds__(256) skinny_nn_kernel(const SkinnyParams p, in
       if (kr < k1 && ina) w[r][0] = ld_stream(row + na);
       if (kr < k1 && inb) w[r][1] = ld_stream(row + nb);
     }
+  };
+  const int kfirst = blockIdx.y * ks + warp * 16;
+  load(kfirst);
+  pdl_wait();
+  pdl_next();
+  for (int k = kfirst; k < k1; k += 128) {
+    uint4 v[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      v[r][0] = w[r][0];
+      v[r][1] = w[r][1];
+    }
+    if (k + 128 < k1) load(k + 128);
     uint32_t x0 = 0, x1 = 0;                           // A[g][2 q ..] and A[g][2 q + 8 ..]; K is a multiple of 8
     if (g < p.M) {
       const __nv_bfloat16* a = p.A + g * p.lda + k + 2 * q;
@@ -79,22 +94,22 @@ __global__ void __launch_bounds__(256) skinny_nn_kernel(const SkinnyParams p, in
       uint32_t f[4];
 #pragma unroll
       for (int x = 0; x < 4; ++x) {                    // a0, a1: rows 2 q, 2 q + 1 of halves 0, 1; a2, a3: the rows 8 further
-        const uint32_t lo = reinterpret_cast<const uint32_t*>(&w[x / 2 * 2][x & 1])[j / 2], hi = reinterpret_cast<const uint32_t*>(&w[x / 2 * 2 + 1][x & 1])[j / 2];
-        f[x] = __byte_perm(lo, hi, j & 1 ? 0x7632 : 0x5410);
+        const uint32_t lo = reinterpret_cast<const uint32_t*>(&v[x / 2 * 2][x & 1])[j / 2], hi = reinterpret_cast<const uint32_t*>(&v[x / 2 * 2 + 1][x & 1])[j / 2];
+        f[x] = HALVES == 1 && (x & 1) ? 0u : __byte_perm(lo, hi, j & 1 ? 0x7632 : 0x5410);
       }
       mma_bf16(acc[j], f, x0, x1);
     }
   }
 #pragma unroll
-  for (int x = 0; x < 4; ++x) {                        // x = 0, 1: column 8 g + j, rows 2 q, 2 q + 1 of A; 2, 3: column 64 + 8 g + j
+  for (int x = 0; x < 2 * HALVES; ++x) {               // x = 0, 1: column 8 g + j, rows 2 q, 2 q + 1 of A; 2, 3: column 64 + 8 g + j
     float* dst = &part[warp][2 * q + (x & 1)][(x >> 1) * 64 + 8 * g];
     *reinterpret_cast<float4*>(dst) = make_float4(acc[0][x], acc[1][x], acc[2][x], acc[3][x]);
     *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[4][x], acc[5][x], acc[6][x], acc[7][x]);
   }
   __syncthreads();
   float* sum = &part[0][0][0];                         // the warps' parts, added up over those of warp 0
-  for (int i = threadIdx.x; i < p.M * 32; i += 256) {
-    const int at = i / 32 * 132 + i % 32 * 4;
+  for (int i = threadIdx.x; i < p.M * 16 * HALVES; i += 256) {
+    const int at = i / (16 * HALVES) * 132 + i % (16 * HALVES) * 4;
     float4 s = *reinterpret_cast<const float4*>(sum + at);
 #pragma unroll
     for (int w = 1; w < 8; ++w) {
@@ -106,8 +121,8 @@ __global__ void __launch_bounds__(256) skinny_nn_kernel(const SkinnyParams p, in
   const int shares = gridDim.y, rank = blockIdx.y;
   if (shares > 1) cluster_sync_all();
   else __syncthreads();
-  for (int i = rank + threadIdx.x * shares; i < p.M * 16; i += 256 * shares) {
-    const int m = i / 16, c = i % 16 * 8;
+  for (int i = rank + threadIdx.x * shares; i < p.M * 8 * HALVES; i += 256 * shares) {
+    const int m = i / (8 * HALVES), c = i % (8 * HALVES) * 8;
     float f[8] = {};
     for (int r = 0; r < shares; ++r) {
       const uint32_t at = smem_u32(sum + m * 132 + c), src = shares > 1 ? map_to_cta(at, r) : at;
@@ -133,6 +148,8 @@ __global__ void __launch_bounds__(256) skinny_nt_kernel(const SkinnyParams p) {
   const bool in0 = n0 + g < p.N, in1 = n0 + g + 8 < p.N;
   const __nv_bfloat16 *b0 = p.B + (n0 + g) * p.ldb + 8 * q, *b1 = b0 + 8 * p.ldb, *a = p.A + g * p.lda + 8 * q;
   float acc[2][4] = {};
+  pdl_wait();
+  pdl_next();
   for (int kb = warp % WK * 32; kb < p.K; kb += WK * UN * 32) {
     uint4 w0[UN], w1[UN], x[UN];
 #pragma unroll
@@ -173,24 +190,16 @@ __global__ void __launch_bounds__(256) skinny_nt_kernel(const SkinnyParams p) {
 int launch_gemm_skinny(const SkinnyParams& p, bool b_mn, cudaStream_t s) {
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   if (!b_mn) {
-    if (p.N >= 64 * sms) skinny_nt_kernel<1><<<(p.N + 127) / 128, 256, 0, s>>>(p);
-    else skinny_nt_kernel<8><<<(p.N + 15) / 16, 256, 0, s>>>(p);
+    if (p.N >= 64 * sms) ELFA_CUDA(launch_chain(skinny_nt_kernel<1>, dim3((p.N + 127) / 128), dim3(256), 0, s, 1, p));
+    else ELFA_CUDA(launch_chain(skinny_nt_kernel<8>, dim3((p.N + 15) / 16), dim3(256), 0, s, 1, p));
   } else {
-    const int tiles = (p.N + 127) / 128;
+    // 64 columns per CTA where 128 would leave SMs idle even with eight slices (1024 x 4096: 64 CTAs)
+    const bool narrow = (p.N + 127) / 128 * 8 < sms;
+    const int tiles = narrow ? (p.N + 63) / 64 : (p.N + 127) / 128;
     int shares = 1;                                    // about two CTAs per SM, at least 128 rows of B each
     while (shares < 8 && tiles * shares < 2 * sms && p.K / (2 * shares) >= 128) shares *= 2;
     const int ks = ((p.K + shares - 1) / shares + 15) / 16 * 16;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(tiles, shares);
-    cfg.blockDim = dim3(256);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = at[0].val.clusterDim.z = 1;
-    at[0].val.clusterDim.y = shares;
-    cfg.attrs = at;
-    cfg.numAttrs = shares > 1 ? 1 : 0;
-    ELFA_CUDA(cudaLaunchKernelEx(&cfg, skinny_nn_kernel, p, ks));
+    ELFA_CUDA(launch_chain(narrow ? skinny_nn_kernel<1> : skinny_nn_kernel<2>, dim3(tiles, shares), dim3(256), 0, s, shares, p, ks));
   }
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);

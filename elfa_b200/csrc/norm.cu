@@ -41,6 +41,8 @@ __global__ void __launch_bounds__(256, NV <= 8 ? (HAS_RES ? 2 : 3) : 1) norm_fwd
   const long long off = (long long)(valid ? row : 0) * D;
   const uint4* xr = reinterpret_cast<const uint4*>(x + off);
   uint4 buf[NV];
+  pdl_wait();
+  pdl_next();
 #pragma unroll
   for (int i = 0; i < NV; ++i) buf[i] = ld_or_zero(xr + t + i * TPR, valid && t + i * TPR < nvec);
   if (HAS_RES) {
@@ -303,15 +305,19 @@ ELFA_API int elfa_norm_fwd(const void* x, const void* res, const void* w, const 
   auto* Y = static_cast<__nv_bfloat16*>(y);
   auto* S = static_cast<__nv_bfloat16*>(sum_out);
   const bool rms = kind == 1, has_res = res != nullptr;
+  cudaError_t err = cudaSuccess;
+  auto launch = [&](auto kernel, int grid) {
+    err = launch_chain(kernel, dim3(grid), dim3(256), 0, s, 1, X, R, W, B, Y, S, mean_out, rstd_out, rows, D, eps);
+  };
 #define LAUNCH_FWD(TPR, NV)                                                                                                  \
   do {                                                                                                                       \
     const int grid = (rows + (256 / TPR) - 1) / (256 / TPR);                                                                 \
     if (rms) {                                                                                                               \
-      if (has_res) norm_fwd_kernel<TPR, NV, true, true><<<grid, 256, 0, s>>>(X, R, W, B, Y, S, mean_out, rstd_out, rows, D, eps);  \
-      else norm_fwd_kernel<TPR, NV, true, false><<<grid, 256, 0, s>>>(X, R, W, B, Y, S, mean_out, rstd_out, rows, D, eps);    \
+      if (has_res) launch(norm_fwd_kernel<TPR, NV, true, true>, grid);                                                       \
+      else launch(norm_fwd_kernel<TPR, NV, true, false>, grid);                                                              \
     } else {                                                                                                                 \
-      if (has_res) norm_fwd_kernel<TPR, NV, false, true><<<grid, 256, 0, s>>>(X, R, W, B, Y, S, mean_out, rstd_out, rows, D, eps); \
-      else norm_fwd_kernel<TPR, NV, false, false><<<grid, 256, 0, s>>>(X, R, W, B, Y, S, mean_out, rstd_out, rows, D, eps);   \
+      if (has_res) launch(norm_fwd_kernel<TPR, NV, false, true>, grid);                                                      \
+      else launch(norm_fwd_kernel<TPR, NV, false, false>, grid);                                                             \
     }                                                                                                                        \
   } while (0)
   // at most 8 vectors (128 bytes) per thread up to D = 16384, so that several rows per SM are in flight
@@ -322,6 +328,7 @@ ELFA_API int elfa_norm_fwd(const void* x, const void* res, const void* w, const 
   else if (D <= 16384) LAUNCH_FWD(256, 8);
   else LAUNCH_FWD(256, 16);
 #undef LAUNCH_FWD
+  ELFA_CUDA(err);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;

@@ -22,6 +22,11 @@ int cuda_fail(cudaError_t e, const char* what) {
 static std::atomic<long long> g_launches{0};
 void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
+static thread_local bool t_pdl = false;
+bool pdl_open() { return t_pdl; }
+PdlScope::PdlScope(bool on) : was(t_pdl) { t_pdl = on; }
+PdlScope::~PdlScope() { t_pdl = was; }
+
 static std::atomic<int> g_deterministic{0};
 bool deterministic_mode() { return g_deterministic.load(std::memory_order_relaxed) != 0; }
 

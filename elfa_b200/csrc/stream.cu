@@ -152,6 +152,9 @@ ELFA_API int elfa_gpt_stream(const unsigned long long* p, const long long* dims,
   const float scale = (float)(1.0 / sqrt((double)m.hd));
   STREAM_CALL(elfa_embedding_fwd(static_cast<const long long*>(at(0)), at(1), m.has_pos ? at(2) : nullptr, w.x[0], rows, D, S, B, (int)m.pos0, 0, (int)m.V,
                                  (int)m.V, stream));
+  // Decoding: the chain of small launches overlaps their starts, and a product's first weights are on their way before its rows are there. The
+  // weights and caches that the chain reads early were written before the ordinary launch above. 
+  const PdlScope chain(m.t > 0);
   int cur = 0;
   for (int l = 0; l < m.layers; ++l) {
     const int q = 8 + 12 * l;
