@@ -11,15 +11,19 @@
 //   MODE_DQ  (CTA owns a query tile, loops over key tiles):
 //       S = Q K^T, dP = dO V^T;  dS -> bf16 in tensor memory;  dQ += dS K
 // P / dS never touch shared memory; the Q / K / V / dO tiles are used K-major or MN-major through
-// the descriptor only, so no transpose is materialised. The inner tiles are double buffered (TMA
-// runs one iteration ahead). Two passes keep every accumulator in tensor memory and make the
-// result deterministic (no floating-point atomics on dQ).
+// the descriptor only, so no transpose is materialised. Two passes keep every accumulator in tensor
+// memory and make the result deterministic (no floating-point atomics on dQ).
+//
+// S 4096, 32 heads of 128, causal: 260 + 192 us and 15 us of row sums. A block pair takes 3900 / 2900 cycles of an SM for 2048 / 1536 cycles of
+// products: the key-tile pass waits on the chain S -> P -> dV -> next S (tensor memory is full: S, dP and two accumulators, so S has one
+// place), the query-tile pass on shared memory (S and dP read 16 KB per 64 cycles of product, and 64 KB arrive per pair). The
+// resident operands in tensor memory instead were slower (212 against 192 us).
 //
 // reference: the op is defined by src/futhark/attention.fut:28-51; the reference ships no
 // attention backward at all.
 //
-// Roles per CTA (320 threads): warp 0 TMA, warp 1 MMA issue, warps 2-9 compute (warps w and w+4
-// share a tensor-memory lane quarter and split the 128 columns in halves).
+// Roles per CTA: warp 0 TMA, warp 1 MMA issue, warp 2 row vectors (key-tile pass), the rest compute (warps w and w + 4 share a
+// tensor-memory lane quarter and split the columns).
 #include <type_traits>
 
 #include "common.cuh"
@@ -33,10 +37,17 @@ int make_qkv_tmap(CUtensorMap* tm, const void* qkv, int S, int B, int H, int hd,
 namespace {
 
 constexpr int SUBB = 128 * 128;
-constexpr int ATTB_CW = 32;                           // columns of a compute warp
-constexpr int ATTB_SPLIT = 128 / ATTB_CW;             // compute warps per tensor-memory lane quarter
-constexpr int ATTB_COMPUTE = 4 * ATTB_SPLIT;          // compute warps
-constexpr int ATTB_THREADS = 32 * (3 + ATTB_COMPUTE);
+// Compute warps per tensor-memory lane quarter, each on its own columns of a block, and the pieces in which they hand P and dS to the MMA warp.
+// Key-tile pass: its chain is P -> dV -> next S, so four warps (a quarter more of the exponentials' rate than two) and halves, of
+// which the first is multiplied while the second is made (260 us against 268 with two warps, 279 without halves; S 4096, 32 heads of 128). Query-tile
+// pass: next S waits for nothing but the read of this one; two warps, whole (192 us; four warps 200).
+template <bool DKV> struct BwdWarps {
+  static constexpr int SPLIT = DKV ? 4 : 2, PIECES = DKV ? 2 : 1;
+  static constexpr int CW = 128 / SPLIT;                // columns of a compute warp
+  static constexpr int HC = CW / PIECES;                // columns of a piece
+  static constexpr int COMPUTE = 4 * SPLIT;             // compute warps
+  static constexpr int THREADS = 32 * (3 + COMPUTE);
+};
 
 // Grouped-query attention (Hkv < H): the key-tile pass runs `nsplit` CTAs (a cluster) per key / value head, each walking the query
 // tiles of its share of the group's query heads one head after the other; the shares are added up in rank order, so dK / dV are summed in a
@@ -46,8 +57,6 @@ struct AttnBwdParams {
   int S, B, H, hd;
   int Hkv;
   int nsplit;             // key-tile pass: CTAs (of one cluster) that share the query heads of a key head
-  const __nv_bfloat16 *qkv, *dout;
-  long long q_stride_s, q_stride_b, o_stride_s, o_stride_b;
   const int* doc_start;   // [B, S] or null
   const float* lse;    // [B, H, S] natural log
   const float* delta;  // [B, H, S]
@@ -59,23 +68,19 @@ struct AttnBwdParams {
   unsigned int* status;
 };
 
-// P and dS are handed over in two halves (the first and second 16 columns of every compute warp): BB_P, BB_DS and the one behind each
-enum { BB_RES0 = 0, BB_RES1, BB_QF0, BB_QE0 = BB_QF0 + 4, BB_OF0 = BB_QE0 + 4, BB_OE0 = BB_OF0 + 3, BB_VF0 = BB_OE0 + 3, BB_S = BB_VF0 + 2,
+// P and dS are handed over in up to two pieces: BB_P, BB_DS and the one behind each
+enum { BB_RES0 = 0, BB_RES1, BB_QF0, BB_QE0 = BB_QF0 + 3, BB_OF0 = BB_QE0 + 3, BB_OE0 = BB_OF0 + 2, BB_VF0 = BB_OE0 + 2, BB_S = BB_VF0 + 2,
        BB_DP, BB_P, BB_DS = BB_P + 2, BB_ACC = BB_DS + 2, BB_COUNT };
 
 template <int HDP, bool DKV>
 struct BwdSmem {
-  // The resident pair is the A operand of S and dP. Where tensor memory has room for it (all but the key-tile pass of 128-wide heads) it is
-  // read from there: from shared memory a 128 x 128 x 16 product reads A and B in exactly the 64 cycles it takes, and the tiles that arrive
-  // and the other products come on top.
-  static constexpr bool RES_TM = !DKV || HDP == 64;
   static constexpr int NSUB = HDP / 64;
   static constexpr int TILE = NSUB * SUBB;
   // rings of the inner tiles: one slot more for the operand that two products far apart read (Q, or K in the query-tile pass)
-  static constexpr int NQ = RES_TM ? 4 : 3, NO = NQ - 1;
+  static constexpr int NQ = 3, NO = 2;
   static constexpr int RES0 = 0;
-  static constexpr int RES1 = RES0 + (RES_TM ? 0 : TILE);
-  static constexpr int INQ = RES1 + (RES_TM ? 0 : TILE);
+  static constexpr int RES1 = RES0 + TILE;
+  static constexpr int INQ = RES1 + TILE;
   static constexpr int INO = INQ + NQ * TILE;
   static constexpr int VEC = 2 * 128 * 4 + 128;            // -lse2, -delta * scale (fp32), document start relative to the key tile (bytes)
   static constexpr int VEC_OFF = INO + NO * TILE;          // [2 slots]
@@ -142,12 +147,21 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
+// a compute warp's columns of a block
+template <int CW>
+__device__ __forceinline__ void load_cols(uint32_t taddr, uint32_t (&r)[CW]) {
+#pragma unroll
+  for (int c = 0; c < CW / 32; ++c) tmem_ld32(taddr + c * 32, reinterpret_cast<uint32_t(&)[32]>(r[c * 32]));
+#pragma unroll
+  for (int c = 0; c < CW / 32; ++c) tmem_ld_wait32(reinterpret_cast<uint32_t(&)[32]>(r[c * 32]));
+}
+
 template <int HDP, bool DKV>
-__global__ void __launch_bounds__(ATTB_THREADS, 1)
+__global__ void __launch_bounds__(BwdWarps<DKV>::THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO, const AttnBwdParams p) {
   using L = BwdSmem<HDP, DKV>;
-  constexpr int NSUB = L::NSUB, NQ = L::NQ, NO = L::NO, CW = ATTB_CW;
-  constexpr bool RES_TM = L::RES_TM;
+  constexpr int NSUB = L::NSUB, NQ = L::NQ, NO = L::NO, CW = BwdWarps<DKV>::CW, HC = BwdWarps<DKV>::HC, PIECES = BwdWarps<DKV>::PIECES,
+                SPLIT = BwdWarps<DKV>::SPLIT, COMPUTE = BwdWarps<DKV>::COMPUTE;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + BB_COUNT);
@@ -197,7 +211,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     prefetch_tmap(&tmQKV);
     prefetch_tmap(&tmDO);
     for (int i = 0; i < BB_COUNT; ++i)      // one arrival per compute warp, or one
-      mbar_init(bar(i), (i >= BB_P && i < BB_ACC) || (RES_TM && i <= BB_RES1) ? ATTB_COMPUTE : 1);
+      mbar_init(bar(i), i >= BB_P && i < BB_ACC ? COMPUTE : 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -209,9 +223,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  // fp32 S (or S^T) and dP (or dP^T); their bf16 successors P / dS overwrite the first 16 of the warp's 32 columns they come from
-  const uint32_t TM_S = tmem_base, TM_DP = tmem_base + 128, TM_ACC0 = tmem_base + 256, TM_ACC1 = tmem_base + 256 + HDP,
-                 TM_RES0 = tmem_base + 384, TM_RES1 = TM_RES0 + HDP / 2;
+  // fp32 S (or S^T) and dP (or dP^T); their bf16 successors P / dS overwrite the first half of the columns of the warp they come from
+  const uint32_t TM_S = tmem_base, TM_DP = tmem_base + 128, TM_ACC0 = tmem_base + 256, TM_ACC1 = tmem_base + 256 + HDP;
 
   // resident pair: (K_j, V_j) in DKV mode, (Q_i, dO_i) in DQ mode; the inner pair is the other one
   const uint32_t sRes0 = sbase + L::RES0, sRes1 = sbase + L::RES1;
@@ -232,9 +245,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         const int hq = hq0 + it / n_in, t = in_begin + it % n_in;
         load(sO(it % NO), DKV ? &tmDO : &tmQKV, DKV ? hq : p.H + p.Hkv + kvh, t, BB_OF0 + it % NO);
       };
-      if (!RES_TM) load(sRes0, &tmQKV, p.H + kvh, outer, BB_RES0);
+      load(sRes0, &tmQKV, DKV ? p.H + kvh : h, outer, BB_RES0);
       load_q(0);
-      if (!RES_TM) load(sRes1, &tmQKV, p.H + p.Hkv + kvh, outer, BB_RES1);
+      load(sRes1, DKV ? &tmQKV : &tmDO, DKV ? p.H + p.Hkv + kvh : h, outer, BB_RES1);
       load_o(0);
       for (int it = 1; it < NQ; ++it) {                   // NO = NQ - 1
         if (it < n_iter) load_q(it);
@@ -265,8 +278,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 #pragma unroll
           for (int kk = 0; kk < HDP / 16; ++kk) {
             const uint32_t off = (kk / 4) * SUBB + (kk % 4) * 32;
-            if (RES_TM) tc_mma_f16_ts(TM_S, TM_RES0 + kk * 8, make_smem_desc(b0 + off, 16, 1024, 2), idesc_s, kk != 0);
-            else tc_mma_f16(TM_S, make_smem_desc(a0 + off, 16, 1024, 2), make_smem_desc(b0 + off, 16, 1024, 2), idesc_s, kk != 0);
+            tc_mma_f16(TM_S, make_smem_desc(a0 + off, 16, 1024, 2), make_smem_desc(b0 + off, 16, 1024, 2), idesc_s, kk != 0);
           }
           tc_commit(bar(BB_S));
         }
@@ -278,8 +290,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 #pragma unroll
           for (int kk = 0; kk < HDP / 16; ++kk) {
             const uint32_t off = (kk / 4) * SUBB + (kk % 4) * 32;
-            if (RES_TM) tc_mma_f16_ts(TM_DP, TM_RES1 + kk * 8, make_smem_desc(b1 + off, 16, 1024, 2), idesc_s, kk != 0);
-            else tc_mma_f16(TM_DP, make_smem_desc(a1 + off, 16, 1024, 2), make_smem_desc(b1 + off, 16, 1024, 2), idesc_s, kk != 0);
+            tc_mma_f16(TM_DP, make_smem_desc(a1 + off, 16, 1024, 2), make_smem_desc(b1 + off, 16, 1024, 2), idesc_s, kk != 0);
           }
           tc_commit(bar(BB_DP));
           if (!DKV) tc_commit(bar(BB_OE0 + it % NO));
@@ -287,12 +298,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         __syncwarp();
       };
       // A (16 columns of P or dS per step, 8 tensor-memory columns) lies in the first half of its compute warp's columns; acc += A B over the
-      // steps that the warps' first (half 0) or second 16 columns make up
-      auto issue_acc = [&](uint32_t acc, uint32_t a, uint32_t b, int half, bool first) {
+      // steps that this piece of every warp's columns makes up
+      auto issue_acc = [&](uint32_t acc, uint32_t a, uint32_t b, int piece, bool first) {
         if (elect_one()) {
 #pragma unroll
-          for (int w = 0; w < ATTB_SPLIT; ++w)
-            tc_mma_f16_ts(acc, a + w * CW + half * 8, make_smem_desc(b + (2 * w + half) * 2048, SUBB, 1024, 2), idesc_acc, !(first && half == 0 && w == 0));
+          for (int i = 0; i < 8 / PIECES; ++i) {
+            const int w = i / (HC / 16), u = i % (HC / 16);
+            tc_mma_f16_ts(acc, a + w * CW + piece * (HC / 2) + u * 8, make_smem_desc(b + ((w * CW + piece * HC) / 16 + u) * 2048, SUBB, 1024, 2), idesc_acc,
+                          !(first && piece == 0 && i == 0));
+          }
         }
         __syncwarp();
       };
@@ -310,11 +324,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         const uint32_t b0 = sQ(it % NQ), b1 = sO(it % NO);
         if (DKV) {          // dV[key, d] += sum_q P^T[key, q] dO[q, d]
 #pragma unroll
-          for (int half = 0; half < 2 && ok; ++half) {
-            ok = wait(BB_P + half, it & 1);
+          for (int piece = 0; piece < PIECES && ok; ++piece) {
+            ok = wait(BB_P + piece, it & 1);
             if (!ok) break;
             tc_fence_after();
-            issue_acc(TM_ACC0, TM_S, b1, half, it == 0);
+            issue_acc(TM_ACC0, TM_S, b1, piece, it == 0);
           }
           if (!ok) break;
           if (elect_one()) tc_commit(bar(BB_OE0 + it % NO));
@@ -328,11 +342,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         }
         // dK[key, d] += sum_q dS^T[key, q] Q[q, d], or dQ[q, d] += sum_key dS[q, key] K[key, d]
 #pragma unroll
-        for (int half = 0; half < 2 && ok; ++half) {
-          ok = wait(BB_DS + half, it & 1);
+        for (int piece = 0; piece < PIECES && ok; ++piece) {
+          ok = wait(BB_DS + piece, it & 1);
           if (!ok) break;
           tc_fence_after();
-          issue_acc(DKV ? TM_ACC1 : TM_ACC0, TM_DP, b0, half, it == 0);
+          issue_acc(DKV ? TM_ACC1 : TM_ACC0, TM_DP, b0, piece, it == 0);
         }
         if (!ok) break;
         if (elect_one()) tc_commit(bar(BB_QE0 + it % NQ));
@@ -404,31 +418,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       }
       if (dstart) doc_last = dstart[min(outer * 128 + 127, p.S - 1)];
     }
-    if (RES_TM) {       // the resident pair into tensor memory: HDP / SPLIT columns of this thread's row, zeros past the end
-      constexpr int VN = HDP / ATTB_SPLIT / 8;
-      const int row = outer * 128 + row_local, e0 = part * (HDP / ATTB_SPLIT);
-      const __nv_bfloat16* r0 = p.qkv + (long long)row * p.q_stride_s + (long long)b * p.q_stride_b + (long long)(DKV ? p.H + kvh : h) * p.hd + e0;
-      const __nv_bfloat16* r1 = DKV ? r0 + (long long)p.Hkv * p.hd : p.dout + (long long)row * p.o_stride_s + (long long)b * p.o_stride_b + (long long)h * p.hd + e0;
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        uint32_t v[VN * 4];
-#pragma unroll
-        for (int i = 0; i < VN; ++i) {
-          uint4 q = make_uint4(0, 0, 0, 0);
-          if (row < p.S && e0 + i * 8 < p.hd) q = *reinterpret_cast<const uint4*>((which ? r1 : r0) + i * 8);
-          v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
-        }
-        const uint32_t dst = (which ? TM_RES1 : TM_RES0) + lane_addr + e0 / 2;
-        if constexpr (VN == 4) tmem_st16(dst, v); else tmem_st8(dst, v);
-      }
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(bar(BB_RES0));
-        mbar_arrive(bar(BB_RES1));
-      }
-    }
     const float sc2 = p.scale_log2;
     const uint64_t sc2x2 = pack_f32x2(sc2, sc2), scx2 = pack_f32x2(p.scale, p.scale);
     for (int it = 0, in_tile = in_begin; it < n_iter; ++it, in_tile = in_tile + 1 < in_end ? in_tile + 1 : in_begin) {
@@ -442,20 +431,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       if (!ok) break;
       tc_fence_after();
       const bool diag = p.causal && in_tile == outer;
-      uint32_t rs[32];                   // S, then the probabilities (fp32, kept for dS)
-      tmem_ld32(TM_S + lane_addr + colw, rs);
-      tmem_ld_wait32(rs);
+      uint32_t rs[CW];                   // S, then the probabilities (fp32, kept for dS)
+      load_cols(TM_S + lane_addr + colw, rs);
       if (!DKV) {                        // the S columns have been read: the next S product may overwrite them
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(BB_P));
       }
-      // ---- phase 1: P = exp2(S * scale - lse), 16 columns at a time. `diag` (and a ragged last tile) is uniform over the CTA: only
+      // ---- phase 1: P = exp2(S * scale - lse), a piece of the columns at a time. `diag` (and a ragged last tile) is uniform over the CTA: only
       // those tiles pay for the per-element mask test. The per-query vectors come from shared memory four at a time.
-      auto phase1 = [&](auto masked_tag, int half) {
+      auto phase1 = [&](auto masked_tag, int piece) {
         constexpr bool MASK = decltype(masked_tag)::value;
 #pragma unroll
-        for (int i = half * 16; i < half * 16 + 16; i += 4) {
+        for (int i = piece * HC; i < piece * HC + HC; i += 4) {
           float l4[4] = {lse2, lse2, lse2, lse2};
           if (DKV) {
             const float4 t4 = *reinterpret_cast<const float4*>(vl + colw + i);
@@ -484,25 +472,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
           }
         }
       };
-      // eight registers of bf16 pairs into tensor memory, then this half is handed to the MMA warp
-      auto hand_over = [&](uint32_t at, const uint32_t (&t)[8], int bar_id, int half) {
-        tmem_st8(at + lane_addr + colw + half * 8, t);
+      // a piece's bf16 pairs into tensor memory, then it is handed to the MMA warp
+      auto hand_over = [&](uint32_t at, const uint32_t (&t)[HC / 2], int bar_id, int piece) {
+        const uint32_t dst = at + lane_addr + colw + piece * (HC / 2);
+        if constexpr (HC == 64) tmem_st32(dst, t); else if constexpr (HC == 32) tmem_st16(dst, t); else tmem_st8(dst, t);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(bar_id + half));
+        if (lane == 0) mbar_arrive(bar(bar_id + piece));
       };
       // a document boundary inside the block pair: the key tile starts before the query tile's last document does
       const bool doc_mask = dstart && (DKV ? vdoc[127] > 0 : k_tile * 128 < doc_last);
       const bool any_mask = diag || doc_mask || (!DKV && (outer + 1) * 128 > p.S);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        if (any_mask) phase1(std::true_type{}, half); else phase1(std::false_type{}, half);
+      for (int piece = 0; piece < PIECES; ++piece) {
+        if (any_mask) phase1(std::true_type{}, piece); else phase1(std::false_type{}, piece);
         if (DKV) {
-          uint32_t t[8];
+          uint32_t t[HC / 2];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) t[i] = pack_bf16(__uint_as_float(rs[half * 16 + 2 * i]), __uint_as_float(rs[half * 16 + 2 * i + 1]));
-          hand_over(TM_S, t, BB_P, half);
+          for (int i = 0; i < HC / 2; ++i) t[i] = pack_bf16(__uint_as_float(rs[piece * HC + 2 * i]), __uint_as_float(rs[piece * HC + 2 * i + 1]));
+          hand_over(TM_S, t, BB_P, piece);
         }
       }
       // ---- phase 2: dS = P * (dP - delta) * scale
@@ -510,14 +499,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      uint32_t rd[32];
-      tmem_ld32(TM_DP + lane_addr + colw, rd);
-      tmem_ld_wait32(rd);
+      uint32_t rd[CW];
+      load_cols(TM_DP + lane_addr + colw, rd);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t t[8];
+      for (int piece = 0; piece < PIECES; ++piece) {
+        uint32_t t[HC / 2];
 #pragma unroll
-        for (int i = half * 16; i < half * 16 + 16; i += 4) {
+        for (int i = piece * HC; i < piece * HC + HC; i += 4) {
           float d4[4] = {dlt, dlt, dlt, dlt};
           if (DKV) {
             const float4 t4 = *reinterpret_cast<const float4*>(vl + 128 + colw + i);
@@ -529,10 +517,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
           const uint64_t t23 = fma_f32x2(pack_f32x2(__uint_as_float(rd[i + 2]), __uint_as_float(rd[i + 3])), scx2, pack_f32x2(d4[2], d4[3]));
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), t01, 0ull), x0, x1);
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[i + 2]), __uint_as_float(rs[i + 3])), t23, 0ull), x2, x3);
-          t[(i - half * 16) >> 1] = pack_bf16(x0, x1);
-          t[((i - half * 16) >> 1) + 1] = pack_bf16(x2, x3);
+          t[(i - piece * HC) >> 1] = pack_bf16(x0, x1);
+          t[((i - piece * HC) >> 1) + 1] = pack_bf16(x2, x3);
         }
-        hand_over(TM_DP, t, BB_DS, half);
+        hand_over(TM_DP, t, BB_DS, piece);
       }
     }
     // ---------------------------------------------------------------- epilogue
@@ -546,7 +534,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       constexpr int CHUNKS = HDP / 32;           // 32-column chunks per accumulator
       constexpr int NACC = DKV ? 2 : 1;
       // split the NACC * CHUNKS chunks between the warps that share this lane quarter
-      for (int idx = part; idx < NACC * CHUNKS; idx += ATTB_SPLIT) {
+      for (int idx = part; idx < NACC * CHUNKS; idx += SPLIT) {
         const int acc = idx / CHUNKS, c = idx % CHUNKS;
         uint32_t r[32];
         tmem_ld32((acc == 0 ? TM_ACC0 : TM_ACC1) + lane_addr + c * 32, r);
@@ -584,7 +572,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     const int rows = 128 / nsplit;
     const uint32_t red = sbase + L::INQ;
     if (!*abort_flag) {
-      for (int i = threadIdx.x; i < rows * (2 * HDP / 8); i += ATTB_THREADS) {
+      for (int i = threadIdx.x; i < rows * (2 * HDP / 8); i += BwdWarps<DKV>::THREADS) {
         const int rl = share * rows + i / (2 * HDP / 8), c = i % (2 * HDP / 8) * 8, d0 = c % HDP;
         const int row = outer * 128 + rl;
         if (row >= p.S || d0 >= p.hd) continue;
@@ -617,7 +605,7 @@ int launch_attn_bwd(const CUtensorMap& tmQKV, const CUtensorMap& tmDO, const Att
   const unsigned nsplit = DKV ? p.nsplit : 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)p.n_tiles * (DKV ? p.Hkv : p.H) * p.B * nsplit);
-  cfg.blockDim = dim3(ATTB_THREADS);
+  cfg.blockDim = dim3(BwdWarps<DKV>::THREADS);
   cfg.dynamicSmemBytes = L::TOTAL;
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
@@ -670,10 +658,6 @@ ELFA_API int elfa_attention_bwd_ex(const void* qkv, long long stride_s, long lon
   p.S = S; p.B = B; p.H = H; p.hd = hd;
   p.Hkv = Hkv;
   p.doc_start = doc_start;
-  p.qkv = static_cast<const __nv_bfloat16*>(qkv);
-  p.dout = static_cast<const __nv_bfloat16*>(dout);
-  p.q_stride_s = stride_s; p.q_stride_b = stride_b;
-  p.o_stride_s = o_stride_s; p.o_stride_b = o_stride_b;
   p.lse = lse; p.delta = delta;
   p.dqkv = static_cast<__nv_bfloat16*>(dqkv);
   p.d_stride_s = d_stride_s; p.d_stride_b = d_stride_b;
