@@ -442,6 +442,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       // those tiles pay for the per-element mask test. The per-query vectors come from shared memory four at a time.
       auto phase1 = [&](auto masked_tag, int piece) {
         constexpr bool MASK = decltype(masked_tag)::value;
+        uint32_t docs[4] = {};           // key-tile pass: document starts of the piece's 16 queries
+        if (DKV && MASK) {
+          const uint4 q4 = *reinterpret_cast<const uint4*>(vdoc + colw + piece * HC);
+          docs[0] = q4.x; docs[1] = q4.y; docs[2] = q4.z; docs[3] = q4.w;
+        }
 #pragma unroll
         for (int i = piece * HC; i < piece * HC + HC; i += 4) {
           float l4[4] = {lse2, lse2, lse2, lse2};
@@ -455,8 +460,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
               const int col = colw + i + u;
               float e = fast_exp2(fmaf(__uint_as_float(rs[i + u]), sc2, l4[u]));
               // DKV: lane = key, column = query -> masked when key > query; DQ: lane = query, column = key
-              bool masked = DKV ? (diag && row_local > col) : (!row_ok || (diag && col > row_local));
-              if (dstart) masked = masked || (DKV ? (row_local < (int)vdoc[col]) : (k_tile * 128 + col < lower));
+              const int j = i + u - piece * HC;
+              const bool masked = DKV ? (diag && row_local > col) || row_local < (int)((docs[(j >> 2) & 3] >> (8 * (j & 3))) & 255u)
+                                      : !row_ok || (diag && col > row_local) || k_tile * 128 + col < lower;
               if (masked) e = 0.f;
               rs[i + u] = __float_as_uint(e);
             }
