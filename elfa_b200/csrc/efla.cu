@@ -320,8 +320,13 @@ __global__ void __launch_bounds__(128) shortconv_ring_bwd_kernel(const __nv_bflo
     shortconv_bwd_again<W>(xb, w + (long long)c * W, gb, ob, pb, t0, t1, T, C);
 }
 
+// A gradient in the type it is wanted in: fp32 sums, rounded once (as two casts behind the kernel would, without their launches)
+__device__ __forceinline__ void put_grad(float* p, float v) { *p = v; }
+__device__ __forceinline__ void put_grad(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
+
 // dw[c, j] = sum over the slices of part[slice][j][c], db[c] from row `taps`. grid (ceil(C / 32), taps + 1), block (32, 16)
-__global__ void __launch_bounds__(512) shortconv_sum_kernel(const float* __restrict__ part, float* __restrict__ dw, float* __restrict__ db,
+template <typename G>
+__global__ void __launch_bounds__(512) shortconv_sum_kernel(const float* __restrict__ part, G* __restrict__ dw, G* __restrict__ db,
                                                             int slices, int C, int taps) {
   __shared__ float red[16][33];
   const int c = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y;
@@ -336,8 +341,8 @@ __global__ void __launch_bounds__(512) shortconv_sum_kernel(const float* __restr
     float tot = 0.f;
 #pragma unroll
     for (int k = 0; k < 16; ++k) tot += red[k][threadIdx.x];
-    if (j < taps) dw[(long long)c * taps + j] = tot;
-    else if (db) db[c] = tot;
+    if (j < taps) put_grad(dw + (long long)c * taps + j, tot);
+    else if (db) put_grad(db + c, tot);
   }
 }
 
@@ -503,6 +508,14 @@ ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, 
 // dx bf16 [B,T,C]; dw fp32 [C,W]; db fp32 [C] or null; part: scratch of elfa_shortconv_bwd_slices() * (W + 1) * C floats (null when 0).
 ELFA_API int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, float* part, int B, int T,
                                 int C, int W, void* stream) {
+  return elfa_shortconv_bwd_as(x, w, dy, dx, dw, db, part, 0, B, T, C, W, stream);
+}
+
+// The same with the weight and bias gradients in bf16 where `grads_bf16`, windows of 4, 8 and 16 only.
+ELFA_API int elfa_shortconv_bwd_as(const void* x, const void* w, const void* dy, void* dx, void* dw_, void* db_, float* part, int grads_bf16,
+                                   int B, int T, int C, int W, void* stream) {
+  float *dw = static_cast<float*>(dw_), *db = static_cast<float*>(db_);
+  ELFA_REQUIRE(!grads_bf16 || shortconv_ring(W), "shortconv_bwd: bf16 gradients for windows of 4, 8 and 16 only");
   ELFA_REQUIRE(x && w && dy && dx && dw && B > 0 && T > 0 && C > 0 && W > 0, "shortconv_bwd: bad arguments");
   ELFA_REQUIRE(C % 2 == 0 && W <= 128, "shortconv_bwd: the channel count must be even and the window at most 128");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -516,7 +529,9 @@ ELFA_API int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, vo
     else if (W == 8) shortconv_ring_bwd_kernel<8><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
     else shortconv_ring_bwd_kernel<16><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
     ELFA_CUDA(cudaGetLastError());
-    shortconv_sum_kernel<<<dim3((C + 31) / 32, W + 1), dim3(32, 16), 0, s>>>(part, dw, db, B * spans, C, W);
+    const dim3 gs((C + 31) / 32, W + 1), bs(32, 16);
+    if (grads_bf16) shortconv_sum_kernel<<<gs, bs, 0, s>>>(part, static_cast<__nv_bfloat16*>(dw_), static_cast<__nv_bfloat16*>(db_), B * spans, C, W);
+    else shortconv_sum_kernel<<<gs, bs, 0, s>>>(part, dw, db, B * spans, C, W);
     ELFA_CUDA(cudaGetLastError());
     ::elfa::count_launches(2);
     return ELFA_OK;
