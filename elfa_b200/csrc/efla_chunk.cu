@@ -1349,22 +1349,25 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 using namespace elfa;
 
 // How many segments a walk over T tokens is cut into (1: none), and with them how large `work` is: 3 * segments * B * H * d * d floats.
-// One walk takes nchunks steps; cut, FIRST takes nchunks / P steps of (2 P - 3) walks per head and column block and REST as many of P - 1. A step
-// costs the latency of a chunk's chain while an SM has one CTA, 1.25 of it with two (its registers hold no third) and whole rounds beyond.
+// One walk takes nchunks steps; cut, FIRST takes nchunks / P steps of (2 P - 3) walks per head and column block and REST as many of P - 1. Measured
+// per head dimension: a step with one CTA per SM, with as many as its registers and shared memory hold (whole rounds beyond), and the
+// two launches and joints more. B 1 x 8192, 16 heads of 64: P 1 355 us, 6 150, 8 146, 10 128, 12 160 (a second round); B 2 x 1531, 8 heads of 128: P 1
+// 109, 4 98, 5 93, 6 101; B 4 x 1024, 8 heads of 128: P 1 78, 3 88 (not cut); B 8 x 2048, 16 heads of 64: P 1 118, 3 165 (not cut).
 ELFA_API int elfa_efla_segments(int B, int T, int H, int d) {
   const int nchunks = (T + EC - 1) / EC, sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const long long units = (long long)B * H * (d == 128 || d == 96 ? 2 : 1);
-  const double step = d == 128 ? 2.0 : (d == 96 ? 1.6 : 1.4), combine = d == 128 ? 1.8 : 0.9;      // microseconds
+  struct Cost { double one, full; int resident; double launches, joint; };      // microseconds
+  const Cost c = d == 128 ? Cost{2.1, 3.6, 2, 16, 4} : (d == 96 ? Cost{1.76, 2.6, 2, 9, 3.5} : (d == 64 ? Cost{1.4, 1.9, 2, 6, 3} : Cost{1.16, 1.4, 4, 4, 1}));
   auto steps = [&](long long walks) {
-    const long long ctas = units * walks, full = ctas / (2 * sms), rest = ctas % (2 * sms);
-    return step * (1.25 * (double)full + (rest == 0 ? 0. : (rest <= sms ? 1. : 1.25)));
+    const long long ctas = units * walks, round = (long long)c.resident * sms, rest = ctas % round;
+    return c.full * (double)(ctas / round) + (rest == 0 ? 0. : (rest <= sms ? c.one : c.full));
   };
-  double best = nchunks * steps(1);
+  double best = 0.95 * nchunks * steps(1);       // cut only where that is clearly less
   int at = 1;
   for (int P = 3; P <= 16 && nchunks / P >= 4; ++P) {
     const int seg = (nchunks + P - 1) / P;
-    const double t = seg * (steps(2 * P - 3) + steps(P - 1)) + 8 + combine * (P - 2);      // two more launches
-    if (t < 0.95 * best) {
+    const double t = seg * (steps(2 * P - 3) + steps(P - 1)) + c.launches + c.joint * (P - 2);
+    if (t < best) {
       best = t;
       at = P;
     }
