@@ -346,6 +346,45 @@ __global__ void __launch_bounds__(512) shortconv_sum_kernel(const float* __restr
   }
 }
 
+// ShortConv of T new positions behind the last `tail` ones of a stream, which the layer keeps: u[b, t] from the tail and the new inputs, and tail and
+// inputs side by side as the next tail's source, in one launch (as copies and the ordinary kernel: four). RING: the order of the sums of the
+// register-ring kernels (even and odd taps apart), otherwise that of the general one, so that the bits do not depend on how a sequence is cut.
+// A block is 64 channel pairs of one position. grid (B * T, ceil(C / 128))
+template <bool RING>
+__global__ void __launch_bounds__(64) shortconv_stream_kernel(const __nv_bfloat16* __restrict__ tail, long long tail_stride,
+                                                              const __nv_bfloat16* __restrict__ n, const __nv_bfloat16* __restrict__ w,
+                                                              const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ xin,
+                                                              __nv_bfloat16* __restrict__ u, int tails, int T, int C, int W) {
+  const int c = (blockIdx.y * 64 + threadIdx.x) * 2, t = blockIdx.x % T, b = blockIdx.x / T;
+  if (c >= C) return;
+  const __nv_bfloat16 *tb = tail + b * tail_stride + c, *nb = n + (long long)b * T * C + c;
+  __nv_bfloat16* xb = xin + (long long)b * (tails + T) * C + c;
+  auto at = [&](int i) {                   // position i of tail and inputs
+    return *reinterpret_cast<const uint32_t*>(i < tails ? tb + (long long)i * C : nb + (long long)(i - tails) * C);
+  };
+  if (t == 0)
+    for (int i = 0; i < tails; ++i) *reinterpret_cast<uint32_t*>(xb + (long long)i * C) = at(i);
+  *reinterpret_cast<uint32_t*>(xb + (long long)(tails + t) * C) = at(tails + t);
+  float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};                            // [chain][channel]
+  if (bias) {
+    s[0][0] = __bfloat162float(bias[c]);
+    s[0][1] = __bfloat162float(bias[c + 1]);
+  }
+  const int taps = min(W, tails + t + 1);
+#pragma unroll 4
+  for (int j = 0; j < taps; ++j) {
+    const uint32_t x = at(tails + t - j);
+    const int k = RING ? j & 1 : 0;
+    s[k][0] = fmaf(bf16_lo(x), __bfloat162float(w[(long long)c * W + j]), s[k][0]);
+    s[k][1] = fmaf(bf16_hi(x), __bfloat162float(w[(long long)(c + 1) * W + j]), s[k][1]);
+  }
+  if (RING) {
+    s[0][0] += s[1][0];
+    s[0][1] += s[1][1];
+  }
+  *reinterpret_cast<uint32_t*>(u + ((long long)b * T + t) * C + c) = pack_bf16(s[0][0], s[0][1]);
+}
+
 // Forward and input gradient share one kernel (DX = false: y[t] = bias + sum_j x[t - j] w[j]; DX = true:
 // dx[t] = sum_j dy[t + j] w[j]). A lane owns a PAIR of adjacent channels (4-byte loads, 128 bytes per warp); the
 // CTA's 64 channels x W weights sit transposed in shared memory (the [C, W] layout read directly would touch a
@@ -500,6 +539,21 @@ ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, 
   shortconv_apply_kernel<false><<<grid, block, (size_t)W * 64 * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(bias),
       static_cast<__nv_bfloat16*>(y), B, T, C, W);
+  ELFA_CUDA(cudaGetLastError());
+  ::elfa::count_launches(1);
+  return ELFA_OK;
+}
+
+// tail [B, tails, C] (batches tail_stride elements apart), n [B, T, C] -> u [B, T, C] = ShortConv of tail and n side by side, its last T positions,
+// and xin [B, tails + T, C], the two side by side.
+ELFA_API int elfa_shortconv_stream(const void* tail, long long tail_stride, const void* n, const void* w, const void* bias, void* xin, void* u, int B,
+                                   int tails, int T, int C, int W, void* stream) {
+  ELFA_REQUIRE(tail && n && w && xin && u && B > 0 && tails > 0 && T > 0 && (long long)B * T < (1ll << 31) && C > 0 && W > 0, "shortconv_stream: bad arguments");
+  ELFA_REQUIRE(C % 2 == 0 && tail_stride % 2 == 0 && W <= 128, "shortconv_stream: channels and batch stride must be even, the window at most 128");
+  auto kernel = shortconv_ring(W) ? shortconv_stream_kernel<true> : shortconv_stream_kernel<false>;
+  const auto h = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
+  kernel<<<dim3((unsigned)(B * T), (C + 127) / 128), 64, 0, static_cast<cudaStream_t>(stream)>>>(h(tail), tail_stride, h(n), h(w), h(bias), static_cast<__nv_bfloat16*>(xin),
+                                                                                   static_cast<__nv_bfloat16*>(u), tails, T, C, W);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;

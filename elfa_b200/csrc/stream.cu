@@ -87,7 +87,7 @@ struct EflaDims {
   long long B, T, D, H, d, F, V, layers, L, W, act, kind, prism, tail;
 };
 struct EflaWork {
-  bf16 *x[2], *r, *n, *k, *v, *o, *e, *u, *uc, *z, *wc, *q, *h, *g, *f, *nmat;
+  bf16 *x[2], *r, *n, *k, *v, *o, *e, *u, *z, *wc, *q, *h, *g, *f, *nmat;
   float *coef, *segw;
 };
 size_t efla_work(const EflaDims& m, unsigned char* base, EflaWork* w, int segments, bool step) {
@@ -101,8 +101,7 @@ size_t efla_work(const EflaDims& m, unsigned char* base, EflaWork* w, int segmen
   w->v = p.take<bf16>(rows * hd);
   w->o = p.take<bf16>(rows * hd);
   w->e = p.take<bf16>(rows * m.D);
-  w->u = p.take<bf16>(m.prism ? m.B * (m.T + m.tail) * m.D : 0);
-  w->uc = p.take<bf16>(m.prism && m.tail ? rows * m.D : 0);
+  w->u = p.take<bf16>(m.prism ? rows * m.D : 0);
   w->z = p.take<bf16>(m.prism ? rows * 3 * m.L * m.d : 0);
   w->wc = p.take<bf16>(m.prism ? m.D * 3 * m.L * m.d : 0);
   w->q = p.take<bf16>(m.prism ? rows * m.D : 0);
@@ -153,7 +152,7 @@ ELFA_API int elfa_gpt_stream(const unsigned long long* p, const long long* dims,
   STREAM_CALL(elfa_embedding_fwd(static_cast<const long long*>(at(0)), at(1), m.has_pos ? at(2) : nullptr, w.x[0], rows, D, S, B, (int)m.pos0, 0, (int)m.V,
                                  (int)m.V, stream));
   // Decoding: the chain of small launches overlaps their starts, and a product's first weights are on their way before its rows are there. The
-  // weights and caches that the chain reads early were written before the ordinary launch above. 
+  // weights and caches that the chain reads early were written before the ordinary launch above.
   const PdlScope chain(m.t > 0);
   int cur = 0;
   for (int l = 0; l < m.layers; ++l) {
@@ -208,8 +207,9 @@ ELFA_API int elfa_efla_stream(const unsigned long long* p, const long long* dims
   efla_work(m, static_cast<unsigned char*>(at(6)), &w, segments, step);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int rows = (int)(m.B * m.T), D = (int)m.D, B = (int)m.B, T = (int)m.T, H = (int)m.H, d = (int)m.d, L = (int)m.L, kind = (int)m.kind, G = D / d;
-  const int hd = H * d, per = 19 + 3 * L, Tt = (int)(m.T + m.tail);
+  const int hd = H * d, per = 19 + 3 * L;
   STREAM_CALL(elfa_embedding_fwd(static_cast<const long long*>(at(0)), at(1), nullptr, w.x[0], rows, D, T, 1, 0, 0, (int)m.V, (int)m.V, stream));
+  const PdlScope chain(m.B * m.T <= 8);        // decoding, as above
   int cur = 0;
   for (int l = 0; l < m.layers; ++l) {
     const int q = 7 + per * l;
@@ -226,26 +226,22 @@ ELFA_API int elfa_efla_stream(const unsigned long long* p, const long long* dims
     STREAM_CALL(linear(w.o, at(q + 4), w.e, rows, hd, D, 0, stream));
     const bf16* y = w.e;
     if (m.prism) {
-      const bf16* u = w.u;
-      if (m.tail) {       // tail and new positions side by side
-        const size_t row = (size_t)D * 2, pitch = (size_t)Tt * row;
-        STREAM_CALL(copy2d(xin, pitch, at(q + 16), (size_t)p[q + 17] * 2, (size_t)m.tail * row, B, s));
-        STREAM_CALL(copy2d(xin + m.tail * D, pitch, n, (size_t)T * row, (size_t)T * row, B, s));
-        STREAM_CALL(elfa_shortconv_fwd(xin, at(q + 6), at(q + 7), w.u, B, Tt, D, (int)m.W, stream));
-        STREAM_CALL(copy2d(w.uc, (size_t)T * row, w.u + m.tail * D, pitch, (size_t)T * row, B, s));
-        u = w.uc;
-      } else {
+      if (m.tail)
+        STREAM_CALL(elfa_shortconv_stream(at(q + 16), (long long)p[q + 17], n, at(q + 6), at(q + 7), xin, w.u, B, (int)m.tail, T, D, (int)m.W, stream));
+      else
         STREAM_CALL(elfa_shortconv_fwd(xin, at(q + 6), at(q + 7), w.u, B, T, D, (int)m.W, stream));
-      }
       ConcatArgs a{};
       for (int i = 0; i < 3 * L; ++i) a.src[i] = static_cast<const uint4*>(at(q + 19 + i));
       const long long vecs = (long long)D * 3 * L * (d / 8);
       concat_cols_kernel<<<(unsigned)((vecs + 255) / 256), 256, 0, s>>>(a, reinterpret_cast<uint4*>(w.wc), D, 3 * L, d / 8);
       ELFA_CUDA(cudaGetLastError());
       ::elfa::count_launches(1);
-      STREAM_CALL(linear(u, w.wc, w.z, rows, D, 3 * L * d, 0, stream));
-      STREAM_CALL(elfa_prism_gated_fwd(u, w.e, w.z, 3 * L * d, w.q, rows, G, d, L, stream));
-      STREAM_CALL(elfa_prism_state(u, w.e, w.z, 3 * L * d, L * d, 2 * L * d, static_cast<const float*>(at(q + 14)), static_cast<float*>(at(q + 15)), B, T, G, d,
+      {       // its matrix was put together by the launch above: nothing of it may be asked for early
+        const PdlScope whole(false);
+        STREAM_CALL(linear(w.u, w.wc, w.z, rows, D, 3 * L * d, 0, stream));
+      }
+      STREAM_CALL(elfa_prism_gated_fwd(w.u, w.e, w.z, 3 * L * d, w.q, rows, G, d, L, stream));
+      STREAM_CALL(elfa_prism_state(w.u, w.e, w.z, 3 * L * d, L * d, 2 * L * d, static_cast<const float*>(at(q + 14)), static_cast<float*>(at(q + 15)), B, T, G, d,
                                    L, forget[l], stream));
       y = w.q;
     }
