@@ -166,7 +166,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   // wait for the MMAs that still read the current ones.
   // BN = 256: two whole accumulators and the scales are 24 columns too many, so the accumulators share 24 columns: columns 232 .. 255 are the last
   // ones of the first and the first ones of the second. The epilogue reads the group of 64 that holds them first and raises over_bar, for
-  // which the next tile's first product waits (some 500 cycles per tile; the rest of the epilogue runs under that tile's products).
+  // which the next tile's first product waits; the rest of the epilogue runs under that tile's products.
   constexpr bool SHARED = BN == 256;
   static_assert(!SHARED || (TWO && !FP4 && !AG), "the 256-wide tile is for CTA pairs");
   constexpr uint32_t TMEM_COLS = 512;
@@ -508,7 +508,8 @@ int launch_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& 
   return ELFA_OK;
 }
 
-// Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile. Measured (us, 192 / 256 wide): 4096 x 11008 x 4096
+// Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile (cycles: the fill of shared memory per K block, and the wait
+// for the shared columns). Of 36 shapes (M 1500 to 16384, N 3072 to 11008, K 1024 to 4096) it misses the faster tile in three, by 3 % at most. Measured (us, 192 / 256 wide): 4096 x 11008 x 4096
 // 155 / 138, 2048 x 4096 x 4096 38 / 31, 1500 x 4096 x 4096 28 / 30 (both one round: the narrow one).
 bool wide_pair(int M, int N, int K) {
   const long long pairs = device_sm_count() / 2, tm = (M + 255) / 256, kt = (K + QBK - 1) / QBK;
