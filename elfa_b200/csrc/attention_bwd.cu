@@ -24,6 +24,7 @@
 //
 // Roles per CTA: warp 0 TMA, warp 1 MMA issue, warp 2 row vectors (key-tile pass), the rest compute (warps w and w + 4 share a
 // tensor-memory lane quarter and split the columns).
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -607,7 +608,13 @@ template <int HDP, bool DKV>
 int launch_attn_bwd(const CUtensorMap& tmQKV, const CUtensorMap& tmDO, const AttnBwdParams& p, cudaStream_t stream) {
   using L = BwdSmem<HDP, DKV>;
   auto kern = attn_bwd_kernel<HDP, DKV>;
-  ELFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+  static std::atomic<unsigned long long> configured{0};      // devices on which the kernel may use this much; asking each time costs the host 1 to 2 us
+  int dev = 0;
+  ELFA_CUDA(cudaGetDevice(&dev));
+  if (dev > 63 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
+    ELFA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+    if (dev <= 63) configured.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
   const unsigned nsplit = DKV ? p.nsplit : 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)p.n_tiles * (DKV ? p.Hkv : p.H) * p.B * nsplit);
