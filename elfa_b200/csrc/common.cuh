@@ -292,7 +292,10 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
   return r;
 }
+// Every thread of a warp has to execute an `.aligned` instruction together, and only __syncwarp brings them together again behind a loop or a
+// branch that some of them left early.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // 16 bytes of any CTA's shared memory (address from map_to_cta)
