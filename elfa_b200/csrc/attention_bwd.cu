@@ -482,6 +482,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       // a piece's bf16 pairs into tensor memory, then it is handed to the MMA warp
       auto hand_over = [&](uint32_t at, const uint32_t (&t)[HC / 2], int bar_id, int piece) {
         const uint32_t dst = at + lane_addr + colw + piece * (HC / 2);
+        __syncwarp();                    // one lane's arrival for the piece before: the stores want the warp together
         if constexpr (HC == 64) tmem_st32(dst, t); else if constexpr (HC == 32) tmem_st16(dst, t); else tmem_st8(dst, t);
         tmem_st_wait();
         tc_fence_before();

@@ -368,6 +368,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(over_bar, 0));
+            __syncwarp();                  // the next loads want the warp together
           }
           if (fl & ELFA_EPI_STORE_PREACT) {
             warp_stage_64cols(stage, ra, rb, alpha, lane);

@@ -22,3 +22,13 @@ def test_a_cluster_barrier_brings_the_warp_together_first():
     for f in sorted(CSRC.glob("*.cu*")):                       # and there is no other place that issues it
         if f.name != "common.cuh":
             assert not re.search(r"barrier\.cluster\.\w+[\w.]*\.aligned", f.read_text()), f.name
+
+
+def test_tensor_memory_is_used_by_whole_warps_after_one_lane_arrived():
+    """``tcgen05.ld`` and ``.st`` are ``.sync.aligned``: behind an arrival by one lane the warp is brought together before the next of them."""
+    text = (CSRC / "attention_bwd.cu").read_text()
+    hand = text[text.index("auto hand_over"):]
+    assert hand.index("__syncwarp()") < hand.index("tmem_st")
+    text = (CSRC / "gemm_mxfp8.cu").read_text()
+    after = text[text.index("if (lane == 0) mbar_arrive_cluster(map_to_cta(over_bar, 0));"):]
+    assert after.index("__syncwarp()") < min(after.index("fl & ELFA_EPI_STORE_PREACT"), after.index("tmem_ld32"))
