@@ -550,6 +550,8 @@ ELFA_API int elfa_shortconv_stream(const void* tail, long long tail_stride, cons
                                    int tails, int T, int C, int W, void* stream) {
   ELFA_REQUIRE(tail && n && w && xin && u && B > 0 && tails > 0 && T > 0 && (long long)B * T < (1ll << 31) && C > 0 && W > 0, "shortconv_stream: bad arguments");
   ELFA_REQUIRE(C % 2 == 0 && tail_stride % 2 == 0 && W <= 128, "shortconv_stream: channels and batch stride must be even, the window at most 128");
+  for (const void* q : {tail, n, static_cast<const void*>(xin), static_cast<const void*>(u)})
+    ELFA_REQUIRE((reinterpret_cast<uintptr_t>(q) & 3) == 0, "shortconv_stream: operands must be 4-byte aligned");
   auto kernel = shortconv_ring(W) ? shortconv_stream_kernel<true> : shortconv_stream_kernel<false>;
   const auto h = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
   kernel<<<dim3((unsigned)(B * T), (C + 127) / 128), 64, 0, static_cast<cudaStream_t>(stream)>>>(h(tail), tail_stride, h(n), h(w), h(bias), static_cast<__nv_bfloat16*>(xin),

@@ -186,7 +186,7 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
             if not pa or p0.requires_grad or (ct is not None) != bool(tail):
                 return None
             if tail and (ct.shape != (B, tail, D) or ct.dtype != torch.bfloat16 or ct.device != dev or ct.stride(2) != 1 or ct.stride(1) != D
-                         or ct.requires_grad):
+                         or ct.requires_grad or ct.data_ptr() % 4 or ct.stride(0) % 2):       # read two channels, four bytes, at a time
                 return None
             p1 = torch.empty_like(p0)
             xin = torch.empty((B, tail + T, D), dtype=torch.bfloat16, device=dev)

@@ -1,0 +1,64 @@
+"""Which streaming calls go to native code, decided on the CPU: the native calls are only recorded, so nothing is launched and a call that must not
+get there shows without a device."""
+import pytest
+import torch
+
+from elfa_b200.config import Config
+from elfa_b200.models import streaming
+from elfa_b200.models.efla_model import EflaModel
+from elfa_b200.models.gpt import GPTModel
+
+
+@pytest.fixture
+def route(monkeypatch):
+    """``route(model, ids, states)``: whether the call is taken by native code."""
+    calls = []
+    monkeypatch.setattr(streaming, "_eager", lambda ids: True)
+    monkeypatch.setattr(streaming, "stream_ptr", lambda t: 0)
+    monkeypatch.setattr(streaming.lib, "call", lambda name, *a: calls.append(name))
+    monkeypatch.setattr(streaming.lib, "raw", lambda name: lambda *a: 1)
+
+    def ask(model, ids, states=None):
+        if states is None:
+            states = fresh(model, ids.shape[0])
+        calls.clear()
+        with torch.no_grad():
+            r = (streaming.efla_stream if isinstance(model, EflaModel) else streaming.gpt_stream)(model, ids, states)
+        assert (r is not None) == (len(calls) == 1)
+        return r is not None
+    return ask
+
+
+def fresh(model, batch):
+    return model.init_states(batch) if isinstance(model, EflaModel) else {"pos": 0, "layers": [{"k": None, "v": None} for _ in model.blocks]}
+
+
+def model(efla, act="gelu", layers=2, prism=True):
+    cfg = Config()
+    m = cfg.model
+    m.dtype, m.efla.enabled, m.prism.enabled = "bf16", efla, efla and prism
+    m.num_layers, m.hidden_dim, m.num_heads, m.num_kv_heads, m.head_dim = layers, 64, 2, 2, 32
+    m.intermediate_dim, m.vocab_size, m.activation, m.norm_type, m.max_seq_len, cfg.data.seq_len = 64, 72, act, "rmsnorm", 32, 32
+    m.prism.num_iterations, m.prism.shortconv_window = 2, 4
+    return (EflaModel if efla else GPTModel)(cfg, device=torch.device("cpu")).eval()
+
+
+IDS = torch.arange(6).view(2, 3)
+
+
+def test_plain_calls_are_taken(route):
+    assert route(model(True), IDS) and route(model(False), IDS) and route(model(True, prism=False), IDS)
+
+
+def test_shortconv_tails_that_the_kernel_cannot_read(route):
+    """It reads two channels at a time: an odd offset or an odd batch stride belongs to the general route."""
+    m, D = model(True), 64
+
+    def tail(offset, pitch):
+        flat = torch.zeros(offset + 2 * pitch + 3 * D, dtype=torch.bfloat16)
+        return flat.as_strided((2, 3, D), (pitch, D, 1), offset)
+    for offset, pitch, taken in ((0, 3 * D, True), (2, 3 * D + 2, True), (1, 3 * D, False), (0, 3 * D + 1, False), (3, 3 * D + 3, False)):
+        states = fresh(m, 2)
+        for s in states:
+            s["conv_tail"] = tail(offset, pitch)
+        assert route(m, IDS, states) == taken, (offset, pitch)

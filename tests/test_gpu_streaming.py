@@ -104,3 +104,19 @@ def test_what_is_left_to_the_general_route(cuda_device, monkeypatch):
     # five rows of four heads to a key head: the cached kernel takes eight
     model = GPTModel(_config(False, H=4, Hkv=1), device=cuda_device).eval()
     _compare(monkeypatch, model, ids, (0, 4, 9, 10), 2)
+
+
+@pytest.mark.parametrize("offset,pitch", [(1, 192), (0, 193), (3, 195)])
+def test_tails_at_odd_places(cuda_device, offset, pitch):
+    """A caller's own ShortConv tail may start and step anywhere: such calls go layer by layer, to the same values."""
+    model = EflaModel(_config(True, H=1, hd=64), device=cuda_device).eval()
+    ids = _ids(2, 9, cuda_device)
+    with torch.no_grad():
+        _, states = model.forward_with_states(ids[:, :5])
+        want, after = model.forward_with_states(ids[:, 5:], states)
+        for s in states:
+            odd = torch.empty(offset + 2 * pitch, dtype=torch.bfloat16, device=cuda_device).as_strided((2, 3, 64), (pitch, 64, 1), offset)
+            s["conv_tail"] = odd.copy_(s["conv_tail"])
+        got, now = model.forward_with_states(ids[:, 5:], states)
+    assert native.status() == 0 and torch.equal(got, want)
+    assert all(torch.equal(a[n], b[n]) for a, b in zip(after, now) for n in a)
