@@ -102,7 +102,7 @@ def gpt_stream(model, ids: torch.Tensor, states: dict):
         a, m, n1, n2 = blk.attn, blk.mlp, blk.ln1, blk.ln2
         if not (_plain(blk, Block) and _plain(a, Attention) and _plain(m, MLP) and _plain(n1, Norm) and _plain(n2, Norm)) \
                 or a.pc.tp_size != 1 or a.pc.cp_size != 1 or _quantised(a.quant) or _quantised(m.quant) or (blk.dropout > 0 and blk.training) \
-                or (a.n_heads, a.n_kv_heads, a.head_dim, m.act) != (H, Hkv, hd, act) or not _same_norms(fin, n1, n2):
+                or (a.n_heads, a.n_kv_heads, a.head_dim, m.act, m.gated) != (H, Hkv, hd, act, act == "swiglu") or not _same_norms(fin, n1, n2):
             return None
         if not _weights(dev, per_layer, (n1.weight, vec), (n1.bias, vec), (a.w_qkv, (D, N)), (a.w_o, (H * hd, D)), (n2.weight, vec), (n2.bias, vec),
                         (m.up, (D, 2 * F if act == "swiglu" else F)), (m.down, (F, D))):
@@ -148,7 +148,7 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
     H, d, act, F = first.efla.H, first.efla.d, first.act, first.mlp_up.shape[1]
     prism = first.prism is not None
     L, W = (first.prism.L, first.prism.conv_weight.shape[1]) if prism else (0, 1)
-    if not _plain(fin, Norm) or len(states) != len(blocks) or act not in _ACTS or d not in (32, 64, 96, 128) or D % d or model.vocab_lo != 0:
+    if not _plain(fin, Norm) or len(states) != len(blocks) or act not in _ACTS or act == "swiglu" or d not in (32, 64, 96, 128) or D % d or model.vocab_lo != 0:
         return None
     if prism and not (1 <= L <= 8 and W <= 128):
         return None

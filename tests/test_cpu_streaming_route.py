@@ -62,3 +62,15 @@ def test_shortconv_tails_that_the_kernel_cannot_read(route):
         for s in states:
             s["conv_tail"] = tail(offset, pitch)
         assert route(m, IDS, states) == taken, (offset, pitch)
+
+
+def test_an_activation_that_the_block_does_not_have(route):
+    """An EFLA block has one up-projection: with SwiGLU written into it the native call would read twice its columns."""
+    m = model(True)
+    for blk in m.blocks:
+        blk.act = "swiglu"
+    assert not route(m, IDS)
+    m = model(False)
+    for blk in m.blocks:
+        blk.mlp.act, blk.mlp.gated = "silu", True               # the layer goes by `gated`
+    assert not route(m, IDS)
