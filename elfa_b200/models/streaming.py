@@ -36,6 +36,10 @@ def _plain(module: nn.Module, kind: type) -> bool:
     return type(module) is kind and "forward" not in d and not d["_forward_hooks"] and not d["_forward_pre_hooks"]
 
 
+def _each_plain(blocks, kind: type) -> bool:
+    return len(blocks) > 0 and all(_plain(b, kind) for b in blocks)
+
+
 def _same_norms(a, *others) -> bool:
     return all(n.kind == a.kind and n.eps == a.eps for n in others)
 
@@ -79,13 +83,17 @@ def gpt_stream(model, ids: torch.Tensor, states: dict):
     tok, pos, fin, blocks = model.embed_tokens, model.pos_embed, model.final_norm, model.blocks
     head = model.lm_head if model.lm_head is not None else tok
     pos0, D = states["pos"], tok.shape[1]
-    if not _plain(fin, Norm) or len(states["layers"]) != len(blocks) or (pos is not None and pos0 + S > pos.shape[0]) or model.vocab_lo != 0:
+    if not _plain(fin, Norm) or not _each_plain(blocks, Block) or len(states["layers"]) != len(blocks) \
+            or any(type(c) is not dict for c in states["layers"]) or (pos is not None and pos0 + S > pos.shape[0]) or model.vocab_lo != 0:
         return None
     first, cache0 = blocks[0], states["layers"][0]
+    if not (_plain(first.attn, Attention) and _plain(first.mlp, MLP)):
+        return None
     at, act = first.attn, first.mlp.act
     H, Hkv, hd, F = at.n_heads, at.n_kv_heads, at.head_dim, first.mlp.down.shape[0]
-    t = cache0["k"].shape[0] if cache0["k"] is not None else 0
-    if (cache0["k"] is not None and not t) or act not in _ACTS or (act == "swiglu" and F % 8):
+    k0 = cache0.get("k")
+    t = k0.shape[0] if k0 is not None else 0
+    if (k0 is not None and not t) or act not in _ACTS or (act == "swiglu" and F % 8):
         return None
     if (hd not in DECODE_HEAD_DIMS or S * (H // Hkv) > DECODE_ROWS) if t else (hd % 8 or hd > 128):
         return None
@@ -100,14 +108,14 @@ def gpt_stream(model, ids: torch.Tensor, states: dict):
     per_layer: List[int] = []
     for blk, cache in zip(blocks, states["layers"]):
         a, m, n1, n2 = blk.attn, blk.mlp, blk.ln1, blk.ln2
-        if not (_plain(blk, Block) and _plain(a, Attention) and _plain(m, MLP) and _plain(n1, Norm) and _plain(n2, Norm)) \
+        if not (_plain(a, Attention) and _plain(m, MLP) and _plain(n1, Norm) and _plain(n2, Norm)) \
                 or a.pc.tp_size != 1 or a.pc.cp_size != 1 or _quantised(a.quant) or _quantised(m.quant) or (blk.dropout > 0 and blk.training) \
                 or (a.n_heads, a.n_kv_heads, a.head_dim, m.act, m.gated) != (H, Hkv, hd, act, act == "swiglu") or not _same_norms(fin, n1, n2):
             return None
         if not _weights(dev, per_layer, (n1.weight, vec), (n1.bias, vec), (a.w_qkv, (D, N)), (a.w_o, (H * hd, D)), (n2.weight, vec), (n2.bias, vec),
                         (m.up, (D, 2 * F if act == "swiglu" else F)), (m.down, (F, D))):
             return None
-        k, v = cache["k"], cache["v"]
+        k, v = cache.get("k"), cache.get("v")
         if t:
             if k is None or v is None or k.shape != (t, B, Hkv, hd) or v.shape != k.shape or k.requires_grad or v.requires_grad:
                 return None
@@ -144,11 +152,15 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
     B, T = ids.shape
     tok, fin, blocks = model.embed_tokens, model.final_norm, model.blocks
     head = model.lm_head if model.lm_head is not None else tok
+    if not _plain(fin, Norm) or not _each_plain(blocks, EflaBlock) or len(states) != len(blocks) or any(type(s) is not dict for s in states):
+        return None
     D, first = tok.shape[1], blocks[0]
+    if not _plain(first.efla, EflaLayer) or (first.prism is not None and not _plain(first.prism, PrismLayer)):
+        return None
     H, d, act, F = first.efla.H, first.efla.d, first.act, first.mlp_up.shape[1]
     prism = first.prism is not None
     L, W = (first.prism.L, first.prism.conv_weight.shape[1]) if prism else (0, 1)
-    if not _plain(fin, Norm) or len(states) != len(blocks) or act not in _ACTS or act == "swiglu" or d not in (32, 64, 96, 128) or D % d or model.vocab_lo != 0:
+    if act not in _ACTS or act == "swiglu" or d not in (32, 64, 96, 128) or D % d or model.vocab_lo != 0:
         return None
     if prism and not (1 <= L <= 8 and W <= 128):
         return None
@@ -163,11 +175,11 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
     new_states = []
     for blk, st in zip(blocks, states):
         e, pr, n1, n2 = blk.efla, blk.prism, blk.ln1, blk.ln2
-        if not (_plain(blk, EflaBlock) and _plain(e, EflaLayer) and _plain(n1, Norm) and _plain(n2, Norm)) or blk.pc.tp_size != 1 or e.pc.tp_size != 1 \
+        if not (_plain(e, EflaLayer) and _plain(n1, Norm) and _plain(n2, Norm)) or blk.pc.tp_size != 1 or e.pc.tp_size != 1 \
                 or (pr is not None) != prism or (prism and not (_plain(pr, PrismLayer) and pr.L == L and pr.d == d)) \
                 or (e.H, e.d, blk.act) != (H, d, act) or not _same_norms(fin, n1, n2):
             return None
-        s0, p0, ct = st["efla"], st["prism"], st.get("conv_tail")
+        s0, p0, ct = st.get("efla"), st.get("prism"), st.get("conv_tail")
         beta = e.beta_param
         sa = _address(s0, dev, torch.float32) if s0 is not None and s0.shape == (B, H, d, d) else 0
         if not sa or type(beta) is not nn.Parameter or beta.dtype != torch.float32 or beta.device != dev or beta.shape != (1,) or s0.requires_grad:

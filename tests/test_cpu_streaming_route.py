@@ -74,3 +74,43 @@ def test_an_activation_that_the_block_does_not_have(route):
     for blk in m.blocks:
         blk.mlp.act, blk.mlp.gated = "silu", True               # the layer goes by `gated`
     assert not route(m, IDS)
+
+
+class _Wrapped(torch.nn.Module):
+    def __init__(self, block):
+        super().__init__()
+        self.inner = block
+
+    def forward(self, *a, **k):
+        return self.inner(*a, **k)
+
+
+@pytest.mark.parametrize("efla", [True, False])
+def test_models_without_layers_or_with_other_ones(route, efla):
+    assert not route(model(efla, layers=0), IDS)
+    for i in (0, 1):
+        m = model(efla)
+        m.blocks[i] = _Wrapped(m.blocks[i])
+        assert not route(m, IDS, fresh(model(efla), 2))
+        m = model(efla)
+        name = "efla" if efla else "mlp"
+        setattr(m.blocks[i], name, _Wrapped(getattr(m.blocks[i], name)))
+        assert not route(m, IDS)
+    if efla:
+        m = model(True)
+        m.blocks[0].prism = _Wrapped(m.blocks[0].prism)
+        assert not route(m, IDS)
+
+
+def test_states_that_leave_things_out(route):
+    """What the layers read with ``get`` may be absent, what they do not read may be too, and a layer without a state has ``None``."""
+    m = model(False)
+    assert route(m, IDS, {"pos": 0, "layers": [{}, {}]})
+    assert not route(m, IDS, {"pos": 0, "layers": [None, None]}) and not route(m, IDS, {"pos": 0, "layers": [{}, None]})
+    m = model(True, prism=False)
+    states = [{"efla": s["efla"]} for s in fresh(m, 2)]
+    assert route(m, IDS, states)
+    assert not route(m, IDS, [None, None]) and not route(m, IDS, [states[0], None])
+    m = model(True)
+    states = [{"efla": s["efla"], "prism": s["prism"]} for s in fresh(m, 2)]
+    assert route(m, IDS, states)
