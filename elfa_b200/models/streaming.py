@@ -100,6 +100,8 @@ def gpt_stream(model, ids: torch.Tensor, states: dict):
     ptrs: List[int] = []
     V, N = head.shape[0], (H + 2 * Hkv) * hd
     vec = (D,)
+    if V != model.cfg.model.vocab_size:
+        return None
     if not _weights(dev, ptrs, (tok, (V, D)), (pos, pos.shape if pos is not None else ()), (fin.weight, vec), (fin.bias, vec), (head, (V, D))):
         return None
     if pos is not None and pos.shape[1] != D:
@@ -168,7 +170,7 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
     tail = tail0.shape[1] if tail0 is not None else 0
     ptrs: List[int] = []
     V, vec = head.shape[0], (D,)
-    if not _weights(dev, ptrs, (tok, (V, D)), (fin.weight, vec), (fin.bias, vec), (head, (V, D))):
+    if V != model.cfg.model.vocab_size or not _weights(dev, ptrs, (tok, (V, D)), (fin.weight, vec), (fin.bias, vec), (head, (V, D))):
         return None
     per_layer: List[int] = []
     forget: List[float] = []

@@ -114,3 +114,12 @@ def test_states_that_leave_things_out(route):
     m = model(True)
     states = [{"efla": s["efla"], "prism": s["prism"]} for s in fresh(m, 2)]
     assert route(m, IDS, states)
+
+
+def test_a_table_that_is_not_the_configured_vocabulary(route):
+    """Ids are checked against the configured vocabulary, the table may have more rows."""
+    for efla in (True, False):
+        m = model(efla)
+        m.embed_tokens = torch.nn.Parameter(torch.zeros(80, 64, dtype=torch.bfloat16))
+        m.lm_head = None
+        assert not route(m, IDS)
