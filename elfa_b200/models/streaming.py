@@ -46,7 +46,7 @@ def _same_norms(a, *others) -> bool:
 
 def _address(t: Optional[torch.Tensor], device, dtype=torch.bfloat16) -> int:
     """Where a contiguous, 16-byte aligned tensor lies; 0 for what the kernels cannot take as it is."""
-    if t.dtype != dtype or t.device != device or not t.is_contiguous():
+    if type(t) not in (torch.Tensor, nn.Parameter) or t.dtype != dtype or t.device != device or not t.is_contiguous():
         return 0
     a = t.data_ptr()
     return a if a % 16 == 0 else 0
@@ -199,7 +199,7 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
             pa = _address(p0, dev, torch.float32) if p0 is not None and p0.shape == (B, D // d, d, d) else 0
             if not pa or p0.requires_grad or (ct is not None) != bool(tail):
                 return None
-            if tail and (ct.shape != (B, tail, D) or ct.dtype != torch.bfloat16 or ct.device != dev or ct.stride(2) != 1 or ct.stride(1) != D
+            if tail and (type(ct) is not torch.Tensor or ct.shape != (B, tail, D) or ct.dtype != torch.bfloat16 or ct.device != dev or ct.stride(2) != 1 or ct.stride(1) != D
                          or ct.requires_grad or ct.data_ptr() % 4 or ct.stride(0) % 2):       # read two channels, four bytes, at a time
                 return None
             p1 = torch.empty_like(p0)

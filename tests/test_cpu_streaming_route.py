@@ -123,3 +123,20 @@ def test_a_table_that_is_not_the_configured_vocabulary(route):
         m.embed_tokens = torch.nn.Parameter(torch.zeros(80, 64, dtype=torch.bfloat16))
         m.lm_head = None
         assert not route(m, IDS)
+
+
+def test_states_of_another_tensor_class(route):
+    class Tagged(torch.Tensor):
+        pass
+    for efla in (True, False):
+        m = model(efla)
+        states = fresh(m, 2)
+        if efla:
+            states[1]["efla"] = states[1]["efla"].as_subclass(Tagged)
+        else:
+            states["pos"] = 1
+            for c in states["layers"]:
+                c["k"], c["v"] = (torch.zeros(1, 2, 2, 32, dtype=torch.bfloat16) for _ in range(2))
+            assert route(m, IDS, {"pos": 1, "layers": [dict(c) for c in states["layers"]]})
+            states["layers"][1]["v"] = states["layers"][1]["v"].as_subclass(Tagged)
+        assert not route(m, IDS, states)
