@@ -13,6 +13,7 @@ from typing import List, Optional
 
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 from torch.nn.modules import module as nn_module
 
 from ..native import lib, stream_ptr
@@ -23,12 +24,17 @@ from ..ops.nn import _EW
 _ACTS = {"swiglu": -1, "gelu": 0, **{k: v[0] for k, v in _EW.items() if k != "gelu"}}
 
 
-def _eager(ids: torch.Tensor) -> bool:
-    """Plain eager execution without a gradient, on CUDA token ids."""
-    return (not torch.is_grad_enabled() and type(ids) is torch.Tensor and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() == 2
-            and ids.numel() > 0 and not nn_module._has_any_global_hook() and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
-            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+def _plain_mode() -> bool:
+    """Eager execution without a gradient: no tracing, no dispatch or function mode, no transform, no forward-mode level (which ``no_grad`` leaves
+    open: a state may be a dual tensor, whose tangent the layers refuse to drop)."""
+    return (not torch.is_grad_enabled() and forward_ad._current_level < 0 and not nn_module._has_any_global_hook() and not torch.jit.is_tracing()
+            and not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
             and torch._C._functorch.peek_interpreter_stack() is None)
+
+
+def _eager(ids: torch.Tensor) -> bool:
+    """CUDA token ids in plain eager execution."""
+    return type(ids) is torch.Tensor and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() == 2 and ids.numel() > 0 and _plain_mode()
 
 
 def _plain(module: nn.Module, kind: type) -> bool:

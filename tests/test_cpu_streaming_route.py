@@ -1,7 +1,10 @@
 """Which streaming calls go to native code, decided on the CPU: the native calls are only recorded, so nothing is launched and a call that must not
 get there shows without a device."""
+import contextlib
+
 import pytest
 import torch
+from torch.autograd import forward_ad
 
 from elfa_b200.config import Config
 from elfa_b200.models import streaming
@@ -140,3 +143,22 @@ def test_states_of_another_tensor_class(route):
             assert route(m, IDS, {"pos": 1, "layers": [dict(c) for c in states["layers"]]})
             states["layers"][1]["v"] = states["layers"][1]["v"].as_subclass(Tagged)
         assert not route(m, IDS, states)
+
+
+def test_modes_that_only_the_layers_know():
+    def under(ctx):
+        with torch.no_grad(), ctx:
+            return streaming._plain_mode()
+    assert under(contextlib.nullcontext())
+    assert not streaming._plain_mode()                             # a gradient may be wanted
+    assert not under(forward_ad.dual_level())
+    assert not under(torch.utils._python_dispatch.TorchDispatchMode()) and not under(torch.overrides.TorchFunctionMode())
+    seen = []
+    with torch.no_grad():
+        torch.func.vmap(lambda x: seen.append(streaming._plain_mode()) or x)(torch.zeros(2))
+        torch.func.jvp(lambda x: seen.append(streaming._plain_mode()) or x, (torch.zeros(2),), (torch.ones(2),))
+        torch.jit.trace(lambda x: seen.append(streaming._plain_mode()) or x, torch.zeros(2), check_trace=False)
+        h = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+        seen.append(streaming._plain_mode())
+        h.remove()
+        assert len(seen) == 4 and not any(seen) and streaming._plain_mode()

@@ -1,6 +1,7 @@
 """``forward_with_states`` from native code against the layer-by-layer route: the same kernels in the same order, so the same bits."""
 import pytest
 import torch
+import torch.autograd.forward_ad as fwd
 
 from elfa_b200 import native
 from elfa_b200.config import Config
@@ -120,3 +121,15 @@ def test_tails_at_odd_places(cuda_device, offset, pitch):
         got, now = model.forward_with_states(ids[:, 5:], states)
     assert native.status() == 0 and torch.equal(got, want)
     assert all(torch.equal(a[n], b[n]) for a, b in zip(after, now) for n in a)
+
+
+def test_a_tangent_is_not_dropped(cuda_device):
+    """Forward mode stays open under ``no_grad``: the scan has no such rule and refuses a dual state."""
+    model = EflaModel(_config(True), device=cuda_device).eval()
+    ids = _ids(1, 4, cuda_device)
+    with torch.no_grad():
+        _, states = model.forward_with_states(ids[:, :3])
+        with fwd.dual_level():
+            states[0]["efla"] = fwd.make_dual(states[0]["efla"], torch.ones_like(states[0]["efla"]))
+            with pytest.raises(NotImplementedError):
+                model.forward_with_states(ids[:, 3:], states)
