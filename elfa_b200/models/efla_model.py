@@ -42,6 +42,7 @@ def _identical(*params):
             p.tp_identical = True
 
 
+@streaming.stands_in_for("forward")
 class EflaLayer(nn.Module):
     """Tensor parallel over the heads: ``w_k`` / ``w_v`` column shards (this rank's heads), ``w_o`` the matching row shard whose
     partial products are summed over the group; the scan runs on the local heads only (reference: per-head weights
@@ -81,6 +82,7 @@ class EflaLayer(nn.Module):
         return tpl.row_parallel_linear(o.reshape(B, T, self.H * self.d).to(x.dtype), self.w_o, self.pc), s
 
 
+@streaming.stands_in_for("forward")
 class PrismLayer(nn.Module):
     def __init__(self, cfg: Config, dtype, device):
         super().__init__()
@@ -135,6 +137,7 @@ class PrismLayer(nn.Module):
         return y, new_state, new_tail
 
 
+@streaming.stands_in_for("forward")
 class EflaBlock(nn.Module):
     def __init__(self, cfg: Config, dtype, device, pc: Optional[ParallelContext] = None):
         super().__init__()
@@ -177,6 +180,7 @@ class EflaBlock(nn.Module):
         return out, new_states
 
 
+@streaming.stands_in_for("hidden_states", "_embed", "_logits")
 class EflaModel(nn.Module):
     def __init__(self, cfg: Config, pc: Optional[ParallelContext] = None, device=None):
         super().__init__()

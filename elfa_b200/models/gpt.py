@@ -37,6 +37,7 @@ def _dtype(name: str) -> torch.dtype:
     return {"fp32": torch.float32, "fp16": torch.float16, "bf16": torch.bfloat16, "fp8_e4m3": torch.bfloat16}[name]
 
 
+@streaming.stands_in_for("forward")
 class Norm(nn.Module):
     def __init__(self, dim: int, kind: str, dtype, device):
         super().__init__()
@@ -67,6 +68,7 @@ def _attend_cached(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.T
     return o.reshape(s_, B, H * hd).to(q.dtype)
 
 
+@streaming.stands_in_for("forward")
 class Attention(nn.Module):
     def __init__(self, cfg: Config, pc: ParallelContext, dtype, device, init_std: float, out_std: float):
         super().__init__()
@@ -122,6 +124,7 @@ class Attention(nn.Module):
         return tpl.row_parallel_linear(o, self.w_o, self.pc, quant=self.quant)        # [S(/tp), B, D]
 
 
+@streaming.stands_in_for("forward")
 class MLP(nn.Module):
     def __init__(self, cfg: Config, pc: ParallelContext, dtype, device):
         super().__init__()
@@ -147,6 +150,7 @@ class MLP(nn.Module):
         return tpl.row_parallel_linear(a, self.down, self.pc, quant=self.quant)
 
 
+@streaming.stands_in_for("forward")
 class Block(nn.Module):
     def __init__(self, cfg: Config, pc: ParallelContext, dtype, device, init_std, out_std):
         super().__init__()
@@ -179,6 +183,7 @@ class Block(nn.Module):
         return x, f
 
 
+@streaming.stands_in_for("hidden_states")
 class GPTModel(nn.Module):
     def __init__(self, cfg: Config, pc: Optional[ParallelContext] = None, device=None):
         super().__init__()

@@ -37,9 +37,32 @@ def _eager(ids: torch.Tensor) -> bool:
     return type(ids) is torch.Tensor and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() == 2 and ids.numel() > 0 and _plain_mode()
 
 
+_METHODS = {}          # class -> {name: function}, as the class was written
+_CALL = nn.Module.__call__
+
+
+def stands_in_for(*names: str):
+    """Marks a class whose methods of these names the native call does the work of: replaced on the class or on an instance, they are called again."""
+    def mark(kind: type) -> type:
+        _METHODS[kind] = {n: vars(kind)[n] for n in names}
+        return kind
+    return mark
+
+
+def _as_written() -> bool:
+    """The marked classes still have the methods that they were written with, and modules are called as ever."""
+    return nn.Module.__call__ is _CALL and all(vars(kind).get(n) is f and "__call__" not in vars(kind)
+                                               for kind, methods in _METHODS.items() for n, f in methods.items())
+
+
+def _own_methods(module: nn.Module, kind: type) -> bool:
+    return type(module) is kind and module.__dict__.keys().isdisjoint(_METHODS[kind])
+
+
 def _plain(module: nn.Module, kind: type) -> bool:
     d = module.__dict__
-    return type(module) is kind and "forward" not in d and not d["_forward_hooks"] and not d["_forward_pre_hooks"]
+    return (_own_methods(module, kind) and not d["_forward_hooks"] and not d["_forward_pre_hooks"]
+            and d.get("_compiled_call_impl") is None)
 
 
 def _each_plain(blocks, kind: type) -> bool:
@@ -82,7 +105,7 @@ def _quantised(q) -> bool:
 def gpt_stream(model, ids: torch.Tensor, states: dict):
     """``(logits [B, T, V], states)`` of :meth:`GPTModel.forward_with_states`, or ``None``."""
     from .gpt import MLP, Attention, Block, GPTModel, Norm
-    if not (_eager(ids) and type(model) is GPTModel and model.dtype == torch.bfloat16 and "hidden_states" not in model.__dict__):
+    if not (_eager(ids) and _as_written() and _own_methods(model, GPTModel) and model.dtype == torch.bfloat16):
         return None
     dev = ids.device
     B, S = ids.shape
@@ -153,8 +176,7 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
     """``(logits [B, T, V], states)`` of :meth:`EflaModel.forward_with_states`, or ``None``."""
     from .efla_model import EflaBlock, EflaLayer, EflaModel, PrismLayer
     from .gpt import Norm
-    if not (_eager(ids) and type(model) is EflaModel and model.dtype == torch.bfloat16 and model.pc.tp_size == 1
-            and "hidden_states" not in model.__dict__):
+    if not (_eager(ids) and _as_written() and _own_methods(model, EflaModel) and model.dtype == torch.bfloat16 and model.pc.tp_size == 1):
         return None
     dev = ids.device
     B, T = ids.shape

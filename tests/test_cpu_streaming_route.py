@@ -162,3 +162,29 @@ def test_modes_that_only_the_layers_know():
         seen.append(streaming._plain_mode())
         h.remove()
         assert len(seen) == 4 and not any(seen) and streaming._plain_mode()
+
+
+@pytest.mark.parametrize("efla", [True, False])
+def test_replaced_methods_are_called(route, monkeypatch, efla):
+    m = model(efla)
+    kinds = {type(x) for x in m.modules() if type(x).__module__.startswith("elfa_b200")}
+    assert len(kinds) == 5
+    for kind in kinds:
+        names = ("hidden_states", "_embed", "_logits") if kind is EflaModel else ("hidden_states",) if kind is GPTModel else ("forward",)
+        for name in names:
+            with monkeypatch.context() as p:                       # on the class
+                p.setattr(kind, name, lambda *a, **k: None)
+                assert not route(m, IDS), (kind, name)
+            x = next(x for x in reversed(list(m.modules())) if type(x) is kind)
+            setattr(x, name, lambda *a, **k: None)                  # on one instance
+            assert not route(m, IDS), (kind, name)
+            delattr(x, name)
+        with monkeypatch.context() as p:
+            p.setattr(kind, "__call__", lambda *a, **k: None, raising=False)
+            assert not route(m, IDS) or kind in (EflaModel, GPTModel), kind
+    with monkeypatch.context() as p:
+        p.setattr(torch.nn.Module, "__call__", lambda *a, **k: None)
+        assert not route(m, IDS)
+    m.blocks[1].ln1.compile(backend="eager")
+    assert not route(m, IDS)
+    assert route(model(efla), IDS)
