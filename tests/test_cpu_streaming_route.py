@@ -10,6 +10,8 @@ from elfa_b200.config import Config
 from elfa_b200.models import streaming
 from elfa_b200.models.efla_model import EflaModel
 from elfa_b200.models.gpt import GPTModel
+from elfa_b200.parallel.mesh import ParallelContext
+from elfa_b200.quant.qat import QuantSpec
 
 
 @pytest.fixture
@@ -188,3 +190,41 @@ def test_replaced_methods_are_called(route, monkeypatch, efla):
     m.blocks[1].ln1.compile(backend="eager")
     assert not route(m, IDS)
     assert route(model(efla), IDS)
+
+
+@pytest.mark.parametrize("efla", [True, False])
+def test_hooks_gradients_quantisers_and_parallel_layers(route, efla):
+    def left(change):
+        m = model(efla)
+        change(m, m.blocks[1])
+        return not route(m, IDS)
+    assert not left(lambda m, b: None)
+    assert left(lambda m, b: b.ln1.register_forward_hook(lambda *a: None)) and left(lambda m, b: b.register_forward_pre_hook(lambda *a: None))
+    assert left(lambda m, b: m.final_norm.register_forward_hook(lambda *a, **k: None, with_kwargs=True))
+    assert left(lambda m, b: setattr(b.ln2, "eps", 0.1)) and left(lambda m, b: setattr(m, "dtype", torch.float32))
+    assert left(lambda m, b: setattr(b.ln2, "weight", torch.nn.Parameter(torch.ones(64))))
+    w = "w_k" if efla else "w_o"
+    layer = lambda b: b.efla if efla else b.attn
+    assert left(lambda m, b: setattr(layer(b), w, torch.nn.Parameter(getattr(layer(b), w).t())))                # another layout
+    assert left(lambda m, b: setattr(getattr(layer(b), w), "_gemm_gather", object()))                           # fetched on use
+    two = ParallelContext(tp_size=2)
+    assert left(lambda m, b: setattr(layer(b), "pc", two))
+    if not efla:
+        assert left(lambda m, b: setattr(b.attn, "quant", QuantSpec(fmt="mxfp8"))) and left(lambda m, b: setattr(b.mlp, "quant", QuantSpec(fmt="mxfp8")))
+        assert left(lambda m, b: (setattr(b, "dropout", 0.1), b.train()))
+    else:
+        assert left(lambda m, b: setattr(m, "pc", two))
+    m = model(efla)
+    states = fresh(m, 2)
+    if efla:
+        states[1]["efla"].requires_grad_(True)
+        assert not route(m, IDS, states)
+        states = fresh(m, 2)
+        states[1]["prism"] = states[1]["prism"].double()
+        assert not route(m, IDS, states)
+    else:
+        kv = [torch.zeros(2, 2, 2, 32, dtype=torch.bfloat16) for _ in range(4)]
+        layers = lambda: [dict(k=kv[0], v=kv[1]), dict(k=kv[2], v=kv[3])]
+        assert route(m, IDS, {"pos": 2, "layers": layers()})
+        kv[3] = kv[3].transpose(0, 1)
+        assert not route(m, IDS, {"pos": 2, "layers": layers()})
