@@ -606,10 +606,17 @@ __device__ __noinline__ void efla_fwd_again(const __nv_bfloat16* k, const __nv_b
 //   (efla_combine_kernel: start of segment p + 1 = A_p start_p + B_p)
 //   REST   segments 1 .. P - 1 from their starts, with their outputs
 // The walk in one piece is compiled apart (CUT = false): asking for what may be absent in it cost 5 us of 94.
-// Three times the work in 2 / P of the steps: worth it where the heads alone leave the chip idle (see efla_segments). The maps contract (the
-// eigenvalues of a token's factor lie in (0, 1]), so an error of a start dies out along its segment.
+// Three times the work in 2 / P of the steps: worth it where the heads alone leave the chip idle (see efla_segments). With beta >= 0 the maps
+// contract (the eigenvalues of a token's factor, exp(-beta |k|^2) and 1, lie in (0, 1]), so an error of a start dies out along its segment.
+// beta is learned and may turn negative: then a map of many tokens grows past the range of fp32 where the states that it would multiply are
+// zero, and the heads are walked in one piece: the first CTA of FIRST takes all chunks and the other launches leave at once. The host does not know
+// beta; the sign of a token's coefficient is that of beta.
 // work: start [P], A [P], B [P], each [B H, d, d] fp32.
 enum { EFLA_FIRST, EFLA_REST };
+
+__device__ __forceinline__ bool efla_in_one_piece(const float* __restrict__ coef, int bh, int nchunks) {
+  return !(coef[(long long)bh * nchunks * EC_COEF] >= 0.f);
+}
 
 __device__ __forceinline__ float* efla_work(float* work, int which, int P, int p, int bh, int dd) {
   return work + (((long long)which * P + p) * gridDim.x + bh) * dd;
@@ -623,7 +630,9 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
     float4* __restrict__ ckpt, float* work, int T, int H, int nchunks, int P, int seg, int phase) {
   const int bh = blockIdx.x, z = blockIdx.z;
   EflaWalk w{0, nchunks, false, state0 ? state0 + (long long)bh * D * D : nullptr, state_out ? state_out + (long long)bh * D * D : nullptr};
-  if (CUT) {
+  const bool whole = !CUT || efla_in_one_piece(coef, bh, nchunks);
+  if (CUT && whole && (phase == EFLA_REST || z > 0)) return;
+  if (!whole) {
     const bool map = phase == EFLA_FIRST && z > 0;                       // a segment's A or B
     const int p = phase == EFLA_REST ? z + 1 : (z > P - 2 ? z - (P - 2) : z);
     w.c0 = p * seg;
@@ -649,13 +658,14 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
 // those of the walks (64-bit comparison, B 1, T 8192, 16 heads of 64, 10
 // segments: final state as in one walk). Grid (B * H, d / 16).
 template <int D>
-__global__ void __launch_bounds__(256) efla_combine_kernel(float* __restrict__ work, int P, int dir) {
+__global__ void __launch_bounds__(256) efla_combine_kernel(const float* __restrict__ coef, float* __restrict__ work, int nchunks, int P, int dir) {
   constexpr int EPT = D / 16, DD = D * D, LD = D + 4, VPT = DD / 1024;       // 16-byte vectors of A per thread
   extern __shared__ __align__(16) unsigned char smem[];
   float* sa = reinterpret_cast<float*>(smem);
   float(*ss)[17] = reinterpret_cast<float(*)[17]>(smem + D * LD * 4);
   const int bh = blockIdx.x, col = threadIdx.x & 15, r0 = (threadIdx.x >> 4) * EPT, c = blockIdx.y * 16 + col;
   int p = dir > 0 ? 1 : P - 2;
+  if (efla_in_one_piece(coef, bh, nchunks)) return;
   const float* s0 = efla_work(work, 0, P, p, bh, DD);
   float4 nxt[VPT];
   float bn[EPT];
@@ -711,11 +721,11 @@ __global__ void __launch_bounds__(256) efla_combine_kernel(float* __restrict__ w
 }
 
 template <int D>
-int launch_combine(float* work, int BH, int P, int dir, cudaStream_t s) {
+int launch_combine(const float* coef, float* work, int BH, int nchunks, int P, int dir, cudaStream_t s) {
   if (P < 3) return ELFA_OK;
   constexpr int bytes = (D * (D + 4) + D * 17) * 4;
   ELFA_CUDA(cudaFuncSetAttribute(efla_combine_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  efla_combine_kernel<D><<<dim3(BH, D / 16), 256, bytes, s>>>(work, P, dir);
+  efla_combine_kernel<D><<<dim3(BH, D / 16), 256, bytes, s>>>(coef, work, nchunks, P, dir);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;
@@ -751,7 +761,7 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
   } else {
     walk(EFLA_FIRST, 2 * P - 3);
     ELFA_CUDA(cudaGetLastError());
-    const int rc = launch_combine<D>(work, B * H, P, 1, s);
+    const int rc = launch_combine<D>(coef, work, B * H, nchunks, P, 1, s);
     if (rc != ELFA_OK) return rc;
     walk(EFLA_REST, P - 1);
   }
@@ -871,7 +881,9 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_bwd_state_kerne
     int nchunks, int P, int seg, int phase) {
   const int bh = blockIdx.x, z = blockIdx.z;
   EflaWalk w{0, nchunks, false, dstate_out ? dstate_out + (long long)bh * D * D : nullptr, dstate0 ? dstate0 + (long long)bh * D * D : nullptr};
-  if (CUT) {
+  const bool whole = !CUT || efla_in_one_piece(coef, bh, nchunks);
+  if (CUT && whole && (phase == EFLA_REST || z > 0)) return;
+  if (!whole) {
     const bool map = phase == EFLA_FIRST && z > 0;
     const int p = phase == EFLA_REST ? z : (z == 0 ? P - 1 : (z > P - 2 ? z - (P - 2) : z));
     w.c0 = p * seg;
@@ -1328,7 +1340,7 @@ int launch_chunk_bwd(const void* k, const void* v, const void* nmat, const float
   } else {
     walk(EFLA_FIRST, 2 * P - 3);
     ELFA_CUDA(cudaGetLastError());
-    const int rc = launch_combine<D>(work, B * H, P, -1, s);
+    const int rc = launch_combine<D>(coef, work, B * H, nchunks, P, -1, s);
     if (rc != ELFA_OK) return rc;
     walk(EFLA_REST, P - 1);
   }

@@ -70,6 +70,24 @@ def test_a_bad_value_stays_behind_its_token_and_in_its_column(cuda_device, bad, 
         assert (a.float() - b.float()).abs().max() <= rel * b.float().abs().max()
 
 
+@pytest.mark.parametrize("d", [32, 128])
+@pytest.mark.parametrize("beta,first", [(-3.0, 500), (-0.02, 0), (-1e-6, 0)])
+def test_negative_beta_is_walked_in_one_piece(cuda_device, d, beta, first):
+    """Its maps grow: those of a whole segment leave fp32 where the zero states before the first value would not."""
+    k, v, b, s0, do, ds = _inputs(cuda_device, 2, 530, 3, d)
+    v[:, :first] = 0
+    if first:
+        s0.zero_()
+        do[:, first:], ds = 0, torch.zeros_like(ds)
+        k[:, first:] *= 0.1
+    ins = (k, v, torch.full_like(b, beta), s0, do, ds)
+    want = _run(1, *ins)
+    assert torch.isfinite(want[0]).all() and torch.isfinite(want[1]).all()
+    for P in (2, 3, 16):
+        for x, y in zip(_run(P, *ins), want):
+            torch.testing.assert_close(x, y, rtol=0, atol=0, equal_nan=True)
+
+
 def test_the_rule_gives_segments_that_fit(cuda_device):
     for B, T, H, d in ((1, 8192, 16, 64), (2, 1531, 8, 128), (8, 2048, 16, 64), (1, 113, 4, 32), (1, 1, 1, 64), (64, 4096, 16, 64)):
         n = lib.raw("elfa_efla_segments")(B, T, H, d)
