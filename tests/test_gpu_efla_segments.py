@@ -88,6 +88,20 @@ def test_negative_beta_is_walked_in_one_piece(cuda_device, d, beta, first):
             torch.testing.assert_close(x, y, rtol=0, atol=0, equal_nan=True)
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 1e30])
+@pytest.mark.parametrize("at", [0, 70, 128, 255, 256, 511])
+def test_a_bad_key_reaches_what_it_reaches_in_one_walk(cuda_device, bad, at):
+    """1e30: its square overflows, which leaves the token without an effect. The segments are joined by maps made from such keys."""
+    k, v, beta, s0, do, ds = _inputs(cuda_device, 1, 512, 2, 64)
+    k[0, at, 0, 5] = bad
+    for got, want, rel in zip(_run(4, k, v, beta, s0, do, ds), _run(1, k, v, beta, s0, do, ds), (2 ** -8, 1e-5, 2 ** -8, 2 ** -8, 1e-5)):
+        ok = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(got), ok)
+        got, want = got[ok].float(), want[ok].float()
+        # of the second head's and the other tokens' largest: the overflowing key itself gives outputs and gradients of its own size
+        assert ((got - want).abs() <= rel * want.abs().clamp(min=want.abs().quantile(0.999).item())).all()
+
+
 def test_the_rule_gives_segments_that_fit(cuda_device):
     for B, T, H, d in ((1, 8192, 16, 64), (2, 1531, 8, 128), (8, 2048, 16, 64), (1, 113, 4, 32), (1, 1, 1, 64), (64, 4096, 16, 64)):
         n = lib.raw("elfa_efla_segments")(B, T, H, d)
