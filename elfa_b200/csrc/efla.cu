@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(512) shortconv_sum_kernel(const float* __restr
 }
 
 // ShortConv of T new positions behind the last `tail` ones of a stream, which the layer keeps: u[b, t] from the tail and the new inputs, and tail and
-// inputs side by side as the next tail's source, in one launch (as copies and the ordinary kernel: four). RING: the order of the sums of the
+// inputs side by side as the next tail's source, in one launch, for short blocks (see shortconv_stream_long). RING: the order of the sums of the
 // register-ring kernels (even and odd taps apart), otherwise that of the general one, so that the bits do not depend on how a sequence is cut.
 // A block is 64 channel pairs of one position. grid (B * T, ceil(C / 128))
 template <bool RING>
@@ -544,18 +544,53 @@ ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, 
   return ELFA_OK;
 }
 
+// Whether T positions behind a tail are long enough for the ordinary kernels: tail and inputs are copied side by side, the outputs of the tail's own
+// positions are made and dropped, with several sequences the others are copied together. The one kernel reads 2 W weights per channel pair and
+// position straight from [C, W], where every lane touches another line: long blocks cost it 5 (W 4), 9 (8), 30 (16), 24 (24), 114 (32) and 226 (64)
+// microseconds per 10^6 values. Measured, one kernel / ordinary ones, microseconds: W 4, 1 sequence 2^20 values 6.9 / 6.5, 2^22 21 / 10, 4 sequences
+// 2^22 21 / 26; W 8 2^20 11 / 7 and 11 / 11; W 16 2^17 6.6 / 6.4 and 6.6 / 8.2, 2^18 10.6 / 6.5 and 10.6 / 8.4, 2^22 125 / 13; W 24 2^18 9 / 13,
+// 2^19 15 / 13; W 32 2^17 18 / 16; W 64 2^16 21 / 23, 2^17 33 / 24, 2^22 948 / 81.
+static bool shortconv_stream_long(int B, int T, int C, int W) {
+  const long long values = (long long)B * T * C;
+  if (W < 8) return B == 1 && values >= 1 << 21;
+  if (W < 16) return values >= 1 << 20;
+  return values >= 1 << (W == 16 ? 18 : (W < 32 ? 19 : 17));
+}
+
+// Positions of scratch (C values each) of elfa_shortconv_stream: all of tail and inputs in the long form, otherwise none.
+ELFA_API int elfa_shortconv_stream_rows(int B, int tails, int T, int C, int W) {
+  return B > 0 && tails > 0 && T > 0 && C > 0 && W > 0 && shortconv_stream_long(B, T, C, W) ? B * (tails + T) : 0;
+}
+
 // tail [B, tails, C] (batches tail_stride elements apart), n [B, T, C] -> u [B, T, C] = ShortConv of tail and n side by side, its last T positions,
-// and xin [B, tails + T, C], the two side by side.
-ELFA_API int elfa_shortconv_stream(const void* tail, long long tail_stride, const void* n, const void* w, const void* bias, void* xin, void* u, int B,
-                                   int tails, int T, int C, int W, void* stream) {
-  ELFA_REQUIRE(tail && n && w && xin && u && B > 0 && tails > 0 && T > 0 && (long long)B * T < (1ll << 31) && C > 0 && W > 0, "shortconv_stream: bad arguments");
+// and xin [B, tails + T, C], the two side by side. full: scratch of elfa_shortconv_stream_rows() positions (null when 0); with one sequence u may
+// be full + tails * C, where the long form leaves it anyway.
+ELFA_API int elfa_shortconv_stream(const void* tail, long long tail_stride, const void* n, const void* w, const void* bias, void* xin, void* u,
+                                   void* full, int B, int tails, int T, int C, int W, void* stream) {
+  ELFA_REQUIRE(tail && n && w && xin && u && B > 0 && tails > 0 && T > 0 && (long long)B * (tails + (long long)T) < (1ll << 31) && C > 0 && W > 0,
+               "shortconv_stream: bad arguments");
   ELFA_REQUIRE(C % 2 == 0 && tail_stride % 2 == 0 && W <= 128, "shortconv_stream: channels and batch stride must be even, the window at most 128");
-  for (const void* q : {tail, n, static_cast<const void*>(xin), static_cast<const void*>(u)})
+  for (const void* q : {tail, n, static_cast<const void*>(xin), static_cast<const void*>(u), static_cast<const void*>(full)})
     ELFA_REQUIRE((reinterpret_cast<uintptr_t>(q) & 3) == 0, "shortconv_stream: operands must be 4-byte aligned");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (shortconv_stream_long(B, T, C, W)) {
+    ELFA_REQUIRE(full, "shortconv_stream: this length needs the scratch buffer");
+    const size_t row = (size_t)C * 2, all = (size_t)(tails + T) * row;
+    auto* x = static_cast<unsigned char*>(xin);
+    const auto* f = static_cast<const unsigned char*>(full) + tails * row;
+    const bool apart = B == 1 || tail_stride >= (long long)tails * C;      // or one tail for several sequences
+    for (int b = 0; b < (apart ? 1 : B); ++b)
+      ELFA_CUDA(cudaMemcpy2DAsync(x + b * all, all, static_cast<const unsigned char*>(tail) + b * tail_stride * 2,
+                                  B > 1 && apart ? (size_t)tail_stride * 2 : tails * row, tails * row, apart ? B : 1, cudaMemcpyDeviceToDevice, s));
+    ELFA_CUDA(cudaMemcpy2DAsync(x + tails * row, all, n, T * row, T * row, B, cudaMemcpyDeviceToDevice, s));
+    const int rc = elfa_shortconv_fwd(xin, w, bias, full, B, tails + T, C, W, stream);
+    if (rc == ELFA_OK && u != f) ELFA_CUDA(cudaMemcpy2DAsync(u, T * row, f, all, T * row, B, cudaMemcpyDeviceToDevice, s));
+    return rc;
+  }
   auto kernel = shortconv_ring(W) ? shortconv_stream_kernel<true> : shortconv_stream_kernel<false>;
   const auto h = [](const void* p) { return static_cast<const __nv_bfloat16*>(p); };
-  kernel<<<dim3((unsigned)(B * T), (C + 127) / 128), 64, 0, static_cast<cudaStream_t>(stream)>>>(h(tail), tail_stride, h(n), h(w), h(bias), static_cast<__nv_bfloat16*>(xin),
-                                                                                   static_cast<__nv_bfloat16*>(u), tails, T, C, W);
+  kernel<<<dim3((unsigned)(B * T), (C + 127) / 128), 64, 0, s>>>(h(tail), tail_stride, h(n), h(w), h(bias), static_cast<__nv_bfloat16*>(xin),
+                                                               static_cast<__nv_bfloat16*>(u), tails, T, C, W);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;

@@ -87,7 +87,7 @@ struct EflaDims {
   long long B, T, D, H, d, F, V, layers, L, W, act, kind, prism, tail;
 };
 struct EflaWork {
-  bf16 *x[2], *r, *n, *k, *v, *o, *e, *u, *z, *wc, *q, *h, *g, *f, *nmat;
+  bf16 *x[2], *r, *n, *k, *v, *o, *e, *full, *u, *z, *wc, *q, *h, *g, *f, *nmat;
   float *coef, *segw;
 };
 size_t efla_work(const EflaDims& m, unsigned char* base, EflaWork* w, int segments, bool step) {
@@ -101,7 +101,9 @@ size_t efla_work(const EflaDims& m, unsigned char* base, EflaWork* w, int segmen
   w->v = p.take<bf16>(rows * hd);
   w->o = p.take<bf16>(rows * hd);
   w->e = p.take<bf16>(rows * m.D);
-  w->u = p.take<bf16>(m.prism ? rows * m.D : 0);
+  const long long positions = m.prism && m.tail ? elfa_shortconv_stream_rows((int)m.B, (int)m.tail, (int)m.T, (int)m.D, (int)m.W) : 0;
+  w->full = p.take<bf16>(positions * m.D);
+  w->u = positions && m.B == 1 ? w->full + m.tail * m.D : p.take<bf16>(m.prism ? rows * m.D : 0);
   w->z = p.take<bf16>(m.prism ? rows * 3 * m.L * m.d : 0);
   w->wc = p.take<bf16>(m.prism ? m.D * 3 * m.L * m.d : 0);
   w->q = p.take<bf16>(m.prism ? rows * m.D : 0);
@@ -227,7 +229,8 @@ ELFA_API int elfa_efla_stream(const unsigned long long* p, const long long* dims
     const bf16* y = w.e;
     if (m.prism) {
       if (m.tail)
-        STREAM_CALL(elfa_shortconv_stream(at(q + 16), (long long)p[q + 17], n, at(q + 6), at(q + 7), xin, w.u, B, (int)m.tail, T, D, (int)m.W, stream));
+        STREAM_CALL(elfa_shortconv_stream(at(q + 16), (long long)p[q + 17], n, at(q + 6), at(q + 7), xin, w.u, w.full, B, (int)m.tail, T, D, (int)m.W,
+                                          stream));
       else
         STREAM_CALL(elfa_shortconv_fwd(xin, at(q + 6), at(q + 7), w.u, B, T, D, (int)m.W, stream));
       ConcatArgs a{};

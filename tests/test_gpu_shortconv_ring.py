@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from elfa_b200 import native
+from elfa_b200.native import lib, stream_ptr
 from elfa_b200.ops import efla as eops
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +66,55 @@ def test_nothing_beyond_the_sequence_is_multiplied(cuda_device, T, W, bad):
         for got, ref in zip((y, dx), clean):
             assert torch.equal(got[:, :, other], ref[:, :, other])
         assert torch.equal(dw[other], clean[2][other])
+
+
+def _behind_tail(tail, n, w, b):
+    """The native streaming form: new outputs, and tail and inputs side by side."""
+    (B, tails, C), T, W = tail.shape, n.shape[1], w.shape[1]
+    xin, u = torch.empty(B, tails + T, C, dtype=n.dtype, device=n.device), torch.empty_like(n)
+    rows = lib.raw("elfa_shortconv_stream_rows")(B, tails, T, C, W)
+    full = torch.empty(rows, C, dtype=n.dtype, device=n.device) if rows else None
+    if rows and B == 1:
+        u = full[tails:].view(n.shape)
+    lib.call("elfa_shortconv_stream", tail, tail.stride(0), n, w, b, xin, u, full, B, tails, T, C, W, stream_ptr(n))
+    return u, xin, rows > 0
+
+
+@pytest.mark.parametrize("W,B,C,short,long", [(4, 1, 1024, 2047, 2048), (4, 3, 1024, 2048, None), (5, 1, 66, 40, 31776), (8, 2, 1024, 511, 512), (16, 1, 130, 2016, 2017),
+                                              (16, 3, 512, 170, 171), (24, 2, 256, 1023, 1024), (64, 1, 64, 2047, 2048), (64, 3, 128, 341, 342)])
+@pytest.mark.parametrize("pitch", ["own", "wide", "shared"])
+def test_behind_a_tail_on_both_sides_of_the_line(cuda_device, W, B, C, short, long, pitch):
+    torch.manual_seed(W + C)
+    r = lambda *s: torch.randn(*s, device=cuda_device).bfloat16()
+    w, b = (r(C, W) * W ** -0.5), r(C)
+    for T in (short, long):
+        if T is None:
+            continue
+        tail = r(B, W - 1, C) if pitch == "own" else r(B, W + 3, C)[:, 2:W + 1] if pitch == "wide" else r(1, W - 1, C).expand(B, -1, -1)
+        n = r(B, T, C)
+        u, xin, in_full = _behind_tail(tail, n, w, b)
+        assert native.status() == 0 and in_full == (T == long)
+        whole = torch.cat([tail, n], 1)
+        assert torch.equal(xin, whole) and torch.equal(u, eops.shortconv(whole, w, b)[:, W - 1:])
+
+
+@pytest.mark.parametrize("W,C,T", [(16, 1024, 8192), (64, 1024, 2048), (4, 512, 16384)])
+def test_a_long_block_behind_a_tail_costs_about_what_the_whole_costs(cuda_device, W, C, T):
+    r = lambda *s: torch.randn(*s, device=cuda_device).bfloat16()
+    tail, n, w, b = r(1, W - 1, C), r(1, T, C), r(C, W), r(C)
+    whole = torch.cat([tail, n], 1)
+
+    def us(f):
+        best = []
+        for _ in range(5):
+            torch.cuda.synchronize()
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            for _ in range(10):
+                f()
+            e[1].record()
+            torch.cuda.synchronize()
+            best.append(e[0].elapsed_time(e[1]))
+        return min(best)
+    with torch.no_grad():       # measured 1.2 to 1.7 with the copies; one block per position was 3.5 to 23
+        assert us(lambda: _behind_tail(tail, n, w, b)) < 3 * us(lambda: eops.shortconv(whole, w, b))
