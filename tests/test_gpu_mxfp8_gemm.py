@@ -61,6 +61,30 @@ def test_mxfp8_gemm_epilogue():
     assert (y.float() - gelu_tanh_ref(ref_pre)).abs().max() <= 2 ** -7 * ref_pre.abs().max() + 1e-3
 
 
+@pytest.mark.parametrize("K", [256, 1536, 1568])                         # 2, 12 and 13 blocks of K: eight epilogue warps up to 12 where 192 wide
+@pytest.mark.parametrize("bn,bias", [(384, False), (384, True), (512, False), (0, False), (0, True)])
+def test_mxfp8_pair_tiles_with_every_epilogue(K, bn, bias):
+    """16 x 16 or 16 x 22 pair tiles, ragged both ways: a pair walks at least three, so that both accumulators and the columns that they share are used
+    again. Bounds as above: the output's rounding, and the activation's hardware tanh."""
+    from elfa_b200 import native
+    from elfa_b200.ops import gemm_mxfp8 as q
+    from elfa_b200.ops.gemm import gelu_tanh_ref
+    M, N = 4000, 4072
+    x, w = _operands(M, N, K, K + bn)
+    x, w = x * 0.05, w * 0.05
+    b = torch.randn(N, device="cuda").bfloat16() if bias else None
+    xq, _ = q.quantize_mxfp8(x)
+    wq, _ = q.quantize_mxfp8(w, right=True)
+    pre = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    y = q.gemm_mxfp8(xq, wq, bias=b, gelu=True, preact=pre, force_bn=bn)
+    plain = q.gemm_mxfp8(xq, wq, bias=b, force_bn=bn)
+    assert native.status() == 0 and torch.equal(plain, pre)
+    ref = (q.dequantize_ref(xq).double() @ q.dequantize_ref(wq).double().t()) + (b.double() if bias else 0)
+    big = ref.abs().max()
+    assert ((pre.double() - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -18 * big).all()
+    assert ((y.double() - gelu_tanh_ref(ref)).abs() <= 2 ** -7 * ref.abs() + 2 ** -18 * big).all()
+
+
 @pytest.mark.parametrize("act", [None, "gelu"])
 def test_quant_linear_block_scaled_path_equals_fake_quant_path(act):
     from elfa_b200.parallel.mesh import ParallelContext
