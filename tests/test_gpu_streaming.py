@@ -8,6 +8,7 @@ from elfa_b200.config import Config
 from elfa_b200.models import streaming
 from elfa_b200.models.efla_model import EflaModel
 from elfa_b200.models.gpt import GPTModel
+from elfa_b200.native import lib
 
 pytestmark = pytest.mark.gpu
 
@@ -75,6 +76,16 @@ def test_softmax_family(cuda_device, monkeypatch, act, norm, H, Hkv, hd, tie, po
 def test_efla_family(cuda_device, monkeypatch, act, norm, hd, L, W, prism, B, cuts):
     torch.manual_seed(0)
     model = EflaModel(_config(True, act, norm, 2, 2, hd, L, W, prism), device=cuda_device).eval()
+    _compare(monkeypatch, model, _ids(B, cuts[-1], cuda_device), cuts, len(cuts) - 1)
+
+
+@pytest.mark.parametrize("B,H,hd,cuts", [(2, 2, 64, (0, 100, 1137, 2210)), (1, 2, 128, (0, 1500, 1501, 2535))])
+def test_efla_calls_that_are_walked_in_segments(cuda_device, monkeypatch, B, H, hd, cuts):
+    """The scratch of the segments is a piece of the one workspace of all layers; carried states, ragged last chunks, a tail in front."""
+    cut = [lib.raw("elfa_efla_segments")(B, hi - lo, H, hd) for lo, hi in zip(cuts, cuts[1:])]
+    assert sum(c > 1 for c in cut) >= 2, cut
+    torch.manual_seed(0)
+    model = EflaModel(_config(True, H=H, hd=hd, W=16), device=cuda_device).eval()
     _compare(monkeypatch, model, _ids(B, cuts[-1], cuda_device), cuts, len(cuts) - 1)
 
 
