@@ -22,8 +22,8 @@
 // reference: the op is defined by src/futhark/attention.fut:28-51; the reference ships no
 // attention backward at all.
 //
-// Roles per CTA: warp 0 TMA, warp 1 MMA issue, warp 2 row vectors (key-tile pass), the rest compute (warps w and w + 4 share a
-// tensor-memory lane quarter and split the columns).
+// Roles per CTA: warp 0 TMA, warp 1 MMA issue, warp 2 row vectors (key-tile pass), the rest compute: the four (key-tile pass) or two warps with
+// the same number modulo 4 share a tensor-memory lane quarter and split the columns.
 #include <atomic>
 #include <type_traits>
 
@@ -483,7 +483,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
       auto hand_over = [&](uint32_t at, const uint32_t (&t)[HC / 2], int bar_id, int piece) {
         const uint32_t dst = at + lane_addr + colw + piece * (HC / 2);
         __syncwarp();                    // one lane's arrival for the piece before: the stores want the warp together
-        if constexpr (HC == 64) tmem_st32(dst, t); else if constexpr (HC == 32) tmem_st16(dst, t); else tmem_st8(dst, t);
+        static_assert(HC == 64 || HC == 16, "the stores that follow");
+        if constexpr (HC == 64) tmem_st32(dst, t); else tmem_st8(dst, t);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();

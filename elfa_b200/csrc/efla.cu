@@ -511,7 +511,7 @@ static int shortconv_span(int B, int T, int C) {
 }
 static bool shortconv_ring(int W) { return W == 4 || W == 8 || W == 16; }
 
-// Slices of the weight-gradient scratch of elfa_shortconv_bwd (slices * (W + 1) * C floats), 0 when it needs none.
+// Slices of the weight-gradient scratch of elfa_shortconv_bwd_as (slices * (W + 1) * C floats), 0 when it needs none.
 ELFA_API int elfa_shortconv_bwd_slices(int B, int T, int C, int W) {
   if (!shortconv_ring(W) || B <= 0 || T <= 0 || C <= 0) return 0;
   const int span = shortconv_span(B, T, C);
@@ -596,13 +596,8 @@ ELFA_API int elfa_shortconv_stream(const void* tail, long long tail_stride, cons
   return ELFA_OK;
 }
 
-// dx bf16 [B,T,C]; dw fp32 [C,W]; db fp32 [C] or null; part: scratch of elfa_shortconv_bwd_slices() * (W + 1) * C floats (null when 0).
-ELFA_API int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, float* part, int B, int T,
-                                int C, int W, void* stream) {
-  return elfa_shortconv_bwd_as(x, w, dy, dx, dw, db, part, 0, B, T, C, W, stream);
-}
-
-// The same with the weight and bias gradients in bf16 where `grads_bf16`, windows of 4, 8 and 16 only.
+// dx bf16 [B,T,C]; dw [C,W] and db [C] (or null) in fp32, or in bf16 where `grads_bf16` (windows of 4, 8 and 16 only); part: scratch of
+// elfa_shortconv_bwd_slices() * (W + 1) * C floats (null when 0).
 ELFA_API int elfa_shortconv_bwd_as(const void* x, const void* w, const void* dy, void* dx, void* dw_, void* db_, float* part, int grads_bf16,
                                    int B, int T, int C, int W, void* stream) {
   float *dw = static_cast<float*>(dw_), *db = static_cast<float*>(db_);

@@ -227,8 +227,6 @@ int elfa_shortconv_stream(const void* tail, long long tail_stride, const void* n
 int elfa_shortconv_bwd_slices(int B, int T, int C, int W);
 int elfa_shortconv_bwd_as(const void* x, const void* w, const void* dy, void* dx, void* dw, void* db, float* part, int grads_bf16, int B, int T,
                           int C, int W, void* stream);
-int elfa_shortconv_bwd(const void* x, const void* w, const void* dy, void* dx, float* dw, float* db, float* part, int B, int T, int C,
-                       int W, void* stream);
 
 // ---- stream.cu ---------------------------------------------------------------------------------
 int elfa_gpt_stream_work(const long long* dims);
