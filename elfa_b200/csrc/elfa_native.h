@@ -97,6 +97,7 @@ int elfa_attention_bwd(const void* qkv, long long stride_s, long long stride_b, 
                        long long d_stride_s, long long d_stride_b, int S, int B, int H, int hd, float scale, int causal,
                        void* stream);
 
+int elfa_attention_bwd_shares(int S, int B, int H, int Hkv, int hd, int causal);
 int elfa_attention_bwd_ex(const void* qkv, long long stride_s, long long stride_b, const void* out, const void* dout,
                           long long o_stride_s, long long o_stride_b, const float* lse, float* delta, void* dqkv,
                           long long d_stride_s, long long d_stride_b, int S, int B, int H, int Hkv, int hd, float scale, int causal,
