@@ -37,40 +37,33 @@ def _eager(ids: torch.Tensor) -> bool:
     return type(ids) is torch.Tensor and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() == 2 and ids.numel() > 0 and _plain_mode()
 
 
-_METHODS = {}          # class -> {name: function}, as the class was written
+_WRITTEN = []           # (attributes of a class, name, function), as the classes were written; live views of the attributes
 _CALL = nn.Module.__call__
 
 
 def stands_in_for(*names: str):
     """Marks a class whose methods of these names the native call does the work of: replaced on the class or on an instance, they are called again."""
     def mark(kind: type) -> type:
-        _METHODS[kind] = {n: vars(kind)[n] for n in names}
+        _WRITTEN.extend((vars(kind), n, vars(kind)[n]) for n in names)
         return kind
     return mark
 
 
 def _as_written() -> bool:
     """The marked classes still have the methods that they were written with, and modules are called as ever."""
-    return nn.Module.__call__ is _CALL and all(vars(kind).get(n) is f and "__call__" not in vars(kind)
-                                               for kind, methods in _METHODS.items() for n, f in methods.items())
-
-
-def _own_methods(module: nn.Module, kind: type) -> bool:
-    return type(module) is kind and module.__dict__.keys().isdisjoint(_METHODS[kind])
+    for attributes, name, f in _WRITTEN:
+        if attributes.get(name) is not f or "__call__" in attributes:
+            return False
+    return nn.Module.__call__ is _CALL
 
 
 def _plain(module: nn.Module, kind: type) -> bool:
     d = module.__dict__
-    return (_own_methods(module, kind) and not d["_forward_hooks"] and not d["_forward_pre_hooks"]
-            and d.get("_compiled_call_impl") is None)
+    return type(module) is kind and "forward" not in d and not d["_forward_hooks"] and not d["_forward_pre_hooks"] and "_compiled_call_impl" not in d
 
 
-def _each_plain(blocks, kind: type) -> bool:
-    return len(blocks) > 0 and all(_plain(b, kind) for b in blocks)
-
-
-def _same_norms(a, *others) -> bool:
-    return all(n.kind == a.kind and n.eps == a.eps for n in others)
+def _same_norms(a, b, c) -> bool:
+    return a.kind == b.kind == c.kind and a.eps == b.eps == c.eps
 
 
 def _address(t: Optional[torch.Tensor], device, dtype=torch.bfloat16) -> int:
@@ -87,8 +80,11 @@ def _weights(device, out: List[int], *params) -> bool:
         if w is None:
             out.append(0)
             continue
-        a = _address(w, device) if type(w) is nn.Parameter and w.shape == shape and not hasattr(w, "_gemm_gather") else 0
-        if not a:
+        if type(w) is not nn.Parameter or w.shape != shape or w.dtype != torch.bfloat16 or w.device != device or not w.is_contiguous() \
+                or "_gemm_gather" in w.__dict__:
+            return False
+        a = w.data_ptr()
+        if a % 16:
             return False
         out.append(a)
     return True
@@ -105,15 +101,15 @@ def _quantised(q) -> bool:
 def gpt_stream(model, ids: torch.Tensor, states: dict):
     """``(logits [B, T, V], states)`` of :meth:`GPTModel.forward_with_states`, or ``None``."""
     from .gpt import MLP, Attention, Block, GPTModel, Norm
-    if not (_eager(ids) and _as_written() and _own_methods(model, GPTModel) and model.dtype == torch.bfloat16):
+    if not (_eager(ids) and _as_written() and type(model) is GPTModel and "hidden_states" not in model.__dict__ and model.dtype == torch.bfloat16):
         return None
     dev = ids.device
     B, S = ids.shape
     tok, pos, fin, blocks = model.embed_tokens, model.pos_embed, model.final_norm, model.blocks
     head = model.lm_head if model.lm_head is not None else tok
     pos0, D = states["pos"], tok.shape[1]
-    if not _plain(fin, Norm) or not _each_plain(blocks, Block) or len(states["layers"]) != len(blocks) \
-            or any(type(c) is not dict for c in states["layers"]) or (pos is not None and pos0 + S > pos.shape[0]) or model.vocab_lo != 0:
+    if not _plain(fin, Norm) or not len(blocks) or not _plain(blocks[0], Block) or len(states["layers"]) != len(blocks) \
+            or type(states["layers"][0]) is not dict or (pos is not None and pos0 + S > pos.shape[0]) or model.vocab_lo != 0:
         return None
     first, cache0 = blocks[0], states["layers"][0]
     if not (_plain(first.attn, Attention) and _plain(first.mlp, MLP)):
@@ -138,6 +134,8 @@ def gpt_stream(model, ids: torch.Tensor, states: dict):
     outs = []
     per_layer: List[int] = []
     for blk, cache in zip(blocks, states["layers"]):
+        if not _plain(blk, Block) or type(cache) is not dict:
+            return None
         a, m, n1, n2 = blk.attn, blk.mlp, blk.ln1, blk.ln2
         if not (_plain(a, Attention) and _plain(m, MLP) and _plain(n1, Norm) and _plain(n2, Norm)) \
                 or a.pc.tp_size != 1 or a.pc.cp_size != 1 or _quantised(a.quant) or _quantised(m.quant) or (blk.dropout > 0 and blk.training) \
@@ -176,13 +174,14 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
     """``(logits [B, T, V], states)`` of :meth:`EflaModel.forward_with_states`, or ``None``."""
     from .efla_model import EflaBlock, EflaLayer, EflaModel, PrismLayer
     from .gpt import Norm
-    if not (_eager(ids) and _as_written() and _own_methods(model, EflaModel) and model.dtype == torch.bfloat16 and model.pc.tp_size == 1):
+    if not (_eager(ids) and _as_written() and type(model) is EflaModel
+            and model.__dict__.keys().isdisjoint(("hidden_states", "_embed", "_logits")) and model.dtype == torch.bfloat16 and model.pc.tp_size == 1):
         return None
     dev = ids.device
     B, T = ids.shape
     tok, fin, blocks = model.embed_tokens, model.final_norm, model.blocks
     head = model.lm_head if model.lm_head is not None else tok
-    if not _plain(fin, Norm) or not _each_plain(blocks, EflaBlock) or len(states) != len(blocks) or any(type(s) is not dict for s in states):
+    if not _plain(fin, Norm) or not len(blocks) or not _plain(blocks[0], EflaBlock) or len(states) != len(blocks) or type(states[0]) is not dict:
         return None
     D, first = tok.shape[1], blocks[0]
     if not _plain(first.efla, EflaLayer) or (first.prism is not None and not _plain(first.prism, PrismLayer)):
@@ -202,8 +201,11 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
         return None
     per_layer: List[int] = []
     forget: List[float] = []
+    numbers, gate = tuple(str(i) for i in range(L)), (D, d)
     new_states = []
     for blk, st in zip(blocks, states):
+        if not _plain(blk, EflaBlock) or type(st) is not dict:
+            return None
         e, pr, n1, n2 = blk.efla, blk.prism, blk.ln1, blk.ln2
         if not (_plain(e, EflaLayer) and _plain(n1, Norm) and _plain(n2, Norm)) or blk.pc.tp_size != 1 or e.pc.tp_size != 1 \
                 or (pr is not None) != prism or (prism and not (_plain(pr, PrismLayer) and pr.L == L and pr.d == d)) \
@@ -234,9 +236,10 @@ def efla_stream(model, ids: torch.Tensor, states: List[dict]):
             xin = torch.empty((B, tail + T, D), dtype=torch.bfloat16, device=dev)
             new_tail = xin[:, -(W - 1):] if W > 1 else None
             per_layer += (pa, p1.data_ptr(), ct.data_ptr() if tail else 0, ct.stride(0) if tail else 0, xin.data_ptr())
-            gates = [(w, (D, d)) for w in (*pr.w_p, *pr.w_beta, *pr.w_k)]
-            if not (len(pr.w_p) == len(pr.w_beta) == len(pr.w_k) == L) or not _weights(dev, per_layer, *gates):
-                return None
+            for ws in (pr.w_p, pr.w_beta, pr.w_k):
+                own = ws._parameters               # by position; indexing the list looks each one up by name, a microsecond apiece
+                if tuple(own) != numbers or len(ws) != L or not _weights(dev, per_layer, *[(w, gate) for w in own.values()]):
+                    return None
             forget.append(float(pr.forget))
         else:
             if p0 is not None:
