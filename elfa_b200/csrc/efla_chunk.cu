@@ -1365,6 +1365,9 @@ using namespace elfa;
 // per head dimension: a step with one CTA per SM, with as many as its registers and shared memory hold (whole rounds beyond), and the
 // two launches and joints more. B 1 x 8192, 16 heads of 64: P 1 355 us, 6 150, 8 146, 10 128, 12 160 (a second round); B 2 x 1531, 8 heads of 128: P 1
 // 109, 4 98, 5 93, 6 101; B 4 x 1024, 8 heads of 128: P 1 78, 3 88 (not cut); B 8 x 2048, 16 heads of 64: P 1 118, 3 165 (not cut).
+// The walk of the state gradient is cut alike: on eleven shapes its best number is the forward walk's, or within 3 % of it (kernels alone, forward /
+// state gradient, us: B 1 x 8192, 16 heads of 64, P 1 337 / 358, 8 126 / 127, 10 109 / 109, 12 140 / 134; B 2 x 1531, 8 heads of 128, P 1 100 / 111, 4 86 / 91,
+// 5 82 / 83, 6 89 / 92; B 4 x 1024, 8 heads of 128, P 1 69 / 75, 3 78 / 81; B 1 x 4096, 16 heads of 32, P 1 161 / 138, 10 42 / 45, 16 39 / 41).
 ELFA_API int elfa_efla_segments(int B, int T, int H, int d) {
   const int nchunks = (T + EC - 1) / EC, sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const long long units = (long long)B * H * (d == 128 || d == 96 ? 2 : 1);

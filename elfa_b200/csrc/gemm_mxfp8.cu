@@ -510,8 +510,9 @@ int launch_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& 
 }
 
 // Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile (cycles: the fill of shared memory per K block, and the wait
-// for the shared columns). Of 36 shapes (M 1500 to 16384, N 3072 to 11008, K 1024 to 4096) it misses the faster tile in three, by 3 % at most. Measured (us, 192 / 256 wide): 4096 x 11008 x 4096
-// 155 / 138, 2048 x 4096 x 4096 38 / 31, 1500 x 4096 x 4096 28 / 30 (both one round: the narrow one).
+// for the shared columns). Of 43 shapes (M 512 to 16384, N 3072 to 11008, K 1024 to 4096) it misses the faster tile in five, by 5 % at most. Measured (us,
+// 192 / 256 wide, GELU): 4096 x 11008 x 4096 160 / 139, 2048 x 4096 x 4096 42 / 32 and 1024 x 4096 x 4096 29 / 19 (two rounds against one),
+// 1500 x 4096 x 4096 31.1 / 30.6 (two rounds each: the narrow one), 512 x 7104 one round each, x 1024 9.9 / 10.2, x 4096 20 / 19 (the narrow one).
 bool wide_pair(int M, int N, int K) {
   const long long pairs = device_sm_count() / 2, tm = (M + 255) / 256, kt = (K + QBK - 1) / QBK;
   const long long r256 = (tm * ((N + 255) / 256) + pairs - 1) / pairs, r192 = (tm * ((N + 191) / 192) + pairs - 1) / pairs;
