@@ -557,6 +557,19 @@ static bool shortconv_stream_long(int B, int T, int C, int W) {
   return values >= 1 << (W == 16 ? 18 : (W < 32 ? 19 : 17));
 }
 
+// `bytes` of each of B batches. One copy of rows wants them apart and a pitch below 2^31 bytes (a block of a million positions of 1024 values is
+// past it); one tail shared by several sequences, and longer blocks, go one by one.
+static cudaError_t copy_batches(void* dst, size_t dpitch, const void* src, size_t spitch, size_t bytes, int B, cudaStream_t s) {
+  if (B > 1 && spitch >= bytes && dpitch < (1ull << 31) && spitch < (1ull << 31))
+    return cudaMemcpy2DAsync(dst, dpitch, src, spitch, bytes, B, cudaMemcpyDeviceToDevice, s);
+  for (int b = 0; b < B; ++b) {
+    const cudaError_t e = cudaMemcpyAsync(static_cast<unsigned char*>(dst) + b * dpitch, static_cast<const unsigned char*>(src) + b * spitch, bytes,
+                                          cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 // Positions of scratch (C values each) of elfa_shortconv_stream: all of tail and inputs in the long form, otherwise none.
 ELFA_API int elfa_shortconv_stream_rows(int B, int tails, int T, int C, int W) {
   return B > 0 && tails > 0 && T > 0 && C > 0 && W > 0 && shortconv_stream_long(B, T, C, W) ? B * (tails + T) : 0;
@@ -578,13 +591,10 @@ ELFA_API int elfa_shortconv_stream(const void* tail, long long tail_stride, cons
     const size_t row = (size_t)C * 2, all = (size_t)(tails + T) * row;
     auto* x = static_cast<unsigned char*>(xin);
     const auto* f = static_cast<const unsigned char*>(full) + tails * row;
-    const bool apart = B == 1 || tail_stride >= (long long)tails * C;      // or one tail for several sequences
-    for (int b = 0; b < (apart ? 1 : B); ++b)
-      ELFA_CUDA(cudaMemcpy2DAsync(x + b * all, all, static_cast<const unsigned char*>(tail) + b * tail_stride * 2,
-                                  B > 1 && apart ? (size_t)tail_stride * 2 : tails * row, tails * row, apart ? B : 1, cudaMemcpyDeviceToDevice, s));
-    ELFA_CUDA(cudaMemcpy2DAsync(x + tails * row, all, n, T * row, T * row, B, cudaMemcpyDeviceToDevice, s));
+    ELFA_CUDA(copy_batches(x, all, tail, (size_t)tail_stride * 2, tails * row, B, s));
+    ELFA_CUDA(copy_batches(x + tails * row, all, n, T * row, T * row, B, s));
     const int rc = elfa_shortconv_fwd(xin, w, bias, full, B, tails + T, C, W, stream);
-    if (rc == ELFA_OK && u != f) ELFA_CUDA(cudaMemcpy2DAsync(u, T * row, f, all, T * row, B, cudaMemcpyDeviceToDevice, s));
+    if (rc == ELFA_OK && u != f) ELFA_CUDA(copy_batches(u, T * row, f, all, T * row, B, s));
     return rc;
   }
   auto kernel = shortconv_ring(W) ? shortconv_stream_kernel<true> : shortconv_stream_kernel<false>;

@@ -118,3 +118,18 @@ def test_a_long_block_behind_a_tail_costs_about_what_the_whole_costs(cuda_device
         return min(best)
     with torch.no_grad():       # measured 1.2 to 1.7 with the copies; one block per position was 3.5 to 23
         assert us(lambda: _behind_tail(tail, n, w, b)) < 3 * us(lambda: eops.shortconv(whole, w, b))
+
+
+@pytest.mark.parametrize("B", [1, 2])
+def test_a_block_of_two_gigabytes_behind_a_tail(cuda_device, B):
+    """Past the largest pitch of a copy of rows. Values that bf16 sums exactly, so that a wrong place cannot hide."""
+    T, C, W = (1 << 20) + 3, 1024, 16
+    ramp = torch.arange(T, device=cuda_device) % 61
+    n = ramp.to(torch.bfloat16).view(1, T, 1).expand(B, T, C).contiguous()
+    tail = torch.full((B, W - 1, C), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    w = torch.zeros(C, W, dtype=torch.bfloat16, device=cuda_device)
+    w[:, W - 1] = 1
+    u, xin, in_full = _behind_tail(tail, n, w, torch.zeros(C, dtype=torch.bfloat16, device=cuda_device))
+    assert native.status() == 0 and in_full
+    assert (xin[:, :W - 1] == 7).all() and torch.equal(xin[:, W - 1:], n)
+    assert (u[:, :W - 1] == 7).all() and torch.equal(u[:, W - 1:], n[:, :T - W + 1])
