@@ -1144,7 +1144,7 @@ ELFA_API int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
   auto whole16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (M <= SKINNY_ROWS && !a_mn_major && K % 8 == 0 && force_bn == 0 && max_ctas <= 0 &&
       !(flags & ~(ELFA_EPI_BIAS | ELFA_EPI_GELU | ELFA_EPI_STORE_PREACT)) && whole16(A) && whole16(B) && whole16(C) &&
-      (!(flags & ELFA_EPI_STORE_PREACT) || whole16(preact))) {
+      (!(flags & ELFA_EPI_STORE_PREACT) || whole16(preact)) && gemm_skinny_better(M, N, K)) {
     const SkinnyParams q{static_cast<const __nv_bfloat16*>(A), static_cast<const __nv_bfloat16*>(B), static_cast<const __nv_bfloat16*>(bias),
                          static_cast<__nv_bfloat16*>(C), static_cast<__nv_bfloat16*>(preact), lda, ldb, ldc, ldpre, M, N, K, alpha, flags};
     return launch_gemm_skinny(q, b_mn_major != 0, static_cast<cudaStream_t>(stream));

@@ -2,8 +2,8 @@
 // operands, fp32 sums. The matrix is read once with 16-byte loads and that read is the cost, so the matrix is the left operand of
 // mma.sync m16n8k16 (its output index runs along the 16 rows) and the rows of A are its eight columns: a loaded vector needs no conversion (or one
 // byte permutation per register) and eight rows cost what one costs. A tcgen05 tile of 128 rows does sixteen rows of padding for each
-// real one and leaves most SMs idle (8 to 32 tiles). Four rows, microseconds here / in such tiles: 1536 x 1024 4.2 / 8.1, 4096 x 1024 5.3 / 8.2, 1024 x 4096
-// 7.0 / 20, 4096 x 11008 20 / 49, and with the contraction contiguous 32000 x 1024 16 / 20; eight rows take 0 to 15 % more. With packed
+// real one and leaves most SMs idle (8 to 32 tiles). Four rows, microseconds here / in such tiles: 1536 x 1024 4.2 / 8.3, 4096 x 1024 5.9 / 8.9, 1024 x 4096
+// 7.4 / 21, 4096 x 11008 20 / 50, and with the contraction contiguous 11008 x 4096 22 / 37, 32000 x 1024 15 / 22; eight rows take 0 to 10 % more. With packed
 // multiply-adds instead of products, eight rows of 4096 x 1024 took 16 us.
 //
 // The sums are short (a warp's share of the contraction) and joined in fp32: of the outputs, as many as lie beside the bf16 value nearest to the 64-bit product,
@@ -14,6 +14,7 @@
 //
 // reference: src/eval/evaluator.zig:419-470 (generation, one token at a time).
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "elfa_native.h"
@@ -143,11 +144,13 @@ __global__ void __launch_bounds__(256) skinny_nn_kernel(const SkinnyParams p, in
 
 // B [N, K], contraction contiguous. A warp owns 16 columns: thread (g, q) loads 16 bytes of rows g and g + 8 of B, k = 8 q .., which are the
 // fragments of two products (k 8 q .. 8 q + 3 and 8 q + 4 .. 8 q + 7 of every q), and the same of row g of A. WK warps of a CTA share 16 columns,
-// 32 values of k each in turn, where there are few columns.
-template <int WK>
+// 32 J values of k each in turn, where there are few columns: with J = 4 or 2 a warp asks for whole lines (J = 1, for short contractions: half of
+// one). N 9480, K 4096: WK 4, J 1 / 2 25 / 20 us; N 32000, K 1024: WK 8, J 1 / 4 16.6 / 15.0 us.
+template <int WK, int J>
 __global__ void __launch_bounds__(256) skinny_nt_kernel(const SkinnyParams p) {
   __shared__ __align__(16) float part[8][8][20];       // [warp][row of A][column]
   constexpr int UN = 4;                                // 32 values of k each, in flight
+  static_assert(UN % J == 0, "steps of a warp");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int group = warp / WK, n0 = (blockIdx.x * (8 / WK) + group) * 16;
   const bool in0 = n0 + g < p.N, in1 = n0 + g + 8 < p.N;
@@ -155,11 +158,11 @@ __global__ void __launch_bounds__(256) skinny_nt_kernel(const SkinnyParams p) {
   float acc[2][4] = {};
   pdl_wait();
   pdl_next();
-  for (int kb = warp % WK * 32; kb < p.K; kb += WK * UN * 32) {
+  for (int kb = warp % WK * (32 * J); kb < p.K; kb += WK * UN * 32) {
     uint4 w0[UN], w1[UN], x[UN];
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
-      const int k = kb + u * WK * 32;
+      const int k = kb + u / J * (WK * 32 * J) + u % J * 32;
       const bool in = k + 8 * q < p.K;
       w0[u] = w1[u] = x[u] = make_uint4(0, 0, 0, 0);
       if (in && in0) w0[u] = ld_stream(b0 + k);
@@ -177,34 +180,100 @@ __global__ void __launch_bounds__(256) skinny_nt_kernel(const SkinnyParams p) {
   for (int i = 0; i < 4; ++i) part[warp][2 * q + (i & 1)][g + (i >> 1) * 8] = acc[0][i] + acc[1][i];
   if (WK > 1) __syncthreads();
   else __syncwarp();
-  for (int i = (WK > 1 ? threadIdx.x : lane); i < p.M * 2; i += WK > 1 ? 256 : 32) {       // WK is 1 or 8
-    const int m = i / 2, c = i % 2 * 8;
+  constexpr int GROUPS = WK > 1 ? 8 / WK : 1;          // of 16 columns, added up by the CTA, or by each warp its own
+  for (int i = (WK > 1 ? threadIdx.x : lane); i < p.M * 2 * GROUPS; i += WK > 1 ? 256 : 32) {
+    const int m = i / (2 * GROUPS), at = i / 2 % GROUPS, c = i % 2 * 8, first = WK > 1 ? at * WK : warp;
+    const int n = WK > 1 ? (blockIdx.x * GROUPS + at) * 16 : n0;
     float f[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      f[j] = part[WK > 1 ? 0 : warp][m][c + j];
+      f[j] = part[first][m][c + j];
 #pragma unroll
-      for (int w = 1; w < WK; ++w) f[j] += part[w][m][c + j];
+      for (int w = 1; w < WK; ++w) f[j] += part[first + w][m][c + j];
     }
-    if (n0 + c < p.N) skinny_store(p, m, n0 + c, f);
+    if (n + c < p.N) skinny_store(p, m, n + c, f);
   }
+}
+
+// Clusters of n CTAs that run at once (0 where the runtime does not say), asked once per width and size: SMs that do not fill a cluster are left out.
+int skinny_room(bool narrow, int n) {
+  static std::atomic<int> known[2][9];
+  int v = known[narrow][n].load(std::memory_order_relaxed);
+  if (v == 0) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1, n);
+    cfg.blockDim = dim3(256);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.y = n;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&v, narrow ? skinny_nn_kernel<1> : skinny_nn_kernel<2>, &cfg) != cudaSuccess || v <= 0) {
+      cudaGetLastError();
+      v = -1;
+    }
+    known[narrow][n].store(v, std::memory_order_relaxed);
+  }
+  return v > 0 ? v : 0;
+}
+
+// How a [K, N] matrix is cut: in as many slices (1, 2, 3, 4 or 8 of at least 256 rows; of 128 where SMs are idle otherwise) as run at once, in the width that
+// fills more of the room; past one round whole columns of 128. One slice too many starts a second round. Four to eight rows, us: N 8192, K 4096, 128 wide
+// 4 / 8 slices 15 / 19; N 11008, K 4096, 3 / 4 20 / 30; N 32000, K 4096, 1 / 2 45 / 52; N 6144, K 2048, 64 wide 4 / 128 wide 8 9.3 / 15;
+// N 12288, K 8192, 64 wide 2 / 128 wide 3 (96 clusters, 93 fit) 43 / 57.
+struct SkinnyPlan {
+  bool narrow;
+  int shares;
+};
+SkinnyPlan skinny_plan(int N, int K, int sms) {
+  const bool few = (N + 127) / 128 * 8 < sms;          // 128 wide would leave SMs idle even with eight slices
+  SkinnyPlan best{few, 1};
+  double fill = 0;
+  for (int w = few ? 1 : 0; w < 2; ++w) {
+    const int tiles = w ? (N + 63) / 64 : (N + 127) / 128;
+    for (int n : {1, 2, 3, 4, 8}) {
+      const int room = skinny_room(w != 0, n);
+      if (n > 1 && (tiles > room || K / n < (K >= 1024 && tiles * n <= sms ? 128 : 256))) continue;
+      if (n == 1 && tiles > room) {                    // several rounds
+        if (!w) return {false, 1};
+        continue;
+      }
+      if ((double)tiles / room > fill) {
+        fill = (double)tiles / room;
+        best = {w != 0, n};
+      }
+    }
+  }
+  return best;
 }
 
 }  // namespace
 
+// The tensor-core tiles are faster for a large matrix whose columns make most of one wave of 128, once A has 64 K values (below, they take half as
+// long again). Eight rows, us here / there: 8192 x 12288 43 / 41, x 14336 48 / 42, x 16384 49 / 45; contraction contiguous, 28672 x 12288 145 / 128,
+// x 16384 161 / 153; outside 8192 x 11008 35 / 41, x 18944 50 / 54, and 4096 x 14336 27 / 35.
+bool gemm_skinny_better(int M, int N, int K) {
+  const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
+  return (long long)M * K < 65536 || N < 80 * sms || N >= 128 * sms;
+}
+
 int launch_gemm_skinny(const SkinnyParams& p, bool b_mn, cudaStream_t s) {
   const int sms = device_sm_count() > 0 ? device_sm_count() : 148;
   if (!b_mn) {
-    if (p.N >= 64 * sms) ELFA_CUDA(launch_chain(skinny_nt_kernel<1>, dim3((p.N + 127) / 128), dim3(256), 0, s, 1, p));
-    else ELFA_CUDA(launch_chain(skinny_nt_kernel<8>, dim3((p.N + 15) / 16), dim3(256), 0, s, 1, p));
+    // Warps per 16 columns: eight; four for the columns that make one round of them and a bit with eight (11008: 52 us against 60 at K 11008); one
+    // where there are many columns and a contraction of a few hundred leaves nothing to share (K 256, N 64000: 7.5 us with one, 9.6 with
+    // four, 13 with eight; N 11008 4.9, 3.2 and 3.4).
+    auto launch = [&](auto kernel, int wk) { return launch_chain(kernel, dim3((p.N + 128 / wk - 1) / (128 / wk)), dim3(256), 0, s, 1, p); };
+    if (p.K <= 512 && p.N >= 192 * sms) ELFA_CUDA(launch(skinny_nt_kernel<1, 1>, 1));
+    else if (p.N >= 64 * sms && (p.K <= 512 || p.N < 80 * sms)) ELFA_CUDA(launch(skinny_nt_kernel<4, 2>, 4));
+    else if (p.K >= 1024) ELFA_CUDA(launch(skinny_nt_kernel<8, 4>, 8));
+    else ELFA_CUDA(launch(skinny_nt_kernel<8, 1>, 8));
   } else {
-    // 64 columns per CTA where 128 would leave SMs idle even with eight slices (1024 x 4096: 64 CTAs)
-    const bool narrow = (p.N + 127) / 128 * 8 < sms;
-    const int tiles = narrow ? (p.N + 63) / 64 : (p.N + 127) / 128;
-    int shares = 1;                                    // about two CTAs per SM, at least 128 rows of B each
-    while (shares < 8 && tiles * shares < 2 * sms && p.K / (2 * shares) >= 128) shares *= 2;
+    const SkinnyPlan plan = skinny_plan(p.N, p.K, sms);
+    const int tiles = plan.narrow ? (p.N + 63) / 64 : (p.N + 127) / 128, shares = plan.shares;
     const int ks = ((p.K + shares - 1) / shares + 15) / 16 * 16;
-    ELFA_CUDA(launch_chain(narrow ? skinny_nn_kernel<1> : skinny_nn_kernel<2>, dim3(tiles, shares), dim3(256), 0, s, shares, p, ks));
+    ELFA_CUDA(launch_chain(plan.narrow ? skinny_nn_kernel<1> : skinny_nn_kernel<2>, dim3(tiles, shares), dim3(256), 0, s, shares, p, ks));
   }
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);

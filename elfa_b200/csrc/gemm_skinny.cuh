@@ -15,6 +15,7 @@ struct SkinnyParams {
   unsigned flags;                          // ELFA_EPI_BIAS, ELFA_EPI_GELU, ELFA_EPI_STORE_PREACT
 };
 
+bool gemm_skinny_better(int M, int N, int K);
 int launch_gemm_skinny(const SkinnyParams& p, bool b_mn, cudaStream_t s);
 
 }  // namespace elfa

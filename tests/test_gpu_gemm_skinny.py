@@ -19,7 +19,8 @@ def _operands(dev, M, N, K, bmn):
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9])                    # 9: the tensor-core form
-@pytest.mark.parametrize("N,K", [(8, 8), (64, 256), (72, 264), (1000, 1104), (1536, 1024), (256, 11008), (32000, 128)])
+@pytest.mark.parametrize("N,K", [(8, 8), (64, 256), (72, 264), (1000, 1104), (1536, 1024), (256, 11008), (32000, 128), (30000, 520), (9480, 1104),
+                                 (11008, 776), (6144, 2056), (14336, 8192)])
 @pytest.mark.parametrize("bmn", [True, False])
 def test_matches_the_product(cuda_device, M, N, K, bmn):
     a, b = _operands(cuda_device, M, N, K, bmn)
@@ -65,3 +66,27 @@ def test_linear_backward_of_a_few_rows(cuda_device):
     dx, dw = torch.autograd.grad(ops.linear(x, w), [x, w], dy)
     for got, want in ((dx, dy.double() @ w.double().t()), (dw, x.double().t() @ dy.double())):
         assert (got.double() - want).abs().max() <= 2 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("bmn,M,N,K", [(False, 8, 9480, 8192), (False, 1, 11008, 4096), (False, 8, 18944, 1024), (True, 8, 6144, 1024), (True, 8, 9480, 1024),
+                                       (True, 8, 14336, 8192), (True, 1, 12288, 4096)])
+def test_no_slower_than_the_tiles(cuda_device, bmn, M, N, K):
+    """The cuts of a matrix at which one round too many, or too few warps, once cost up to three times the tensor-core tiles' time."""
+    ops_ = [_operands(cuda_device, M, N, K, bmn) for _ in range(max(2, min(8, 300_000_000 // (N * K * 2))))]
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=cuda_device)
+
+    def us(bn):
+        run = lambda: [gemm(a, b, b_mn=bmn, out=out, force_bn=bn) for a, b in ops_]
+        run()
+        g, best = torch.cuda.CUDAGraph(), []
+        with torch.cuda.graph(g):
+            run()
+        for _ in range(6):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            g.replay()
+            e[1].record()
+            torch.cuda.synchronize()
+            best.append(e[0].elapsed_time(e[1]))
+        return min(best)
+    assert us(0) < 1.15 * us(512 if N >= 18944 else 128)
