@@ -324,7 +324,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
   } else if (warp < 2 + EPI) {
     // ------------------------------------------------------------------ epilogue
-    const int q = warp & 3, part = (warp - 2) >> 2;
+    const int q = warp & 3, part = PARTS == 1 ? 0 : (warp - 2) >> 2;      // known to be 0 where one warp takes a quarter: its columns are constants
     uint32_t tile_iter = 0;
     const unsigned fl = p.flags;
     float alpha = 1.f;
