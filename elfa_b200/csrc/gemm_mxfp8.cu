@@ -509,14 +509,15 @@ int launch_q(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& 
   return ELFA_OK;
 }
 
-// Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile (cycles: the fill of shared memory per K block, and the wait
-// for the shared columns). Of 43 shapes (M 512 to 16384, N 3072 to 11008, K 1024 to 4096) it misses the faster tile in five, by 5 % at most. Measured (us,
-// 192 / 256 wide, GELU): 4096 x 11008 x 4096 160 / 139, 2048 x 4096 x 4096 42 / 32 and 1024 x 4096 x 4096 29 / 19 (two rounds against one),
-// 1500 x 4096 x 4096 31.1 / 30.6 (two rounds each: the narrow one), 512 x 7104 one round each, x 1024 9.9 / 10.2, x 4096 20 / 19 (the narrow one).
-bool wide_pair(int M, int N, int K) {
+// Whether 256 x 256 pair tiles beat 256 x 192: rounds over the pairs times the cost of a tile (cycles: the fill of shared memory per K block, the ends, and
+// the wait for the shared columns, which a plain output makes longer: it has nothing else to do meanwhile). 165 shapes (M 1500 to 8192, N 3072 to 11008, K 256
+// to 4096): within 0.1 % of the faster tile on average with GELU, 4 % at most; plain within 0.5 %, at most 2.5 % behind the narrow one.
+// Measured (us, 192 / 256 wide): GELU 4096 x 11008 x 4096 160 / 139, 2048 x 4096 x 4096 42 / 32 (two rounds against one), 3000 x 11008 x 256
+// 40 / 32; plain 8192 x 6144 x 1024 52 / 57, 4096 x 11008 x 1024 48 / 51.
+bool wide_pair(int M, int N, int K, bool gelu) {
   const long long pairs = device_sm_count() / 2, tm = (M + 255) / 256, kt = (K + QBK - 1) / QBK;
   const long long r256 = (tm * ((N + 255) / 256) + pairs - 1) / pairs, r192 = (tm * ((N + 191) / 192) + pairs - 1) / pairs;
-  return r256 * (632 * kt + 700) < r192 * (566 * kt);
+  return r256 * (gelu ? 632 * kt + 2000 : 660 * kt + 3000) < r192 * (566 * kt + 1500);
 }
 
 // Tensor map over a scale tensor viewed as [atoms, 128] 32-bit words, box = `box_atoms` rows. Small cache:
@@ -718,7 +719,7 @@ ELFA_API int elfa_gemm_mxfp8(const void* A, const void* sfa, const void* B, cons
   ELFA_REQUIRE(force_bn != 512 || !(flags & ELFA_EPI_BIAS), "gemm_mxfp8: the 256-wide tile takes no bias");
   const bool pair = force_bn == 384 || force_bn == 512 ||
                     (force_bn == 0 && N > 128 && (long long)((M + 255) / 256) * ((N + 191) / 192) >= device_sm_count() / 2);
-  const bool wide = force_bn == 512 || (force_bn == 0 && pair && !(flags & ELFA_EPI_BIAS) && wide_pair(M, N, K));
+  const bool wide = force_bn == 512 || (force_bn == 0 && pair && !(flags & ELFA_EPI_BIAS) && wide_pair(M, N, K, (flags & ELFA_EPI_GELU) != 0));
   const int BN = pair ? (wide ? 256 : 192) : ((force_bn == 128 || force_bn == 192) ? force_bn : (N <= 128 ? 128 : 192));
   CUtensorMap tmA, tmB;
   int rc = shared_tmap(&tmA, A, 1, (uint64_t)M, (uint64_t)K, (uint64_t)K, QBM, QBK);
@@ -748,9 +749,10 @@ ELFA_API int elfa_gemm_mxfp8(const void* A, const void* sfa, const void* B, cons
   p.status = st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // Eight epilogue warps where a tile's products take less time than four need to write it (with GELU about 5 us for 192 columns, 7 for 256; a K block
-  // 0.34 us); their staging costs a stage of the ring. 4096 x 11008 x 1024: 192 wide 65 -> 57 us, 256 wide 73 -> 57; x 4096: 192 wide 155 -> 158.
+  // 0.34 us); their staging costs a stage of the ring. 4096 x 11008 x 1024: 192 wide 65 -> 57 us, 256 wide 73 -> 57; x 4096: 192 wide 155 -> 158. A plain
+  // output is written by four in time (192 wide, K 256 to 1536: eight take 1 to 6 % longer); with a bias, which is added from registers, eight win by 16 to 19 %.
   if (wide) return launch_q<256, 5, true, false, false, 8>(tmA, tmB, tmSFA, tmSFB, p, s);
-  if (pair && kt <= 12) return launch_q<192, 6, true, false, false, 8>(tmA, tmB, tmSFA, tmSFB, p, s);
+  if (pair && kt <= 12 && (flags & (ELFA_EPI_GELU | ELFA_EPI_BIAS))) return launch_q<192, 6, true, false, false, 8>(tmA, tmB, tmSFA, tmSFB, p, s);
   if (pair) return launch_q<192, 7, true>(tmA, tmB, tmSFA, tmSFB, p, s);
   if (BN == 192) return launch_q<192, 5, false>(tmA, tmB, tmSFA, tmSFB, p, s);
   return launch_q<128, 6, false>(tmA, tmB, tmSFA, tmSFB, p, s);
