@@ -23,6 +23,7 @@
 //
 // reference: kernels/cuda/efla.cu:121-271,534-552 (chunks are scanned one after the other, the bf16 state in global memory).
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "elfa_native.h"
@@ -720,11 +721,23 @@ __global__ void __launch_bounds__(256) efla_combine_kernel(const float* __restri
   }
 }
 
+// The shared memory that a kernel may use, set once per device: asking on every call costs the host 1 to 2 us, up to five times in a pass
+template <auto Kernel>
+cudaError_t allow_shared(int bytes) {
+  static std::atomic<unsigned long long> configured{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev <= 63 && (configured.load(std::memory_order_relaxed) >> dev & 1))) return e;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev <= 63) configured.fetch_or(1ull << dev, std::memory_order_relaxed);
+  return e;
+}
+
 template <int D>
 int launch_combine(const float* coef, float* work, int BH, int nchunks, int P, int dir, cudaStream_t s) {
   if (P < 3) return ELFA_OK;
   constexpr int bytes = (D * (D + 4) + D * 17) * 4;
-  ELFA_CUDA(cudaFuncSetAttribute(efla_combine_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  ELFA_CUDA(allow_shared<efla_combine_kernel<D>>(bytes));
   efla_combine_kernel<D><<<dim3(BH, D / 16), 256, bytes, s>>>(coef, work, nchunks, P, dir);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
@@ -748,7 +761,7 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
     P = (nchunks + seg - 1) / seg;
   }
   auto kernel = P > 1 ? efla_chunk_fwd_kernel<D, true> : efla_chunk_fwd_kernel<D, false>;
-  ELFA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  ELFA_CUDA((P > 1 ? allow_shared<efla_chunk_fwd_kernel<D, true>>(bytes) : allow_shared<efla_chunk_fwd_kernel<D, false>>(bytes)));
   auto walk = [&](int phase, int walks) {
     kernel<<<dim3(B * H, D / L::VC, walks), 32 * ec_warps<D>(), bytes, s>>>(
         static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), static_cast<const __nv_bfloat16*>(nmat), coef, state0,
@@ -1322,14 +1335,14 @@ int launch_chunk_bwd(const void* k, const void* v, const void* nmat, const float
   const auto* K = static_cast<const __nv_bfloat16*>(k);
   const auto* O = static_cast<const __nv_bfloat16*>(dout);
   const auto* N = static_cast<const __nv_bfloat16*>(nmat);
-  ELFA_CUDA(cudaFuncSetAttribute(efla_chunk_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::BYTES));
+  ELFA_CUDA(allow_shared<efla_chunk_bwd_kernel<D>>(M::BYTES));
   int seg = nchunks;
   if (P > 1) {
     seg = (nchunks + P - 1) / P;
     P = (nchunks + seg - 1) / seg;
   }
   auto kernel = P > 1 ? efla_chunk_bwd_state_kernel<D, true> : efla_chunk_bwd_state_kernel<D, false>;
-  ELFA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes1));
+  ELFA_CUDA((P > 1 ? allow_shared<efla_chunk_bwd_state_kernel<D, true>>(bytes1) : allow_shared<efla_chunk_bwd_state_kernel<D, false>>(bytes1)));
   auto walk = [&](int phase, int walks) {
     kernel<<<dim3(B * H, D / L::VC, walks), 32 * ec_warps<D>(), bytes1, s>>>(
         K, O, N, coef, dstate_out, reinterpret_cast<float4*>(dckpt), dstate0, work, T, H, nchunks, P, seg, phase);
@@ -1368,7 +1381,9 @@ using namespace elfa;
 // The walk of the state gradient is cut alike: on eleven shapes its best number is the forward walk's, or within 3 % of it (kernels alone, forward /
 // state gradient, us: B 1 x 8192, 16 heads of 64, P 1 337 / 358, 8 126 / 127, 10 109 / 109, 12 140 / 134; B 2 x 1531, 8 heads of 128, P 1 100 / 111, 4 86 / 91,
 // 5 82 / 83, 6 89 / 92; B 4 x 1024, 8 heads of 128, P 1 69 / 75, 3 78 / 81; B 1 x 4096, 16 heads of 32, P 1 161 / 138, 10 42 / 45, 16 39 / 41).
-ELFA_API int elfa_efla_segments(int B, int T, int H, int d) {
+// A cut costs the host two launches and an allocation per walk (6 to 8 us), which only a walk longer than the host's part of the call pays for: about 30 us
+// without a gradient, 70 with one, where the rest of the pass runs meanwhile (B 1 x 500, 8 heads of 32, training, cut whatever its length: 159 -> 208 us).
+static int efla_segments(int B, int T, int H, int d, double least) {
   const int nchunks = (T + EC - 1) / EC, sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const long long units = (long long)B * H * (d == 128 || d == 96 ? 2 : 1);
   struct Cost { double one, full; int resident; double launches, joint; };      // microseconds
@@ -1377,7 +1392,9 @@ ELFA_API int elfa_efla_segments(int B, int T, int H, int d) {
     const long long ctas = units * walks, round = (long long)c.resident * sms, rest = ctas % round;
     return c.full * (double)(ctas / round) + (rest == 0 ? 0. : (rest <= sms ? c.one : c.full));
   };
-  double best = 0.95 * nchunks * steps(1);       // cut only where that is clearly less
+  const double whole = nchunks * steps(1);
+  if (whole < least) return 1;
+  double best = 0.9 * whole;                     // cut only where that is clearly less
   int at = 1;
   for (int P = 3; P <= 16 && nchunks / P >= 4; ++P) {
     const int seg = (nchunks + P - 1) / P;
@@ -1389,6 +1406,8 @@ ELFA_API int elfa_efla_segments(int B, int T, int H, int d) {
   }
   return at;
 }
+ELFA_API int elfa_efla_segments(int B, int T, int H, int d) { return efla_segments(B, T, H, d, 30); }
+ELFA_API int elfa_efla_segments_train(int B, int T, int H, int d) { return efla_segments(B, T, H, d, 70); }
 
 // k, v, o: [B, T, H, d] bf16, 16-byte aligned; beta: 1 float; state0 (optional) / state_out: [B, H, d, d] fp32; ckpt: null or
 // B * H * ceil(T / 32) * d * d floats (chunk-start states in the kernels' own order, needed by backward). nmat: [B * H * ceil(T / 32), 3, 32, 32] bf16 and

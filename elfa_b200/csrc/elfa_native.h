@@ -211,6 +211,7 @@ int elfa_efla_scan_fwd(const void* k, const void* v, const float* beta, const fl
                        int B, int T, int H, int d, void* stream);
 // ---- efla_chunk.cu -----------------------------------------------------------------------------
 int elfa_efla_segments(int B, int T, int H, int d);
+int elfa_efla_segments_train(int B, int T, int H, int d);
 int elfa_efla_chunk_fwd(const void* k, const void* v, const float* beta, const float* state0, void* o, float* state_out,
                         float* ckpt, void* nmat, float* coef, int B, int T, int H, int d, void* stream);
 int elfa_efla_chunk_bwd(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,

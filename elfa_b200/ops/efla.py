@@ -20,6 +20,7 @@ Math restated from the reference (all three are host loops there):
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -111,10 +112,15 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-def _efla_segments(k: torch.Tensor, B: int, T: int, H: int, d: int):
-    """Into how many segments the kernels cut the walk over the chunks, and the scratch that takes (start, map and offset of each)."""
-    n = lib.raw("elfa_efla_segments")(B, T, H, d)
-    return n, torch.empty(3 * n * B * H * d * d, dtype=torch.float32, device=k.device) if n > 1 else None
+@functools.lru_cache(maxsize=1024)
+def _efla_segments(B: int, T: int, H: int, d: int, train: bool) -> int:
+    """Into how many segments the kernels cut the walk over the chunks: a rule on the sizes alone, asked once for each."""
+    return lib.raw("elfa_efla_segments_train" if train else "elfa_efla_segments")(B, T, H, d)
+
+
+def _efla_scratch(n: int, k: torch.Tensor, B: int, H: int, d: int) -> torch.Tensor:
+    """Start, map and offset of each segment."""
+    return torch.empty(3 * n * B * H * d * d, dtype=torch.float32, device=k.device)
 
 
 class _EflaScan(torch.autograd.Function):
@@ -137,9 +143,9 @@ class _EflaScan(torch.autograd.Function):
         ckpt = torch.empty(B * H * nchunks * d * d, dtype=torch.float32, device=k.device) if want_grad else None
         nmat = torch.empty((B, H, nchunks, 3, _EFLA_CHUNK, _EFLA_CHUNK), dtype=torch.bfloat16, device=k.device)
         coef = torch.empty((B, H, nchunks, 4, _EFLA_CHUNK), dtype=torch.float32, device=k.device)
-        cut, work = _efla_segments(kc, B, T, H, d)
+        cut = _efla_segments(B, T, H, d, want_grad)
         if cut > 1:
-            lib.call("elfa_efla_chunk_fwd_cut", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, work, cut, B, T, H, d, stream_ptr(kc))
+            lib.call("elfa_efla_chunk_fwd_cut", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, _efla_scratch(cut, kc, B, H, d), cut, B, T, H, d, stream_ptr(kc))
         else:
             lib.call("elfa_efla_chunk_fwd", kc, vc, bt, st0, o, s_out, ckpt, nmat, coef, B, T, H, d, stream_ptr(kc))
         if want_grad:
@@ -157,10 +163,10 @@ class _EflaScan(torch.autograd.Function):
         ds0 = torch.empty((B, H, d, d), dtype=torch.float32, device=kc.device) if has_state else None
         dckpt = torch.empty_like(ckpt)
         dso = ds_out.float().contiguous() if ds_out is not None else None
-        cut, work = _efla_segments(kc, B, T, H, d)
+        cut = _efla_segments(B, T, H, d, True)
         if cut > 1:
-            lib.call("elfa_efla_chunk_bwd_cut", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt, work, cut, B, T, H, d,
-                     stream_ptr(kc))
+            lib.call("elfa_efla_chunk_bwd_cut", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt,
+                     _efla_scratch(cut, kc, B, H, d), cut, B, T, H, d, stream_ptr(kc))
         else:
             lib.call("elfa_efla_chunk_bwd", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt, B, T, H, d, stream_ptr(kc))
         return dk, dv, dbeta.sum().reshape(1), ds0, None

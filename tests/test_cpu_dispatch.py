@@ -45,3 +45,11 @@ def test_a_host_tensor_has_no_stream(monkeypatch):
                                           ((4096, 1, 32, 32, 128, 1), 1), ((300, 2, 6, 2, 64, 1), 1)])
 def test_shares_of_a_key_head(shape, shares):
     assert native.lib.raw("elfa_attention_bwd_shares")(*shape) == shares
+
+
+@pytest.mark.parametrize("shape,forward,train", [((1, 384, 8, 64), False, False), ((1, 500, 16, 32), False, False), ((1, 1000, 2, 64), True, False), ((1, 1400, 2, 64), True, False),
+                                                 ((1, 2000, 8, 64), True, True), ((1, 8192, 16, 64), True, True), ((2, 1531, 8, 128), True, True),
+                                                 ((8, 1400, 8, 64), False, False), ((8, 2048, 16, 64), False, False)])
+def test_walks_that_are_cut(shape, forward, train):
+    """Two launches and an allocation more: not for a walk that ends before the host has issued the rest of the call."""
+    assert (native.lib.raw("elfa_efla_segments")(*shape) > 1, native.lib.raw("elfa_efla_segments_train")(*shape) > 1) == (forward, train)
