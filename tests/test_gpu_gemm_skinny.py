@@ -3,6 +3,10 @@
 Bound: bf16 operands, fp32 sums of K terms in any order (K 2^-24 of the sum of magnitudes at worst; 2^-12 of the largest output covers K <= 11008 of
 random signs) and one rounding of the output to bf16 (2^-9 of itself): 2^-8 of the largest.
 """
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -90,3 +94,16 @@ def test_no_slower_than_the_tiles(cuda_device, bmn, M, N, K):
             best.append(e[0].elapsed_time(e[1]))
         return min(best)
     assert us(0) < 1.15 * us(512 if N >= 18944 else 128)
+
+
+def test_first_few_rows_of_a_process_under_capture(cuda_device):
+    """The clusters that run at once are asked for on the first such call, which may be inside a graph capture (the library's status word is made by
+    the product of 16 rows before it)."""
+    code = ("import torch\nfrom elfa_b200.ops.gemm import gemm\n"
+            "a, b = torch.randn(4, 1024, device='cuda').bfloat16(), torch.randn(1024, 4096, device='cuda').bfloat16()\n"
+            "y = torch.zeros(4, 4096, dtype=torch.bfloat16, device='cuda')\ng = torch.cuda.CUDAGraph()\n"
+            "gemm(torch.cat([a] * 4), b, b_mn=True)\n"
+            "with torch.cuda.graph(g):\n    gemm(a, b, b_mn=True, out=y)\n"
+            "g.replay()\nz = gemm(a, b, b_mn=True)\ntorch.cuda.synchronize()\nassert torch.equal(y, z) and y.abs().max() > 0\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-2000:]
