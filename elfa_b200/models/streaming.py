@@ -2,7 +2,8 @@
 a Python step, an autograd call and an allocation per kernel. A decoding step of 4 layers took 1.1 ms to issue that way for 0.3 ms of kernels.
 
 Each function returns ``None`` for what it does not handle - a gradient wanted, another type, layout or device, tensor or context parallelism,
-quantised layers, parameters that are fetched on use, hooks or replaced methods, transforms and tracing - and the model takes the general route.
+quantised layers, parameters that are fetched on use, hooks or replaced methods, transforms, forward mode and tracing, states that are not plain - and the
+model takes the general route.
 
 reference: ``src/model/model.zig:415-454`` (streaming with carried states), ``src/eval/evaluator.zig:419-470``.
 """
