@@ -13,125 +13,18 @@
 // pass over the rows per (32 channels, 4 taps) without atomics.
 #include <type_traits>
 
-#include "common.cuh"
+#include "efla_step.cuh"
 #include "elfa_native.h"
 
 namespace elfa {
 namespace {
 
-__device__ __forceinline__ float efla_coeff(float beta, float lam) {
-  // expm1f: 1 - exp would cancel for short keys (at beta lam = 1e-6 one step of fp32 is 6 %, and the chunked form has c in fp64)
-  return lam < 1e-30f ? beta : -expm1f(-beta * lam) / lam;
-}
-
-// Token by token, for short blocks without a gradient (generation; the line is in ops/efla.py): one launch, nothing else to prepare.
-// k, v, o: [B, T, H, D] bf16. state0 / state_out: [B, H, D, D] fp32.
-// The columns of S evolve independently (column j needs k_t, c_t and v_t[j] only), so a CTA owns 32 value columns:
-// grid (B*H, D/32). Its four warps split the D key rows: warp w keeps rows [w D/4, (w+1) D/4) of the 32 columns in
-// registers (lane = column), so the dependent instruction chain of a step is a quarter as long and the four
-// schedulers of the SM all have a warp. A step costs one block barrier: the warps exchange their partial dot
-// products through a parity-double-buffered shared array. Time is walked in tiles of EFLA_TT tokens: every warp
-// fetches eight of the tile's rows with all loads in flight together (keys as fp32, the CTA's 32 value columns),
-// warp 0 computes lam / c for the whole tile (lane r owns token r), and the sequential part touches global memory
-// only for the output.
-constexpr int EFLA_TT = 32;
-constexpr int EFLA_W = 4;
-
-template <int D>
-__device__ __forceinline__ void efla_load_tile(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-                                               float (*sk)[D], float (*sv)[32], float* sc, float* slam, float beta, long long row0,
-                                               long long row_stride, int col, int n, int warp, int lane) {
-  __syncthreads();                                       // the previous tile has been consumed
-  const int r0 = warp * (EFLA_TT / EFLA_W);
-  if (r0 < n) {
-    __nv_bfloat16 kq[8][D / 32], vq[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const long long row = row0 + (long long)min(r0 + u, n - 1) * row_stride;      // clamped: rows past the end re-read the last one
-#pragma unroll
-      for (int c = 0; c < D / 32; ++c) kq[u][c] = k[row + c * 32 + lane];
-      vq[u] = v[row + col];
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-#pragma unroll
-      for (int c = 0; c < D / 32; ++c) sk[r0 + u][c * 32 + lane] = __bfloat162float(kq[u][c]);
-      sv[r0 + u][lane] = __bfloat162float(vq[u]);
-    }
-  }
-  __syncthreads();
-  if (warp == 0 && lane < n) {                           // the rotated index keeps the banks apart
-    float lam = 0.f;
-#pragma unroll 8
-    for (int c = 0; c < D; ++c) {
-      const float x = sk[lane][(c + lane) % D];
-      lam += x * x;
-    }
-    sc[lane] = efla_coeff(beta, lam);
-    slam[lane] = lam;
-  }
-  __syncthreads();
-}
-
-// One step of the recurrence for this warp's R rows: returns p (complete, after the exchange) and applies the update.
-template <int R>
-__device__ __forceinline__ float efla_step(float (&S)[R], const float* __restrict__ krow, float c_, float vj, float* part, int warp,
-                                           int lane) {
-  const float4* kr = reinterpret_cast<const float4*>(krow);
-  float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
-#pragma unroll
-  for (int i = 0; i < R / 4; ++i) {
-    const float4 kk = kr[i];
-    p0 += kk.x * S[4 * i];
-    p1 += kk.y * S[4 * i + 1];
-    p2 += kk.z * S[4 * i + 2];
-    p3 += kk.w * S[4 * i + 3];
-  }
-  part[warp * 32 + lane] = (p0 + p1) + (p2 + p3);
-  __syncthreads();
-  const float p = (part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]);
-  const float ce = c_ * (vj - p);
-#pragma unroll
-  for (int i = 0; i < R / 4; ++i) {
-    const float4 kk = kr[i];
-    S[4 * i] += kk.x * ce;
-    S[4 * i + 1] += kk.y * ce;
-    S[4 * i + 2] += kk.z * ce;
-    S[4 * i + 3] += kk.w * ce;
-  }
-  return p;
-}
-
 template <int D>
 __global__ void __launch_bounds__(32 * EFLA_W) efla_scan_fwd_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
                                                                     const float* __restrict__ beta_ptr, const float* __restrict__ state0,
                                                                     __nv_bfloat16* __restrict__ o, float* __restrict__ state_out, int T, int H) {
-  constexpr int R = D / EFLA_W;
-  __shared__ __align__(16) float sk[EFLA_TT][D];
-  __shared__ float sv[EFLA_TT][32];
-  __shared__ float sc[EFLA_TT], slam[EFLA_TT];
-  __shared__ float spart[2][EFLA_W * 32];
-  const int bh = blockIdx.x, b = bh / H, h = bh % H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col = blockIdx.y * 32 + lane, i0 = warp * R;
-  const float beta = *beta_ptr;
-  float S[R];
-#pragma unroll
-  for (int i = 0; i < R; ++i) S[i] = state0 ? state0[((long long)bh * D + i0 + i) * D + col] : 0.f;
-  for (int t0 = 0; t0 < T; t0 += EFLA_TT) {
-    const int n = min(EFLA_TT, T - t0);
-    efla_load_tile<D>(k, v, sk, sv, sc, slam, beta, (((long long)b * T + t0) * H + h) * D, (long long)H * D, col, n,
-                      warp, lane);
-    for (int r = 0; r < n; ++r) {
-      const int t = t0 + r;
-      const float c_ = sc[r], vj = sv[r][lane];
-      const float p = efla_step<R>(S, sk[r] + i0, c_, vj, spart[r & 1], warp, lane);
-      if (warp == 0) o[(((long long)b * T + t) * H + h) * D + col] = __float2bfloat16(p + c_ * slam[r] * (vj - p));
-    }
-  }
-  if (state_out) {
-#pragma unroll
-    for (int i = 0; i < R; ++i) state_out[((long long)bh * D + i0 + i) * D + col] = S[i];
-  }
+  __shared__ EflaStepScratch<D, EFLA_TT> sm;
+  efla_scan_block<D, EFLA_TT>(k, v, beta_ptr, state0, o, state_out, T, H, blockIdx.x, blockIdx.y, sm, threadIdx.x, [] { __syncthreads(); });
 }
 
 // ------------------------------------------------------------------------------------ ShortConv
@@ -358,31 +251,9 @@ __global__ void __launch_bounds__(64) shortconv_stream_kernel(const __nv_bfloat1
   const int c = (blockIdx.y * 64 + threadIdx.x) * 2, t = blockIdx.x % T, b = blockIdx.x / T;
   if (c >= C) return;
   const __nv_bfloat16 *tb = tail + b * tail_stride + c, *nb = n + (long long)b * T * C + c;
-  __nv_bfloat16* xb = xin + (long long)b * (tails + T) * C + c;
-  auto at = [&](int i) {                   // position i of tail and inputs
+  shortconv_stream_pair<RING>([&](int i) {                             // position i of tail and inputs
     return *reinterpret_cast<const uint32_t*>(i < tails ? tb + (long long)i * C : nb + (long long)(i - tails) * C);
-  };
-  if (t == 0)
-    for (int i = 0; i < tails; ++i) *reinterpret_cast<uint32_t*>(xb + (long long)i * C) = at(i);
-  *reinterpret_cast<uint32_t*>(xb + (long long)(tails + t) * C) = at(tails + t);
-  float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};                            // [chain][channel]
-  if (bias) {
-    s[0][0] = __bfloat162float(bias[c]);
-    s[0][1] = __bfloat162float(bias[c + 1]);
-  }
-  const int taps = min(W, tails + t + 1);
-#pragma unroll 4
-  for (int j = 0; j < taps; ++j) {
-    const uint32_t x = at(tails + t - j);
-    const int k = RING ? j & 1 : 0;
-    s[k][0] = fmaf(bf16_lo(x), __bfloat162float(w[(long long)c * W + j]), s[k][0]);
-    s[k][1] = fmaf(bf16_hi(x), __bfloat162float(w[(long long)(c + 1) * W + j]), s[k][1]);
-  }
-  if (RING) {
-    s[0][0] += s[1][0];
-    s[0][1] += s[1][1];
-  }
-  *reinterpret_cast<uint32_t*>(u + ((long long)b * T + t) * C + c) = pack_bf16(s[0][0], s[0][1]);
+  }, w, bias, xin + (long long)b * (tails + T) * C + c, u + ((long long)b * T + t) * C + c, tails, t, c, C, W);
 }
 
 // Forward and input gradient share one kernel (DX = false: y[t] = bias + sum_j x[t - j] w[j]; DX = true:

@@ -222,11 +222,7 @@ int skinny_room(bool narrow, int n, int sms) {
 // fills more of the room; past one round whole columns of 128. One slice too many starts a second round. Four to eight rows, us: N 8192, K 4096, 128 wide
 // 4 / 8 slices 15 / 19; N 11008, K 4096, 3 / 4 20 / 30; N 32000, K 4096, 1 / 2 45 / 52; N 6144, K 2048, 64 wide 4 / 128 wide 8 9.3 / 15;
 // N 12288, K 8192, 64 wide 2 / 128 wide 3 (96 clusters, 93 fit) 43 / 57.
-struct SkinnyPlan {
-  bool narrow;
-  int shares;
-};
-SkinnyPlan skinny_plan(int N, int K, int sms) {
+SkinnyPlan plan_for(int N, int K, int sms) {
   const bool few = (N + 127) / 128 * 8 < sms;          // 128 wide would leave SMs idle even with eight slices
   SkinnyPlan best{few, 1};
   double fill = 0;
@@ -250,6 +246,8 @@ SkinnyPlan skinny_plan(int N, int K, int sms) {
 
 }  // namespace
 
+SkinnyPlan skinny_plan(int N, int K) { return plan_for(N, K, device_sm_count() > 0 ? device_sm_count() : 148); }
+
 // The tensor-core tiles are faster for a large matrix whose columns make most of one wave of 128, once A has 64 K values (below, they take half as
 // long again). Eight rows, us here / there: 8192 x 12288 43 / 41, x 14336 48 / 42, x 16384 49 / 45; contraction contiguous, 28672 x 12288 145 / 128,
 // x 16384 161 / 153; outside 8192 x 11008 35 / 41, x 18944 50 / 54, and 4096 x 14336 27 / 35.
@@ -270,10 +268,9 @@ int launch_gemm_skinny(const SkinnyParams& p, bool b_mn, cudaStream_t s) {
     else if (p.K >= 1024) ELFA_CUDA(launch(skinny_nt_kernel<8, 4>, 8));
     else ELFA_CUDA(launch(skinny_nt_kernel<8, 1>, 8));
   } else {
-    const SkinnyPlan plan = skinny_plan(p.N, p.K, sms);
-    const int tiles = plan.narrow ? (p.N + 63) / 64 : (p.N + 127) / 128, shares = plan.shares;
-    const int ks = ((p.K + shares - 1) / shares + 15) / 16 * 16;
-    ELFA_CUDA(launch_chain(plan.narrow ? skinny_nn_kernel<1> : skinny_nn_kernel<2>, dim3(tiles, shares), dim3(256), 0, s, shares, p, ks));
+    const SkinnyPlan plan = plan_for(p.N, p.K, sms);
+    ELFA_CUDA(launch_chain(plan.narrow ? skinny_nn_kernel<1> : skinny_nn_kernel<2>, dim3(plan.tiles(p.N), plan.shares), dim3(256), 0, s, plan.shares, p,
+                           plan.ks(p.K)));
   }
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);

@@ -8,8 +8,8 @@
 // reference has no LayerNorm backward kernel and reduces weight gradients with atomics; here the
 // weight/bias gradients are reduced in two deterministic passes through a [blocks, D] fp32
 // scratch buffer supplied by the caller.
-#include "common.cuh"
 #include "elfa_native.h"
+#include "norm.cuh"
 
 namespace elfa {
 namespace {
@@ -52,24 +52,13 @@ __global__ void __launch_bounds__(256, NV <= 8 ? (HAS_RES ? 2 : 3) : 1) norm_fwd
     for (int i = 0; i < NV; ++i) rb[i] = ld_or_zero(rr + t + i * TPR, valid && t + i * TPR < nvec);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      uint32_t* pv = reinterpret_cast<uint32_t*>(&buf[i]);
-      const uint32_t* pr = reinterpret_cast<const uint32_t*>(&rb[i]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) pv[j] = pack_bf16(bf16_lo(pv[j]) + bf16_lo(pr[j]), bf16_hi(pv[j]) + bf16_hi(pr[j]));
+      buf[i] = norm_add(buf[i], rb[i]);
       if (valid && t + i * TPR < nvec) reinterpret_cast<uint4*>(sum_out + off)[t + i * TPR] = buf[i];
     }
   }
   float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const uint32_t* pv = reinterpret_cast<const uint32_t*>(&buf[i]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float a = bf16_lo(pv[j]), c = bf16_hi(pv[j]);
-      s1 += a + c;
-      s2 += a * a + c * c;
-    }
-  }
+  for (int i = 0; i < NV; ++i) norm_sums(buf[i], s1, s2);
   s1 = warp_sum(s1);
   s2 = warp_sum(s2);
   if (ROW_WARPS > 1) {
@@ -81,11 +70,8 @@ __global__ void __launch_bounds__(256, NV <= 8 ? (HAS_RES ? 2 : 3) : 1) norm_fwd
 #pragma unroll
     for (int i = 0; i < ROW_WARPS; ++i) { s1 += red[0][w0 + i]; s2 += red[1][w0 + i]; }
   }
-  const float inv_d = 1.0f / (float)D;
-  float mean = RMS ? 0.f : s1 * inv_d;
-  float var = s2 * inv_d - mean * mean;
-  var = fmaxf(var, 0.f);
-  const float rstd = rsqrtf(var + eps);
+  float mean, rstd;
+  norm_moments<RMS>(s1, s2, D, eps, mean, rstd);
   if (t == 0 && valid) {
     if (mean_out) mean_out[row] = mean;
     if (rstd_out) rstd_out[row] = rstd;
@@ -97,21 +83,7 @@ __global__ void __launch_bounds__(256, NV <= 8 ? (HAS_RES ? 2 : 3) : 1) norm_fwd
   for (int i = 0; i < NV; ++i) {
     const int vi = t + i * TPR;
     if (valid && vi < nvec) {
-      const uint32_t* pv = reinterpret_cast<const uint32_t*>(&buf[i]);
-      uint4 wq = wv[vi];
-      const uint32_t* pw = reinterpret_cast<const uint32_t*>(&wq);
-      uint4 bq = make_uint4(0, 0, 0, 0);
-      if (!RMS && b) bq = bv[vi];
-      const uint32_t* pb = reinterpret_cast<const uint32_t*>(&bq);
-      uint4 o;
-      uint32_t* po = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float lo = (bf16_lo(pv[j]) - mean) * rstd * bf16_lo(pw[j]) + bf16_lo(pb[j]);
-        const float hi = (bf16_hi(pv[j]) - mean) * rstd * bf16_hi(pw[j]) + bf16_hi(pb[j]);
-        po[j] = pack_bf16(lo, hi);
-      }
-      yr[vi] = o;
+      yr[vi] = norm_scale(buf[i], mean, rstd, wv[vi], !RMS && b ? bv[vi] : make_uint4(0, 0, 0, 0));
     }
   }
 }

@@ -10,13 +10,11 @@
 // One thread owns one (token, channel-in-group) pair and walks over the G groups, so the gradient of
 // p_l (a sum over groups) is accumulated in registers: no atomics, deterministic. Consecutive
 // threads touch consecutive channels: every access is coalesced. The backward recomputes r_l.
-#include "common.cuh"
 #include "elfa_native.h"
+#include "prism_step.cuh"
 
 namespace elfa {
 namespace {
-
-constexpr int PRISM_MAX_L = 8;
 
 struct PrismPtrs {
   const __nv_bfloat16* p[PRISM_MAX_L];   // [tokens, d] each
@@ -102,12 +100,6 @@ int prism_grid(long long n) {
 // and the carried fp32 state are as far from 64 bits as with PyTorch's functions (state: 5.5e-8 to 8.2e-7 relative against 6.0e-8 to 8.2e-7). Bound by the special
 // functions (two per element and iteration) and memory about equally: 16384 tokens x 1024 channels, two iterations: 40 us forward (100 MB),
 // 47 us backward (168 MB). With fp32 gates the layer ran PyTorch's elementwise kernels before: 2.85 ms forward and backward, 0.79 with these.
-__device__ __forceinline__ float prism_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-// -> sigmoid(2u) of the tanh-form GELU at x
-__device__ __forceinline__ float prism_gelu_gate(float x) {
-  return prism_sigmoid(1.5957691216057308f * x * fmaf(0.044715f * x, x, 1.f));
-}
-
 template <int VEC> struct PrismVec;
 template <> struct PrismVec<8> { using T = uint4; };
 template <> struct PrismVec<4> { using T = uint2; };
@@ -168,7 +160,7 @@ __global__ void __launch_bounds__(256) prism_gated_fwd_kernel(const __nv_bfloat1
             float res = r[x] - uu[x], refined = 0.f;
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-              const float a = p[l][x] * res, delta = a * prism_gelu_gate(a);
+              const float delta = prism_delta(p[l][x], res);
               res -= delta;
               refined += delta;
             }
@@ -330,92 +322,24 @@ __global__ void __launch_bounds__(256) prism_weight_sum_kernel(const float* __re
 // formed in parallel in shared memory first, so the serial part of a token is about D / 2 + L D / 4 multiply-adds per thread.
 // (B 2, 16 groups of 64, two iterations: 13 us per call on average over one block of 64 tokens and four single ones; the host loop issued
 // several launches per token and iteration: two such layers, 64 tokens and four steps, 33.6 ms with it and 5.3 with this.)
-constexpr int PS_TT = 8;
-
 template <int D>
 __global__ void __launch_bounds__(4 * D) prism_state_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ v,
                                                             const __nv_bfloat16* __restrict__ z, long long ldz, int off_b, int off_k,
                                                             const float* __restrict__ state, float* __restrict__ out, int T, int G, int L,
                                                             float forget) {
   extern __shared__ __align__(16) float ps_smem[];
-  float* sk = ps_smem;                          // [PS_TT][L][D]
-  float* sd = sk + PS_TT * L * D;               // [PS_TT][L][D]  b * delta
-  float* sb = sd + PS_TT * L * D;               // [PS_TT][L]
-  const int bg = blockIdx.x, b = bg / G, g = bg % G;
-  const int row = threadIdx.x >> 2, part = threadIdx.x & 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const PrismTile<D> sm(ps_smem, PS_TT, L);
+  const PrismSource in{u, v, z, ldz, off_b, off_k, T, G, L};
+  const int bg = blockIdx.x, row = threadIdx.x >> 2, part = threadIdx.x & 3;
   float S[D / 4];
-  const float* sp = state + ((long long)bg * D + row) * D;
-#pragma unroll
-  for (int m = 0; m < D / 16; ++m)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) S[4 * m + x] = sp[m * 16 + part * 4 + x];
+  prism_state_load<D>(S, state + ((long long)bg * D + row) * D, part);
   for (int t0 = 0; t0 < T; t0 += PS_TT) {
     const int n = min(PS_TT, T - t0);
     __syncthreads();                            // the previous tokens have been consumed
-    for (int i = warp; i < n * L; i += D / 8) {
-      const int tt = i / L, l = i % L;
-      const __nv_bfloat16* zr = z + ((long long)b * T + t0 + tt) * ldz + l * D;
-      float kx[D / 32], ss = 0.f, sm = 0.f;
-#pragma unroll
-      for (int m = 0; m < D / 32; ++m) {
-        kx[m] = __bfloat162float(zr[off_k + m * 32 + lane]);
-        ss += kx[m] * kx[m];
-        sm += __bfloat162float(zr[off_b + m * 32 + lane]);
-      }
-      ss = sqrtf(warp_sum(ss));
-      sm = warp_sum(sm);
-      const float inv = ss < 1e-12f ? 1.f : 1.f / ss;
-#pragma unroll
-      for (int m = 0; m < D / 32; ++m) sk[i * D + m * 32 + lane] = kx[m] * inv;
-      if (lane == 0) sb[i] = prism_sigmoid(sm / (float)D);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n * D; i += 4 * D) {
-      const int tt = i / D, c = i % D;
-      const long long r0 = (long long)b * T + t0 + tt, at = (r0 * G + g) * D + c;
-      float r = __bfloat162float(v[at]) - __bfloat162float(u[at]);
-      for (int l = 0; l < L; ++l) {
-        const float a = prism_sigmoid(__bfloat162float(z[r0 * ldz + l * D + c])) * r, delta = a * prism_gelu_gate(a);
-        r -= delta;
-        sd[(tt * L + l) * D + c] = sb[tt * L + l] * delta;
-      }
-    }
-    __syncthreads();
-    for (int i = 0; i < n * L; ++i) {
-      const float4* kr = reinterpret_cast<const float4*>(sk + i * D);
-      float coef = sd[i * D + row];
-      if (i % L == 0) {
-        float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
-#pragma unroll
-        for (int m = 0; m < D / 16; ++m) {
-          const float4 kk = kr[m * 4 + part];
-          p0 += kk.x * S[4 * m];
-          p1 += kk.y * S[4 * m + 1];
-          p2 += kk.z * S[4 * m + 2];
-          p3 += kk.w * S[4 * m + 3];
-        }
-        float p = (p0 + p1) + (p2 + p3);
-        p += __shfl_xor_sync(0xffffffffu, p, 1);
-        p += __shfl_xor_sync(0xffffffffu, p, 2);
-        coef -= sb[i] * forget * p;
-#pragma unroll
-        for (int m = 0; m < D / 4; ++m) S[m] *= forget;
-      }
-#pragma unroll
-      for (int m = 0; m < D / 16; ++m) {
-        const float4 kk = kr[m * 4 + part];
-        S[4 * m] += coef * kk.x;
-        S[4 * m + 1] += coef * kk.y;
-        S[4 * m + 2] += coef * kk.z;
-        S[4 * m + 3] += coef * kk.w;
-      }
-    }
+    prism_state_prepare<D, 4 * D>(in, sm, bg, t0, n, threadIdx.x, [] { __syncthreads(); });
+    prism_state_rows<D>(S, sm, n, L, row, part, forget);
   }
-  float* op = out + ((long long)bg * D + row) * D;
-#pragma unroll
-  for (int m = 0; m < D / 16; ++m)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) op[m * 16 + part * 4 + x] = S[4 * m + x];
+  prism_state_store<D>(S, out + ((long long)bg * D + row) * D, part);
 }
 
 template <int D>

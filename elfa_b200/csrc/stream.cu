@@ -7,6 +7,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "decode.cuh"
 #include "elfa_native.h"
 
 namespace elfa {
@@ -48,9 +49,6 @@ __global__ void __launch_bounds__(256) concat_cols_kernel(const ConcatArgs a, ui
   out[i] = a.src[m][i / ((long long)dv * n) * dv + c];
 }
 
-// the activation of an MLP by its number: -1 SwiGLU, 0 GELU in the product's epilogue, else an operation of elfa_elementwise
-constexpr int ACT_SWIGLU = -1, ACT_GELU = 0;
-
 // f = act(n W_up) W_down
 int mlp(const bf16* n, const void* up, const void* down, bf16* h, bf16* g, bf16* f, long long rows, int D, int F, int act, void* s) {
   int rc = linear(n, up, h, rows, D, act == ACT_SWIGLU ? 2 * F : F, act == ACT_GELU ? ELFA_EPI_GELU : 0, s);
@@ -83,13 +81,6 @@ size_t gpt_work(const GptDims& m, unsigned char* base, GptWork* w) {
   return p.used;
 }
 
-struct EflaDims {
-  long long B, T, D, H, d, F, V, layers, L, W, act, kind, prism, tail;
-};
-struct EflaWork {
-  bf16 *x[2], *r, *n, *k, *v, *o, *e, *full, *u, *z, *wc, *q, *h, *g, *f, *nmat;
-  float *coef, *segw;
-};
 size_t efla_work(const EflaDims& m, unsigned char* base, EflaWork* w, int segments, bool step) {
   Pieces p{base};
   const long long rows = m.B * m.T, hd = m.H * m.d, chunks = (m.T + 31) / 32;
@@ -113,6 +104,7 @@ size_t efla_work(const EflaDims& m, unsigned char* base, EflaWork* w, int segmen
   w->nmat = p.take<bf16>(step ? 0 : m.B * m.H * chunks * 3 * 32 * 32);
   w->coef = p.take<float>(step ? 0 : m.B * m.H * chunks * 4 * 32);
   w->segw = p.take<float>(!step && segments > 1 ? 3 * segments * m.B * m.H * m.d * m.d : 0);
+  w->arrived = p.take<unsigned int>(DECODE_COUNTERS);
   return p.used;
 }
 
@@ -210,6 +202,11 @@ ELFA_API int elfa_efla_stream(const unsigned long long* p, const long long* dims
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int rows = (int)(m.B * m.T), D = (int)m.D, B = (int)m.B, T = (int)m.T, H = (int)m.H, d = (int)m.d, L = (int)m.L, kind = (int)m.kind, G = D / d;
   const int hd = H * d, per = 19 + 3 * L;
+  if (step && efla_decode_fits(m)) {
+    STREAM_CALL(efla_decode(p, m, w, forget, eps, s));
+    const PdlScope head(true);
+    return logits(w.n, at(4), at(5), rows, D, (int)m.V, stream);
+  }
   STREAM_CALL(elfa_embedding_fwd(static_cast<const long long*>(at(0)), at(1), nullptr, w.x[0], rows, D, T, 1, 0, 0, (int)m.V, (int)m.V, stream));
   const PdlScope chain(m.B * m.T <= 8);        // decoding, as above
   int cur = 0;
