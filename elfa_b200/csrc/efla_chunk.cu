@@ -76,10 +76,6 @@ __global__ void __launch_bounds__(64) efla_prep_kernel(const __nv_bfloat16* __re
   for (int mi = 0; mi < 2; ++mi) {
     float acc[4][4];
 #pragma unroll
-    for (int nj = 0; nj < 4; ++nj)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[nj][e] = 0.f;
-#pragma unroll
     for (int kk = 0; kk < D / 16; ++kk) {
       uint32_t a[4];
       ldsm4(a, ks + ((mi * 16 + (lane & 15)) * LD + kk * 16 + (lane >> 4) * 8) * 2);
@@ -87,8 +83,13 @@ __global__ void __launch_bounds__(64) efla_prep_kernel(const __nv_bfloat16* __re
       for (int np = 0; np <= mi; ++np) {   // token columns 16 np .. 16 np + 15: the strictly upper tiles are not needed
         uint32_t bq[4];
         ldsm4(bq, ks + ((np * 16 + (lane & 7) + (lane >> 4) * 8) * LD + kk * 16 + ((lane >> 3) & 1) * 8) * 2);
-        mma_bf16(acc[2 * np], a, bq[0], bq[1]);
-        mma_bf16(acc[2 * np + 1], a, bq[2], bq[3]);
+        if (kk == 0) {
+          mma_bf16_first(acc[2 * np], a, bq[0], bq[1]);
+          mma_bf16_first(acc[2 * np + 1], a, bq[2], bq[3]);
+        } else {
+          mma_bf16(acc[2 * np], a, bq[0], bq[1]);
+          mma_bf16(acc[2 * np + 1], a, bq[2], bq[3]);
+        }
       }
     }
 #pragma unroll
@@ -207,10 +208,6 @@ __device__ __forceinline__ void efla_apply_n(float (&e)[4][4], uint32_t nbase, i
   // the four token tiles advance together: a dependent mma.sync waits for the one before it, and there is one warp per scheduler
   float acc[4][4];
 #pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) acc[nt][x] = 0.f;
-#pragma unroll
   for (int p = 2; p >= 0; --p) {           // splits of N, small ones first
     uint32_t bf[4][4];
 #pragma unroll
@@ -225,23 +222,20 @@ __device__ __forceinline__ void efla_apply_n(float (&e)[4][4], uint32_t nbase, i
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
           if (TRANS ? (nt >= 2 && ks == 0) : (nt < 2 && ks == 1)) continue;                 // zero blocks of the triangle
-          mma_bf16(acc[nt], m == 0 ? ah[ks] : (m == 1 ? am[ks] : al[ks]), bf[nt][2 * ks], bf[nt][2 * ks + 1]);
+          if (p == 2 && ks == (TRANS && nt >= 2)) mma_bf16_first(acc[nt], ah[ks], bf[nt][2 * ks], bf[nt][2 * ks + 1]);
+          else mma_bf16(acc[nt], m == 0 ? ah[ks] : (m == 1 ? am[ks] : al[ks]), bf[nt][2 * ks], bf[nt][2 * ks + 1]);
         }
   }
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-    for (int x = 0; x < 4; ++x) e[nt][x] += acc[nt][x];
+    for (int hf = 0; hf < 2; ++hf) put_pair(e[nt], hf, add_f32x2(pair_of(e[nt], hf), pair_of(acc[nt], hf)));
 }
 
 // p[16 x 32] = S^T K^T for the warp's S^T tiles (rows = value columns, columns = tokens)
 template <int D>
 __device__ __forceinline__ void efla_state_times_k(float (&p)[4][4], const float (&S)[D / 8][4], uint32_t kbase, int lane) {
   constexpr int LD = EflaStage<D>::KLD;
-#pragma unroll
-  for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) p[nt][x] = 0.f;
 #pragma unroll
   for (int k2 = 0; k2 < D / 32; ++k2) {
     uint32_t bq[4][4];
@@ -252,7 +246,10 @@ __device__ __forceinline__ void efla_state_times_k(float (&p)[4][4], const float
       uint32_t hi[4], mid[4], lo[4];
       split3_a(hi, mid, lo, S[4 * k2 + 2 * u], S[4 * k2 + 2 * u + 1]);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) mma_bf16(p[nt], lo, bq[nt][2 * u], bq[nt][2 * u + 1]);
+      for (int nt = 0; nt < 4; ++nt) {
+        if (k2 == 0 && u == 0) mma_bf16_first(p[nt], lo, bq[nt][0], bq[nt][1]);
+        else mma_bf16(p[nt], lo, bq[nt][2 * u], bq[nt][2 * u + 1]);
+      }
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) mma_bf16(p[nt], mid, bq[nt][2 * u], bq[nt][2 * u + 1]);
 #pragma unroll
@@ -273,22 +270,23 @@ __device__ __forceinline__ void efla_state_update(float (&S)[D / 8][4], const fl
     uint32_t bq[4][4];
     float acc[4][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      ldsm4_t(bq[n], kbase + (lane * LD + (n0 + n) * 8) * 2);
-#pragma unroll
-      for (int x = 0; x < 4; ++x) acc[n][x] = 0.f;
-    }
+    for (int n = 0; n < 4; ++n) ldsm4_t(bq[n], kbase + (lane * LD + (n0 + n) * 8) * 2);
 #pragma unroll
     for (int p = 0; p < 3; ++p)
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
-          mma_bf16(acc[n], p == 0 ? lo[ks] : (p == 1 ? mid[ks] : hi[ks]), bq[n][2 * ks], bq[n][2 * ks + 1]);
+        for (int n = 0; n < 4; ++n) {
+          if (p == 0 && ks == 0) mma_bf16_first(acc[n], lo[0], bq[n][0], bq[n][1]);
+          else mma_bf16(acc[n], p == 0 ? lo[ks] : (p == 1 ? mid[ks] : hi[ks]), bq[n][2 * ks], bq[n][2 * ks + 1]);
+        }
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) S[n0 + n][x] = SUB ? S[n0 + n][x] - acc[n][x] : S[n0 + n][x] + acc[n][x];
+      for (int hf = 0; hf < 2; ++hf) {
+        const uint64_t s = pair_of(S[n0 + n], hf), a = pair_of(acc[n], hf);
+        put_pair(S[n0 + n], hf, SUB ? fma_f32x2(a, pack_f32x2(-1.f, -1.f), s) : add_f32x2(s, a));
+      }
   }
 }
 
@@ -454,7 +452,8 @@ __device__ __forceinline__ void efla_errors(float (&e)[4][4], const uint32_t (&v
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-    for (int x = 0; x < 4; ++x) e[nt][x] = ((x & 1) ? bf16_hi(vq[x >> 1][nt]) : bf16_lo(vq[x >> 1][nt])) - e[nt][x];
+    for (int hf = 0; hf < 2; ++hf)
+      put_pair(e[nt], hf, fma_f32x2(pair_of(e[nt], hf), pack_f32x2(-1.f, -1.f), pack_f32x2(bf16_lo(vq[hf][nt]), bf16_hi(vq[hf][nt]))));
 }
 
 // Chunk-boundary states are stored as the warps hold them: [B, H, chunk][d / 16 value blocks][d / 8 tiles][lane] float4.
@@ -545,9 +544,10 @@ __device__ __forceinline__ bool efla_fwd_walk(
       const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-        oq[hf][nt] = pack_bf16(fmaf(-ex.x, e[nt][2 * hf], bf16_lo(vq[hf][nt])), fmaf(-ex.y, e[nt][2 * hf + 1], bf16_hi(vq[hf][nt])));
-        e[nt][2 * hf] *= cc.x;
-        e[nt][2 * hf + 1] *= cc.y;
+        float o0, o1;
+        unpack_f32x2(fma_f32x2(pack_f32x2(-ex.x, -ex.y), pair_of(e[nt], hf), pack_f32x2(bf16_lo(vq[hf][nt]), bf16_hi(vq[hf][nt]))), o0, o1);
+        oq[hf][nt] = pack_bf16(o0, o1);
+        put_pair(e[nt], hf, mul_f32x2(pair_of(e[nt], hf), pack_f32x2(cc.x, cc.y)));
       }
     }
     if (bad) {
@@ -790,9 +790,12 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
 //   dlam_t = c_t sum_j (dO E)_tj + dc_t dc/dlam,   dbeta = sum_t dc_t ex_t
 // Only dS is sequential: efla_chunk_bwd_state_kernel walks the chunks backwards with dS in registers and writes the dS1 of every chunk;
 // efla_chunk_bwd_kernel then handles all chunks in parallel from the two chunk-boundary states.
-// B 8, T 2048, 16 heads of 64: 92 us and 253 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
+// B 8, T 2048, 16 heads of 64: 91 us and 255 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
 // finish). The parallel kernel issues about 400 mma.sync per warp and chunk (94 us of tensor time at 8.3 cycles each) and reads 370 MB
-// (55 us); a third CTA per SM, at 168 registers, did not make it faster.
+// (55 us); it is bound by the chain of its two warps per scheduler (five cycles per instruction of a warp, a third of the issue slots). A third CTA
+// per SM, at 168 registers, did not make it faster; nor did a tenth fewer instructions (packed remainders of the splits, first products without zeroed
+// sums, per-token sums halved from lane to lane) with 64-wide heads. With 128-wide ones, one CTA per SM, these, the start's states asked for into L2 one
+// round of CTAs ahead and read a second time behind the products of the other term took it from 99 to 91.5 us (B 2, T 1531, 8 heads).
 template <int D, bool CHECKED, bool CUT>
 __device__ __forceinline__ bool efla_bwd_walk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ nmat,
@@ -850,8 +853,8 @@ __device__ __forceinline__ bool efla_bwd_walk(
       const float2 ex = *reinterpret_cast<const float2*>(cf + EC + nt * 8 + 2 * q);
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-        e[nt][2 * hf] = cc.x * e[nt][2 * hf] - ex.x * bf16_lo(oq[hf][nt]);
-        e[nt][2 * hf + 1] = cc.y * e[nt][2 * hf + 1] - ex.y * bf16_hi(oq[hf][nt]);
+        const uint64_t o = mul_f32x2(pack_f32x2(-ex.x, -ex.y), pack_f32x2(bf16_lo(oq[hf][nt]), bf16_hi(oq[hf][nt])));
+        put_pair(e[nt], hf, fma_f32x2(pack_f32x2(cc.x, cc.y), pair_of(e[nt], hf), o));
       }
     }
     efla_apply_n<true>(e, st + L::N, lane);
@@ -962,9 +965,10 @@ __device__ __forceinline__ void efla_get_b(uint32_t (&b)[3][4], uint32_t scr, in
   for (int p = 0; p < 3; ++p) ldsm4_t(b[p], scr + (p * 16 * LD + (lane & 15) * LD + np * 16 + (lane >> 4) * 8) * 2);
 }
 // the i-th of the six products of two split operands, small ones first
-__device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int o, int i) {
+__device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int o, int i, bool first) {
   const int ai = i == 0 || i == 3 ? 1 : (i == 1 ? 2 : 0), bi = i == 0 || i == 4 ? 1 : (i == 2 ? 2 : 0);
-  mma_bf16(acc, a[ai], b[bi][o], b[bi][o + 1]);
+  if (first) mma_bf16_first(acc, a[ai], b[bi][o], b[bi][o + 1]);
+  else mma_bf16(acc, a[ai], b[bi][o], b[bi][o + 1]);
 }
 
 template <int D, bool CHECKED>
@@ -972,7 +976,7 @@ __device__ __forceinline__ bool efla_bwd_chunk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ dout,
     const __nv_bfloat16* __restrict__ nmat, const float* __restrict__ coef, const float4* __restrict__ ckpt,
     const float4* __restrict__ dckpt, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-    float* __restrict__ dbeta_tok, int T, int H, int nchunks) {
+    float* __restrict__ dbeta_tok, int T, int H, int nchunks, int ahead) {
   using L = EflaBwdSmem<D>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
@@ -1007,12 +1011,17 @@ __device__ __forceinline__ bool efla_bwd_chunk(
     const float4 f = sp[i * 32];
     S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
   }
+  if (tid == 0 && id + ahead < gridDim.x) {                             // the states of the chunk that follows on this SM, into L2
+    const long long at = (id + ahead) * (D * D);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const float*>(ckpt) + at), "r"(D * D * 4) : "memory");
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const float*>(dckpt) + at), "r"(D * D * 4) : "memory");
+  }
   cp_async_wait<0>();
   __syncthreads();
 
   float* sG = reinterpret_cast<float*>(smem + L::G);
   if (warp < 2) {                          // rows 16 warp .. of the Gram matrix, lower tiles
-    float acc[4][4] = {};
+    float acc[4][4];
 #pragma unroll
     for (int kk = 0; kk < D / 16; ++kk) {
       uint32_t a[4];
@@ -1021,8 +1030,13 @@ __device__ __forceinline__ bool efla_bwd_chunk(
       for (int np = 0; np < 2; ++np) {
         uint32_t bq[4];
         ldsm4(bq, base + L::K + ((np * 16 + (lane & 7) + (lane >> 4) * 8) * L::LD + kk * 16 + ((lane >> 3) & 1) * 8) * 2);
-        mma_bf16(acc[2 * np], a, bq[0], bq[1]);
-        mma_bf16(acc[2 * np + 1], a, bq[2], bq[3]);
+        if (kk == 0) {
+          mma_bf16_first(acc[2 * np], a, bq[0], bq[1]);
+          mma_bf16_first(acc[2 * np + 1], a, bq[2], bq[3]);
+        } else {
+          mma_bf16(acc[2 * np], a, bq[0], bq[1]);
+          mma_bf16(acc[2 * np + 1], a, bq[2], bq[3]);
+        }
       }
     }
 #pragma unroll
@@ -1052,6 +1066,7 @@ __device__ __forceinline__ bool efla_bwd_chunk(
   efla_state_times_k<D>(de, S, base + L::K, lane);
   float* ssum = reinterpret_cast<float*>(smem + L::SUM) + warp * 2 * EC;
   auto sums_and_de = [&]() {               // the sums of Y E and dO E over the warp's columns; de: from Y to dE
+    float t[16];                           // [Y E, dO E][token tile][token 2 q, 2 q + 1]
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
@@ -1068,17 +1083,25 @@ __device__ __forceinline__ bool efla_bwd_chunk(
         de[nt][2 * hf + 1] = cc.y * de[nt][2 * hf + 1] - ex.y * o1;
       }
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
-#pragma unroll
-        for (int m = 4; m < 32; m <<= 1) {
-          ye[x] += __shfl_xor_sync(0xffffffffu, ye[x], m);
-          oe[x] += __shfl_xor_sync(0xffffffffu, oe[x], m);
-        }
-      if (g == 0) {
-        *reinterpret_cast<float2*>(ssum + nt * 8 + 2 * q) = make_float2(ye[0], ye[1]);
-        *reinterpret_cast<float2*>(ssum + EC + nt * 8 + 2 * q) = make_float2(oe[0], oe[1]);
+      for (int x = 0; x < 2; ++x) {
+        t[nt * 2 + x] = ye[x];
+        t[8 + nt * 2 + x] = oe[x];
       }
     }
+    // over the eight lanes of a q: every step adds half of the sums and hands the others to the lane that adds them (14 exchanges, not 48)
+#pragma unroll
+    for (int st = 0; st < 3; ++st) {
+      const int n = 8 >> st, m = 4 << st;
+      const bool upper = lane & m;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float give = upper ? t[i] : t[i + n], keep = upper ? t[i + n] : t[i];
+        t[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+      }
+    }
+    // lane bits 2, 3, 4 say which: Y E or dO E, upper or lower two token tiles, which of the two
+    const int nt = (lane >> 3 & 1) * 2 + (lane >> 4 & 1);
+    *reinterpret_cast<float2*>(ssum + (lane >> 2 & 1) * EC + nt * 8 + 2 * q) = make_float2(t[0], t[1]);
   };
   sums_and_de();
   efla_apply_n<true>(de, base + L::N, lane);
@@ -1136,12 +1159,6 @@ __device__ __forceinline__ bool efla_bwd_chunk(
   }
   // dK partial (2 x d / 8 tiles) = U dS1^T - dE0 S0^T
   float acc[2][D / 8][4];
-#pragma unroll
-  for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) acc[mi][i][x] = 0.f;
   uint32_t a[2][3][4];
 #pragma unroll
   for (int term = 0; term < 2; ++term) {
@@ -1151,13 +1168,6 @@ __device__ __forceinline__ bool efla_bwd_chunk(
       const float2 cc = *reinterpret_cast<const float2*>(cf + nt * 8 + 2 * q);
 #pragma unroll
       for (int x = 0; x < 4; ++x) w[nt][x] = term == 0 ? e[nt][x] * ((x & 1) ? cc.y : cc.x) : -de[nt][x];
-    }
-    if (term == 1) {
-#pragma unroll
-      for (int i = 0; i < D / 8; ++i) {
-        const float4 f = sp[i * 32];
-        S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
-      }
     }
     efla_put_tokens(scr_e, w, lane);
 #pragma unroll
@@ -1171,6 +1181,13 @@ __device__ __forceinline__ bool efla_bwd_chunk(
         for (int p = 0; p < 3; ++p)
           stsm4(scr_s + (p * 16 * L::LD + (hf * 8 + (lane & 7)) * L::LD + i4 * 32 + (lane >> 3) * 8) * 2, s[p][0], s[p][1], s[p][2], s[p][3]);
       }
+    if (term == 0) {                       // S0 once more, on its way while these products run
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i) {
+        const float4 f = sp[i * 32];
+        S[i][0] = f.x; S[i][1] = f.y; S[i][2] = f.z; S[i][3] = f.w;
+      }
+    }
     __syncwarp();
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi) efla_get_a(a[mi], scr_e, mi, lane);
@@ -1182,8 +1199,8 @@ __device__ __forceinline__ bool efla_bwd_chunk(
       for (int i = 0; i < 6; ++i)
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi) {
-          mma_split(acc[mi][2 * np], a[mi], bq, 0, i);
-          mma_split(acc[mi][2 * np + 1], a[mi], bq, 2, i);
+          mma_split(acc[mi][2 * np], a[mi], bq, 0, i, term == 0 && i == 0);
+          mma_split(acc[mi][2 * np + 1], a[mi], bq, 2, i, term == 0 && i == 0);
         }
     }
     __syncwarp();
@@ -1200,9 +1217,9 @@ __device__ __forceinline__ bool efla_bwd_chunk(
     for (int mi = np; mi < 2; ++mi)
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        float da[4] = {0.f, 0.f, 0.f, 0.f};
+        float da[4];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) mma_split(da, a[mi], bq, 2 * u, i);
+        for (int i = 0; i < 6; ++i) mma_split(da, a[mi], bq, 2 * u, i, i == 0);
         *reinterpret_cast<float2*>(&sda[(mi * 16 + g) * L::GLD + np * 16 + u * 8 + 2 * q]) = make_float2(da[0], da[1]);
         *reinterpret_cast<float2*>(&sda[(mi * 16 + g + 8) * L::GLD + np * 16 + u * 8 + 2 * q]) = make_float2(da[2], da[3]);
       }
@@ -1255,12 +1272,6 @@ __device__ __forceinline__ bool efla_bwd_chunk(
   // key rows 16 warp ..: dK = sum of the partials + sym K
   float dkt[2][2][4];
 #pragma unroll
-  for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) dkt[mi][u][x] = 0.f;
-#pragma unroll
   for (int ks = 0; ks < 2; ++ks) {
     uint32_t b0[4];
     ldsm4_t(b0, base + L::K + ((ks * 16 + (lane & 15)) * L::LD + warp * 16 + (lane >> 4) * 8) * 2);
@@ -1276,7 +1287,8 @@ __device__ __forceinline__ bool efla_bwd_chunk(
       for (int x = 0; x < 4; ++x) split3(f[x].x, f[x].y, hi[x], mid[x], lo[x]);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        mma_bf16(dkt[mi][u], lo, b0[2 * u], b0[2 * u + 1]);
+        if (ks == 0) mma_bf16_first(dkt[mi][u], lo, b0[2 * u], b0[2 * u + 1]);
+        else mma_bf16(dkt[mi][u], lo, b0[2 * u], b0[2 * u + 1]);
         mma_bf16(dkt[mi][u], mid, b0[2 * u], b0[2 * u + 1]);
         mma_bf16(dkt[mi][u], hi, b0[2 * u], b0[2 * u + 1]);
       }
@@ -1309,7 +1321,7 @@ template <int D>
 __device__ __noinline__ void efla_bwd_chunk_again(const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* dout,
                                                   const __nv_bfloat16* nmat, const float* coef, const float4* ckpt, const float4* dckpt,
                                                   __nv_bfloat16* dk, __nv_bfloat16* dv, float* dbeta_tok, int T, int H, int nchunks) {
-  efla_bwd_chunk<D, true>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks);
+  efla_bwd_chunk<D, true>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks, 1 << 30);
 }
 
 template <int D>
@@ -1317,8 +1329,8 @@ __global__ void __launch_bounds__(2 * D, D <= 64 ? 2 : 1) efla_chunk_bwd_kernel(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ dout,
     const __nv_bfloat16* __restrict__ nmat, const float* __restrict__ coef, const float4* __restrict__ ckpt,
     const float4* __restrict__ dckpt, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-    float* __restrict__ dbeta_tok, int T, int H, int nchunks) {
-  if (__syncthreads_or(efla_bwd_chunk<D, false>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks)))
+    float* __restrict__ dbeta_tok, int T, int H, int nchunks, int ahead) {
+  if (__syncthreads_or(efla_bwd_chunk<D, false>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks, ahead)))
     efla_bwd_chunk_again<D>(k, v, dout, nmat, coef, ckpt, dckpt, dk, dv, dbeta_tok, T, H, nchunks);
 }
 
@@ -1360,7 +1372,8 @@ int launch_chunk_bwd(const void* k, const void* v, const void* nmat, const float
   ELFA_CUDA(cudaGetLastError());
   efla_chunk_bwd_kernel<D><<<(unsigned)total, 2 * D, M::BYTES, s>>>(
       K, static_cast<const __nv_bfloat16*>(v), O, N, coef, reinterpret_cast<const float4*>(ckpt),
-      reinterpret_cast<const float4*>(dckpt), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), dbeta_tok, T, H, nchunks);
+      reinterpret_cast<const float4*>(dckpt), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), dbeta_tok, T, H, nchunks,
+      (D <= 64 ? 2 : 1) * (device_sm_count() > 0 ? device_sm_count() : 148));
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;

@@ -17,6 +17,12 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// c = a b, the first product of a sum: nothing has to be set to zero before
+__device__ __forceinline__ void mma_bf16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -41,12 +47,20 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // x = hi + mid + lo, each a bf16 (8 significant bits): 24 bits, i.e. fp32 without loss. Two values per register.
+// The remainders of both are one packed operation each (exact: -1 times a part, added to what it was taken from).
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint64_t minus = pack_f32x2(-1.f, -1.f);
   hi = pack_bf16(x, y);
-  const float x1 = x - bf16_lo(hi), y1 = y - bf16_hi(hi);
-  mid = pack_bf16(x1, y1);
-  lo = pack_bf16(x1 - bf16_lo(mid), y1 - bf16_hi(mid));
+  uint64_t rest = fma_f32x2(pack_f32x2(bf16_lo(hi), bf16_hi(hi)), minus, pack_f32x2(x, y));
+  unpack_f32x2(rest, x, y);
+  mid = pack_bf16(x, y);
+  rest = fma_f32x2(pack_f32x2(bf16_lo(mid), bf16_hi(mid)), minus, rest);
+  unpack_f32x2(rest, x, y);
+  lo = pack_bf16(x, y);
 }
+// two neighbouring values of an accumulator tile as a packed pair
+__device__ __forceinline__ uint64_t pair_of(const float (&t)[4], int hf) { return pack_f32x2(t[2 * hf], t[2 * hf + 1]); }
+__device__ __forceinline__ void put_pair(float (&t)[4], int hf, uint64_t v) { unpack_f32x2(v, t[2 * hf], t[2 * hf + 1]); }
 // The A operand (three splits) of two neighbouring accumulator tiles.
 __device__ __forceinline__ void split3_a(uint32_t (&hi)[4], uint32_t (&mid)[4], uint32_t (&lo)[4], const float (&t0)[4], const float (&t1)[4]) {
   split3(t0[0], t0[1], hi[0], mid[0], lo[0]);
