@@ -654,70 +654,106 @@ __global__ void __launch_bounds__(32 * ec_warps<D>()) efla_chunk_fwd_kernel(
     efla_fwd_again<D, CUT>(k, v, nmat, coef, o, ckpt, T, H, nchunks, w);
 }
 
-// start[p + dir] = A[p] start[p] + B[p] for the P - 2 inner segments, in order; a CTA owns 16 columns of a head, a thread D / 16 rows of one
-// column. The next A is on its way while this one is used. fp32 sums in four parts of D / 4: the errors that this adds to a start stay below
-// those of the walks (64-bit comparison, B 1, T 8192, 16 heads of 64, 10
-// segments: final state as in one walk). Grid (B * H, d / 16).
+// the i-th of the six products of two split operands, small ones first
+__device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int o, int i, bool first) {
+  const int ai = i == 0 || i == 3 ? 1 : (i == 1 ? 2 : 0), bi = i == 0 || i == 4 ? 1 : (i == 2 ? 2 : 0);
+  if (first) mma_bf16_first(acc, a[ai], b[bi][o], b[bi][o + 1]);
+  else mma_bf16(acc, a[ai], b[bi][o], b[bi][o + 1]);
+}
+
+// start[p + dir] = A[p] start[p] + B[p] for the P - 2 inner segments, in order, on the tensor cores: a CTA owns 16 columns of a head, warp w the rows
+// 16 w .. 16 w + 15. Both operands are split in three (24 bits each; the six products above 2^-24, small ones first, in three sums joined at the end), so a
+// start is as close to the 64-bit one as with fp32 multiply-adds (which the walks' errors hide either way: final state, B 1, T 8192, 16 heads of 64, 10
+// segments, 2.2e-7 relative). The next A is copied to shared memory while this one is used; the start goes to the next step as splits in shared memory.
+// Bound by the chain of a step: the sums, the splits of the start, one barrier. Per step of 128 and 64 rows 1.9 and 1.1 us, with fp32 multiply-adds 6.3 and
+// 1.6. Grid (B * H, d / 16).
 template <int D>
-__global__ void __launch_bounds__(256) efla_combine_kernel(const float* __restrict__ coef, float* __restrict__ work, int nchunks, int P, int dir) {
-  constexpr int EPT = D / 16, DD = D * D, LD = D + 4, VPT = DD / 1024;       // 16-byte vectors of A per thread
+struct EflaCombineSmem {
+  static constexpr int ALD = D + 8, SLD = D + 8;                             // A fp32; splits of the start, a row per column
+  static constexpr int A = 0, S = 2 * D * ALD * 4, BYTES = S + 2 * 3 * 16 * SLD * 2;
+};
+template <int D>
+__global__ void __launch_bounds__(2 * D) efla_combine_kernel(const float* __restrict__ coef, float* __restrict__ work, int nchunks, int P, int dir) {
+  using L = EflaCombineSmem<D>;
   extern __shared__ __align__(16) unsigned char smem[];
-  float* sa = reinterpret_cast<float*>(smem);
-  float(*ss)[17] = reinterpret_cast<float(*)[17]>(smem + D * LD * 4);
-  const int bh = blockIdx.x, col = threadIdx.x & 15, r0 = (threadIdx.x >> 4) * EPT, c = blockIdx.y * 16 + col;
-  int p = dir > 0 ? 1 : P - 2;
+  const uint32_t base = smem_u32(smem);
+  const int bh = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, r0 = warp * 16 + g, c0 = blockIdx.y * 16 + 2 * q;
   if (efla_in_one_piece(coef, bh, nchunks)) return;
-  const float* s0 = efla_work(work, 0, P, p, bh, DD);
-  float4 nxt[VPT];
-  float bn[EPT];
-  auto fetch = [&](int at) {
-    const float4* a = reinterpret_cast<const float4*>(efla_work(work, 1, P, at, bh, DD));
-    const float* bb = efla_work(work, 2, P, at, bh, DD);
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) nxt[i] = a[threadIdx.x + i * 256];
-#pragma unroll
-    for (int i = 0; i < EPT; ++i) bn[i] = bb[(r0 + i) * D + c];
+  int p = dir > 0 ? 1 : P - 2;
+  auto fetch = [&](int n, int at) {                    // A of the n-th step
+    const float* a = efla_work(work, 1, P, at, bh, D * D);
+    for (int i = threadIdx.x; i < D * D / 4; i += 2 * D)
+      cp_async16(base + L::A + ((n & 1) * D * L::ALD + i / (D / 4) * L::ALD + i % (D / 4) * 4) * 4, a + i * 4, true);
+    cp_async_commit();
   };
-  fetch(p);
+  // tile j of eight columns, half hf of the warp's rows: row r0 + 8 hf, columns c0 + 8 j and the next
+  auto put_start = [&](int n, const float (&s)[2][4]) {
+    uint32_t t[3][4];
 #pragma unroll
-  for (int i = 0; i < EPT; ++i) ss[r0 + i][col] = s0[(r0 + i) * D + c];
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) split3(s[j][2 * hf], s[j][2 * hf + 1], t[0][2 * j + hf], t[1][2 * j + hf], t[2][2 * j + hf]);
+    const int col = (lane >> 4) * 8 + (lane & 7), row = warp * 16 + (lane >> 3 & 1) * 8;
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+      stsm4_t(base + L::S + (((n & 1) * 3 + x) * 16 * L::SLD + col * L::SLD + row) * 2, t[x][0], t[x][1], t[x][2], t[x][3]);
+  };
+  auto at = [&](float* m, int j, int hf) { return reinterpret_cast<float2*>(m + (r0 + 8 * hf) * D + c0 + 8 * j); };
+  fetch(0, p);
+  float s[2][4], bn[2][4];
+  auto read = [&](float (&to)[2][4], float* m) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const float2 f = *at(m, j, hf);
+        to[j][2 * hf] = f.x;
+        to[j][2 * hf + 1] = f.y;
+      }
+  };
+  read(s, efla_work(work, 0, P, p, bh, D * D));
+  read(bn, efla_work(work, 2, P, p, bh, D * D));
+  put_start(0, s);
   for (int n = 0; n < P - 2; ++n, p += dir) {
+    cp_async_wait<0>();
+    __syncthreads();                                   // A and the start have landed; the buffers of the step before are free
+    float b[2][4];
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int at = (threadIdx.x + i * 256) * 4;
-      *reinterpret_cast<float4*>(sa + at / D * LD + at % D) = nxt[i];
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) b[j][x] = bn[j][x];
+    if (n + 1 < P - 2) {
+      fetch(n + 1, p + dir);
+      read(bn, efla_work(work, 2, P, p + dir, bh, D * D));
     }
-    float sum[EPT];
+    float acc[3][2][4];                                // the smallest products, the middle ones, the large ones
+    const float* sa = reinterpret_cast<const float*>(smem + L::A) + (n & 1) * D * L::ALD;
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) sum[i] = bn[i];
-    __syncthreads();
-    if (n + 1 < P - 2) fetch(p + dir);
+    for (int k = 0; k < D / 16; ++k) {
+      uint32_t a[3][4], f[3][4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float acc[EPT];
-#pragma unroll
-      for (int i = 0; i < EPT; ++i) acc[i] = 0.f;
-#pragma unroll 2
-      for (int j = q * (D / 4); j < (q + 1) * (D / 4); j += 4) {
-        float x[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) x[u] = ss[j + u][col];
-#pragma unroll
-        for (int i = 0; i < EPT; ++i) {
-          const float4 a = *reinterpret_cast<const float4*>(sa + (r0 + i) * LD + j);
-          acc[i] += a.x * x[0] + a.y * x[1] + (a.z * x[2] + a.w * x[3]);
-        }
+      for (int x = 0; x < 4; ++x) {                    // a0, a1: rows g, g + 8; a2, a3: the columns 8 further
+        const float2 v = *reinterpret_cast<const float2*>(sa + (r0 + (x & 1) * 8) * L::ALD + k * 16 + (x >> 1) * 8 + 2 * q);
+        split3(v.x, v.y, a[0][x], a[1][x], a[2][x]);
       }
 #pragma unroll
-      for (int i = 0; i < EPT; ++i) sum[i] += acc[i];
-    }
-    __syncthreads();
-    float* out = efla_work(work, 0, P, p + dir, bh, DD);
+      for (int x = 0; x < 3; ++x)
+        ldsm4(f[x], base + L::S + (((n & 1) * 3 + x) * 16 * L::SLD + ((lane >> 4) * 8 + (lane & 7)) * L::SLD + k * 16 + (lane >> 3 & 1) * 8) * 2);
 #pragma unroll
-    for (int i = 0; i < EPT; ++i) {
-      out[(r0 + i) * D + c] = sum[i];
-      ss[r0 + i][col] = sum[i];
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma_split(acc[i < 3 ? 0 : (i < 5 ? 1 : 2)][j], a, f, 2 * j, i, k == 0 && (i == 0 || i == 3 || i == 5));
     }
+    float* out = efla_work(work, 0, P, p + dir, bh, D * D);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+        for (int x = 2 * hf; x < 2 * hf + 2; ++x) s[j][x] = ((acc[0][j][x] + acc[1][j][x]) + acc[2][j][x]) + b[j][x];
+        *at(out, j, hf) = make_float2(s[j][2 * hf], s[j][2 * hf + 1]);
+      }
+    if (n + 1 < P - 2) put_start(n + 1, s);
   }
 }
 
@@ -736,9 +772,9 @@ cudaError_t allow_shared(int bytes) {
 template <int D>
 int launch_combine(const float* coef, float* work, int BH, int nchunks, int P, int dir, cudaStream_t s) {
   if (P < 3) return ELFA_OK;
-  constexpr int bytes = (D * (D + 4) + D * 17) * 4;
+  constexpr int bytes = EflaCombineSmem<D>::BYTES;
   ELFA_CUDA(allow_shared<efla_combine_kernel<D>>(bytes));
-  efla_combine_kernel<D><<<dim3(BH, D / 16), 256, bytes, s>>>(coef, work, nchunks, P, dir);
+  efla_combine_kernel<D><<<dim3(BH, D / 16), 2 * D, bytes, s>>>(coef, work, nchunks, P, dir);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;
@@ -964,13 +1000,6 @@ __device__ __forceinline__ void efla_get_b(uint32_t (&b)[3][4], uint32_t scr, in
 #pragma unroll
   for (int p = 0; p < 3; ++p) ldsm4_t(b[p], scr + (p * 16 * LD + (lane & 15) * LD + np * 16 + (lane >> 4) * 8) * 2);
 }
-// the i-th of the six products of two split operands, small ones first
-__device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int o, int i, bool first) {
-  const int ai = i == 0 || i == 3 ? 1 : (i == 1 ? 2 : 0), bi = i == 0 || i == 4 ? 1 : (i == 2 ? 2 : 0);
-  if (first) mma_bf16_first(acc, a[ai], b[bi][o], b[bi][o + 1]);
-  else mma_bf16(acc, a[ai], b[bi][o], b[bi][o + 1]);
-}
-
 template <int D, bool CHECKED>
 __device__ __forceinline__ bool efla_bwd_chunk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ dout,
@@ -1400,7 +1429,7 @@ static int efla_segments(int B, int T, int H, int d, double least) {
   const int nchunks = (T + EC - 1) / EC, sms = device_sm_count() > 0 ? device_sm_count() : 148;
   const long long units = (long long)B * H * (d == 128 || d == 96 ? 2 : 1);
   struct Cost { double one, full; int resident; double launches, joint; };      // microseconds
-  const Cost c = d == 128 ? Cost{2.1, 3.6, 2, 16, 4} : (d == 96 ? Cost{1.76, 2.6, 2, 9, 3.5} : (d == 64 ? Cost{1.4, 1.9, 2, 6, 3} : Cost{1.16, 1.4, 4, 4, 1}));
+  const Cost c = d == 128 ? Cost{2.1, 3.6, 2, 16, 2.2} : (d == 96 ? Cost{1.76, 2.6, 2, 9, 1.6} : (d == 64 ? Cost{1.4, 1.9, 2, 6, 0.9} : Cost{1.16, 1.4, 4, 4, 0.5}));
   auto steps = [&](long long walks) {
     const long long ctas = units * walks, round = (long long)c.resident * sms, rest = ctas % round;
     return c.full * (double)(ctas / round) + (rest == 0 ? 0. : (rest <= sms ? c.one : c.full));
