@@ -14,10 +14,9 @@ from typing import List, Optional
 
 import torch
 import torch.nn as nn
-from torch.autograd import forward_ad
 from torch.nn.modules import module as nn_module
 
-from ..native import lib, stream_ptr
+from ..native import lib, plain_eager, stream_ptr
 from ..ops import efla as eops
 from ..ops.attention import DECODE_HEAD_DIMS, DECODE_ROWS
 from ..ops.nn import _EW
@@ -26,11 +25,8 @@ _ACTS = {"swiglu": -1, "gelu": 0, **{k: v[0] for k, v in _EW.items() if k != "ge
 
 
 def _plain_mode() -> bool:
-    """Eager execution without a gradient: no tracing, no dispatch or function mode, no transform, no forward-mode level (which ``no_grad`` leaves
-    open: a state may be a dual tensor, whose tangent the layers refuse to drop)."""
-    return (not torch.is_grad_enabled() and forward_ad._current_level < 0 and not nn_module._has_any_global_hook() and not torch.jit.is_tracing()
-            and not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
-            and torch._C._functorch.peek_interpreter_stack() is None)
+    """Eager execution without a gradient (a state may be a dual tensor, whose tangent the layers refuse to drop), and no hooks on all modules."""
+    return plain_eager() and not nn_module._has_any_global_hook()
 
 
 def _eager(ids: torch.Tensor) -> bool:

@@ -14,6 +14,7 @@ from pathlib import Path
 from typing import Any, Dict, Optional
 
 import torch
+from torch.autograd import forward_ad
 
 _PKG = Path(__file__).resolve().parent
 # ELFA_BOUNDS=1 selects the checked variant of the library (see build.build(bounds=True)): in-kernel index checks that record
@@ -147,6 +148,14 @@ def stream_ptr(t: Optional[torch.Tensor] = None) -> int:
     if i < 0:            # the index of a host tensor, which stands for the current device: no kernel may be given such a tensor
         raise ValueError(f"Expected a cuda device, but got: {t.device}")
     return torch._C._cuda_getCurrentRawStream(i)
+
+
+def plain_eager() -> bool:
+    """Eager execution without a gradient: no tracing, no dispatch or function mode, no transform, no forward-mode level (which ``no_grad`` leaves
+    open). An operation may then call its kernel without an autograd function around it, for tensors that are no subclass."""
+    return (not torch.is_grad_enabled() and forward_ad._current_level < 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None)
 
 
 def status() -> int:

@@ -131,7 +131,6 @@ def test_lion_muon_update_replayed_from_a_cuda_graph_equals_eager(cuda_device, m
 
 
 def test_prism_refine_kernel_matches_reference(cuda_device):
-    from elfa_b200.ops import efla as eops
     torch.manual_seed(0)
     B, T, G, d, L = 2, 64, 8, 64, 3
     u = (torch.randn(B, T, G * d, device=cuda_device) * 0.5).bfloat16().requires_grad_(True)
@@ -148,3 +147,27 @@ def test_prism_refine_kernel_matches_reference(cuda_device):
     want = [y2.detach(), u2.grad, v2.grad] + [p.grad for p in ps2]
     for a, b in zip(got, want):
         assert (a - b).abs().max() <= 0.02 * b.abs().max() + 0.02, ((a - b).abs().max(), b.abs().max())
+
+
+def test_calls_without_a_gradient_take_what_the_autograd_function_takes(cuda_device):
+    """The direct route gives the bits of the other one, for every layout, type and length that it sees; transforms, tangents and subclasses keep
+    going through the function."""
+    import torch.autograd.forward_ad as fwd
+    g = torch.Generator(device=cuda_device).manual_seed(0)
+    r = lambda *s: torch.randn(*s, generator=g, device=cuda_device)
+    beta = torch.full((1,), 0.4, device=cuda_device)
+    for T in (1, 17, 113, 300):
+        k, v, s0 = (r(2, T, 2, 64) * 0.4).bfloat16(), r(2, T, 2, 64).bfloat16(), r(2, 2, 64, 64) * 0.3
+        odd = torch.empty(2 * T * 2 * 64 + 3, dtype=torch.bfloat16, device=cuda_device)[3:].view(2, T, 2, 64).copy_(k)
+        for kk, vv, b, s in ((k, v, beta, s0), (odd, v.transpose(1, 2).contiguous().transpose(1, 2), beta.reshape(()), None), (k, v, beta, s0.transpose(2, 3)),
+                             (k, v, beta, s0.double()), (k, v, beta.double(), s0.bfloat16())):
+            want = eops.efla_scan(kk, vv, b, s)                                # gradients on, none wanted: the function
+            with torch.no_grad():
+                got = eops.efla_scan(kk, vv, b, s)
+            assert all(torch.equal(x, y) and x.stride() == y.stride() for x, y in zip(got, want))
+    with torch.no_grad(), fwd.dual_level():
+        with pytest.raises(NotImplementedError):
+            eops.efla_scan(fwd.make_dual(k, torch.ones_like(k)), v, beta, s0)
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        torch.func.vmap(lambda x: eops.efla_scan(x, v, beta, s0)[0])(torch.stack((k, k)))
+    assert native.status() == 0
