@@ -33,9 +33,13 @@ namespace elfa {
 namespace {
 
 constexpr int EC = 32;                     // tokens of a chunk
-constexpr int EN_LD = 40;                  // row pitch of N in shared memory (bf16)
-constexpr int EN_ELEMS = 3 * EC * EC;      // one chunk's N: [split][t][s] bf16 in global memory
+constexpr int EN_LD = 40;                  // row pitch of a warp's split tiles in shared memory (bf16)
+constexpr int EN_ELEMS = 3 * EC * EC;      // one chunk's N: [split][t][s] bf16, the four 16-byte pieces of a row exchanged (efla_n_piece)
 constexpr int EC_COEF = 4 * EC;            // one chunk's coefficients in global memory
+
+// Byte offset of piece c (columns 8 c ..) of row t of one split of N, in global and in shared memory alike: eight rows of 64 bytes, read at one
+// piece by ldmatrix, lie in different banks, and a chunk's N is one contiguous copy
+__device__ __forceinline__ int efla_n_piece(int t, int c) { return t * 64 + ((c ^ (t >> 1 & 3)) << 4); }
 
 // ------------------------------------------------------------------------------------------------ state-independent part
 // One warp per (batch, head, chunk): Gram matrix by mma.sync (exact bf16 products), then lane s eliminates column s of the unit
@@ -150,10 +154,10 @@ __global__ void __launch_bounds__(64) efla_prep_kernel(const __nv_bfloat16* __re
     x[t] = t < lane ? 0.f : (t == lane ? 1.f : -s);
   }
   // neighbouring lanes trade halves so that a store carries two columns: even lanes write row t, odd lanes row t + 1
-  uint32_t* out = reinterpret_cast<uint32_t*>(nmat + id * EN_ELEMS) + (lane & 1) * (EC / 2) + (lane >> 1);
+  uint32_t* out = reinterpret_cast<uint32_t*>(nmat + id * EN_ELEMS) + (lane >> 1 & 3);
   auto put = [&](int split, int t, uint32_t v) {
     const uint32_t w = __shfl_xor_sync(0xffffffffu, v, 1);
-    out[(split * EC + t) * (EC / 2)] = (lane & 1) ? __byte_perm(w, v, 0x7632) : __byte_perm(v, w, 0x5410);
+    out[split * (EC * EC / 2) + efla_n_piece(t + (lane & 1), lane >> 3) / 4] = (lane & 1) ? __byte_perm(w, v, 0x7632) : __byte_perm(v, w, 0x5410);
   };
 #pragma unroll
   for (int t = 0; t < EC; t += 2) {
@@ -175,28 +179,60 @@ template <int D>
 struct EflaStage {                         // byte offsets inside one stage of the shared-memory ring
   static constexpr int VC = 16 * ec_warps<D>();
   static constexpr int KLD = D + 8, VLD = VC + 8;
-  static constexpr int K = 0, V = K + EC * KLD * 2, N = V + EC * VLD * 2, C = N + 3 * EC * EN_LD * 2, BYTES = C + 2 * EC * 4;
+  static constexpr int K = 0, V = K + EC * KLD * 2, N = V + EC * VLD * 2, C = N + EN_ELEMS * 2, BYTES = C + 2 * EC * 4;
 };
 
-template <int D, bool CUT>
-__device__ __forceinline__ void efla_stage_load(uint32_t st, const __nv_bfloat16* __restrict__ kb, const __nv_bfloat16* __restrict__ vb,
-                                                const __nv_bfloat16* __restrict__ nm, const float* __restrict__ cf, long long row_stride,
-                                                int n) {
+// A thread's place in the copies of a chunk's K and V tiles: it takes 16 bytes of every KR-th row of K, every VR-th row of V. N and the
+// coefficients are copied as they lie. With indices worked out per copy (and N in rows of a wider pitch) the copies took 690 of the 2600 cycles of a
+// chunk to issue; the walks are chains that nothing hides it behind.
+template <int D>
+struct EflaLoader {
   using L = EflaStage<D>;
-  constexpr int NT = 32 * ec_warps<D>();
-  for (int i = threadIdx.x; i < EC * (D / 8); i += NT) {
-    const int r = i / (D / 8), c = i % (D / 8);
-    cp_async16(st + L::K + (r * L::KLD + c * 8) * 2, kb + (r < n ? r : 0) * row_stride + c * 8, r < n);
+  static constexpr int NT = 32 * ec_warps<D>(), KR = NT / (D / 8), VR = NT / (L::VC / 8);
+  static_assert(NT % (D / 8) == 0 && NT % (L::VC / 8) == 0 && EC % KR == 0 && EC % VR == 0, "whole passes");
+  const __nv_bfloat16 *k, *v;              // this thread's vectors in the first chunk's first rows; v: null without values
+  const __nv_bfloat16* n;
+  const float* c;
+  long long rs;
+  uint32_t ring;
+  int krow, vrow, T;
+  __device__ __forceinline__ EflaLoader(const __nv_bfloat16* kb, const __nv_bfloat16* vb, const __nv_bfloat16* nb, const float* cb, long long rs_,
+                                        uint32_t ring_, int T_)
+      : n(nb + threadIdx.x * 8), c(cb + threadIdx.x * 4), rs(rs_), ring(ring_), krow(threadIdx.x / (D / 8)), vrow(threadIdx.x / (L::VC / 8)), T(T_) {
+    k = kb + krow * rs + threadIdx.x % (D / 8) * 8;
+    v = vb ? vb + vrow * rs + threadIdx.x % (L::VC / 8) * 8 : nullptr;
   }
-  for (int i = threadIdx.x; i < EC * (L::VC / 8); i += NT) {           // CUT: without values zeros
-    const int r = i / (L::VC / 8), c = i % (L::VC / 8);
-    const bool has = !CUT || vb;
-    cp_async16(st + L::V + (r * L::VLD + c * 8) * 2, has ? vb + (r < n ? r : 0) * row_stride + c * 8 : kb, has && r < n);
+  // chunk ch as the it-th of the ring's uses
+  __device__ __forceinline__ void operator()(int it, int ch) const {
+    const uint32_t st = ring + it % EC_STAGES * L::BYTES;
+    const __nv_bfloat16* ns = n + (long long)ch * EN_ELEMS;
+    static_assert(EN_ELEMS / 8 % NT == 0, "whole passes");
+#pragma unroll
+    for (int p = 0; p < EN_ELEMS / 8 / NT; ++p) cp_async16(st + L::N + (threadIdx.x + p * NT) * 16, ns + p * NT * 8, true);
+    if (threadIdx.x < 2 * EC / 4) cp_async16(st + L::C + threadIdx.x * 16, c + (long long)ch * EC_COEF, true);
+    const int rows = T - ch * EC;
+    const long long at = (long long)ch * EC * rs;
+    const uint32_t kd = st + L::K + (krow * L::KLD + threadIdx.x % (D / 8) * 8) * 2, vd = st + L::V + (vrow * L::VLD + threadIdx.x % (L::VC / 8) * 8) * 2;
+    if (rows >= EC && v) {
+      const __nv_bfloat16 *ks = k + at, *vs = v + at;
+#pragma unroll
+      for (int p = 0; p < EC / KR; ++p) cp_async16(kd + p * KR * L::KLD * 2, ks + p * KR * rs, true);
+#pragma unroll
+      for (int p = 0; p < EC / VR; ++p) cp_async16(vd + p * VR * L::VLD * 2, vs + p * VR * rs, true);
+    } else {                               // rows past the end, and values where there are none, become zero
+#pragma unroll
+      for (int p = 0; p < EC / KR; ++p) {
+        const bool in = krow + p * KR < rows;
+        cp_async16(kd + p * KR * L::KLD * 2, in ? k + at + p * KR * rs : n, in);
+      }
+#pragma unroll
+      for (int p = 0; p < EC / VR; ++p) {
+        const bool in = v && vrow + p * VR < rows;
+        cp_async16(vd + p * VR * L::VLD * 2, in ? v + at + p * VR * rs : n, in);
+      }
+    }
   }
-  for (int i = threadIdx.x; i < 3 * EC * 4; i += NT)
-    cp_async16(st + L::N + ((i / 4) * EN_LD + (i % 4) * 8) * 2, nm + i * 8, true);
-  if (threadIdx.x < 2 * EC / 4) cp_async16(st + L::C + threadIdx.x * 16, cf + threadIdx.x * 4, true);
-}
+};
 
 // e += N e for a warp's 16 x 32 tile (four C tiles, columns = tokens): six products of the splits, small ones first.
 // TRANS: the transposed matrix (e_r += sum_t N[t][r] e_t), for the gradient.
@@ -212,8 +248,8 @@ __device__ __forceinline__ void efla_apply_n(float (&e)[4][4], uint32_t nbase, i
     uint32_t bf[4][4];
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      if (TRANS) ldsm4_t(bf[nt], nbase + (p * EC * EN_LD + lane * EN_LD + nt * 8) * 2);      // rows t, columns r of tile nt
-      else ldsm4(bf[nt], nbase + (p * EC * EN_LD + (nt * 8 + (lane & 7)) * EN_LD + (lane >> 3) * 8) * 2);
+      if (TRANS) ldsm4_t(bf[nt], nbase + p * (EC * EC * 2) + efla_n_piece(lane, nt));        // rows t, columns r of tile nt
+      else ldsm4(bf[nt], nbase + p * (EC * EC * 2) + efla_n_piece(nt * 8 + (lane & 7), lane >> 3));
     }
 #pragma unroll
     for (int m = 2 - p; m >= 0; --m)       // splits of e that still count against this split of N
@@ -502,20 +538,20 @@ __device__ __forceinline__ bool efla_fwd_walk(
       S[n][x] = CUT && w.identity ? (row == col ? 1.f : 0.f) : (w.state0 ? w.state0[row * D + col] : 0.f);
     }
 
+  const EflaLoader<D> load(kb, vb, nb, cb, rs, ring, T);
   auto fetch = [&](int ch) {
-    if (ch < c1)
-      efla_stage_load<D, CUT>(ring + (ch % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, !CUT || vb ? vb + (long long)ch * EC * rs : nullptr,
-                         nb + (long long)ch * EN_ELEMS, cb + (long long)ch * EC_COEF, rs, min(EC, T - ch * EC));
+    if (ch < c1) load(ch, ch);
     cp_async_commit();
   };
 #pragma unroll
   for (int i = 0; i < EC_STAGES - 1; ++i) fetch(c0 + i);
   for (int ch = c0; ch < c1; ++ch) {
+    const int stage = ch % EC_STAGES;
     cp_async_wait<EC_STAGES - 2>();
     __syncthreads();                       // chunk ch has landed for every thread; the stage of chunk ch - 1 is free
     fetch(ch + EC_STAGES - 1);
-    const uint32_t st = ring + (ch % EC_STAGES) * L::BYTES;
-    const float* cf = reinterpret_cast<const float*>(smem + (ch % EC_STAGES) * L::BYTES + L::C);
+    const uint32_t st = ring + stage * L::BYTES;
+    const float* cf = reinterpret_cast<const float*>(smem + stage * L::BYTES + L::C);
     if (ckpt) {
       float4* dst = ckpt + efla_state_slot<D>((long long)bh * nchunks + ch, wcol / 16, lane);
 #pragma unroll
@@ -557,16 +593,16 @@ __device__ __forceinline__ bool efla_fwd_walk(
         for (int x = 0; x < 4; ++x)
           if (first[x >> 1] < EC) e[nt][x] = 0.f;                     // the walk below moves these columns
     }
-    efla_state_update<D, false>(S, e, st + L::K, lane);
-    if (!CUT || o) {
+    if (!CUT || o) {                       // the outputs change their layout while the state is updated
       const uint32_t so = smem_u32(stage_o);
       __syncwarp();
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) stsm4_t(so + (lane * 24 + hf * 8) * 2, oq[hf][0], oq[hf][1], oq[hf][2], oq[hf][3]);
       __syncwarp();
     }
+    efla_state_update<D, false>(S, e, st + L::K, lane);
     if (bad) {
-      const unsigned char* sst = smem + (ch % EC_STAGES) * L::BYTES;
+      const unsigned char* sst = smem + stage * L::BYTES;
       float sl[D / 2];
 #pragma unroll
       for (int n = 0; n < D / 2; ++n) sl[n] = S[n / 4][n % 4];
@@ -858,21 +894,21 @@ __device__ __forceinline__ bool efla_bwd_walk(
       S[n][x] = CUT && w.identity ? (row == col ? 1.f : 0.f) : (w.state0 ? w.state0[row * D + col] : 0.f);
     }
 
+  const EflaLoader<D> load(kb, ob, nb, cb, rs, ring, T);
   auto fetch = [&](int i) {                // i-th chunk from the end
     const int ch = c1 - 1 - i;
-    if (ch >= c0)
-      efla_stage_load<D, CUT>(ring + (i % EC_STAGES) * L::BYTES, kb + (long long)ch * EC * rs, !CUT || ob ? ob + (long long)ch * EC * rs : nullptr,
-                         nb + (long long)ch * EN_ELEMS, cb + (long long)ch * EC_COEF, rs, min(EC, T - ch * EC));
+    if (ch >= c0) load(i, ch);
     cp_async_commit();
   };
 #pragma unroll
   for (int i = 0; i < EC_STAGES - 1; ++i) fetch(i);
   for (int i = 0; i < c1 - c0; ++i) {
+    const int stage = i % EC_STAGES;
     cp_async_wait<EC_STAGES - 2>();
     __syncthreads();
     fetch(i + EC_STAGES - 1);
-    const uint32_t st = ring + (i % EC_STAGES) * L::BYTES;
-    const float* cf = reinterpret_cast<const float*>(smem + (i % EC_STAGES) * L::BYTES + L::C);
+    const uint32_t st = ring + stage * L::BYTES;
+    const float* cf = reinterpret_cast<const float*>(smem + stage * L::BYTES + L::C);
     if (!CUT || dckpt) {
       float4* dst = dckpt + efla_state_slot<D>((long long)bh * nchunks + c1 - 1 - i, wcol / 16, lane);
 #pragma unroll
@@ -900,7 +936,7 @@ __device__ __forceinline__ bool efla_bwd_walk(
       float sl[D / 2], unused[16];
 #pragma unroll
       for (int n = 0; n < D / 2; ++n) sl[n] = S[n / 4][n % 4];
-      const unsigned char* sst = smem + (i % EC_STAGES) * L::BYTES;
+      const unsigned char* sst = smem + stage * L::BYTES;
       efla_walk_back<D, L::KLD, L::VLD>(sl, unused, reinterpret_cast<const __nv_bfloat16*>(sst + L::K),
                                         reinterpret_cast<const __nv_bfloat16*>(sst + L::V) + warp * 16, cf,
                                         min(EC, T - (c1 - 1 - i) * EC));
@@ -967,7 +1003,7 @@ struct EflaBwdSmem {
   static constexpr int SCR_E = 3 * 16 * EN_LD * 2, SCR_S = 3 * 16 * LD * 2, RED_LD = D + 4;
   static constexpr int SCR = SCR_E + SCR_S > EC * RED_LD * 4 ? SCR_E + SCR_S : EC * RED_LD * 4;
   static constexpr int GLD = 36;
-  static constexpr int K = 0, V = K + TILE, O = V + TILE, N = O + TILE, C = N + 3 * EC * EN_LD * 2, G = C + EC_COEF * 4,
+  static constexpr int K = 0, V = K + TILE, O = V + TILE, N = O + TILE, C = N + EN_ELEMS * 2, G = C + EC_COEF * 4,
                        DA = G + EC * GLD * 4, SUM = DA + W * EC * GLD * 4, DC = SUM + W * 2 * EC * 4, SCRATCH = DC + W * EC * 4,
                        BYTES = SCRATCH + W * SCR;
 };
@@ -1024,7 +1060,7 @@ __device__ __forceinline__ bool efla_bwd_chunk(
     cp_async16(base + L::V + dst, v + src, r < n);
     cp_async16(base + L::O + dst, dout + src, r < n);
   }
-  for (int i = tid; i < 3 * EC * 4; i += 2 * D) cp_async16(base + L::N + ((i / 4) * EN_LD + (i % 4) * 8) * 2, nmat + id * EN_ELEMS + i * 8, true);
+  for (int i = tid; i < 3 * EC * 4; i += 2 * D) cp_async16(base + L::N + i * 16, nmat + id * EN_ELEMS + i * 8, true);
   if (tid < EC_COEF / 4) cp_async16(base + L::C + tid * 16, coef + id * EC_COEF + tid * 4, true);
   const float4* sp = ckpt + efla_state_slot<D>(id, warp, lane);
   const uint32_t scr_e = base + L::SCRATCH + warp * L::SCR, scr_s = scr_e + L::SCR_E;
