@@ -205,63 +205,58 @@ ELFA_API int elfa_cast(const void* src, int src_type, void* dst, int dst_type, l
 
 // ---- gated activation ---------------------------------------------------------------------------------
 // h [rows, 2 F] = [gate | up] -> a [rows, F] = silu(gate) * up, and its gradient in one pass each, straight from the projection's output:
-// no copies of the halves, no intermediate in bf16. Memory bound (3 F and 5 F bf16 per row); two vectors per operand in flight:
-// 4096 rows, F 8192: 45 and 65 us (4.5 and 5.2 TB/s), as separate copies, activation, product and their gradients about 370.
+// no copies of the halves, no intermediate in bf16. Memory bound (3 F and 5 F bf16 per row). One vector per operand and thread, 32 blocks per SM's worth of
+// grid: 4096 rows, F 8192 (L2 flushed, events included): 43 and 59 us; two vectors in flight and 8 blocks 47 and 68, one and 16 43 and 61.5, one and a block
+// for every 256 vectors 45 and 61, four 47 and 86. As separate copies, activation, product and their gradients about 370.
 namespace elfa {
 namespace {
 
-template <bool BWD>
+// Index: 32-bit where the vectors allow it (the row of a vector is a division).
+template <bool BWD, typename Index>
 __global__ void __launch_bounds__(256) swiglu_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ da,
-                                                     __nv_bfloat16* __restrict__ out, long long rows, int F) {
-  constexpr int U = 2;
-  const int per = F / 8;
-  const long long n = rows * per, stride = (long long)gridDim.x * blockDim.x;
-  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += U * stride) {
-    uint4 gq[U], uq[U], dq[U];
-    long long at[U];
+                                                     __nv_bfloat16* __restrict__ out, Index n, Index per) {
+  const Index stride = (Index)gridDim.x * blockDim.x;
+  for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const Index r = i / per, c = i - r * per;
+    const long long at = (long long)r * 2 * per + c;   // vector index in h: gate half; the other half is `per` further
+    const uint4 gq = reinterpret_cast<const uint4*>(h)[at], uq = reinterpret_cast<const uint4*>(h)[at + per];
+    const uint4 dq = BWD ? reinterpret_cast<const uint4*>(da)[i] : make_uint4(0, 0, 0, 0);
+    const uint32_t *pg = reinterpret_cast<const uint32_t*>(&gq), *pu = reinterpret_cast<const uint32_t*>(&uq),
+                   *pd = reinterpret_cast<const uint32_t*>(&dq);
+    uint4 o0, o1;
+    uint32_t *p0 = reinterpret_cast<uint32_t*>(&o0), *p1 = reinterpret_cast<uint32_t*>(&o1);
 #pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const long long i = i0 + k * stride, r = i / per, c = i - r * per;
-      at[k] = r * 2 * per + c;                       // vector index in h: gate half; the other half is `per` further
-      if (i < n) {
-        gq[k] = reinterpret_cast<const uint4*>(h)[at[k]];
-        uq[k] = reinterpret_cast<const uint4*>(h)[at[k] + per];
-        if (BWD) dq[k] = reinterpret_cast<const uint4*>(da)[i];
-      }
-    }
+    for (int j = 0; j < 4; ++j) {
+      float a[2], b[2];
 #pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const long long i = i0 + k * stride;
-      if (i >= n) continue;
-      const uint32_t *pg = reinterpret_cast<const uint32_t*>(&gq[k]), *pu = reinterpret_cast<const uint32_t*>(&uq[k]),
-                     *pd = reinterpret_cast<const uint32_t*>(&dq[k]);
-      uint4 o0, o1;
-      uint32_t *p0 = reinterpret_cast<uint32_t*>(&o0), *p1 = reinterpret_cast<uint32_t*>(&o1);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float a[2], b[2];
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const float g = x ? bf16_hi(pg[j]) : bf16_lo(pg[j]), u = x ? bf16_hi(pu[j]) : bf16_lo(pu[j]);
-          if (!BWD) {
-            a[x] = apply<OP_SILU>(g, 0.f, 1.f) * u;
-          } else {
-            const float d = x ? bf16_hi(pd[j]) : bf16_lo(pd[j]);
-            a[x] = apply<OP_SILU_BWD>(g, d * u, 1.f);
-            b[x] = d * apply<OP_SILU>(g, 0.f, 1.f);
-          }
+      for (int x = 0; x < 2; ++x) {
+        const float g = x ? bf16_hi(pg[j]) : bf16_lo(pg[j]), u = x ? bf16_hi(pu[j]) : bf16_lo(pu[j]);
+        if (!BWD) {
+          a[x] = apply<OP_SILU>(g, 0.f, 1.f) * u;
+        } else {
+          const float d = x ? bf16_hi(pd[j]) : bf16_lo(pd[j]);
+          a[x] = apply<OP_SILU_BWD>(g, d * u, 1.f);
+          b[x] = d * apply<OP_SILU>(g, 0.f, 1.f);
         }
-        p0[j] = pack_bf16(a[0], a[1]);
-        if (BWD) p1[j] = pack_bf16(b[0], b[1]);
       }
-      if (!BWD) {
-        reinterpret_cast<uint4*>(out)[i] = o0;
-      } else {
-        reinterpret_cast<uint4*>(out)[at[k]] = o0;
-        reinterpret_cast<uint4*>(out)[at[k] + per] = o1;
-      }
+      p0[j] = pack_bf16(a[0], a[1]);
+      if (BWD) p1[j] = pack_bf16(b[0], b[1]);
+    }
+    if (!BWD) {
+      reinterpret_cast<uint4*>(out)[i] = o0;
+    } else {
+      reinterpret_cast<uint4*>(out)[at] = o0;
+      reinterpret_cast<uint4*>(out)[at + per] = o1;
     }
   }
+}
+
+template <bool BWD>
+void launch_swiglu(const __nv_bfloat16* h, const __nv_bfloat16* da, __nv_bfloat16* out, long long rows, int F, int grid, cudaStream_t s) {
+  const long long n = rows * (F / 8);
+  // (the index after the last one stays below 2^32 too)
+  if (n < (1ll << 31)) swiglu_kernel<BWD, unsigned int><<<grid, 256, 0, s>>>(h, da, out, (unsigned int)n, (unsigned int)(F / 8));
+  else swiglu_kernel<BWD, long long><<<grid, 256, 0, s>>>(h, da, out, n, F / 8);
 }
 
 }  // namespace
@@ -276,9 +271,10 @@ ELFA_API int elfa_swiglu(const void* h, const void* da, void* out, long long row
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const auto *H = static_cast<const __nv_bfloat16*>(h), *D = static_cast<const __nv_bfloat16*>(da);
   auto* O = static_cast<__nv_bfloat16*>(out);
-  const int g = ew_grid(rows * F);
-  if (da) elfa::swiglu_kernel<true><<<g, 256, 0, s>>>(H, D, O, rows, F);
-  else elfa::swiglu_kernel<false><<<g, 256, 0, s>>>(H, D, O, rows, F);
+  const long long blocks = (rows * (F / 8) + 255) / 256;
+  const int g = (int)(blocks < 148 * 32 ? blocks : 148 * 32);
+  if (da) elfa::launch_swiglu<true>(H, D, O, rows, F, g, s);
+  else elfa::launch_swiglu<false>(H, D, O, rows, F, g, s);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;
