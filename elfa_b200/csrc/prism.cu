@@ -125,14 +125,14 @@ __device__ __forceinline__ typename PrismVec<VEC>::T prism_pack(const float (&f)
 template <int L, int VEC>
 __global__ void __launch_bounds__(256) prism_gated_fwd_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ v,
                                                               const __nv_bfloat16* __restrict__ z, long long ldz,
-                                                              __nv_bfloat16* __restrict__ y, long long tokens, int G, int d) {
+                                                              __nv_bfloat16* __restrict__ y, long long tokens, int G, int d, int parts) {
   using V = typename PrismVec<VEC>::T;
   constexpr int UG = 4;
-  const int per = d / VEC;
-  const long long n = tokens * per;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / per;
-    const int c = (int)(i - t * per) * VEC;
+  const int per = d / VEC, each = ((G + parts - 1) / parts + UG - 1) / UG * UG;           // groups of a thread
+  const long long n = tokens * per * parts;
+  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
+    const long long i = j % (tokens * per), t = i / per;
+    const int c = (int)(i - t * per) * VEC, from = (int)(j / (tokens * per)) * each, to = min(G, from + each);
     float p[L][VEC];
 #pragma unroll
     for (int l = 0; l < L; ++l) {
@@ -141,17 +141,17 @@ __global__ void __launch_bounds__(256) prism_gated_fwd_kernel(const __nv_bfloat1
       for (int x = 0; x < VEC; ++x) p[l][x] = prism_sigmoid(p[l][x]);
     }
     const long long base = t * (long long)G * d + c;
-    for (int g0 = 0; g0 < G; g0 += UG) {
+    for (int g0 = from; g0 < to; g0 += UG) {
       V uq[UG], vq[UG];
 #pragma unroll
       for (int k = 0; k < UG; ++k)
-        if (g0 + k < G) {
+        if (g0 + k < to) {
           uq[k] = *reinterpret_cast<const V*>(u + base + (long long)(g0 + k) * d);
           vq[k] = *reinterpret_cast<const V*>(v + base + (long long)(g0 + k) * d);
         }
 #pragma unroll
       for (int k = 0; k < UG; ++k)
-        if (g0 + k < G) {
+        if (g0 + k < to) {
           float uu[VEC], r[VEC];
           prism_unpack<VEC>(uu, uq[k]);
           prism_unpack<VEC>(r, vq[k]);
@@ -261,8 +261,16 @@ int launch_prism_gated(const void* u, const void* v, const void* z, long long ld
   if (dy)
     prism_gated_bwd_kernel<L, VEC><<<grid, 256, 0, s>>>(U, X, Z, ldz, static_cast<const __nv_bfloat16*>(dy), O,
                                                         static_cast<__nv_bfloat16*>(dv), static_cast<__nv_bfloat16*>(dz), tokens, G, d);
-  else
-    prism_gated_fwd_kernel<L, VEC><<<grid, 256, 0, s>>>(U, X, Z, ldz, O, tokens, G, d);
+  else {
+    // few tokens: the groups are spread over threads too, four each (the gates are formed again for every four). 128 tokens, 16 groups of 64, two iterations:
+    // one thread per token and vector for all groups 16 us (four blocks), spread 6; from two blocks per SM on the gates would cost more than it gains.
+    const int quads = (G + 3) / 4;
+    int parts = 1;
+    while (parts < quads && blocks * parts < 2 * 148) parts *= 2;
+    parts = parts < quads ? parts : quads;
+    const long long all = (tokens * (d / VEC) * parts + 255) / 256;
+    prism_gated_fwd_kernel<L, VEC><<<(int)(all < 148 * 16 ? all : 148 * 16), 256, 0, s>>>(U, X, Z, ldz, O, tokens, G, d, parts);
+  }
   ELFA_CUDA(cudaGetLastError());
   count_launches(1);
   return ELFA_OK;
@@ -318,25 +326,25 @@ __global__ void __launch_bounds__(256) prism_weight_sum_kernel(const float* __re
 //   k = z_k / |z_k|, b = sigmoid(mean z_b), delta_l as in the refinement
 //   l = 0: S <- forget S + b (delta - forget S k) k^T        l > 0: S <- S + b delta k^T
 // The rows of S never meet, so a quad of threads owns a row (D / 4 columns each, in registers for the whole block of tokens; the dot
-// product is two shuffles) and one CTA of 4 D threads owns a (batch, group). Keys, gates and deltas of PS_TT tokens at a time are
-// formed in parallel in shared memory first, so the serial part of a token is about D / 2 + L D / 4 multiply-adds per thread.
-// (B 2, 16 groups of 64, two iterations: 13 us per call on average over one block of 64 tokens and four single ones; the host loop issued
-// several launches per token and iteration: two such layers, 64 tokens and four steps, 33.6 ms with it and 5.3 with this.)
+// product is two shuffles) and one CTA of 4 D threads owns a (batch, group). Keys, gates and deltas of a tile of tokens are
+// formed in parallel in shared memory first, so the serial part of a token is about D / 2 + L D / 4 multiply-adds per thread. Tiles of up to 64 tokens,
+// four items of a warp or thread in flight: with tiles of eight, one item at a time and a division per iteration the preparation of a block of 64 tokens took
+// twice as long as its walk. (B 2, 16 groups of 64, two iterations, 64 tokens: 33 us, with tiles of eight 51.)
 template <int D>
 __global__ void __launch_bounds__(4 * D) prism_state_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ v,
                                                             const __nv_bfloat16* __restrict__ z, long long ldz, int off_b, int off_k,
                                                             const float* __restrict__ state, float* __restrict__ out, int T, int G, int L,
-                                                            float forget) {
+                                                            float forget, int tile) {
   extern __shared__ __align__(16) float ps_smem[];
-  const PrismTile<D> sm(ps_smem, PS_TT, L);
+  const PrismTile<D> sm(ps_smem, tile, L);
   const PrismSource in{u, v, z, ldz, off_b, off_k, T, G, L};
   const int bg = blockIdx.x, row = threadIdx.x >> 2, part = threadIdx.x & 3;
   float S[D / 4];
   prism_state_load<D>(S, state + ((long long)bg * D + row) * D, part);
-  for (int t0 = 0; t0 < T; t0 += PS_TT) {
-    const int n = min(PS_TT, T - t0);
-    __syncthreads();                            // the previous tokens have been consumed
-    prism_state_prepare<D, 4 * D>(in, sm, bg, t0, n, threadIdx.x, [] { __syncthreads(); });
+  for (int t0 = 0; t0 < T; t0 += tile) {
+    const int n = min(tile, T - t0);
+    if (t0) __syncthreads();                    // the previous tokens have been consumed
+    prism_state_prepare<D, 4 * D, 4>(in, sm, bg, t0, n, threadIdx.x, [] { __syncthreads(); });
     prism_state_rows<D>(S, sm, n, L, row, part, forget);
   }
   prism_state_store<D>(S, out + ((long long)bg * D + row) * D, part);
@@ -345,10 +353,12 @@ __global__ void __launch_bounds__(4 * D) prism_state_kernel(const __nv_bfloat16*
 template <int D>
 int launch_prism_state(const void* u, const void* v, const void* z, long long ldz, int off_b, int off_k, const float* state, float* out,
                        int B, int T, int G, int L, float forget, cudaStream_t s) {
-  const int bytes = (2 * PS_TT * L * D + PS_TT * L) * (int)sizeof(float);
+  // tokens of a tile: up to 64 (a multiple of four: the tile's parts start on 16 bytes) in half of an SM's shared memory
+  const int token = (2 * D + 1) * L * (int)sizeof(float), tile = T < 4 ? 4 : (T < 64 ? (T + 3) / 4 * 4 : 64), most = 110 * 1024 / token / 4 * 4;
+  const int tokens = tile < most ? tile : most, bytes = tokens * token;
   ELFA_CUDA(cudaFuncSetAttribute(prism_state_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   prism_state_kernel<D><<<B * G, 4 * D, bytes, s>>>(static_cast<const __nv_bfloat16*>(u), static_cast<const __nv_bfloat16*>(v),
-                                                    static_cast<const __nv_bfloat16*>(z), ldz, off_b, off_k, state, out, T, G, L, forget);
+                                                    static_cast<const __nv_bfloat16*>(z), ldz, off_b, off_k, state, out, T, G, L, forget, tokens);
   ELFA_CUDA(cudaGetLastError());
   count_launches(1);
   return ELFA_OK;

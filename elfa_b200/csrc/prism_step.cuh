@@ -17,8 +17,6 @@ __device__ __forceinline__ float prism_delta(float p, float res) {
   return a * prism_gelu_gate(a);
 }
 
-constexpr int PS_TT = 8;                        // tokens of a tile of the state's walk
-
 struct PrismSource {
   const __nv_bfloat16 *u, *v, *z;
   long long ldz;
@@ -46,39 +44,67 @@ __device__ __forceinline__ void prism_state_store(const float (&S)[D / 4], float
     for (int x = 0; x < 4; ++x) op[m * 16 + part * 4 + x] = S[4 * m + x];
 }
 
-// keys, gates and deltas of tokens t0 .. t0 + n - 1 of (batch, group) bg by NT threads (tid); ends with a barrier
-template <int D, int NT, typename Sync>
+// keys, gates and deltas of tokens t0 .. t0 + n - 1 of (batch, group) bg by NT threads (tid), U items of a warp or thread at a time so that their loads are
+// in flight together; ends with a barrier
+template <int D, int NT, int U, typename Sync>
 __device__ __forceinline__ void prism_state_prepare(const PrismSource& in, const PrismTile<D>& sm, int bg, int t0, int n, int tid, Sync together) {
-  const int b = bg / in.G, g = bg % in.G, warp = tid >> 5, lane = tid & 31, L = in.L;
-  const long long ldz = in.ldz;
+  const int b = bg / in.G, g = bg % in.G, warp = tid >> 5, lane = tid & 31, L = in.L, items = n * L;
+  const long long ldz = in.ldz, first = (long long)b * in.T + t0;
 #pragma unroll 1
-  for (int i = warp; i < n * L; i += NT / 32) {
-    const int tt = i / L, l = i % L;
-    const __nv_bfloat16* zr = in.z + ((long long)b * in.T + t0 + tt) * ldz + l * D;
-    float kx[D / 32], ss = 0.f, sum = 0.f;
+  for (int i0 = warp; i0 < items; i0 += NT / 32 * U) {
+    __nv_bfloat16 kz[U][D / 32], bz[U][D / 32];
 #pragma unroll
-    for (int m = 0; m < D / 32; ++m) {
-      kx[m] = __bfloat162float(zr[in.off_k + m * 32 + lane]);
-      ss += kx[m] * kx[m];
-      sum += __bfloat162float(zr[in.off_b + m * 32 + lane]);
+    for (int y = 0; y < U; ++y) {
+      const int i = min(i0 + y * (NT / 32), items - 1), tt = i / L;
+      const __nv_bfloat16* zr = in.z + (first + tt) * ldz + (i - tt * L) * D + lane;
+#pragma unroll
+      for (int m = 0; m < D / 32; ++m) {
+        kz[y][m] = zr[in.off_k + m * 32];
+        bz[y][m] = zr[in.off_b + m * 32];
+      }
     }
-    ss = sqrtf(warp_sum(ss));
-    sum = warp_sum(sum);
-    const float inv = ss < 1e-12f ? 1.f : 1.f / ss;
 #pragma unroll
-    for (int m = 0; m < D / 32; ++m) sm.k[i * D + m * 32 + lane] = kx[m] * inv;
-    if (lane == 0) sm.b[i] = prism_sigmoid(sum / (float)D);
+    for (int y = 0; y < U; ++y) {
+      const int i = i0 + y * (NT / 32);
+      if (i >= items) break;
+      float kx[D / 32], ss = 0.f, sum = 0.f;
+#pragma unroll
+      for (int m = 0; m < D / 32; ++m) {
+        kx[m] = __bfloat162float(kz[y][m]);
+        ss += kx[m] * kx[m];
+        sum += __bfloat162float(bz[y][m]);
+      }
+      ss = sqrtf(warp_sum(ss));
+      sum = warp_sum(sum);
+      const float inv = ss < 1e-12f ? 1.f : 1.f / ss;
+#pragma unroll
+      for (int m = 0; m < D / 32; ++m) sm.k[i * D + m * 32 + lane] = kx[m] * inv;
+      if (lane == 0) sm.b[i] = prism_sigmoid(sum / (float)D);
+    }
   }
 #pragma unroll 1
-  for (int i = NT - 1 - tid; i < n * D; i += NT) {          // beside the keys, from the last warp on
-    const int tt = i / D, c = i % D;
-    const long long r0 = (long long)b * in.T + t0 + tt, at = (r0 * in.G + g) * D + c;
-    float r = __bfloat162float(in.v[at]) - __bfloat162float(in.u[at]);
+  for (int i0 = NT - 1 - tid; i0 < n * D; i0 += NT * U) {   // beside the keys, from the last warp on
+    float r[U];
+    long long row[U];
+#pragma unroll
+    for (int y = 0; y < U; ++y) {
+      const int i = min(i0 + y * NT, n * D - 1), c = i % D;
+      row[y] = first + i / D;
+      const long long at = (row[y] * in.G + g) * D + c;
+      r[y] = __bfloat162float(in.v[at]) - __bfloat162float(in.u[at]);
+    }
 #pragma unroll 1
     for (int l = 0; l < L; ++l) {
-      const float delta = prism_delta(prism_sigmoid(__bfloat162float(in.z[r0 * ldz + l * D + c])), r);
-      r -= delta;
-      sm.d[(tt * L + l) * D + c] = delta;
+      __nv_bfloat16 z[U];
+#pragma unroll
+      for (int y = 0; y < U; ++y) z[y] = in.z[row[y] * ldz + l * D + (i0 + y * NT) % D];
+#pragma unroll
+      for (int y = 0; y < U; ++y) {
+        const float delta = prism_delta(prism_sigmoid(__bfloat162float(z[y])), r[y]);
+        r[y] -= delta;
+        const int i = i0 + y * NT;
+        if (i < n * D) sm.d[(i / D * L + l) * D + i % D] = delta;
+      }
     }
   }
   together();
@@ -87,27 +113,8 @@ __device__ __forceinline__ void prism_state_prepare(const PrismSource& in, const
 // one row of the state, a quad of threads, over the n tokens of a tile
 template <int D>
 __device__ __forceinline__ void prism_state_rows(float (&S)[D / 4], const PrismTile<D>& sm, int n, int L, int row, int part, float forget) {
-#pragma unroll 1
-  for (int i = 0; i < n * L; ++i) {
+  auto add = [&](int i, float coef) {
     const float4* kr = reinterpret_cast<const float4*>(sm.k + i * D);
-    float coef = sm.b[i] * sm.d[i * D + row];
-    if (i % L == 0) {
-      float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
-#pragma unroll
-      for (int m = 0; m < D / 16; ++m) {
-        const float4 kk = kr[m * 4 + part];
-        p0 += kk.x * S[4 * m];
-        p1 += kk.y * S[4 * m + 1];
-        p2 += kk.z * S[4 * m + 2];
-        p3 += kk.w * S[4 * m + 3];
-      }
-      float p = (p0 + p1) + (p2 + p3);
-      p += __shfl_xor_sync(0xffffffffu, p, 1);
-      p += __shfl_xor_sync(0xffffffffu, p, 2);
-      coef -= sm.b[i] * forget * p;
-#pragma unroll
-      for (int m = 0; m < D / 4; ++m) S[m] *= forget;
-    }
 #pragma unroll
     for (int m = 0; m < D / 16; ++m) {
       const float4 kk = kr[m * 4 + part];
@@ -116,6 +123,29 @@ __device__ __forceinline__ void prism_state_rows(float (&S)[D / 4], const PrismT
       S[4 * m + 2] += coef * kk.z;
       S[4 * m + 3] += coef * kk.w;
     }
+  };
+#pragma unroll 1
+  for (int t = 0, i = 0; t < n; ++t) {
+    const float4* kr = reinterpret_cast<const float4*>(sm.k + i * D);
+    float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+#pragma unroll
+    for (int m = 0; m < D / 16; ++m) {
+      const float4 kk = kr[m * 4 + part];
+      p0 += kk.x * S[4 * m];
+      p1 += kk.y * S[4 * m + 1];
+      p2 += kk.z * S[4 * m + 2];
+      p3 += kk.w * S[4 * m + 3];
+    }
+    float p = (p0 + p1) + (p2 + p3);
+    p += __shfl_xor_sync(0xffffffffu, p, 1);
+    p += __shfl_xor_sync(0xffffffffu, p, 2);
+    const float coef = sm.b[i] * sm.d[i * D + row] - sm.b[i] * forget * p;
+#pragma unroll
+    for (int m = 0; m < D / 4; ++m) S[m] *= forget;
+    add(i, coef);
+    ++i;
+#pragma unroll 1
+    for (int l = 1; l < L; ++l, ++i) add(i, sm.b[i] * sm.d[i * D + row]);
   }
 }
 

@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from elfa_b200 import native
+from elfa_b200.native import lib, stream_ptr
 from elfa_b200.ops import efla as eops, linear
 
 pytestmark = pytest.mark.gpu
@@ -106,3 +107,35 @@ def test_split_product_adds_up(cuda_device, M, N, K, pieces):
     want = a.double().t() @ b.double()
     assert native.status() == 0
     assert (parts.double().sum(0)[:M] - want).abs().max() <= 2 ** -20 * want.abs().max() * max(1, K / 256) ** 0.5
+
+
+@pytest.mark.parametrize("tokens,G,d,L", [(1, 16, 64, 2), (37, 5, 32, 1), (129, 3, 64, 8), (40, 1, 128, 3), (700, 16, 64, 2), (1200, 7, 8, 4)])
+def test_few_tokens_spread_their_groups(cuda_device, tokens, G, d, L):
+    """A call of few tokens spreads the groups over threads: the bits of the same rows inside a call that does not."""
+    g = torch.Generator(device=cuda_device).manual_seed(tokens)
+    rows = 148 * 2 * 256 // (d // 8) + tokens + 8                     # two blocks per SM without spreading
+    u, v, z = (torch.randn(rows, n, generator=g, device=cuda_device).bfloat16() for n in (G * d, G * d, L * d))
+    whole, few = torch.empty_like(u), torch.full_like(u[:tokens + 1], 7.0)
+    for y, n in ((whole, rows), (few, tokens)):
+        lib.call("elfa_prism_gated_fwd", u, v, z, z.stride(0), y, n, G, d, L, stream_ptr(u))
+    assert native.status() == 0 and torch.equal(few[:tokens], whole[:tokens]) and (few[tokens:] == 7).all()
+
+
+@pytest.mark.parametrize("d,L", [(32, 1), (64, 2), (96, 3), (128, 8)])          # the last one: tiles of twelve tokens
+@pytest.mark.parametrize("T", [1, 5, 64, 65, 131])
+def test_the_state_does_not_depend_on_the_tiles(cuda_device, d, L, T):
+    """Tiles of up to 64 tokens; one call and calls of a few tokens each leave the same state."""
+    B, G = 2, 3
+    g = torch.Generator(device=cuda_device).manual_seed(T + d)
+    u, v, z = (torch.randn(B, T, n, generator=g, device=cuda_device).bfloat16() for n in (G * d, G * d, 3 * L * d))
+    s0 = torch.randn(B, G, d, d, generator=g, device=cuda_device)
+
+    def state(lo, hi, s):
+        a, b, c = (x[:, lo:hi].contiguous() for x in (u, v, z))
+        out = torch.empty_like(s)
+        lib.call("elfa_prism_state", a, b, c, 3 * L * d, L * d, 2 * L * d, s, out, B, hi - lo, G, d, L, 0.9, stream_ptr(a))
+        return out
+    cut = s0
+    for lo in range(0, T, 7):
+        cut = state(lo, min(T, lo + 7), cut)
+    assert native.status() == 0 and torch.equal(state(0, T, s0), cut) and torch.isfinite(cut).all()
