@@ -1155,7 +1155,11 @@ ELFA_API int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
   const int pairs = sm_count() / 2;
   const bool pair = force_bn == 512 ||
                     (force_bn == 0 && N >= 256 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= pairs && (max_ctas <= 0 || max_ctas >= sm_count()));
-  const int BN = pair ? 256 : pick_bn(M, N, force_bn);
+  int BN = pair ? 256 : pick_bn(M, N, force_bn);
+  // A product that makes no more than one wave of 64-wide tiles takes those: its time is that of one CTA's walk over the contraction, and a block of
+  // such a tile brings 24 KB for 32 (M 128, B [K, N]: N 1024, K 1024 9.3 -> 8.2 us, N 1024, K 4096 21.5 -> 20.2, N 4096, K 1024 10.8 -> 9.3; past one wave, M 260, N 4096,
+  // 16.4 -> 18.5 with the timing's events). The sums keep their order. (fp32 outputs, whose contraction is split by the number of tiles, keep theirs.)
+  if (BN == 128 && force_bn == 0 && !(flags & ELFA_EPI_OUT_F32) && (long long)((M + BM - 1) / BM) * ((N + 63) / 64) <= sm_count()) BN = 64;
   CUtensorMap tmA, tmB;
   int rc;
   if (!a_mn_major) rc = cached_tmap_bf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, BK);

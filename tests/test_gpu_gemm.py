@@ -156,3 +156,15 @@ def test_gemm_cta_pair_epilogues_and_persistence(cuda_device):
     _close(pre, base, K)
     _close(out, ops.gelu_tanh_ref(base), K)
     assert native.status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 72, 264), (128, 4096, 72), (129, 4736, 64), (520, 1024, 200), (1160, 1096, 1032), (2368, 512, 136)])
+@pytest.mark.parametrize("b_mn", [True, False])
+def test_one_wave_of_narrow_tiles_has_the_bits_of_the_wide_ones(cuda_device, M, N, K, b_mn):
+    """Products around one wave of 64-wide tiles: which width is taken changes no sum."""
+    g = torch.Generator(device=cuda_device).manual_seed(M + N)
+    a = torch.randn(M, K, generator=g, device=cuda_device).bfloat16()
+    b = torch.randn(*((K, N) if b_mn else (N, K)), generator=g, device=cuda_device).bfloat16()
+    y = ops.gemm(a, b, b_mn=b_mn, gelu=True)
+    assert native.status() == 0
+    assert torch.equal(y, ops.gemm(a, b, b_mn=b_mn, gelu=True, force_bn=64)) and torch.equal(y, ops.gemm(a, b, b_mn=b_mn, gelu=True, force_bn=128))
