@@ -18,8 +18,8 @@
 // ones, and V and dO their own columns only (for dV; a row of dK adds up all columns). Inside a chunk the products of the chunked form
 // would carry 0 x NaN to the other tokens, so every kernel asks at its end whether a state or a key gradient came out not finite and, if so,
 // runs once more in a checked form that walks the chunks concerned token by token (efla_walk) and overwrites its results. On finite data
-// that costs one barrier. (Asked for inside the walk over the chunks it stood in the chain of dependent products: forward 105 us against 94
-// now, state gradient 98 against 92 at B 8, T 2048, 16 heads of 64.) Gradients of such tokens are not finite; whether infinity or NaN is not kept.
+// that costs one barrier. (Asked for inside the walk over the chunks it stood in the chain of dependent products: forward 105 us against 94,
+// state gradient 98 against 92 at B 8, T 2048, 16 heads of 64, when it was moved.) Gradients of such tokens are not finite; whether infinity or NaN is not kept.
 //
 // reference: kernels/cuda/efla.cu:121-271,534-552 (chunks are scanned one after the other, the bf16 state in global memory).
 #include <algorithm>
@@ -509,8 +509,8 @@ struct EflaWalk {
 
 // k, v, o: [B, T, H, d] bf16; v and o may be null (see EflaWalk). ckpt (or null): the state at the start of every chunk.
 // Bound by the dependent chain of a chunk (132 mma.sync and about 880 instructions of one warp per scheduler), not by memory. With the
-// preparation, B 1, T 8192, 16 heads of 64, no gradient: 354 us in one walk, token by token (with its checkpoints) 2364 us; in the training step
-// of B 8, T 2048 the forward went from about 750 to 94 us and 28 us for the preparation.
+// preparation, B 1, T 8192, 16 heads of 64, no gradient: 342 us in one walk, token by token (with its checkpoints) 2364 us; in the training step
+// of B 8, T 2048 the forward went from about 750 to 85 us and 28 us for the preparation.
 template <int D, bool CHECKED, bool CUT>
 __device__ __forceinline__ bool efla_fwd_walk(
     const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v, const __nv_bfloat16* __restrict__ nmat,
@@ -862,7 +862,7 @@ int launch_chunk_fwd(const void* k, const void* v, const float* beta, const floa
 //   dlam_t = c_t sum_j (dO E)_tj + dc_t dc/dlam,   dbeta = sum_t dc_t ex_t
 // Only dS is sequential: efla_chunk_bwd_state_kernel walks the chunks backwards with dS in registers and writes the dS1 of every chunk;
 // efla_chunk_bwd_kernel then handles all chunks in parallel from the two chunk-boundary states.
-// B 8, T 2048, 16 heads of 64: 91 us and 255 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
+// B 8, T 2048, 16 heads of 64: 76 us and 257 us (token by token, the states of a chunk through a global workspace: 2352 us and 130 us more to
 // finish). The parallel kernel issues about 400 mma.sync per warp and chunk (94 us of tensor time at 8.3 cycles each) and reads 370 MB
 // (55 us); it is bound by the chain of its two warps per scheduler (five cycles per instruction of a warp, a third of the issue slots). A third CTA
 // per SM, at 168 registers, did not make it faster; nor did a tenth fewer instructions (packed remainders of the splits, first products without zeroed
@@ -1454,11 +1454,10 @@ using namespace elfa;
 // How many segments a walk over T tokens is cut into (1: none), and with them how large `work` is: 3 * segments * B * H * d * d floats.
 // One walk takes nchunks steps; cut, FIRST takes nchunks / P steps of (2 P - 3) walks per head and column block and REST as many of P - 1. Measured
 // per head dimension: a step with one CTA per SM, with as many as its registers and shared memory hold (whole rounds beyond), and the
-// two launches and joints more. B 1 x 8192, 16 heads of 64: P 1 355 us, 6 150, 8 146, 10 128, 12 160 (a second round); B 2 x 1531, 8 heads of 128: P 1
-// 109, 4 98, 5 93, 6 101; B 4 x 1024, 8 heads of 128: P 1 78, 3 88 (not cut); B 8 x 2048, 16 heads of 64: P 1 118, 3 165 (not cut).
-// The walk of the state gradient is cut alike: on eleven shapes its best number is the forward walk's, or within 3 % of it (kernels alone, forward /
-// state gradient, us: B 1 x 8192, 16 heads of 64, P 1 337 / 358, 8 126 / 127, 10 109 / 109, 12 140 / 134; B 2 x 1531, 8 heads of 128, P 1 100 / 111, 4 86 / 91,
-// 5 82 / 83, 6 89 / 92; B 4 x 1024, 8 heads of 128, P 1 69 / 75, 3 78 / 81; B 1 x 4096, 16 heads of 32, P 1 161 / 138, 10 42 / 45, 16 39 / 41).
+// two launches and joints more. Kernels and joints, forward / state gradient, us: B 1 x 8192, 16 heads of 64, P 1 328 / 292, 6 122 / 117, 8 117 / 114,
+// 10 100 / 97, 12 128 / 122 (a second round); B 2 x 1531, 8 heads of 128, P 1 106 / 95, 4 82 / 80, 5 74 / 69, 6 79 / 78; B 1 x 4096, 16 heads of 32, P 1
+// 110 / 117, 10 33 / 31, 16 33 / 32; not cut: B 4 x 1024, 8 heads of 128, 72 / 65; B 8 x 2048, 16 heads of 64, 86 / 78. Both walks are cut alike: on
+// eleven shapes the rule's number is the best for both, or within 5 % of it.
 // A cut costs the host two launches and an allocation per walk (6 to 8 us), which only a walk longer than the host's part of the call pays for: about 30 us
 // without a gradient, 70 with one, where the rest of the pass runs meanwhile (B 1 x 500, 8 heads of 32, training, cut whatever its length: 159 -> 208 us).
 static int efla_segments(int B, int T, int H, int d, double least) {
