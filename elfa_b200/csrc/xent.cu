@@ -27,12 +27,16 @@ __device__ __forceinline__ void online_combine(float& m, float& s, float m2, flo
   m = nm;
 }
 
-// the same with base-2 maxima
-__device__ __forceinline__ void online_combine2(float& m, float& s, float m2, float s2) {
-  const float nm = fmaxf(m, m2);
-  if (nm == -INFINITY) return;
-  s = s * fast_exp2(m - nm) + s2 * fast_exp2(m2 - nm);
-  m = nm;
+// Sums relative to the (base 2) maxima of 2 FROM lanes, joined: the maximum first, so each lane takes one exponential and not two per step.
+template <int FROM>
+__device__ __forceinline__ void join_sums2(float& m, float& s) {
+  float top = m;
+#pragma unroll
+  for (int o = FROM; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  s *= fast_exp2(m - (top == -INFINITY ? 0.f : top));        // nothing but empty sums: zero, as they are
+#pragma unroll
+  for (int o = FROM; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  m = top;
 }
 
 struct StatPeers {      // vocabulary-parallel exchange: every rank's [slices][rows] statistics table (peer-addressable)
@@ -155,8 +159,8 @@ __global__ void __launch_bounds__(XENT_THREADS) xent_grad_kernel(__nv_bfloat16* 
 // Loss and gradient of whole rows in one pass: the row waits in shared memory between the statistics and the gradient (every thread
 // copies in and reads back its own 16-byte vectors, so the copies need no barrier), and the logits are read from memory once and written
 // once - the two-kernel form reads them twice. At V = 32000 a row takes 64 KB: three rows per SM, one loading while the others
-// compute; more than 32768 columns would leave two. 8192 x 32000: 212 us (1.05 GB, 5.0 TB/s; the exponentials alone take 116), as two
-// kernels about 300.
+// compute; more than 32768 columns would leave two. 8192 x 32000: 181 us (1.05 GB, 5.8 TB/s; the exponentials alone take 116), with two
+// exponentials per step of the joints (40 per thread beside its 125) 203, as two kernels about 300. 8192 x 8192: 88 and 109 us.
 constexpr int XENT_ROW_MAX = 8 * 8 * XENT_THREADS;
 
 // The row of xent_row_kernel when its maximum leaves base 2 (|x| log2(e) past the largest float: rows of the type's lowest value, for one; or
@@ -231,16 +235,18 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
       for (int j = 0; j < 4; ++j) sx += bf16_lo(p[j]) + bf16_hi(p[j]);
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    online_combine2(m2, s, __shfl_xor_sync(0xffffffffu, m2, o), __shfl_xor_sync(0xffffffffu, s, o));
-    sx += __shfl_xor_sync(0xffffffffu, sx, o);
-  }
+  join_sums2<16>(m2, s);
+  if (smoothing != 0.f) sx = warp_sum(sx);
   if (lane == 0) { sm[0][wid] = m2; sm[1][wid] = s; sm[2][wid] = sx; }
   __syncthreads();
-  float M2 = sm[0][0], S = sm[1][0], SX = sm[2][0];
+  // every warp joins the warps' sums for itself, a lane (two, with the same) per sum
+  static_assert(XENT_THREADS == 512);
+  float M2 = sm[0][lane & 15], S = sm[1][lane & 15], SX = 0.f;
+  join_sums2<8>(M2, S);
+  if (smoothing != 0.f) {
 #pragma unroll
-  for (int i = 1; i < XENT_THREADS / 32; ++i) { online_combine2(M2, S, sm[0][i], sm[1][i]); SX += sm[2][i]; }
+    for (int i = 0; i < XENT_THREADS / 32; ++i) SX += sm[2][i];
+  }
   const float ls = log2f(S), lse2 = M2 + ls;
   const bool valid = t >= 0 && t < V;
   if (threadIdx.x == 0 && !valid && t != -100) atomicOr(status, (unsigned)ELFA_ST_BAD_TARGET);
