@@ -160,23 +160,24 @@ __global__ void __launch_bounds__(XENT_THREADS) xent_grad_kernel(__nv_bfloat16* 
 // copies in and reads back its own 16-byte vectors, so the copies need no barrier), and the logits are read from memory once and written
 // once - the two-kernel form reads them twice. At V = 32000 a row takes 64 KB: three rows per SM, one loading while the others
 // compute; more than 32768 columns would leave two. 8192 x 32000: 181 us (1.05 GB, 5.8 TB/s; the exponentials alone take 116), with two
-// exponentials per step of the joints (40 per thread beside its 125) 203, as two kernels about 300. 8192 x 8192: 88 and 109 us.
+// exponentials per step of the joints (40 per thread beside its 125) 203, as two kernels about 300.
 constexpr int XENT_ROW_MAX = 8 * 8 * XENT_THREADS;
 
 // The row of xent_row_kernel when its maximum leaves base 2 (|x| log2(e) past the largest float: rows of the type's lowest value, for one; or
 // infinite logits): in natural units, everything relative to the maximum.
+template <int NT>
 __device__ __noinline__ void xent_row_huge(__nv_bfloat16* x, const uint4* xrow, int nvec, int V, bool valid, float tl, int tv, int tj,
-                                           float smoothing, float grad_scale, float* loss, float (*red)[XENT_THREADS / 32]) {
+                                           float smoothing, float grad_scale, float* loss, float (*red)[NT / 32]) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float m = -INFINITY;
-  for (int i = threadIdx.x; i < nvec * 8; i += XENT_THREADS) m = fmaxf(m, __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xrow)[i]));
+  for (int i = threadIdx.x; i < nvec * 8; i += NT) m = fmaxf(m, __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xrow)[i]));
   m = warp_max(m);
   __syncthreads();
   if (lane == 0) red[0][wid] = m;
   __syncthreads();
-  for (int i = 0; i < XENT_THREADS / 32; ++i) m = fmaxf(m, red[0][i]);
+  for (int i = 0; i < NT / 32; ++i) m = fmaxf(m, red[0][i]);
   float s = 0.f, sx = 0.f;
-  for (int i = threadIdx.x; i < nvec * 8; i += XENT_THREADS) {
+  for (int i = threadIdx.x; i < nvec * 8; i += NT) {
     const float f = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xrow)[i]) - m;
     s += expf(f);
     sx += f / (float)V;                    // the plain sum would overflow
@@ -186,27 +187,28 @@ __device__ __noinline__ void xent_row_huge(__nv_bfloat16* x, const uint4* xrow, 
   if (lane == 0) { red[1][wid] = s; red[2][wid] = sx; }
   __syncthreads();
   s = sx = 0.f;
-  for (int i = 0; i < XENT_THREADS / 32; ++i) { s += red[1][i]; sx += red[2][i]; }
+  for (int i = 0; i < NT / 32; ++i) { s += red[1][i]; sx += red[2][i]; }
   if (threadIdx.x == 0) {
     float l = (1.f - smoothing) * (tl - m - logf(s));
     if (smoothing != 0.f) l += smoothing * (sx - logf(s));
     *loss = valid ? -l : 0.f;
   }
   const float gs = valid ? grad_scale : 0.f, off = -gs * (smoothing / (float)V), tg = gs * (1.f - smoothing);
-  for (int i = threadIdx.x; i < nvec * 8; i += XENT_THREADS) {
+  for (int i = threadIdx.x; i < nvec * 8; i += NT) {
     const float f = expf(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(xrow)[i]) - m) / s * gs + off;
     x[i] = __float2bfloat16(f - (valid && i == tv * 8 + tj ? tg : 0.f));
   }
 }
 
-__global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16* __restrict__ logits, long long ld,
+template <int NT>
+__global__ void __launch_bounds__(NT, NT < 64 ? 32 : 3 * XENT_THREADS / NT) xent_row_kernel(__nv_bfloat16* __restrict__ logits, long long ld,
                                                                    const long long* __restrict__ targets, float* __restrict__ loss_out, int V,
                                                                    float smoothing, float grad_scale, unsigned int* status) {
   extern __shared__ __align__(16) uint4 xrow[];
-  __shared__ float sm[3][XENT_THREADS / 32];
+  __shared__ float sm[3][NT / 32];
   const int row = blockIdx.x, nvec = V / 8, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __nv_bfloat16* x = logits + (long long)row * ld;
-  for (int v = threadIdx.x; v < nvec; v += XENT_THREADS) cp_async16(smem_u32(xrow + v), x + v * 8, true);
+  for (int v = threadIdx.x; v < nvec; v += NT) cp_async16(smem_u32(xrow + v), x + v * 8, true);
   cp_async_commit();
   const long long t = targets[row];
   const float tl = t >= 0 && t < V ? __bfloat162float(x[t]) : 0.f;                 // read before any thread overwrites the row
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
   constexpr float L2E = 1.4426950408889634f;
   __nv_bfloat162 mp = __halves2bfloat162(__ushort_as_bfloat16(0xff80), __ushort_as_bfloat16(0xff80));     // -inf
 #pragma unroll 2
-  for (int v = threadIdx.x; v < nvec; v += XENT_THREADS) {
+  for (int v = threadIdx.x; v < nvec; v += NT) {
     const uint4 q = xrow[v];
     const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q);
     mp = __hmax2(mp, __hmax2(__hmax2(p[0], p[1]), __hmax2(p[2], p[3])));
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
   float m2 = fmaxf(__low2float(mp), __high2float(mp)) * L2E, s = 0.f, sx = 0.f;
   const float nm2 = m2 == -INFINITY ? 0.f : -m2;
 #pragma unroll 2
-  for (int v = threadIdx.x; v < nvec; v += XENT_THREADS) {
+  for (int v = threadIdx.x; v < nvec; v += NT) {
     const uint4 q = xrow[v];
     const uint32_t* p = reinterpret_cast<const uint32_t*>(&q);
     float e[4];
@@ -239,22 +241,22 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
   if (smoothing != 0.f) sx = warp_sum(sx);
   if (lane == 0) { sm[0][wid] = m2; sm[1][wid] = s; sm[2][wid] = sx; }
   __syncthreads();
-  // every warp joins the warps' sums for itself, a lane (two, with the same) per sum
-  static_assert(XENT_THREADS == 512);
-  float M2 = sm[0][lane & 15], S = sm[1][lane & 15], SX = 0.f;
-  join_sums2<8>(M2, S);
+  // every warp joins the warps' sums for itself, a lane (or several, with the same) per sum
+  constexpr int NW = NT / 32;
+  float M2 = sm[0][lane & (NW - 1)], S = sm[1][lane & (NW - 1)], SX = 0.f;
+  join_sums2<NW / 2>(M2, S);
   if (smoothing != 0.f) {
 #pragma unroll
-    for (int i = 0; i < XENT_THREADS / 32; ++i) SX += sm[2][i];
+    for (int i = 0; i < NT / 32; ++i) SX += sm[2][i];
   }
   const float ls = log2f(S), lse2 = M2 + ls;
   const bool valid = t >= 0 && t < V;
   if (threadIdx.x == 0 && !valid && t != -100) atomicOr(status, (unsigned)ELFA_ST_BAD_TARGET);
   if (fabsf(M2) == INFINITY) {             // (a thread whose own maximum overflows downwards rightly adds nothing to a larger one)
-    xent_row_huge(x, xrow, nvec, V, valid, tl, valid ? (int)(t >> 3) : -1, (int)(t & 7), smoothing, grad_scale, loss_out + row, sm);
+    xent_row_huge<NT>(x, xrow, nvec, V, valid, tl, valid ? (int)(t >> 3) : -1, (int)(t & 7), smoothing, grad_scale, loss_out + row, sm);
     return;
   }
-  if (threadIdx.x == XENT_THREADS - 1) {     // the thread with the fewest vectors
+  if (threadIdx.x == NT - 1) {     // the thread with the fewest vectors
     // the loss in natural units, from the maximum as it is: M2 carries the rounding of M log2(e), and a result in base 2 would be rounded at
     // 1.44 times its size (up to 1.5 times the error against 64 bits). M is a bf16 number, so M2 ln(2) rounds to it.
     constexpr float LN2 = 0.6931471805599453f;
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
   const float gs = valid ? grad_scale : 0.f, off = -gs * (smoothing / (float)V), tg = gs * (1.f - smoothing);
   const int tv = valid ? (int)(t >> 3) : -1, tj = (int)(t & 7);
 #pragma unroll 2
-  for (int v = threadIdx.x; v < nvec; v += XENT_THREADS) {
+  for (int v = threadIdx.x; v < nvec; v += NT) {
     const uint4 q = xrow[v];
     const uint32_t* p = reinterpret_cast<const uint32_t*>(&q);
     float f[8];
@@ -282,6 +284,16 @@ __global__ void __launch_bounds__(XENT_THREADS, 3) xent_row_kernel(__nv_bfloat16
     }
     reinterpret_cast<uint4*>(x)[v] = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
   }
+}
+
+template <int NT>
+int launch_xent_row(void* logits, long long ld, const long long* targets, float* loss_out, int rows, int V, float smoothing, float grad_scale,
+                    unsigned int* st, cudaStream_t s) {
+  ELFA_CUDA(cudaFuncSetAttribute(xent_row_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, XENT_ROW_MAX * 2));
+  xent_row_kernel<NT><<<rows, NT, V * 2, s>>>(static_cast<__nv_bfloat16*>(logits), ld, targets, loss_out, V, smoothing, grad_scale, st);
+  ELFA_CUDA(cudaGetLastError());
+  ::elfa::count_launches(1);
+  return ELFA_OK;
 }
 
 }  // namespace
@@ -347,6 +359,10 @@ ELFA_API int elfa_xent_row_max(void) { return XENT_ROW_MAX; }
 
 // Both passes in one for whole rows (no vocabulary split): the logits become d loss / d logits * grad_scale in place, loss_out gets the
 // per-token loss. V a multiple of 8 and at most elfa_xent_row_max(), rows on 16-byte boundaries.
+// Threads per row: what a thread does once (the joints, the logarithm, two barriers) should be little beside its share of the row, and rows in different phases
+// should share an SM. 16384 rows, us, 32 / 64 / 128 / 256 / 512 threads: V 256 17 / 20 / 27 / 45 / 89; 1000 27 / 29 / 35 / 51 / 94; 2048 36 / 34 / 45 / 61 /
+// 101; 4096 55 / 51 / 60 / 78 / 123; 8000 119 / 94 / 95 / 108 / 160; 12000 198 / 143 / 135 / 136 / 183; 16384 305 / 216 / 192 / 167 / 218. 4096 rows: 8192
+// 42 / 34 / 34 / 35 / 47; 24000 160 / 114 / 90 / 74 / 80; 32000 266 / 162 / 125 / 98 / 94. 64 and 300 rows: the numbers taken are the best there, or within 1 us.
 ELFA_API int elfa_xent_row(void* logits, long long ld, const long long* targets, float* loss_out, int rows, int V, float smoothing,
                            float grad_scale, void* stream) {
   ELFA_REQUIRE(logits && targets && loss_out && rows > 0 && V > 0, "xent_row: bad arguments");
@@ -354,10 +370,10 @@ ELFA_API int elfa_xent_row(void* logits, long long ld, const long long* targets,
                "xent_row: V must be a multiple of 8 and at most 32768, rows 16-byte aligned");
   unsigned int* st = status_word();
   ELFA_REQUIRE(st != nullptr, "xent: no status word");
-  ELFA_CUDA(cudaFuncSetAttribute(xent_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XENT_ROW_MAX * 2));
-  xent_row_kernel<<<rows, XENT_THREADS, V * 2, static_cast<cudaStream_t>(stream)>>>(static_cast<__nv_bfloat16*>(logits), ld, targets, loss_out,
-                                                                                  V, smoothing, grad_scale, st);
-  ELFA_CUDA(cudaGetLastError());
-  ::elfa::count_launches(1);
-  return ELFA_OK;
+  auto* s = static_cast<cudaStream_t>(stream);
+  if (V <= 1024) return launch_xent_row<32>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
+  if (V <= 4096) return launch_xent_row<64>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
+  if (V <= 8192) return launch_xent_row<128>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
+  if (V <= 24576) return launch_xent_row<256>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
+  return launch_xent_row<512>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
 }

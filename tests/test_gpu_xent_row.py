@@ -79,3 +79,10 @@ def test_loss_is_as_close_to_64_bits_as_in_two_kernels(cuda_device, V, scale):
     ref = torch.cat([torch.nn.functional.cross_entropy(x[i:i + 256].double(), t[i:i + 256], reduction="none") for i in range(0, rows, 256)])
     err = [(e.double() - ref).norm().item() for e in (one, two)]
     assert err[0] <= 1.02 * err[1]                     # the same roundings in another order: 2 % for the sample
+
+
+@pytest.mark.parametrize("V", [1024, 1032, 8192, 8200, 24576, 24584])
+def test_edges_of_the_thread_counts(cuda_device, V):
+    """Rows of 32, 64, 128, 256 and 512 threads, at the widths where the number changes."""
+    test_cross_entropy_widths(cuda_device, V, 0.1)
+    test_logits_near_the_largest_float(cuda_device, V, 0.0)
