@@ -9,8 +9,9 @@
 // src/model/efla.zig:27-49,275-329).
 //
 // ShortConv: y[b,t,c] = bias[c] + sum_w x[b,t-w,c] weight[c,w] (reference:
-// kernels/cuda/convolution.cu:4-57,126-189; src/model/prism.zig:948-973). The weight gradient is one
-// pass over the rows per (32 channels, 4 taps) without atomics.
+// kernels/cuda/convolution.cu:4-57,126-189; src/model/prism.zig:948-973). The weight gradient is
+// summed in slices of the rows, which are added up in order (no atomics).
+#include <algorithm>
 #include <type_traits>
 
 #include "efla_step.cuh"
@@ -32,11 +33,11 @@ __global__ void __launch_bounds__(32 * EFLA_W) efla_scan_fwd_kernel(const __nv_b
 // the last W inputs and the W weights in registers (the loop is unrolled W steps, so the window is a ring with fixed register names);
 // every input element is loaded once per span plus the W - 1 steps of the seam, the next W rows are in flight while the current
 // ones are summed, and the sums run on packed fp32 pairs. Other windows (larger rings do not fit the registers) take
-// shortconv_apply_kernel / shortconv_bwd_dw_kernel below.
+// shortconv_tile_kernel / shortconv_dw_kernel below.
 // Backward is one walk from late to early: with dy[t .. t + W - 1] as the window, dx[t] = sum_j w[j] dy[t + j] and
 // dw[j] += x[t] dy[t + j]; every warp writes its dw / db sums as one slice of part [slices][W + 1][C], added up in order afterwards.
 // B 8, T 2048, C 1024, W 16: 27 us forward (67 MB; bound by the packed multiply-adds and the latency of 202- and 126-register warps), 45 + 6 us
-// backward; the layer that contains them went from 789 to 454 us when they replaced the general kernels below.
+// backward; the layer that contains them went from 789 to 454 us when they replaced kernels that took a tap at a time.
 // A lane's weights are 4 W consecutive bytes; one at a time they would cost 2 W loads that touch 32 lines each, more than the
 // inputs (31.5 against 26.5 us forward).
 template <int W>
@@ -256,94 +257,237 @@ __global__ void __launch_bounds__(64) shortconv_stream_kernel(const __nv_bfloat1
   }, w, bias, xin + (long long)b * (tails + T) * C + c, u + ((long long)b * T + t) * C + c, tails, t, c, C, W);
 }
 
-// Forward and input gradient share one kernel (DX = false: y[t] = bias + sum_j x[t - j] w[j]; DX = true:
-// dx[t] = sum_j dy[t + j] w[j]). A lane owns a PAIR of adjacent channels (4-byte loads, 128 bytes per warp); the
-// CTA's 64 channels x W weights sit transposed in shared memory (the [C, W] layout read directly would touch a
-// different cache line in every lane); a warp walks SC_ROWS / 8 consecutive time steps, so the W - 1 re-reads of an
-// input element come from L1. grid (ceil(B T / SC_ROWS), ceil(C / 64)), block (32, 8), dynamic smem W * 64 floats.
-constexpr int SC_ROWS = 64;
+// ---- any other window of up to 128 taps, 16 taps and 16 time steps at a time, a channel pair per lane: the 31 inputs that such a block meets wait in
+// registers (a ring of 32 slots, unrolled twice, so that their names are fixed), the 16 that the next one adds are under way meanwhile, and 256 packed
+// multiply-adds work on 16 independent sums.
+// B 8, T 2048, C 1024, W 64 (1.07 G multiply-adds each: 30 us at the chip's fp32 rate): output 72 us, input gradient 69,
+// weight gradient 77 + 10 for the joint; one tap of one position at a time they took 268, 270 and 1047. The multiply-adds are 45 % of the instructions (the
+// others load, unpack and go round), half of the issue slots are taken. W 32 139 for 865 us in all, W 5 81 for 402, W 128 402 for 2927; 2 x 1655 x 256,
+// W 64: 29 for 96. Loads with a test and a 64-bit multiplication each, and weights stored 32 lanes to a bank, cost half as much again (342 us at W 64).
+constexpr int SC_TILE = 16;
+constexpr int SC_WARPS = 8;
+constexpr int SC_WLD = 66;                               // floats of a tap's 64 weights: channel by channel stores meet two to a bank
 
-template <bool DX>
-__global__ void __launch_bounds__(256) shortconv_apply_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w,
-                                                              const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out,
-                                                              int B, int T, int C, int W) {
-  extern __shared__ float sw[];                          // [W][64]
-  const int lane = threadIdx.x, warp = threadIdx.y;
-  const int c0 = blockIdx.y * 64;
-  for (int i = warp * 32 + lane; i < W * 64; i += 256) {
-    const int cl = i / W, j = i % W;                     // consecutive threads read consecutive weights of a channel
-    sw[j * 64 + cl] = c0 + cl < C ? __bfloat162float(w[(long long)(c0 + cl) * W + j]) : 0.f;
-  }
-  __syncthreads();
-  const int c = c0 + 2 * lane;
-  if (c >= C) return;
-  const long long rows = (long long)B * T;
-  const long long r0 = (long long)blockIdx.x * SC_ROWS + warp * (SC_ROWS / 8);
-  float b0 = 0.f, b1 = 0.f;
-  if (!DX && bias) {
-    b0 = __bfloat162float(bias[c]);
-    b1 = __bfloat162float(bias[c + 1]);
-  }
-  for (long long r = r0; r < min(rows, r0 + SC_ROWS / 8); ++r) {
-    const int t = (int)(r % T);
-    const int taps = DX ? min(W, T - t) : min(W, t + 1);
-    const __nv_bfloat162* src = reinterpret_cast<const __nv_bfloat162*>(in + r * C + c);
-    const long long step = DX ? (long long)(C / 2) : -(long long)(C / 2);
-    float a0 = b0, a1 = b1;
-#pragma unroll 4
-    for (int j = 0; j < taps; ++j) {
-      const float2 xv = __bfloat1622float2(src[j * step]);
-      const float2 wv = *reinterpret_cast<const float2*>(sw + j * 64 + 2 * lane);
-      a0 += xv.x * wv.x;
-      a1 += xv.y * wv.y;
-    }
-    *reinterpret_cast<__nv_bfloat162*>(out + r * C + c) = __floats2bfloat162_rn(a0, a1);
+// Rows row, row + dir, ... of 16 steps; `inside`: all of them exist (a test and a multiplication less per load), otherwise those of ok(i).
+template <class Ok>
+__device__ __forceinline__ void ld_rows(uint32_t (&q)[SC_TILE], const __nv_bfloat16* base, long long row, long long C, int dir, bool inside, Ok ok) {
+  if (inside) {
+    const __nv_bfloat16* p = base + row * C;
+    const long long step = dir * C;
+#pragma unroll
+    for (int i = 0; i < SC_TILE; ++i, p += step) q[i] = *reinterpret_cast<const uint32_t*>(p);
+  } else {
+#pragma unroll
+    for (int i = 0; i < SC_TILE; ++i) q[i] = ld_pair(base, row + dir * i, C, ok(i));
   }
 }
 
-// dw[c,w] = sum_{b,t>=w} dy[b,t,c] x[b,t-w,c]; db[c] = sum dy. A CTA owns 32 channels (lane = channel) and SC_TAPS taps;
-// its 32 warps stride over all B T rows (four rows in flight per warp), every row's dy is read once and multiplied with
-// the SC_TAPS shifted inputs; the warps' partial sums are added in warp order (no atomics). grid (ceil(C / 32),
-// ceil(W / SC_TAPS)), block (32, 32); the CTAs with blockIdx.y == 0 also produce the bias gradient.
-constexpr int SC_TAPS = 4;
+// One output of the block kernel below as it is meant, for weights that are not finite: no product with what lies outside the sequence.
+template <bool DX>
+__device__ __noinline__ void shortconv_rows(const __nv_bfloat16* ib, const __nv_bfloat16* wc, uint64_t b2, __nv_bfloat16* ob, int s0, int T, int C, int W) {
+  for (int s = s0; s < min(T, s0 + SC_TILE); ++s) {
+    float a0, a1;
+    unpack_f32x2(b2, a0, a1);
+    for (int j = 0; j < min(W, s + 1); ++j) {
+      const uint32_t v = ld_pair(ib, DX ? T - 1 - s + j : s - j, C, true);
+      a0 = fmaf(bf16_lo(v), __bfloat162float(wc[j]), a0);
+      a1 = fmaf(bf16_hi(v), __bfloat162float(wc[W + j]), a1);
+    }
+    *reinterpret_cast<uint32_t*>(ob + (long long)(DX ? T - 1 - s : s) * C) = pack_bf16(a0, a1);
+  }
+}
 
-__global__ void __launch_bounds__(1024) shortconv_bwd_dw_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                                                                float* __restrict__ dw, float* __restrict__ db, int B, int T, int C,
-                                                                int W) {
-  __shared__ float sm[32][SC_TAPS + 1][33];
-  const int lane = threadIdx.x, warp = threadIdx.y;
-  const int c = blockIdx.x * 32 + lane;
-  const int w0 = blockIdx.y * SC_TAPS;
-  float acc[SC_TAPS], accb = 0.f;
+// Forward (y[t] = bias + sum_j x[t - j] w[j]) and, walked from late to early, the input gradient (dx[t] = sum_j dy[t + j] w[j]); step s is time s or
+// T - 1 - s. The sum of an output runs over j in order, as in shortconv_stream_kernel. What lies outside the sequence is zero, which finite weights leave
+// so. grid (ceil(B * tiles / SC_WARPS), ceil(C / 64)), block (32, SC_WARPS), dynamic shared memory: the weights, W by SC_WLD floats.
+template <bool DX>
+__global__ void __launch_bounds__(32 * SC_WARPS, 2) shortconv_tile_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w,
+                                                                          const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out,
+                                                                          int B, int T, int C, int W, int tiles) {
+  extern __shared__ __align__(16) float sw[];
+  const int lane = threadIdx.x, warp = threadIdx.y, c0 = blockIdx.y * 64;
+  float z = 0.f;
+  for (int j = lane; j < W; j += 32) {                   // consecutive lanes read consecutive weights of a channel
 #pragma unroll
-  for (int u = 0; u < SC_TAPS; ++u) acc[u] = 0.f;
-  if (c < C) {
-    const long long rows = (long long)B * T;
-#pragma unroll 4
-    for (long long r = warp; r < rows; r += 32) {
-      const int t = (int)(r % T);
-      const float g = __bfloat162float(dy[r * C + c]);
-      accb += g;
+    for (int i = 0; i < 64 / SC_WARPS; ++i) {
+      const int cl = warp + i * SC_WARPS;
+      const float f = c0 + cl < C ? __bfloat162float(w[(long long)(c0 + cl) * W + j]) : 0.f;
+      sw[j * SC_WLD + cl] = f;
+      z = fmaf(f, 0.f, z);
+    }
+  }
+  const bool bad = __syncthreads_or(z != 0.f);
+  const int c = c0 + 2 * lane;
+  const long long unit = (long long)blockIdx.x * SC_WARPS + warp;
+  if (c >= C || unit >= (long long)B * tiles) return;
+  const long long off = unit / tiles * T * C + c;
+  const int s0 = (int)(unit % tiles) * SC_TILE;
+  const __nv_bfloat16* ib = in + off;
+  __nv_bfloat16* ob = out + off;
+  const uint64_t b2 = !DX && bias ? pack_f32x2(__bfloat162float(bias[c]), __bfloat162float(bias[c + 1])) : 0ull;
+  if (bad) {
+    shortconv_rows<DX>(ib, w + (long long)c * W, b2, ob, s0, T, C, W);
+    return;
+  }
+  // steps s, s - 1, ..., s - 15
+  auto get = [&](uint32_t (&q)[SC_TILE], int s) {
+    ld_rows(q, ib, DX ? T - 1 - s : s, C, DX ? 1 : -1, s < T && s >= SC_TILE - 1, [&](int i) { return s - i < T && s - i >= 0; });
+  };
+  uint64_t win[2 * SC_TILE], acc[SC_TILE];               // step s0 + p is in slot p mod 32
+  {
+    uint32_t q[2][SC_TILE];
+    get(q[0], s0 + SC_TILE - 1);
+    get(q[1], s0 - 1);
 #pragma unroll
-      for (int u = 0; u < SC_TAPS; ++u) {
-        const int wj = w0 + u;
-        if (wj < W && t >= wj) acc[u] += g * __bfloat162float(x[(r - wj) * C + c]);
+    for (int i = 0; i < SC_TILE; ++i) {
+      win[SC_TILE - 1 - i] = pair_f32x2(q[0][i]);
+      win[2 * SC_TILE - 1 - i] = pair_f32x2(q[1][i]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < SC_TILE; ++r) acc[r] = b2;
+  auto block = [&](auto half, auto whole, int j0) {
+    constexpr int H = decltype(half)::value * SC_TILE;
+    uint32_t nx[SC_TILE];
+    if (j0 + SC_TILE < W) {
+      get(nx, s0 - j0 - SC_TILE);
+    } else {
+#pragma unroll
+      for (int i = 0; i < SC_TILE; ++i) nx[i] = 0u;
+    }
+#pragma unroll
+    for (int jj = 0; jj < SC_TILE; ++jj) {
+      if (!whole.value && j0 + jj >= W) break;           // an input that is not finite would make NaN of a tap of zero
+      const uint64_t wv = *reinterpret_cast<const uint64_t*>(sw + (j0 + jj) * SC_WLD + 2 * lane);
+#pragma unroll
+      for (int r = 0; r < SC_TILE; ++r) acc[r] = fma_f32x2(win[(r - jj - H) & 31], wv, acc[r]);
+    }
+#pragma unroll
+    for (int i = 0; i < SC_TILE; ++i) win[(-H - SC_TILE - i) & 31] = pair_f32x2(nx[i]);
+  };
+  using Even = std::integral_constant<int, 0>;
+  using Odd = std::integral_constant<int, 1>;
+  const int full = W / (2 * SC_TILE) * (2 * SC_TILE);
+  for (int j0 = 0; j0 < full; j0 += 2 * SC_TILE) {
+    block(Even{}, std::true_type{}, j0);
+    block(Odd{}, std::true_type{}, j0 + SC_TILE);
+  }
+  if (full < W) block(Even{}, std::false_type{}, full);
+  if (full + SC_TILE < W) block(Odd{}, std::false_type{}, full + SC_TILE);
+  __nv_bfloat16* o = ob + (long long)(DX ? T - 1 - s0 : s0) * C;
+  const long long step = DX ? -(long long)C : C;
+#pragma unroll
+  for (int r = 0; r < SC_TILE; ++r, o += step) {
+    float lo, hi;
+    unpack_f32x2(acc[r], lo, hi);
+    if (s0 + r < T) *reinterpret_cast<uint32_t*>(o) = pack_bf16(lo, hi);
+  }
+}
+
+// The sums of 16 taps over a span of one sequence as they are meant, where those of shortconv_dw_kernel came out not finite: zeros stand in there for
+// what lies outside the span and the sequence.
+__device__ __noinline__ void shortconv_dw_again(const __nv_bfloat16* x, const __nv_bfloat16* dy, float* pb, int b0, int b1, int t0, int t1, int T, int C, int W,
+                                                int j0) {
+  for (int ch = 0; ch < 2; ++ch)
+    for (int j = j0; j < min(W, j0 + SC_TILE); ++j) {
+      float s = 0.f;
+      for (int b = b0; b < b1; ++b)
+        for (int t = max(t0, j); t < t1; ++t)
+          s = fmaf(__bfloat162float(x[((long long)b * T + t - j) * C + ch]), __bfloat162float(dy[((long long)b * T + t) * C + ch]), s);
+      pb[(long long)j * C + ch] = s;
+    }
+}
+
+// part[slice][j][c] = sum over the slice's steps of dy[t, c] x[t - j, c], part[slice][W][c] that of dy. A warp takes 64 channels, 16 taps and a slice: a span of
+// one sequence, or with many sequences all of `seqs`. grid (ceil(slices / 4), ceil(C / 64), ceil(W / 16)), block (32, 4)
+__global__ void __launch_bounds__(128, 3) shortconv_dw_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+                                                              float* __restrict__ part, int B, int T, int C, int W, int span, int spans, int seqs, int slices) {
+  const int c = blockIdx.y * 64 + 2 * threadIdx.x, j0 = blockIdx.z * SC_TILE, unit = blockIdx.x * 4 + threadIdx.y;
+  if (c >= C || unit >= slices) return;
+  const int b0 = unit / spans * seqs, b1 = min(B, b0 + seqs), t0 = unit % spans * span, t1 = min(T, t0 + span);
+  uint64_t acc[SC_TILE], accb = 0ull;
+#pragma unroll
+  for (int j = 0; j < SC_TILE; ++j) acc[j] = 0ull;
+  for (int b = b0; b < b1; ++b) {
+    const __nv_bfloat16 *xb = x + (long long)b * T * C + c, *gb = dy + (long long)b * T * C + c;
+    uint64_t win[2 * SC_TILE];                           // input t0 - j0 + p is in slot p mod 32
+    uint32_t nx[SC_TILE], ng[SC_TILE];
+    auto get_x = [&](int t) {
+      ld_rows(nx, xb, t - j0, C, 1, t >= j0 && t + SC_TILE <= t1, [&](int r) { return t - j0 + r >= 0 && t + r < t1; });
+    };
+    auto get_g = [&](int t) { ld_rows(ng, gb, t, C, 1, t + SC_TILE <= t1, [&](int r) { return t + r < t1; }); };
+    get_x(t0 - SC_TILE);
+#pragma unroll
+    for (int r = 0; r < SC_TILE; ++r) win[SC_TILE + r] = pair_f32x2(nx[r]);
+    get_x(t0);
+    get_g(t0);
+    auto block = [&](auto half, int t) {
+      constexpr int H = decltype(half)::value * SC_TILE;
+      uint32_t cg[SC_TILE];
+#pragma unroll
+      for (int r = 0; r < SC_TILE; ++r) {
+        win[r + H] = pair_f32x2(nx[r]);
+        cg[r] = ng[r];
       }
-    }
-  }
+      get_x(t + SC_TILE);
+      get_g(t + SC_TILE);
 #pragma unroll
-  for (int u = 0; u < SC_TAPS; ++u) sm[warp][u][lane] = acc[u];
-  sm[warp][SC_TAPS][lane] = accb;
-  __syncthreads();
-  if (warp <= SC_TAPS && c < C) {                        // warp u adds up tap u, warp SC_TAPS the bias column
-    float s = 0.f;
-    for (int i = 0; i < 32; ++i) s += sm[i][warp][lane];
-    if (warp == SC_TAPS) {
-      if (db && blockIdx.y == 0) db[c] = s;
-    } else if (w0 + warp < W) {
-      dw[(long long)c * W + w0 + warp] = s;
+      for (int r = 0; r < SC_TILE; ++r) {
+        const uint64_t g = pair_f32x2(cg[r]);
+        accb = add_f32x2(accb, g);
+#pragma unroll
+        for (int j = 0; j < SC_TILE; ++j) acc[j] = fma_f32x2(win[(r - j + H) & 31], g, acc[j]);
+      }
+    };
+    for (int t = t0; t < t1; t += 2 * SC_TILE) {
+      block(std::integral_constant<int, 0>{}, t);
+      if (t + SC_TILE < t1) block(std::integral_constant<int, 1>{}, t + SC_TILE);
     }
   }
+  float* pb = part + (long long)unit * (W + 1) * C + c;
+  uint64_t z = 0ull;
+#pragma unroll
+  for (int j = 0; j < SC_TILE; ++j) {
+    float lo, hi;
+    unpack_f32x2(acc[j], lo, hi);
+    if (j0 + j < W) *reinterpret_cast<float2*>(pb + (long long)(j0 + j) * C) = make_float2(lo, hi);
+    z = fma_f32x2(acc[j], 0ull, z);
+  }
+  if (j0 == 0) {
+    float lo, hi;
+    unpack_f32x2(accb, lo, hi);
+    *reinterpret_cast<float2*>(pb + (long long)W * C) = make_float2(lo, hi);
+  }
+  if (not_finite_f32x2(z)) shortconv_dw_again(x + c, dy + c, pb, b0, b1, t0, t1, T, C, W, j0);
+}
+
+template <bool DX>
+int launch_shortconv_tile(const __nv_bfloat16* in, const __nv_bfloat16* w, const __nv_bfloat16* bias, __nv_bfloat16* out, int B, int T, int C, int W,
+                          cudaStream_t s) {
+  const int tiles = (T + SC_TILE - 1) / SC_TILE;
+  const dim3 grid((unsigned)(((long long)B * tiles + SC_WARPS - 1) / SC_WARPS), (C + 63) / 64), block(32, SC_WARPS);
+  shortconv_tile_kernel<DX><<<grid, block, (size_t)W * SC_WLD * sizeof(float), s>>>(in, w, bias, out, B, T, C, W, tiles);
+  ELFA_CUDA(cudaGetLastError());
+  ::elfa::count_launches(1);
+  return ELFA_OK;
+}
+
+// The slices of shortconv_dw_kernel: no sum longer than SC_CHAIN steps (its error grows with its length: in one wave of warps, up to 2048 steps, it was
+// twice that of sums of 512), in whole waves of its warps (12 of them per SM).
+constexpr int SC_CHAIN = 256;
+struct ShortConvSlices {
+  int span, spans, seqs, slices;
+};
+ShortConvSlices shortconv_slices(int B, int T, int C, int W) {
+  const long long per = (long long)((C + 63) / 64) * ((W + SC_TILE - 1) / SC_TILE), wave = 12ll * 148;        // warps of a slice; of the chip
+  const long long least = ((long long)B * T + SC_CHAIN - 1) / SC_CHAIN, want = std::max(1ll, (least * per + wave - 1) / wave * wave / per);
+  const int tiles = (T + SC_TILE - 1) / SC_TILE, cut = (int)std::min<long long>(tiles, std::max<long long>((T + SC_CHAIN - 1) / SC_CHAIN, want / B));
+  ShortConvSlices q;
+  q.span = (tiles + cut - 1) / cut * SC_TILE;
+  q.spans = (T + q.span - 1) / q.span;
+  q.seqs = (int)std::min(std::max(1ll, (B + want - 1) / want), (long long)std::max(1, SC_CHAIN / T));
+  q.slices = (B + q.seqs - 1) / q.seqs * q.spans;
+  return q;
 }
 
 template <int D>
@@ -382,9 +526,10 @@ static int shortconv_span(int B, int T, int C) {
 }
 static bool shortconv_ring(int W) { return W == 4 || W == 8 || W == 16; }
 
-// Slices of the weight-gradient scratch of elfa_shortconv_bwd_as (slices * (W + 1) * C floats), 0 when it needs none.
+// Slices of the weight-gradient scratch of elfa_shortconv_bwd_as (slices * (W + 1) * C floats).
 ELFA_API int elfa_shortconv_bwd_slices(int B, int T, int C, int W) {
-  if (!shortconv_ring(W) || B <= 0 || T <= 0 || C <= 0) return 0;
+  if (B <= 0 || T <= 0 || C <= 0 || W <= 0) return 0;
+  if (!shortconv_ring(W)) return shortconv_slices(B, T, C, W).slices;
   const int span = shortconv_span(B, T, C);
   return B * ((T + span - 1) / span);
 }
@@ -405,22 +550,16 @@ ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, 
     ::elfa::count_launches(1);
     return ELFA_OK;
   }
-  const long long rows = (long long)B * T;
-  dim3 grid((unsigned)((rows + SC_ROWS - 1) / SC_ROWS), (C + 63) / 64), block(32, 8);
-  shortconv_apply_kernel<false><<<grid, block, (size_t)W * 64 * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(bias),
-      static_cast<__nv_bfloat16*>(y), B, T, C, W);
-  ELFA_CUDA(cudaGetLastError());
-  ::elfa::count_launches(1);
-  return ELFA_OK;
+  return launch_shortconv_tile<false>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(bias),
+                                      static_cast<__nv_bfloat16*>(y), B, T, C, W, static_cast<cudaStream_t>(stream));
 }
 
 // Whether T positions behind a tail are long enough for the ordinary kernels: tail and inputs are copied side by side, the outputs of the tail's own
 // positions are made and dropped, with several sequences the others are copied together. The one kernel reads 2 W weights per channel pair and
 // position straight from [C, W], where every lane touches another line: long blocks cost it 5 (W 4), 9 (8), 30 (16), 24 (24), 114 (32) and 226 (64)
 // microseconds per 10^6 values. Measured, one kernel / ordinary ones, microseconds: W 4, 1 sequence 2^20 values 6.9 / 6.5, 2^22 21 / 10, 4 sequences
-// 2^22 21 / 26; W 8 2^20 11 / 7 and 11 / 11; W 16 2^17 6.6 / 6.4 and 6.6 / 8.2, 2^18 10.6 / 6.5 and 10.6 / 8.4, 2^22 125 / 13; W 24 2^18 9 / 13,
-// 2^19 15 / 13; W 32 2^17 18 / 16; W 64 2^16 21 / 23, 2^17 33 / 24, 2^22 948 / 81.
+// 2^22 21 / 26; W 8 2^20 11 / 7 and 11 / 11; W 16 2^17 6.6 / 6.4 and 6.6 / 8.2, 2^18 10.6 / 6.5 and 10.6 / 8.4, 2^22 125 / 13; W 24 2^18 10 / 12,
+// 2^19 19 / 12 and 19 / 18; W 32 2^16 13 / 12 and 14 / 17, 2^17 21 / 12 and 21 / 17; W 64 2^15 17 / 14 and 19 / 22, 2^16 23 / 15 and 25 / 22, 2^20 245 / 17.
 static bool shortconv_stream_long(int B, int T, int C, int W) {
   const long long values = (long long)B * T * C;
   if (W < 8) return B == 1 && values >= 1 << 21;
@@ -477,39 +616,37 @@ ELFA_API int elfa_shortconv_stream(const void* tail, long long tail_stride, cons
   return ELFA_OK;
 }
 
-// dx bf16 [B,T,C]; dw [C,W] and db [C] (or null) in fp32, or in bf16 where `grads_bf16` (windows of 4, 8 and 16 only); part: scratch of
-// elfa_shortconv_bwd_slices() * (W + 1) * C floats (null when 0).
+// dx bf16 [B,T,C]; dw [C,W] and db [C] (or null) in fp32, or in bf16 where `grads_bf16`; part: scratch of
+// elfa_shortconv_bwd_slices() * (W + 1) * C floats.
 ELFA_API int elfa_shortconv_bwd_as(const void* x, const void* w, const void* dy, void* dx, void* dw_, void* db_, float* part, int grads_bf16,
                                    int B, int T, int C, int W, void* stream) {
   float *dw = static_cast<float*>(dw_), *db = static_cast<float*>(db_);
-  ELFA_REQUIRE(!grads_bf16 || shortconv_ring(W), "shortconv_bwd: bf16 gradients for windows of 4, 8 and 16 only");
   ELFA_REQUIRE(x && w && dy && dx && dw && B > 0 && T > 0 && C > 0 && W > 0, "shortconv_bwd: bad arguments");
   ELFA_REQUIRE(C % 2 == 0 && W <= 128, "shortconv_bwd: the channel count must be even and the window at most 128");
+  ELFA_REQUIRE(part, "shortconv_bwd: the scratch buffer is missing");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const auto *X = static_cast<const __nv_bfloat16*>(x), *Wt = static_cast<const __nv_bfloat16*>(w), *G = static_cast<const __nv_bfloat16*>(dy);
+  auto* DX = static_cast<__nv_bfloat16*>(dx);
+  int slices;
   if (shortconv_ring(W)) {
-    ELFA_REQUIRE(part, "shortconv_bwd: this window needs the scratch buffer");
-    const auto *X = static_cast<const __nv_bfloat16*>(x), *Wt = static_cast<const __nv_bfloat16*>(w), *G = static_cast<const __nv_bfloat16*>(dy);
-    auto* DX = static_cast<__nv_bfloat16*>(dx);
     const int span = shortconv_span(B, T, C), spans = (T + span - 1) / span;
     const dim3 g((unsigned)(((long long)B * spans + 3) / 4), (C + 63) / 64), blk(32, 4);
     if (W == 4) shortconv_ring_bwd_kernel<4><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
     else if (W == 8) shortconv_ring_bwd_kernel<8><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
     else shortconv_ring_bwd_kernel<16><<<g, blk, 0, s>>>(X, Wt, G, DX, part, B, T, C, span, spans);
-    ELFA_CUDA(cudaGetLastError());
-    const dim3 gs((C + 31) / 32, W + 1), bs(32, 16);
-    if (grads_bf16) shortconv_sum_kernel<<<gs, bs, 0, s>>>(part, static_cast<__nv_bfloat16*>(dw_), static_cast<__nv_bfloat16*>(db_), B * spans, C, W);
-    else shortconv_sum_kernel<<<gs, bs, 0, s>>>(part, dw, db, B * spans, C, W);
-    ELFA_CUDA(cudaGetLastError());
-    ::elfa::count_launches(2);
-    return ELFA_OK;
+    slices = B * spans;
+  } else {
+    const int rc = launch_shortconv_tile<true>(G, Wt, nullptr, DX, B, T, C, W, s);
+    if (rc != ELFA_OK) return rc;
+    const ShortConvSlices q = shortconv_slices(B, T, C, W);
+    shortconv_dw_kernel<<<dim3((q.slices + 3) / 4, (C + 63) / 64, (W + SC_TILE - 1) / SC_TILE), dim3(32, 4), 0, s>>>(X, G, part, B, T, C, W, q.span, q.spans,
+                                                                                                                  q.seqs, q.slices);
+    slices = q.slices;
   }
-  const long long rows = (long long)B * T;
-  dim3 grid((unsigned)((rows + SC_ROWS - 1) / SC_ROWS), (C + 63) / 64), block(32, 8);
-  shortconv_apply_kernel<true><<<grid, block, (size_t)W * 64 * sizeof(float), s>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(w), nullptr, static_cast<__nv_bfloat16*>(dx), B, T, C, W);
-  dim3 grid2((C + 31) / 32, (W + SC_TAPS - 1) / SC_TAPS), block2(32, 32);
-  shortconv_bwd_dw_kernel<<<grid2, block2, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), dw, db, B,
-                                                   T, C, W);
+  ELFA_CUDA(cudaGetLastError());
+  const dim3 gs((C + 31) / 32, W + 1), bs(32, 16);
+  if (grads_bf16) shortconv_sum_kernel<<<gs, bs, 0, s>>>(part, static_cast<__nv_bfloat16*>(dw_), static_cast<__nv_bfloat16*>(db_), slices, C, W);
+  else shortconv_sum_kernel<<<gs, bs, 0, s>>>(part, dw, db, slices, C, W);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(2);
   return ELFA_OK;

@@ -133,3 +133,32 @@ def test_a_block_of_two_gigabytes_behind_a_tail(cuda_device, B):
     assert native.status() == 0 and in_full
     assert (xin[:, :W - 1] == 7).all() and torch.equal(xin[:, W - 1:], n)
     assert (u[:, :W - 1] == 7).all() and torch.equal(u[:, W - 1:], n[:, :T - W + 1])
+
+
+@pytest.mark.parametrize("W", [1, 15, 17, 32, 33, 48, 100, 128])
+@pytest.mark.parametrize("B,T,C", [(1, 1, 2), (3, 16, 66), (2, 47, 64), (300, 3, 2), (1, 700, 64)])
+def test_other_windows(cuda_device, B, T, C, W):
+    """Windows, lengths and channels around whole blocks of 16 taps, 16 steps and 64 channels; many sequences to a slice, many slices to a sequence."""
+    test_shortconv_edges(cuda_device, B, T, C, W, True)
+
+
+@pytest.mark.parametrize("W", [15, 17, 33, 64])
+@pytest.mark.parametrize("T", [1, 17, 40, 130])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nothing_beyond_the_sequence_is_multiplied_by_other_windows(cuda_device, T, W, bad):
+    test_nothing_beyond_the_sequence_is_multiplied(cuda_device, T, W, bad)
+
+
+def test_weight_gradient_of_long_sequences_keeps_its_error(cuda_device):
+    """fp32 sums against 64 bits: chains of 256 terms and a sum of their results; random signs let 2^-24 grow with the root of a chain's length (16 times),
+    and the first sum is no nearer than its own rounding."""
+    B, T, C, W = 4, 4096, 64, 33
+    torch.manual_seed(1)
+    x, dy = (torch.randn(B, T, C, device=cuda_device).bfloat16() for _ in range(2))
+    w = torch.randn(C, W, device=cuda_device).bfloat16()
+    slices = lib.raw("elfa_shortconv_bwd_slices")(B, T, C, W)
+    part, dw, db = (torch.empty(*s, device=cuda_device) for s in ((slices, W + 1, C), (C, W), (C,)))
+    lib.call("elfa_shortconv_bwd_as", x, w, dy, torch.empty_like(x), dw, db, part, 0, B, T, C, W, stream_ptr(x))
+    ref = torch.stack([(dy[:, j:].double() * x[:, :T - j].double()).sum((0, 1)) for j in range(W)], 1)
+    assert ((dw.double() - ref).norm() / ref.norm()).item() < 16 * 2.0 ** -24
+
