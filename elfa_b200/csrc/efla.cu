@@ -36,8 +36,9 @@ __global__ void __launch_bounds__(32 * EFLA_W) efla_scan_fwd_kernel(const __nv_b
 // shortconv_tile_kernel / shortconv_dw_kernel below.
 // Backward is one walk from late to early: with dy[t .. t + W - 1] as the window, dx[t] = sum_j w[j] dy[t + j] and
 // dw[j] += x[t] dy[t + j]; every warp writes its dw / db sums as one slice of part [slices][W + 1][C], added up in order afterwards.
-// B 8, T 2048, C 1024, W 16: 27 us forward (67 MB; bound by the packed multiply-adds and the latency of 202- and 126-register warps), 45 + 6 us
-// backward; the layer that contains them went from 789 to 454 us when they replaced kernels that took a tap at a time.
+// B 8, T 2048, C 1024, W 16: 25 us forward (67 MB; bound by the packed multiply-adds and the latency of 202- and 128-register warps; 27 with a test and
+// a 64-bit multiplication per load, which are kept in backward: 45 us with them, 50 without), 45 + 6 us backward; the
+// layer that contains them went from 789 to 454 us when they replaced kernels that took a tap at a time.
 // A lane's weights are 4 W consecutive bytes; one at a time they would cost 2 W loads that touch 32 lines each, more than the
 // inputs (31.5 against 26.5 us forward).
 template <int W>
@@ -62,6 +63,19 @@ __device__ __forceinline__ void shortconv_weights(uint64_t (&wf)[W], const __nv_
 }
 __device__ __forceinline__ uint32_t ld_pair(const __nv_bfloat16* base, long long row, long long C, bool ok) {
   return ok ? *reinterpret_cast<const uint32_t*>(base + row * C) : 0u;
+}
+// Rows row, row + dir, ...; `inside`: all of them exist (a test and a multiplication less per load), otherwise those of ok(i).
+template <int N, class Ok>
+__device__ __forceinline__ void ld_rows(uint32_t (&q)[N], const __nv_bfloat16* base, long long row, long long C, int dir, bool inside, Ok ok) {
+  if (inside) {
+    const __nv_bfloat16* p = base + row * C;
+    const long long step = dir * C;
+#pragma unroll
+    for (int i = 0; i < N; ++i, p += step) q[i] = *reinterpret_cast<const uint32_t*>(p);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) q[i] = ld_pair(base, row + dir * i, C, ok(i));
+  }
 }
 __device__ __forceinline__ uint64_t pair_f32x2(uint32_t v) { return pack_f32x2(bf16_lo(v), bf16_hi(v)); }
 
@@ -121,13 +135,12 @@ __global__ void __launch_bounds__(128) shortconv_ring_fwd_kernel(const __nv_bflo
   uint32_t nx[W];
 #pragma unroll
   for (int r = 0; r < W; ++r) nx[r] = ld_pair(xb, t0 + r, C, t0 + r < t1);
+  __nv_bfloat16* yt = yb + (long long)t0 * C;
   auto block = [&](auto edge, int t) {
     uint32_t cur[W];
 #pragma unroll
-    for (int r = 0; r < W; ++r) {
-      cur[r] = nx[r];
-      nx[r] = ld_pair(xb, t + W + r, C, t + W + r < t1);
-    }
+    for (int r = 0; r < W; ++r) cur[r] = nx[r];
+    ld_rows(nx, xb, t + W, C, 1, t + 2 * W <= t1, [&](int r) { return t + W + r < t1; });
 #pragma unroll
     for (int r = 0; r < W; ++r) {
       win[r] = pair_f32x2(cur[r]);
@@ -139,7 +152,8 @@ __global__ void __launch_bounds__(128) shortconv_ring_fwd_kernel(const __nv_bflo
       }
       float lo, hi;
       unpack_f32x2(add_f32x2(s0, s1), lo, hi);
-      if (t + r < t1) *reinterpret_cast<uint32_t*>(yb + (long long)(t + r) * C) = pack_bf16(lo, hi);
+      if (t + r < t1) *reinterpret_cast<uint32_t*>(yt) = pack_bf16(lo, hi);
+      yt += C;
     }
   };
   int t = t0;
@@ -267,20 +281,6 @@ __global__ void __launch_bounds__(64) shortconv_stream_kernel(const __nv_bfloat1
 constexpr int SC_TILE = 16;
 constexpr int SC_WARPS = 8;
 constexpr int SC_WLD = 66;                               // floats of a tap's 64 weights: channel by channel stores meet two to a bank
-
-// Rows row, row + dir, ... of 16 steps; `inside`: all of them exist (a test and a multiplication less per load), otherwise those of ok(i).
-template <class Ok>
-__device__ __forceinline__ void ld_rows(uint32_t (&q)[SC_TILE], const __nv_bfloat16* base, long long row, long long C, int dir, bool inside, Ok ok) {
-  if (inside) {
-    const __nv_bfloat16* p = base + row * C;
-    const long long step = dir * C;
-#pragma unroll
-    for (int i = 0; i < SC_TILE; ++i, p += step) q[i] = *reinterpret_cast<const uint32_t*>(p);
-  } else {
-#pragma unroll
-    for (int i = 0; i < SC_TILE; ++i) q[i] = ld_pair(base, row + dir * i, C, ok(i));
-  }
-}
 
 // One output of the block kernel below as it is meant, for weights that are not finite: no product with what lies outside the sequence.
 template <bool DX>
@@ -540,7 +540,8 @@ ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, 
   if (shortconv_ring(W)) {
     const auto *X = static_cast<const __nv_bfloat16*>(x), *Wt = static_cast<const __nv_bfloat16*>(w), *Bi = static_cast<const __nv_bfloat16*>(bias);
     auto* Y = static_cast<__nv_bfloat16*>(y);
-    const int span = shortconv_span(B, T, C), spans = (T + span - 1) / span;
+    // four taps: the seam is three rows, and more warps keep more loads in flight (B 4, T 4096, C 512: 20 -> 16 us, B 2, T 1531, C 1024: 12 -> 10)
+    const int span = W == 4 ? 16 : shortconv_span(B, T, C), spans = (T + span - 1) / span;
     const dim3 g((unsigned)(((long long)B * spans + 3) / 4), (C + 63) / 64), blk(32, 4);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (W == 4) shortconv_ring_fwd_kernel<4><<<g, blk, 0, s>>>(X, Wt, Bi, Y, B, T, C, span, spans);
