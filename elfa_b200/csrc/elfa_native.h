@@ -222,6 +222,9 @@ int elfa_efla_chunk_fwd_cut(const void* k, const void* v, const float* beta, con
 int elfa_efla_chunk_bwd_cut(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
                             const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0, float* dckpt, float* work,
                             int segments, int B, int T, int H, int d, void* stream);
+int elfa_efla_chunk_bwd_sum(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
+                            const float* dstate_out, void* dk, void* dv, float* dbeta_terms, float* dbeta, float* dstate0, float* dckpt,
+                            float* work, int segments, int B, int T, int H, int d, void* stream);
 int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, void* y, int B, int T, int C, int W, void* stream);
 int elfa_shortconv_stream_rows(int B, int tails, int T, int C, int W);
 int elfa_shortconv_stream(const void* tail, long long tail_stride, const void* n, const void* w, const void* bias, void* xin, void* u, void* full,

@@ -178,17 +178,15 @@ class _EflaScan(torch.autograd.Function):
         B, T, H, d, has_state = ctx.cfg
         dk = torch.empty_like(kc)
         dv = torch.empty_like(vc)
-        dbeta = torch.empty(B * T * H, dtype=torch.float32, device=kc.device)            # per-token terms, summed below
+        dbeta = torch.empty(1, dtype=torch.float32, device=kc.device)
+        terms = torch.empty(B * H * ((T + 31) // 32), dtype=torch.float32, device=kc.device)          # of dbeta, one per chunk
         ds0 = torch.empty((B, H, d, d), dtype=torch.float32, device=kc.device) if has_state else None
         dckpt = torch.empty_like(ckpt)
         dso = ds_out.float().contiguous() if ds_out is not None else None
         cut = _efla_segments(B, T, H, d, True)
-        if cut > 1:
-            lib.call("elfa_efla_chunk_bwd_cut", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt,
-                     _efla_scratch(cut, kc, B, H, d), cut, B, T, H, d, stream_ptr(kc))
-        else:
-            lib.call("elfa_efla_chunk_bwd", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, dbeta, ds0, dckpt, B, T, H, d, stream_ptr(kc))
-        return dk, dv, dbeta.sum().reshape(1), ds0, None
+        lib.call("elfa_efla_chunk_bwd_sum", kc, vc, nmat, coef, ckpt, _aligned(do), dso, dk, dv, terms, dbeta, ds0, dckpt,
+                 _efla_scratch(cut, kc, B, H, d) if cut > 1 else None, cut, B, T, H, d, stream_ptr(kc))
+        return dk, dv, dbeta, ds0, None
 
 
 def efla_scan(k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, state: Optional[torch.Tensor] = None, chunk: int = 16

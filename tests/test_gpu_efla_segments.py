@@ -107,3 +107,20 @@ def test_the_rule_gives_segments_that_fit(cuda_device):
         n = lib.raw("elfa_efla_segments")(B, T, H, d)
         assert 1 <= n <= 16 and (n == 1 or (T + 31) // 32 >= 4 * n)
     assert lib.raw("elfa_efla_segments")(1, 8192, 16, 64) > 1 and lib.raw("elfa_efla_segments")(64, 4096, 16, 64) == 1
+
+
+@pytest.mark.parametrize("B,T,H,d", [(1, 1, 1, 32), (3, 33, 5, 64), (2, 300, 4, 96), (1, 97, 2, 128), (8, 1100, 16, 32)])
+def test_beta_gradient_is_the_sum_of_its_terms(cuda_device, B, T, H, d):
+    """Added up per chunk and then over the chunks (1, few and more than 4096 of them), in 64 bits: a rounding of each chunk's sum and one of the result,
+    2^-24 of what they are."""
+    k, v, beta, _, do, _ = _inputs(cuda_device, B, T, H, d)
+    n = (T + 31) // 32
+    new = lambda *s, dt=torch.float32: torch.empty(*s, dtype=dt, device=k.device)
+    ckpt, dckpt, coef, nmat, s = new(B * H * n * d * d), new(B * H * n * d * d), new(B, H, n, 4, 32), new(B, H, n, 3, 32, 32, dt=torch.bfloat16), new(B, H, d, d)
+    o, dk, dv, terms, tok, db = torch.empty_like(k), torch.empty_like(k), torch.empty_like(k), new(B * H * n), new(B * T * H), new(1)
+    lib.call("elfa_efla_chunk_fwd", k, v, beta, None, o, s, ckpt, nmat, coef, B, T, H, d, stream_ptr(k))
+    lib.call("elfa_efla_chunk_bwd", k, v, nmat, coef, ckpt, do, None, dk, dv, tok, None, dckpt, B, T, H, d, stream_ptr(k))
+    lib.call("elfa_efla_chunk_bwd_sum", k, v, nmat, coef, ckpt, do, None, dk, dv, terms, db, None, dckpt, None, 1, B, T, H, d, stream_ptr(k))
+    tok = tok.double()
+    assert abs(db.item() - tok.sum().item()) <= 2 ** -24 * (tok.abs().sum() + tok.sum().abs()).item()
+
