@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define ELFA_API extern "C" __attribute__((visibility("default")))
 
 // Return codes of every exported function.
@@ -65,6 +67,18 @@ int make_tmap_nd_bf16(CUtensorMap* out, const void* base, int ndim, const uint64
 int shared_tmap(CUtensorMap* out, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t ld_elems,
                 uint32_t box_rows, uint32_t box_cols);
 int device_sm_count();
+// The shared memory that a kernel may use, set once per device: asking on every call costs the host 1 to 2 us, up to five times in a pass. `bytes` is the
+// most that any call asks for: the limit belongs to the kernel, and a call's own size would be in force when another thread's larger launch comes.
+template <auto Kernel>
+cudaError_t allow_shared(int bytes) {
+  static std::atomic<unsigned long long> configured{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev <= 63 && (configured.load(std::memory_order_relaxed) >> dev & 1))) return e;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev <= 63) configured.fetch_or(1ull << dev, std::memory_order_relaxed);
+  return e;
+}
 // While a scope is open on this thread, the kernels that ask for it are launched with programmatic stream serialisation: their blocks may start
 // before the launch ahead of them has finished and wait inside (pdl_wait). Only for a chain in which nothing that a kernel reads before its
 // pdl_wait is written by the chain, and whose first launch is an ordinary one.

@@ -23,7 +23,6 @@
 //
 // reference: kernels/cuda/efla.cu:121-271,534-552 (chunks are scanned one after the other, the bf16 state in global memory).
 #include <algorithm>
-#include <atomic>
 
 #include "common.cuh"
 #include "elfa_native.h"
@@ -791,18 +790,6 @@ __global__ void __launch_bounds__(2 * D) efla_combine_kernel(const float* __rest
       }
     if (n + 1 < P - 2) put_start(n + 1, s);
   }
-}
-
-// The shared memory that a kernel may use, set once per device: asking on every call costs the host 1 to 2 us, up to five times in a pass
-template <auto Kernel>
-cudaError_t allow_shared(int bytes) {
-  static std::atomic<unsigned long long> configured{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess || (dev <= 63 && (configured.load(std::memory_order_relaxed) >> dev & 1))) return e;
-  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess && dev <= 63) configured.fetch_or(1ull << dev, std::memory_order_relaxed);
-  return e;
 }
 
 template <int D>

@@ -350,13 +350,14 @@ __global__ void __launch_bounds__(4 * D) prism_state_kernel(const __nv_bfloat16*
   prism_state_store<D>(S, out + ((long long)bg * D + row) * D, part);
 }
 
+constexpr int PS_SHARED = 110 * 1024;           // most that a tile takes: half of an SM's
 template <int D>
 int launch_prism_state(const void* u, const void* v, const void* z, long long ldz, int off_b, int off_k, const float* state, float* out,
                        int B, int T, int G, int L, float forget, cudaStream_t s) {
-  // tokens of a tile: up to 64 (a multiple of four: the tile's parts start on 16 bytes) in half of an SM's shared memory
-  const int token = (2 * D + 1) * L * (int)sizeof(float), tile = T < 4 ? 4 : (T < 64 ? (T + 3) / 4 * 4 : 64), most = 110 * 1024 / token / 4 * 4;
+  // tokens of a tile: up to 64 (a multiple of four: the tile's parts start on 16 bytes) in PS_SHARED
+  const int token = (2 * D + 1) * L * (int)sizeof(float), tile = T < 4 ? 4 : (T < 64 ? (T + 3) / 4 * 4 : 64), most = PS_SHARED / token / 4 * 4;
   const int tokens = tile < most ? tile : most, bytes = tokens * token;
-  ELFA_CUDA(cudaFuncSetAttribute(prism_state_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  ELFA_CUDA(allow_shared<prism_state_kernel<D>>(PS_SHARED));
   prism_state_kernel<D><<<B * G, 4 * D, bytes, s>>>(static_cast<const __nv_bfloat16*>(u), static_cast<const __nv_bfloat16*>(v),
                                                     static_cast<const __nv_bfloat16*>(z), ldz, off_b, off_k, state, out, T, G, L, forget, tokens);
   ELFA_CUDA(cudaGetLastError());

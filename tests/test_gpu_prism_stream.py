@@ -1,8 +1,12 @@
 """PRISM state carry in one kernel against the token-by-token update. fp32 on both sides: 1e-5 of the largest covers 40 tokens."""
+import sys
+import threading
+
 import pytest
 import torch
 
 from elfa_b200 import native, ops
+from elfa_b200.native import lib
 from elfa_b200.ops import efla as eops
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +48,34 @@ def test_state_of_any_stride(cuda_device, order):
     want = eops.prism_stream(u, v, wp, wb, wk, s0, 0.97, d)
     got = eops.prism_stream(u, v, wp, wb, wk, view, 0.97, d)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def test_lengths_of_several_threads(cuda_device):
+    """Two threads with tiles of twelve tokens, two with tiles of four: how much shared memory one call takes is no limit for another one's launch (where
+    it was, one launch in sixty failed)."""
+    d, L, failed = 128, 8, [0] * 4
+    f = lib.raw("elfa_prism_state")
+
+    def run(i, T):
+        u, v, z = (torch.randn(1, T, n, device=cuda_device).bfloat16() for n in (d, d, 3 * L * d))
+        s0 = torch.randn(1, 1, d, d, device=cuda_device)
+        s1 = torch.empty_like(s0)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            here = torch.cuda.current_stream()
+            here.wait_stream(torch.cuda.default_stream())
+            for k in range(4096):
+                failed[i] += f(u.data_ptr(), v.data_ptr(), z.data_ptr(), 3 * L * d, L * d, 2 * L * d, s0.data_ptr(), s1.data_ptr(), 1, T, 1, d, L, 0.9,
+                               here.cuda_stream) != 0
+                if k % 64 == 63:
+                    here.synchronize()
+    threads = [threading.Thread(target=run, args=(i, T)) for i, T in enumerate((12, 1, 12, 4))]
+    switch = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(switch)
+    assert failed == [0] * 4 and native.status() == 0
