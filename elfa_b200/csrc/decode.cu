@@ -5,9 +5,10 @@
 // small and elementwise - norms, residual sums, activations, PRISM's refinement - is done again by every CTA on the rows that it needs while it copies them to
 // shared memory:
 //   norm, w_k and w_v, ShortConv | scan, gate logits | w_o | refinement, norm, w_up | activation, w_down, PRISM's state
-// Scan and state belong to the CTAs that have no tile of their phase's product. A phase's weights do not depend on the phases before it: the blocks that fit
-// are copied to shared memory between the arrival at the barrier and the wait, and each CTA asks for its part of the next layer's into L2 there. The phases
-// go through one copy of the code, in loops rather than unrolled: a warp that meets straight-line code for the first time takes about eight cycles
+// Scan and state belong to the CTAs that have no tile of their phase's product, where those are enough for them. A phase's weights do not depend on the
+// phases before it: the blocks that fit are copied to shared memory between the arrival at the barrier and the wait, and each CTA asks for its part of the
+// next layer's into L2 there. The phases go through one copy of the code, in loops rather than unrolled: a warp that meets straight-line code for the first
+// time takes about eight cycles
 // per instruction. Two layers, 1024 wide, B 2: a step 67 us (and 17 for the logits); prompt of 64 tokens and
 // four steps 1131 us with the chain, 788 with this.
 //
@@ -320,12 +321,16 @@ __device__ __forceinline__ void product(const Team& c, const Cut& u, const Weigh
     }
   }
 }
-// Other work beside a product: it belongs to the CTAs of the clusters that have no tile, numbered from 0, or to all of them ahead of the product.
-__device__ __forceinline__ bool free_ctas(const Team& c, const Cut& u, int& at, int& n) {
-  const bool some = u.used < c.clusters;
-  at = some ? c.cta - u.used * CL : c.cta;
-  n = some ? c.ctas - u.used * CL : c.ctas;
-  return at >= 0;
+// Other work beside a product, `items` equal pieces: it belongs to the CTAs of the clusters that have no tile, where those take no more rounds than all
+// CTAs would, and otherwise to all of them, ahead of the product, those without a tile first. Two layers, eight rows, us, all on the CTAs without a tile / so: 2048 wide,
+// 16 heads of 128, w_down leaves eight CTAs for 128 states, 450 / 245; 1024 wide, 8 heads of 128, no PRISM, no product beside the scan, 147 / 95.
+// (-> the CTA has a part; its number and how many there are)
+__device__ __forceinline__ bool side_work(const Team& c, const Cut& u, int items, int& at, int& n) {
+  const int free = c.ctas - u.used * CL;
+  n = free > 0 && (items + free - 1) / free <= (items + c.ctas - 1) / c.ctas ? free : c.ctas;
+  at = c.cta - u.used * CL;
+  if (at < 0) at += c.ctas;
+  return at < n;
 }
 
 // ------------------------------------------------------------------------------------------------ rows
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(NT, 2) efla_decode_kernel(const __grid_constan
     const Cut& u = p.cut[ph];
     const bool multiply = ph != 1 || p.prism;
     int at, n;                                         // the CTAs of what goes on beside a product
-    if (ph == 1 && free_ctas(c, u, at, n)) {           // the scan, beside the gates' logits: 128 threads per 32 columns of a head
+    if (ph == 1 && side_work(c, u, (p.B * p.H * (HD / 32) + 1) / 2, at, n)) {           // the scan, beside the gates' logits: 128 threads per 32 columns of a head
       typedef EflaStepScratch<HD, EFLA_TOKENS> Scratch;
       static_assert(2 * sizeof(Scratch) <= part_bytes(1), "scratch of the scan");
       const int group = c.tid / 128;
@@ -540,7 +545,7 @@ __global__ void __launch_bounds__(NT, 2) efla_decode_kernel(const __grid_constan
       }
       __syncthreads();
     }
-    if (ph == 4 && p.prism && free_ctas(c, u, at, n)) {
+    if (ph == 4 && p.prism && side_work(c, u, p.B * G, at, n)) {
       // PRISM's state, which nothing of this call reads: a CTA per (batch, group), 64 rows at a time
       const PrismTile<HD> sm(c.part, p.T, p.L);
       const PrismSource in{p.w.u, p.w.e, p.w.z, ldz, p.L * HD, 2 * p.L * HD, p.T, G, p.L};
@@ -707,6 +712,7 @@ int launch(P& p, int bytes, cudaStream_t s) {
 void efla_cuts(const EflaDims& m, Cut* cut) {
   cut[0] = cut_of(m.H * m.d, m.D, 2);
   cut[1] = m.prism ? cut_of(3 * m.L * m.d, m.D) : cut[0];
+  if (!m.prism) cut[1].total = 0;                      // the scan alone
   cut[2] = cut_of(m.D, m.H * m.d);
   cut[3] = cut_of(m.F, m.D);
   cut[4] = cut_of(m.D, m.F);

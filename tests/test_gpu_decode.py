@@ -61,6 +61,37 @@ def test_matches_the_layers(cuda_device, monkeypatch, H, hd, F, layers, act, nor
     _check(EflaModel(cfg, device=cuda_device).eval(), B, cuts, cuda_device, monkeypatch, launches)
 
 
+def _us(model, ids, states):
+    """A step on the device, its launches queued ahead."""
+    best = []
+    with torch.no_grad():
+        for _ in range(6):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda._sleep(8_000_000)
+            e[0].record()
+            for _ in range(10):
+                model.forward_with_states(ids, states)
+            e[1].record()
+            torch.cuda.synchronize()
+            best.append(100 * e[0].elapsed_time(e[1]))
+    return min(best)
+
+
+@pytest.mark.parametrize("H,hd,prism,most", [(16, 128, True, 2.1), (8, 128, False, 1.55)])
+def test_scan_and_state_are_spread(cuda_device, H, hd, prism, most):
+    """Eight sequences against one. 2048 wide the product beside the states leaves eight CTAs without a tile, 128 states are too many for those; without PRISM no
+    product goes beside the scan. Measured 1.6 and 1.3; with everything on those few CTAs 3.0 and 2.0."""
+    torch.manual_seed(0)
+    m = EflaModel(_config(2, H, hd, 4 * H * hd, prism=prism), device=cuda_device).eval()
+    us = []
+    for B in (1, 8):
+        ids = torch.randint(0, 264, (B, 5), generator=torch.Generator().manual_seed(1)).to(cuda_device)
+        with torch.no_grad():
+            _, states = m.forward_with_states(ids[:, :4])
+        us.append(_us(m, ids[:, 4:], states))
+    assert us[1] < most * us[0]
+
+
 def test_under_capture_and_on_two_streams(cuda_device):
     """A captured step replays; two streams decode side by side, each call with its own barrier."""
     m = EflaModel(_config(2, 4, 64, 256), device=cuda_device).eval()
