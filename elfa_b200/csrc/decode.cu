@@ -718,6 +718,18 @@ void efla_cuts(const EflaDims& m, Cut* cut) {
   cut[4] = cut_of(m.D, m.F);
 }
 
+// Whether a layer takes less time here than as a chain: what the launches cost, against what every CTA does again on the rows (M D values) and the half
+// blocks of further rounds of tiles, where the chain's own grids take one. Microseconds, from 328 shapes (256 to 4096 wide, 1, 2, 4 and 8 rows, MLPs 2, 8 / 3
+// and 4 times as wide, heads of 64 and 128, with PRISM and without): the slower form is taken at 17 of them, by up to 9 %. Two layers, chain / kernel: 1024 wide,
+// MLP 4096, PRISM, B 1 155 / 70, B 8 151 / 102, without PRISM, B 8 90 / 79; 2048 wide, MLP 8192, PRISM, B 1 180 / 127, B 8 197 / 202, without, B 1 122 / 109, B 8
+// 138 / 155; 2560 wide, MLP 10240, PRISM, B 4 209 / 238, without, B 8 157 / 260; 4096 wide, MLP 8192, PRISM, B 1 252 / 196, B 4 252 / 286.
+bool efla_decode_better(const EflaDims& m, const Cut* cut) {
+  int again = 0;
+  for (int i = 0; i < 5; ++i)
+    if (cut[i].rounds > 1) again += (cut[i].rounds - 1) * ((cut[i].ks + BLOCK_ROWS - 1) / BLOCK_ROWS) * (cut[i].narrow ? 1 : 2);
+  return (m.prism ? 28 : 17) > 1.4 * (double)(m.B * m.T * m.D) / 1024 + again;
+}
+
 }  // namespace
 
 bool efla_decode_fits(const EflaDims& m) {
@@ -732,8 +744,12 @@ bool efla_decode_fits(const EflaDims& m) {
   Cut cut[5];
   efla_cuts(m, cut);
   const int lda = pitch_of((int)m.D, cut, 5), bytes = shared_bytes((int)M, lda, ring_halves((int)M, lda));
-  return (m.d == 32 ? room<efla_decode_kernel<32>>(bytes)
-                    : (m.d == 64 ? room<efla_decode_kernel<64>>(bytes) : (m.d == 96 ? room<efla_decode_kernel<96>>(bytes) : room<efla_decode_kernel<128>>(bytes)))) > 0;
+  const int clusters = m.d == 32 ? room<efla_decode_kernel<32>>(bytes)
+                                 : (m.d == 64 ? room<efla_decode_kernel<64>>(bytes)
+                                              : (m.d == 96 ? room<efla_decode_kernel<96>>(bytes) : room<efla_decode_kernel<128>>(bytes)));
+  if (clusters <= 0) return false;
+  deal_out(cut, 5, clusters);
+  return efla_decode_better(m, cut);
 }
 
 int efla_decode(const unsigned long long* p, const EflaDims& m, const EflaWork& w, const float* forget, float eps, cudaStream_t s) {

@@ -61,6 +61,25 @@ def test_matches_the_layers(cuda_device, monkeypatch, H, hd, F, layers, act, nor
     _check(EflaModel(cfg, device=cuda_device).eval(), B, cuts, cuda_device, monkeypatch, launches)
 
 
+@pytest.mark.parametrize("H,hd,F,L,W,prism,B,cuts", [
+    (20, 128, 5120, 2, 4, False, 8, (0, 3, 4, 5)),      # two and three rounds of tiles where the chain's products take one: half as long again in one kernel
+    (40, 64, 10240, 2, 4, True, 4, (0, 9, 10)),
+    (24, 128, 264, 2, 4, True, 8, (0, 5, 6)),      # eight rows of 3072 do not fit beside the weights
+    (2, 128, 264, 8, 16, True, 1, (0, 20, 23, 26)),      # nor three tokens of eight iterations in the states' scratch
+    (4, 96, 264, 8, 16, True, 1, (0, 2, 6, 10)),      # (a tail shorter than the window)
+])
+def test_the_chain_where_the_kernel_does_not_fit_or_is_slower(cuda_device, monkeypatch, H, hd, F, L, W, prism, B, cuts):
+    torch.manual_seed(0)
+    m = EflaModel(_config(1, H, hd, F, L=L, W=W, prism=prism), device=cuda_device).eval()
+    ids = torch.randint(0, 264, (B, cuts[-1]), generator=torch.Generator().manual_seed(B)).to(cuda_device)
+    with torch.no_grad():
+        _, states = m.forward_with_states(ids[:, :cuts[1]])
+        lib.raw("elfa_launch_count")(1)
+        m.forward_with_states(ids[:, cuts[1]:cuts[2]], states)
+        assert lib.raw("elfa_launch_count")(0) > 8
+    _check(m, B, cuts, cuda_device, monkeypatch, None)
+
+
 def _us(model, ids, states):
     """A step on the device, its launches queued ahead."""
     best = []
