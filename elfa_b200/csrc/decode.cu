@@ -772,6 +772,7 @@ int efla_decode(const unsigned long long* p, const EflaDims& m, const EflaWork& 
   a.lda = pitch_of(a.D, a.cut, 5);
   a.eps = eps;
   a.status = status_word();
+  ELFA_REQUIRE(a.status != nullptr, "decode: no status word");
   a.halves = ring_halves((int)(m.B * m.T), a.lda);
   const int bytes = shared_bytes((int)(m.B * m.T), a.lda, a.halves), per = 19 + 3 * (int)m.L;
   ELFA_CUDA(cudaMemsetAsync(w.arrived, 0, DECODE_COUNTERS * 4, s));

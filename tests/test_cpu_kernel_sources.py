@@ -32,3 +32,11 @@ def test_tensor_memory_is_used_by_whole_warps_after_one_lane_arrived():
     text = (CSRC / "gemm_mxfp8.cu").read_text()
     after = text[text.index("if (lane == 0) mbar_arrive_cluster(map_to_cta(over_bar, 0));"):]
     assert after.index("__syncwarp()") < min(after.index("fl & ELFA_EPI_STORE_PREACT"), after.index("tmem_ld32"))
+
+
+def test_no_kernel_is_given_a_status_word_that_is_not_there():
+    """It is allocated on first use, which fails during a stream capture, for one; a kernel that records an error would write to address zero."""
+    for f in sorted(CSRC.glob("*.cu")):
+        for m in re.finditer(r"(\S+) = (?:elfa::)?status_word\(\);", f.read_text()):
+            behind = f.read_text()[m.end():][:160]
+            assert re.match(rf"\s*(ELFA_REQUIRE\({re.escape(m[1])}( != nullptr|,)|if \(!{re.escape(m[1])}\))", behind), (f.name, behind)
