@@ -419,17 +419,14 @@ __device__ __forceinline__ void put_activation(const Team& c, int M, const Cut& 
     put_slice(c, M, u, h);
     return;
   }
-  const int k0 = slice_of(c, u), nvec = (min(u.K, k0 + u.ks) - k0) / 8, gated = act == ACT_SWIGLU;
+  const int k0 = slice_of(c, u), nvec = (min(u.K, k0 + u.ks) - k0) / 8;
   each_vector(c, M, nvec, [&](int row, int vi) {
-    const bf16* at = h + (long long)row * u.K * (1 + gated) + k0 + vi * 8;
-    const uint4 gq = ld_l2(at), uq = gated ? ld_l2(at + u.K) : make_uint4(0, 0, 0, 0);
-    const uint32_t *pg = reinterpret_cast<const uint32_t*>(&gq), *pu = reinterpret_cast<const uint32_t*>(&uq);
+    const uint4 hq = ld_l2(h + (long long)row * u.K + k0 + vi * 8);
+    const uint32_t* ph = reinterpret_cast<const uint32_t*>(&hq);
     uint4 o;
     uint32_t* po = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll 1
-    for (int j = 0; j < 4; ++j)
-      po[j] = gated ? pack_bf16(apply<OP_SILU>(bf16_lo(pg[j]), 0.f, 1.f) * bf16_lo(pu[j]), apply<OP_SILU>(bf16_hi(pg[j]), 0.f, 1.f) * bf16_hi(pu[j]))
-                    : pack_bf16(activate(act, bf16_lo(pg[j])), activate(act, bf16_hi(pg[j])));
+    for (int j = 0; j < 4; ++j) po[j] = pack_bf16(activate(act, bf16_lo(ph[j])), activate(act, bf16_hi(ph[j])));
     *reinterpret_cast<uint4*>(c.a + row * c.lda + vi * 8) = o;
   });
   __syncthreads();

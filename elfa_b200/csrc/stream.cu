@@ -194,6 +194,7 @@ ELFA_API int elfa_efla_stream(const unsigned long long* p, const long long* dims
   ELFA_REQUIRE(p && dims && forget, "efla_stream: null argument");
   const EflaDims& m = *reinterpret_cast<const EflaDims*>(dims);
   ELFA_REQUIRE(m.B > 0 && m.T > 0 && m.D > 0 && m.layers > 0 && m.L >= 0 && m.L <= 8 && m.tail >= 0 && m.B * m.T < (1ll << 31), "efla_stream: bad sizes");
+  ELFA_REQUIRE(m.act != ACT_SWIGLU, "efla_stream: the block's MLP is not gated");       // (its buffers are F wide)
   auto at = [&](int i) { return reinterpret_cast<void*>(p[i]); };
   const int segments = elfa_efla_segments((int)m.B, (int)m.T, (int)m.H, (int)m.d);
   const bool step = m.T <= step_tokens;

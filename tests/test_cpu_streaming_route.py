@@ -1,11 +1,13 @@
 """Which streaming calls go to native code, decided on the CPU: the native calls are only recorded, so nothing is launched and a call that must not
 get there shows without a device."""
 import contextlib
+import ctypes
 
 import pytest
 import torch
 from torch.autograd import forward_ad
 
+from elfa_b200 import native
 from elfa_b200.config import Config
 from elfa_b200.models import streaming
 from elfa_b200.models.efla_model import EflaModel
@@ -228,3 +230,11 @@ def test_hooks_gradients_quantisers_and_parallel_layers(route, efla):
         assert route(m, IDS, {"pos": 2, "layers": layers()})
         kv[3] = kv[3].transpose(0, 1)
         assert not route(m, IDS, {"pos": 2, "layers": layers()})
+
+
+def test_a_gated_mlp_is_refused_natively():
+    """The EFLA block has none: rows of 2 F would leave a workspace of F. Refused before anything is issued."""
+    dims = (ctypes.c_longlong * 14)(1, 1, 64, 2, 32, 64, 32, 1, 0, 1, streaming._ACTS["swiglu"], 0, 0, 0)
+    p = (ctypes.c_uint64 * 26)()
+    with pytest.raises(native.NativeError, match="not gated"):
+        native.lib.call("elfa_efla_stream", ctypes.addressof(p), ctypes.addressof(dims), ctypes.addressof((ctypes.c_float * 1)()), 1e-5, 16, 0)
