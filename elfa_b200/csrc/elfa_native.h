@@ -40,6 +40,7 @@ int elfa_pinned_free(void* p);
 int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                    long long ldc, int a_mn_major, int b_mn_major, const void* bias, const void* aux, long long ldaux,
                    void* preact, long long ldpre, float alpha, unsigned flags, int force_bn, int max_ctas, void* stream);
+int elfa_gemm_bf16_tile(int M, int N, unsigned flags, int force_bn, int max_ctas);
 int elfa_gemm_bf16_parts_count(int M, int N, int K);
 int elfa_gemm_bf16_parts(const void* A, const void* B, float* parts, int M, int N, int K, long long lda, long long ldb, void* stream);
 

@@ -1125,6 +1125,20 @@ int pick_bn(int M, int N, int forced) {
 
 using namespace elfa;
 
+// Columns of a tile for a product of more than a few rows; 512 is the CTA-pair kernel (256 x 256 tiles per pair), which is used when the problem fills at
+// least one wave of pairs with such tiles, or where force_bn says so.
+ELFA_API int elfa_gemm_bf16_tile(int M, int N, unsigned flags, int force_bn, int max_ctas) {
+  const int ctas = (max_ctas > 0 && max_ctas < sm_count()) ? max_ctas : sm_count();
+  if (force_bn == 512 ||
+      (force_bn == 0 && N >= 256 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= sm_count() / 2 && (max_ctas <= 0 || max_ctas >= sm_count())))
+    return 512;
+  const int BN = pick_bn(M, N, force_bn);
+  // A product that makes no more than one wave of 64-wide tiles takes those: its time is that of one CTA's walk over the contraction, and a block of
+  // such a tile brings 24 KB for 32 (M 128, B [K, N]: N 1024, K 1024 9.3 -> 8.2 us, N 1024, K 4096 21.5 -> 20.2, N 4096, K 1024 10.8 -> 9.3; past one wave, M 260, N 4096,
+  // 16.4 -> 18.5 with the timing's events). The sums keep their order. (fp32 outputs, whose contraction is split by the number of tiles, keep theirs.)
+  return BN == 128 && force_bn == 0 && !(flags & ELFA_EPI_OUT_F32) && (long long)((M + BM - 1) / BM) * ((N + 63) / 64) <= ctas ? 64 : BN;
+}
+
 ELFA_API int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                             long long ldc, int a_mn_major, int b_mn_major, const void* bias, const void* aux,
                             long long ldaux, void* preact, long long ldpre, float alpha, unsigned flags, int force_bn,
@@ -1150,16 +1164,8 @@ ELFA_API int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
     return launch_gemm_skinny(q, b_mn_major != 0, static_cast<cudaStream_t>(stream));
   }
 
-  // force_bn 512 selects the CTA-pair kernel (256 x 256 tiles per pair); by default it is used when the
-  // problem fills at least one wave of pairs with such tiles
-  const int pairs = sm_count() / 2;
-  const bool pair = force_bn == 512 ||
-                    (force_bn == 0 && N >= 256 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= pairs && (max_ctas <= 0 || max_ctas >= sm_count()));
-  int BN = pair ? 256 : pick_bn(M, N, force_bn);
-  // A product that makes no more than one wave of 64-wide tiles takes those: its time is that of one CTA's walk over the contraction, and a block of
-  // such a tile brings 24 KB for 32 (M 128, B [K, N]: N 1024, K 1024 9.3 -> 8.2 us, N 1024, K 4096 21.5 -> 20.2, N 4096, K 1024 10.8 -> 9.3; past one wave, M 260, N 4096,
-  // 16.4 -> 18.5 with the timing's events). The sums keep their order. (fp32 outputs, whose contraction is split by the number of tiles, keep theirs.)
-  if (BN == 128 && force_bn == 0 && !(flags & ELFA_EPI_OUT_F32) && (long long)((M + BM - 1) / BM) * ((N + 63) / 64) <= sm_count()) BN = 64;
+  const int tile = elfa_gemm_bf16_tile(M, N, flags, force_bn, max_ctas), BN = std::min(tile, 256);
+  const bool pair = tile == 512;
   CUtensorMap tmA, tmB;
   int rc;
   if (!a_mn_major) rc = cached_tmap_bf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, BK);

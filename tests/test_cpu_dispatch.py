@@ -53,3 +53,14 @@ def test_shares_of_a_key_head(shape, shares):
 def test_walks_that_are_cut(shape, forward, train):
     """Two launches and an allocation more: not for a walk that ends before the host has issued the rest of the call."""
     assert (native.lib.raw("elfa_efla_segments")(*shape) > 1, native.lib.raw("elfa_efla_segments_train")(*shape) > 1) == (forward, train)
+
+
+# M, N, most CTAs -> columns of a tile, 148 SMs
+@pytest.mark.parametrize("shape,width", [((128, 4096, 0), 64), ((128, 4096, 200), 64), ((128, 4096, 64), 64), ((128, 4096, 63), 128), ((260, 4096, 0), 128),
+                                         ((520, 1024, 80), 64), ((520, 1024, 79), 128), ((128, 64, 1), 64), ((4096, 4096, 0), 512), ((4096, 4096, 100), 256)])
+def test_a_wave_of_narrow_tiles_is_one_of_the_launch(shape, width):
+    """64 CTAs make 64 narrow tiles in one wave; fewer would go round twice."""
+    M, N, most = shape
+    tile = native.lib.raw("elfa_gemm_bf16_tile")
+    assert tile(M, N, 0, 0, most) == width
+    assert [tile(M, N, 0, n, most) for n in (64, 128, 256, 512)] == [64, 128, 256, 512]
