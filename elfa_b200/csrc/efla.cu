@@ -560,12 +560,13 @@ ELFA_API int elfa_shortconv_fwd(const void* x, const void* w, const void* bias, 
 // position straight from [C, W], where every lane touches another line: long blocks cost it 5 (W 4), 9 (8), 30 (16), 24 (24), 114 (32) and 226 (64)
 // microseconds per 10^6 values. Measured, one kernel / ordinary ones, microseconds: W 4, 1 sequence 2^20 values 6.9 / 6.5, 2^22 21 / 10, 4 sequences
 // 2^22 21 / 26; W 8 2^20 11 / 7 and 11 / 11; W 16 2^17 6.6 / 6.4 and 6.6 / 8.2, 2^18 10.6 / 6.5 and 10.6 / 8.4, 2^22 125 / 13; W 24 2^18 10 / 12,
-// 2^19 19 / 12 and 19 / 18; W 32 2^16 13 / 12 and 14 / 17, 2^17 21 / 12 and 21 / 17; W 64 2^15 17 / 14 and 19 / 22, 2^16 23 / 15 and 25 / 22, 2^20 245 / 17.
+// 2^19 19 / 12 and 19 / 18; W 32 2^16 13 / 12 and 14 / 17, 2^17 21 / 12 and 21 / 17; W 48 2^17 17 / 13 and 17 / 19;
+// W 64 2^15 17 / 14 and 19 / 22, 2^16 23 / 15 and 25 / 22, 2^20 245 / 17; W 100 2^16 23 / 17 and 23 / 23; W 128 2^16 41 / 20 and 41 / 25.
 static bool shortconv_stream_long(int B, int T, int C, int W) {
   const long long values = (long long)B * T * C;
   if (W < 8) return B == 1 && values >= 1 << 21;
   if (W < 16) return values >= 1 << 20;
-  return values >= 1 << (W == 16 ? 18 : (W < 32 ? 19 : 17));
+  return values >= 1 << (W == 16 ? 18 : (W < 32 ? 19 : (W < 64 ? 17 : 16)));
 }
 
 // `bytes` of each of B batches. One copy of rows wants them apart and a pitch below 2^31 bytes (a block of a million positions of 1024 values is
