@@ -261,10 +261,10 @@ class _ShortConv(torch.autograd.Function):
         dyc = dy.contiguous()
         dx = torch.empty_like(xc)
         slices = lib.raw("elfa_shortconv_bwd_slices")(B, T, C, W)
-        kind = torch.bfloat16 if slices and weight.dtype == torch.bfloat16 else torch.float32      # the last sum rounds, or a cast behind it
+        kind = torch.bfloat16 if weight.dtype == torch.bfloat16 else torch.float32      # the last sum rounds
         dw = torch.empty((C, W), dtype=kind, device=xc.device)
         db = torch.empty(C, dtype=kind, device=xc.device) if ctx.has_bias else None
-        part = torch.empty((slices, W + 1, C), dtype=torch.float32, device=xc.device) if slices else None
+        part = torch.empty((slices, W + 1, C), dtype=torch.float32, device=xc.device)
         lib.call("elfa_shortconv_bwd_as", xc, weight, dyc, dx, dw, db, part, int(kind == torch.bfloat16), B, T, C, W, stream_ptr(xc))
         return dx, dw.to(weight.dtype), (db.to(weight.dtype) if db is not None else None)
 
