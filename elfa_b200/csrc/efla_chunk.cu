@@ -1540,7 +1540,8 @@ ELFA_API int elfa_efla_chunk_bwd(const void* k, const void* v, const void* nmat,
   return elfa_efla_chunk_bwd_cut(k, v, nmat, coef, ckpt, dout, dstate_out, dk, dv, dbeta_tok, dstate0, dckpt, nullptr, 1, B, T, H, d, stream);
 }
 
-// The same in segments, see elfa_efla_chunk_fwd_cut.
+// The same in segments, see elfa_efla_chunk_fwd_cut. (Training takes the sum below; these two are for callers that want the terms of beta's gradient per
+// token, the tests of that sum among them.)
 ELFA_API int elfa_efla_chunk_bwd_cut(const void* k, const void* v, const void* nmat, const float* coef, const float* ckpt, const void* dout,
                                      const float* dstate_out, void* dk, void* dv, float* dbeta_tok, float* dstate0,
                                      float* dckpt, float* work, int segments, int B, int T, int H, int d, void* stream) {

@@ -22,7 +22,8 @@ def _inputs(dev, B, T, H, d):
 
 
 def _run(P, k, v, beta, s0, do, ds):
-    """Forward and backward through the native entry points with the walk in P segments."""
+    """Forward and backward through the native entry points with the walk in P segments; backward in both of its forms, with beta's terms per token and, as
+    training calls it, with their sum (bounded as below)."""
     B, T, H, d = k.shape
     n = (T + 31) // 32
     new = lambda *s, dt=torch.float32: torch.empty(*s, dtype=dt, device=k.device)
@@ -31,7 +32,14 @@ def _run(P, k, v, beta, s0, do, ds):
     o, s, dk, dv, ds0, db = torch.empty_like(k), torch.empty_like(s0), torch.empty_like(k), torch.empty_like(k), torch.empty_like(s0), new(B * T * H)
     lib.call("elfa_efla_chunk_fwd_cut", k, v, beta, s0, o, s, ckpt, nmat, coef, work, P, B, T, H, d, stream_ptr(k))
     lib.call("elfa_efla_chunk_bwd_cut", k, v, nmat, coef, ckpt, do, ds, dk, dv, db, ds0, dckpt, work, P, B, T, H, d, stream_ptr(k))
+    dk2, dv2, ds2, terms, total = torch.empty_like(dk), torch.empty_like(dv), torch.empty_like(ds0), new(B * H * n), new(1)
+    lib.call("elfa_efla_chunk_bwd_sum", k, v, nmat, coef, ckpt, do, ds, dk2, dv2, terms, total, ds2, dckpt, work, P, B, T, H, d, stream_ptr(k))
     assert native.status() == 0
+    for a, b in ((dk, dk2), (dv, dv2), (ds0, ds2)):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    db = db.double()
+    if torch.isfinite(db).all():
+        assert abs(total.item() - db.sum().item()) <= 2 ** -24 * (db.abs().sum() + db.sum().abs()).item()
     return o, s, dk, dv, ds0
 
 
