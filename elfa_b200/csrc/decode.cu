@@ -701,7 +701,13 @@ int launch(P& p, int bytes, cudaStream_t s) {
   at[1].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  ELFA_CUDA(cudaLaunchKernelEx(&cfg, Kernel, p));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, Kernel, p);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {       // the stream has a part of the SMs only (a green context)
+    cudaGetLastError();
+    set_last_error("decode: the CTAs do not run at once on this stream");
+    return ELFA_ERR_UNSUPPORTED;
+  }
+  ELFA_CUDA(e);
   ::elfa::count_launches(1);
   return ELFA_OK;
 }

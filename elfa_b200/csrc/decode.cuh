@@ -17,7 +17,8 @@ struct EflaWork {
 constexpr int ACT_SWIGLU = -1, ACT_GELU = 0;
 constexpr int DECODE_COUNTERS = 64;        // barrier counters: one per launch
 
-// Whether a call can take the one-kernel form; if so efla_decode issues it up to and with the final norm, whose rows are left in w.n.
+// Whether a call can take the one-kernel form; if so efla_decode issues it up to and with the final norm, whose rows are left in w.n. ELFA_ERR_UNSUPPORTED:
+// the stream has too few SMs for it, and the call is the chain's after all (which writes everything anew).
 bool efla_decode_fits(const EflaDims& m);
 int efla_decode(const unsigned long long* p, const EflaDims& m, const EflaWork& w, const float* forget, float eps, cudaStream_t s);
 

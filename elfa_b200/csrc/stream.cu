@@ -204,9 +204,12 @@ ELFA_API int elfa_efla_stream(const unsigned long long* p, const long long* dims
   const int rows = (int)(m.B * m.T), D = (int)m.D, B = (int)m.B, T = (int)m.T, H = (int)m.H, d = (int)m.d, L = (int)m.L, kind = (int)m.kind, G = D / d;
   const int hd = H * d, per = 19 + 3 * L;
   if (step && efla_decode_fits(m)) {
-    STREAM_CALL(efla_decode(p, m, w, forget, eps, s));
-    const PdlScope head(true);
-    return logits(w.n, at(4), at(5), rows, D, (int)m.V, stream);
+    const int rc = efla_decode(p, m, w, forget, eps, s);
+    if (rc == ELFA_OK) {
+      const PdlScope head(true);
+      return logits(w.n, at(4), at(5), rows, D, (int)m.V, stream);
+    }
+    if (rc != ELFA_ERR_UNSUPPORTED) return rc;
   }
   STREAM_CALL(elfa_embedding_fwd(static_cast<const long long*>(at(0)), at(1), nullptr, w.x[0], rows, D, T, 1, 0, 0, (int)m.V, (int)m.V, stream));
   const PdlScope chain(m.B * m.T <= 8);        // decoding, as above

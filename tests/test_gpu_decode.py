@@ -136,3 +136,28 @@ def test_under_capture_and_on_two_streams(cuda_device):
             assert torch.equal(out, want)
         del graph
     assert native.status() == 0
+
+
+def test_on_a_part_of_the_gpu(cuda_device):
+    """A stream of a green context has fewer SMs than the one-kernel form needs at once: the chain, and no error is left behind."""
+    green = pytest.importorskip("torch.cuda.green_contexts")
+    m = EflaModel(_config(2, 4, 64, 256), device=cuda_device).eval()
+    ids = torch.randint(0, 264, (2, 10), generator=torch.Generator().manual_seed(1)).to(cuda_device)
+    with torch.no_grad():
+        _, states = m.forward_with_states(ids[:, :9])
+        want, _ = m.forward_with_states(ids[:, 9:], states)
+        torch.cuda.synchronize()
+        try:
+            part = green.GreenContext.create(num_sms=32, device_id=cuda_device.index or 0)
+        except RuntimeError as e:
+            pytest.skip(str(e))
+        with torch.cuda.stream(part.Stream()):
+            got, _ = m.forward_with_states(ids[:, 9:], states)
+        torch.cuda.synchronize()
+        part.set_context()
+        try:
+            also, _ = m.forward_with_states(ids[:, 9:], states)
+            torch.cuda.synchronize()
+        finally:
+            part.pop_context()
+    assert torch.equal(got, want) and torch.equal(also, want) and native.status() == 0
