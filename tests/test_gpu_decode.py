@@ -54,6 +54,10 @@ def _check(model, B, cuts, dev, monkeypatch, launches):
     (32, 96, 264, 1, "gelu", "layernorm", 8, 16, True, 1, (0, 20, 21, 23), 2),      # 3072 wide; several rounds of gate logits
     (4, 64, 256, 9, "relu", "rmsnorm", 2, 4, True, 1, (0, 4, 12), 3),      # a layer more than one launch holds, eight tokens
     (4, 64, 256, 2, "gelu", "rmsnorm", 1, 1, False, 4, (0, 2, 4), 2),
+    (4, 64, 264, 1, "gelu", "layernorm", 2, 4, True, 3, (0, 6, 7), 2),      # rows that end inside a pair of the fragments' columns
+    (8, 32, 256, 1, "silu", "rmsnorm", 1, 8, True, 5, (0, 7, 8), 2),
+    (2, 96, 200, 1, "relu", "rmsnorm", 2, 16, True, 7, (0, 17, 18), 2),
+    (2, 128, 264, 1, "gelu", "rmsnorm", 1, 1, False, 7, (0, 2, 3), 2),
 ])
 def test_matches_the_layers(cuda_device, monkeypatch, H, hd, F, layers, act, norm, L, W, prism, B, cuts, launches):
     torch.manual_seed(0)
