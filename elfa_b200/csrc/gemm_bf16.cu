@@ -1134,9 +1134,12 @@ ELFA_API int elfa_gemm_bf16_tile(int M, int N, unsigned flags, int force_bn, int
     return 512;
   const int BN = pick_bn(M, N, force_bn);
   // A product that makes no more than one wave of 64-wide tiles takes those: its time is that of one CTA's walk over the contraction, and a block of
-  // such a tile brings 24 KB for 32 (M 128, B [K, N]: N 1024, K 1024 9.3 -> 8.2 us, N 1024, K 4096 21.5 -> 20.2, N 4096, K 1024 10.8 -> 9.3; past one wave, M 260, N 4096,
-  // 16.4 -> 18.5 with the timing's events). The sums keep their order. (fp32 outputs, whose contraction is split by the number of tiles, keep theirs.)
-  return BN == 128 && force_bn == 0 && !(flags & ELFA_EPI_OUT_F32) && (long long)((M + BM - 1) / BM) * ((N + 63) / 64) <= ctas ? 64 : BN;
+  // such a tile brings 24 KB for 32 (M 128, B [K, N]: N 1024, K 1024 9.3 -> 8.2 us, N 1024, K 4096 21.5 -> 20.2, N 4096, K 1024 10.8 -> 9.3; past one wave, M 260,
+  // N 4096, 16.4 -> 18.5 with the timing's events). Not where many of them ask for the same few rows of A at once: M 16, K 1024, N 9216 10.3 us 128 wide, 12.3
+  // 64 wide; M 9, K 4096, N 4096 20 % longer; A [K, M], M 24, N 5120 up to 25 %; 48 tiles and fewer are never slower, and from 64 rows on none are. The sums
+  // keep their order. (fp32 outputs, whose contraction is split by the number of tiles, keep theirs.)
+  const long long across = (N + 63) / 64, narrow = (long long)((M + BM - 1) / BM) * across;
+  return BN == 128 && force_bn == 0 && !(flags & ELFA_EPI_OUT_F32) && narrow <= ctas && (M >= 64 || across <= 48) ? 64 : BN;
 }
 
 ELFA_API int elfa_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,

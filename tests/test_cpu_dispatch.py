@@ -57,9 +57,10 @@ def test_walks_that_are_cut(shape, forward, train):
 
 # M, N, most CTAs -> columns of a tile, 148 SMs
 @pytest.mark.parametrize("shape,width", [((128, 4096, 0), 64), ((128, 4096, 200), 64), ((128, 4096, 64), 64), ((128, 4096, 63), 128), ((260, 4096, 0), 128),
-                                         ((520, 1024, 80), 64), ((520, 1024, 79), 128), ((128, 64, 1), 64), ((4096, 4096, 0), 512), ((4096, 4096, 100), 256)])
+                                         ((520, 1024, 80), 64), ((520, 1024, 79), 128), ((128, 64, 1), 64), ((4096, 4096, 0), 512), ((4096, 4096, 100), 256),
+                                         ((9, 3072, 0), 64), ((16, 3080, 0), 128), ((63, 9216, 0), 128), ((64, 9216, 0), 64)])
 def test_a_wave_of_narrow_tiles_is_one_of_the_launch(shape, width):
-    """64 CTAs make 64 narrow tiles in one wave; fewer would go round twice."""
+    """64 CTAs make 64 narrow tiles in one wave; fewer would go round twice. Few rows, which all of them ask for, go to fewer tiles."""
     M, N, most = shape
     tile = native.lib.raw("elfa_gemm_bf16_tile")
     assert tile(M, N, 0, 0, most) == width
