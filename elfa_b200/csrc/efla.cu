@@ -297,17 +297,97 @@ __device__ __noinline__ void shortconv_rows(const __nv_bfloat16* ib, const __nv_
   }
 }
 
+// Sequences of up to N steps (2, or SC_FEW), 16 / N of them in flight, forward and input gradient: step s is time s or T - 1 - s, all of a sequence's
+// outputs from its registers, and no other products than those of the sums, which run over j in order as below. A warp takes sequence after sequence, its
+// weights in registers; bound by memory (4096 sequences of two steps, 1024 channels, W 5: 34 MB in 8.3 us). A block of 16 taps by 16 steps is made whatever
+// the sequence fills of it. us, output / all gradients, in such blocks -> so: W 5, 4096 x 2 x 1024 92 / 361 -> 8 / 25, 1024 x 4 x 1024 27 / 79 -> 8 / 23,
+// 512 x 8 x 1024 16.5 / 45 -> 8 / 21; W 64 298 / 1143 -> 12 / 52, 80 / 361 -> 17 / 50, 43 / 189 -> 21 / 49. (From nine steps on the blocks: 512 x 9 x 1024,
+// W 5, 16.5 / 46.) grid (any, ceil(C / 64)), block (32, SC_WARPS)
+constexpr int SC_FEW = 8;
+template <bool DX, int N>
+__global__ void __launch_bounds__(32 * SC_WARPS) shortconv_few_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w,
+                                                                      const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, int B, int T,
+                                                                      int C, int W) {
+  const int c = blockIdx.y * 64 + 2 * threadIdx.x, taps = min(W, T);
+  if (c >= C) return;
+  uint64_t wv[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    wv[j] = j < taps ? pack_f32x2(__bfloat162float(w[(long long)c * W + j]), __bfloat162float(w[(long long)(c + 1) * W + j])) : 0ull;
+  const uint64_t b2 = !DX && bias ? pack_f32x2(__bfloat162float(bias[c]), __bfloat162float(bias[c + 1])) : 0ull;
+#pragma unroll (16 / N)
+  for (int b = blockIdx.x * SC_WARPS + threadIdx.y; b < B; b += gridDim.x * SC_WARPS) {
+    const __nv_bfloat16* ib = in + (long long)b * T * C + c;
+    __nv_bfloat16* ob = out + (long long)b * T * C + c;
+    uint32_t q[N];
+#pragma unroll
+    for (int s = 0; s < N; ++s) q[s] = ld_pair(ib, DX ? T - 1 - s : s, C, s < T);
+#pragma unroll
+    for (int s = 0; s < N; ++s)
+      if (s < T) {
+        uint64_t a = b2;
+#pragma unroll
+        for (int j = 0; j <= s; ++j)
+          if (j < taps) a = fma_f32x2(pair_f32x2(q[s - j]), wv[j], a);
+        float lo, hi;
+        unpack_f32x2(a, lo, hi);
+        *reinterpret_cast<uint32_t*>(ob + (long long)(DX ? T - 1 - s : s) * C) = pack_bf16(lo, hi);
+      }
+  }
+}
+// and the weight gradient, as shortconv_dw_kernel leaves it. grid (ceil(slices / 4), ceil(C / 64)), block (32, 4)
+template <int N>
+__global__ void __launch_bounds__(128) shortconv_few_dw_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+                                                               float* __restrict__ part, int B, int T, int C, int W, int seqs, int slices) {
+  const int c = blockIdx.y * 64 + 2 * threadIdx.x, unit = blockIdx.x * 4 + threadIdx.y;
+  if (c >= C || unit >= slices) return;
+  uint64_t acc[N], accb = 0ull;
+#pragma unroll
+  for (int j = 0; j < N; ++j) acc[j] = 0ull;
+  const int b1 = min(B, (unit + 1) * seqs);
+#pragma unroll (16 / N)
+  for (int b = unit * seqs; b < b1; ++b) {
+    const __nv_bfloat16 *xb = x + (long long)b * T * C + c, *gb = dy + (long long)b * T * C + c;
+    uint32_t xq[N], gq[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      xq[t] = ld_pair(xb, t, C, t < T);
+      gq[t] = ld_pair(gb, t, C, t < T);
+    }
+#pragma unroll
+    for (int t = 0; t < N; ++t)
+      if (t < T) {
+        const uint64_t g = pair_f32x2(gq[t]);
+        accb = add_f32x2(accb, g);
+#pragma unroll
+        for (int j = 0; j <= t; ++j) acc[j] = fma_f32x2(pair_f32x2(xq[t - j]), g, acc[j]);
+      }
+  }
+  float* pb = part + (long long)unit * (W + 1) * C + c;
+  auto put = [&](int j, uint64_t v) {
+    float lo, hi;
+    unpack_f32x2(v, lo, hi);
+    *reinterpret_cast<float2*>(pb + (long long)j * C) = make_float2(lo, hi);
+  };
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (j < W) put(j, acc[j]);
+  for (int j = N; j < W; ++j) put(j, 0ull);
+  put(W, accb);
+}
+
 // Forward (y[t] = bias + sum_j x[t - j] w[j]) and, walked from late to early, the input gradient (dx[t] = sum_j dy[t + j] w[j]); step s is time s or
 // T - 1 - s. The sum of an output runs over j in order, as in shortconv_stream_kernel. What lies outside the sequence is zero, which finite weights leave
-// so. grid (ceil(B * tiles / SC_WARPS), ceil(C / 64)), block (32, SC_WARPS), dynamic shared memory: the weights, W by SC_WLD floats.
+// so. taps: those that a sequence meets, min(W, T). grid (ceil(B * tiles / SC_WARPS), ceil(C / 64)), block (32, SC_WARPS), dynamic shared memory: the
+// weights, taps by SC_WLD floats.
 template <bool DX>
 __global__ void __launch_bounds__(32 * SC_WARPS, 2) shortconv_tile_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w,
                                                                           const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out,
-                                                                          int B, int T, int C, int W, int tiles) {
+                                                                          int B, int T, int C, int W, int taps, int tiles) {
   extern __shared__ __align__(16) float sw[];
   const int lane = threadIdx.x, warp = threadIdx.y, c0 = blockIdx.y * 64;
   float z = 0.f;
-  for (int j = lane; j < W; j += 32) {                   // consecutive lanes read consecutive weights of a channel
+  for (int j = lane; j < taps; j += 32) {                   // consecutive lanes read consecutive weights of a channel
 #pragma unroll
     for (int i = 0; i < 64 / SC_WARPS; ++i) {
       const int cl = warp + i * SC_WARPS;
@@ -349,7 +429,7 @@ __global__ void __launch_bounds__(32 * SC_WARPS, 2) shortconv_tile_kernel(const 
   auto block = [&](auto half, auto whole, int j0) {
     constexpr int H = decltype(half)::value * SC_TILE;
     uint32_t nx[SC_TILE];
-    if (j0 + SC_TILE < W) {
+    if (j0 + SC_TILE < taps) {
       get(nx, s0 - j0 - SC_TILE);
     } else {
 #pragma unroll
@@ -357,7 +437,7 @@ __global__ void __launch_bounds__(32 * SC_WARPS, 2) shortconv_tile_kernel(const 
     }
 #pragma unroll
     for (int jj = 0; jj < SC_TILE; ++jj) {
-      if (!whole.value && j0 + jj >= W) break;           // an input that is not finite would make NaN of a tap of zero
+      if (!whole.value && j0 + jj >= taps) break;        // an input that is not finite would make NaN of a tap of zero
       const uint64_t wv = *reinterpret_cast<const uint64_t*>(sw + (j0 + jj) * SC_WLD + 2 * lane);
 #pragma unroll
       for (int r = 0; r < SC_TILE; ++r) acc[r] = fma_f32x2(win[(r - jj - H) & 31], wv, acc[r]);
@@ -367,13 +447,13 @@ __global__ void __launch_bounds__(32 * SC_WARPS, 2) shortconv_tile_kernel(const 
   };
   using Even = std::integral_constant<int, 0>;
   using Odd = std::integral_constant<int, 1>;
-  const int full = W / (2 * SC_TILE) * (2 * SC_TILE);
+  const int full = taps / (2 * SC_TILE) * (2 * SC_TILE);
   for (int j0 = 0; j0 < full; j0 += 2 * SC_TILE) {
     block(Even{}, std::true_type{}, j0);
     block(Odd{}, std::true_type{}, j0 + SC_TILE);
   }
-  if (full < W) block(Even{}, std::false_type{}, full);
-  if (full + SC_TILE < W) block(Odd{}, std::false_type{}, full + SC_TILE);
+  if (full < taps) block(Even{}, std::false_type{}, full);
+  if (full + SC_TILE < taps) block(Odd{}, std::false_type{}, full + SC_TILE);
   __nv_bfloat16* o = ob + (long long)(DX ? T - 1 - s0 : s0) * C;
   const long long step = DX ? -(long long)C : C;
 #pragma unroll
@@ -408,7 +488,7 @@ __global__ void __launch_bounds__(128, 3) shortconv_dw_kernel(const __nv_bfloat1
   uint64_t acc[SC_TILE], accb = 0ull;
 #pragma unroll
   for (int j = 0; j < SC_TILE; ++j) acc[j] = 0ull;
-  for (int b = b0; b < b1; ++b) {
+  for (int b = j0 < T ? b0 : b1; b < b1; ++b) {          // (taps longer than the sequence: zero)
     const __nv_bfloat16 *xb = x + (long long)b * T * C + c, *gb = dy + (long long)b * T * C + c;
     uint64_t win[2 * SC_TILE];                           // input t0 - j0 + p is in slot p mod 32
     uint32_t nx[SC_TILE], ng[SC_TILE];
@@ -464,9 +544,18 @@ __global__ void __launch_bounds__(128, 3) shortconv_dw_kernel(const __nv_bfloat1
 template <bool DX>
 int launch_shortconv_tile(const __nv_bfloat16* in, const __nv_bfloat16* w, const __nv_bfloat16* bias, __nv_bfloat16* out, int B, int T, int C, int W,
                           cudaStream_t s) {
-  const int tiles = (T + SC_TILE - 1) / SC_TILE;
+  const int tiles = (T + SC_TILE - 1) / SC_TILE, taps = std::min(W, T);
+  if (T <= SC_FEW) {
+    const long long groups = (C + 63) / 64, all = ((long long)B + SC_WARPS - 1) / SC_WARPS, room = std::max(1ll, 148 * 8 / groups);
+    const dim3 g((unsigned)std::min(all, room), (unsigned)groups), blk(32, SC_WARPS);
+    if (T <= 2) shortconv_few_kernel<DX, 2><<<g, blk, 0, s>>>(in, w, bias, out, B, T, C, W);
+    else shortconv_few_kernel<DX, SC_FEW><<<g, blk, 0, s>>>(in, w, bias, out, B, T, C, W);
+    ELFA_CUDA(cudaGetLastError());
+    ::elfa::count_launches(1);
+    return ELFA_OK;
+  }
   const dim3 grid((unsigned)(((long long)B * tiles + SC_WARPS - 1) / SC_WARPS), (C + 63) / 64), block(32, SC_WARPS);
-  shortconv_tile_kernel<DX><<<grid, block, (size_t)W * SC_WLD * sizeof(float), s>>>(in, w, bias, out, B, T, C, W, tiles);
+  shortconv_tile_kernel<DX><<<grid, block, (size_t)taps * SC_WLD * sizeof(float), s>>>(in, w, bias, out, B, T, C, W, taps, tiles);
   ELFA_CUDA(cudaGetLastError());
   ::elfa::count_launches(1);
   return ELFA_OK;
@@ -641,8 +730,14 @@ ELFA_API int elfa_shortconv_bwd_as(const void* x, const void* w, const void* dy,
     const int rc = launch_shortconv_tile<true>(G, Wt, nullptr, DX, B, T, C, W, s);
     if (rc != ELFA_OK) return rc;
     const ShortConvSlices q = shortconv_slices(B, T, C, W);
-    shortconv_dw_kernel<<<dim3((q.slices + 3) / 4, (C + 63) / 64, (W + SC_TILE - 1) / SC_TILE), dim3(32, 4), 0, s>>>(X, G, part, B, T, C, W, q.span, q.spans,
-                                                                                                                  q.seqs, q.slices);
+    const dim3 few((q.slices + 3) / 4, (C + 63) / 64);
+    if (T <= 2)
+      shortconv_few_dw_kernel<2><<<few, dim3(32, 4), 0, s>>>(X, G, part, B, T, C, W, q.seqs, q.slices);
+    else if (T <= SC_FEW)
+      shortconv_few_dw_kernel<SC_FEW><<<few, dim3(32, 4), 0, s>>>(X, G, part, B, T, C, W, q.seqs, q.slices);
+    else
+      shortconv_dw_kernel<<<dim3((q.slices + 3) / 4, (C + 63) / 64, (W + SC_TILE - 1) / SC_TILE), dim3(32, 4), 0, s>>>(X, G, part, B, T, C, W, q.span, q.spans,
+                                                                                                                    q.seqs, q.slices);
     slices = q.slices;
   }
   ELFA_CUDA(cudaGetLastError());
