@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(NT, 2) efla_decode_kernel(const __grid_constan
         float S[HD / 4];                               // the first rows are on their way while keys and deltas are formed
         int row = c.tid >> 2;
         if (row < HD) prism_state_load<HD>(S, y.p0 + ((long long)bg * HD + row) * HD, part);
-        prism_state_prepare<HD, NT, 1>(in, sm, bg, 0, p.T, c.tid, [] { __syncthreads(); });
+        prism_state_prepare<HD, NT, 1, 1>(in, sm, bg, 0, p.T, c.tid, [] { __syncthreads(); });
 #pragma unroll 1
         for (; row < HD; row += NT / 4) {
           if (row >= NT / 4) prism_state_load<HD>(S, y.p0 + ((long long)bg * HD + row) * HD, part);

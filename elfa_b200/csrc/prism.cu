@@ -10,6 +10,8 @@
 // One thread owns one (token, channel-in-group) pair and walks over the G groups, so the gradient of
 // p_l (a sum over groups) is accumulated in registers: no atomics, deterministic. Consecutive
 // threads touch consecutive channels: every access is coalesced. The backward recomputes r_l.
+#include <algorithm>
+
 #include "elfa_native.h"
 #include "prism_step.cuh"
 
@@ -329,8 +331,10 @@ __global__ void __launch_bounds__(256) prism_weight_sum_kernel(const float* __re
 // product is two shuffles) and one CTA of 4 D threads owns a (batch, group). Keys, gates and deltas of a tile of tokens are
 // formed in parallel in shared memory first, so the serial part of a token is about D / 2 + L D / 4 multiply-adds per thread. Tiles of up to 64 tokens,
 // four items of a warp or thread in flight: with tiles of eight, one item at a time and a division per iteration the preparation of a block of 64 tokens took
-// twice as long as its walk. (B 2, 16 groups of 64, two iterations, 64 tokens: 33 us, with tiles of eight 51.)
-template <int D>
+// twice as long as its walk. (B 2, 16 groups of 64, two iterations, 64 tokens: 33 us, with tiles of eight 51.) Tiles below 16 have no four items: one, and four
+// iterations of its loads in flight (one token of 16 groups of 64, eight iterations: 6.5 us, four items 10.5). Where the states are several to an SM a tile
+// takes its part of the shared memory (2048 of 32, eight iterations, 64 tokens: 352 us; half of an SM's whatever their number 830, tiles of eight 468).
+template <int D, int U>
 __global__ void __launch_bounds__(4 * D) prism_state_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ v,
                                                             const __nv_bfloat16* __restrict__ z, long long ldz, int off_b, int off_k,
                                                             const float* __restrict__ state, float* __restrict__ out, int T, int G, int L,
@@ -344,25 +348,34 @@ __global__ void __launch_bounds__(4 * D) prism_state_kernel(const __nv_bfloat16*
   for (int t0 = 0; t0 < T; t0 += tile) {
     const int n = min(tile, T - t0);
     if (t0) __syncthreads();                    // the previous tokens have been consumed
-    prism_state_prepare<D, 4 * D, 4>(in, sm, bg, t0, n, threadIdx.x, [] { __syncthreads(); });
+    prism_state_prepare<D, 4 * D, U, U == 1 ? 4 : 1>(in, sm, bg, t0, n, threadIdx.x, [] { __syncthreads(); });
     prism_state_rows<D>(S, sm, n, L, row, part, forget);
   }
   prism_state_store<D>(S, out + ((long long)bg * D + row) * D, part);
 }
 
 constexpr int PS_SHARED = 110 * 1024;           // most that a tile takes: half of an SM's
-template <int D>
-int launch_prism_state(const void* u, const void* v, const void* z, long long ldz, int off_b, int off_k, const float* state, float* out,
-                       int B, int T, int G, int L, float forget, cudaStream_t s) {
-  // tokens of a tile: up to 64 (a multiple of four: the tile's parts start on 16 bytes) in PS_SHARED
-  const int token = (2 * D + 1) * L * (int)sizeof(float), tile = T < 4 ? 4 : (T < 64 ? (T + 3) / 4 * 4 : 64), most = PS_SHARED / token / 4 * 4;
-  const int tokens = tile < most ? tile : most, bytes = tokens * token;
-  ELFA_CUDA(allow_shared<prism_state_kernel<D>>(PS_SHARED));
-  prism_state_kernel<D><<<B * G, 4 * D, bytes, s>>>(static_cast<const __nv_bfloat16*>(u), static_cast<const __nv_bfloat16*>(v),
-                                                    static_cast<const __nv_bfloat16*>(z), ldz, off_b, off_k, state, out, T, G, L, forget, tokens);
+template <int D, int U>
+int launch_prism_state_as(const void* u, const void* v, const void* z, long long ldz, int off_b, int off_k, const float* state, float* out,
+                          int B, int T, int G, int L, float forget, int tile, int bytes, cudaStream_t s) {
+  ELFA_CUDA((allow_shared<prism_state_kernel<D, U>>(PS_SHARED)));
+  prism_state_kernel<D, U><<<B * G, 4 * D, bytes, s>>>(static_cast<const __nv_bfloat16*>(u), static_cast<const __nv_bfloat16*>(v),
+                                                       static_cast<const __nv_bfloat16*>(z), ldz, off_b, off_k, state, out, T, G, L, forget, tile);
   ELFA_CUDA(cudaGetLastError());
   count_launches(1);
   return ELFA_OK;
+}
+template <int D>
+int launch_prism_state(const void* u, const void* v, const void* z, long long ldz, int off_b, int off_k, const float* state, float* out,
+                       int B, int T, int G, int L, float forget, cudaStream_t s) {
+  // tokens of a tile, a multiple of four (its parts start on 16 bytes): up to 64, as the CTAs that an SM will have, by the registers at most 1024 threads,
+  // leave room for, at least eight
+  const int token = (2 * D + 1) * L * (int)sizeof(float);
+  const long long ctas = std::min<long long>(std::max(2, 1024 / (4 * D)), std::max<long long>(2, ((long long)B * G + 147) / 148));
+  const int room = std::min(PS_SHARED, (int)(220 * 1024 / ctas)), least = std::min(8, PS_SHARED / token / 4 * 4);
+  const int most = std::max(least, std::min(64, room / token / 4 * 4)), tile = std::min(most, std::max(4, (T + 3) / 4 * 4));
+  return tile < 16 ? launch_prism_state_as<D, 1>(u, v, z, ldz, off_b, off_k, state, out, B, T, G, L, forget, tile, tile * token, s)
+                   : launch_prism_state_as<D, 4>(u, v, z, ldz, off_b, off_k, state, out, B, T, G, L, forget, tile, tile * token, s);
 }
 
 }  // namespace

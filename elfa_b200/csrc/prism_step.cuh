@@ -45,8 +45,8 @@ __device__ __forceinline__ void prism_state_store(const float (&S)[D / 4], float
 }
 
 // keys, gates and deltas of tokens t0 .. t0 + n - 1 of (batch, group) bg by NT threads (tid), U items of a warp or thread at a time so that their loads are
-// in flight together; ends with a barrier
-template <int D, int NT, int U, typename Sync>
+// in flight together, and of a delta's iterations LU; ends with a barrier
+template <int D, int NT, int U, int LU, typename Sync>
 __device__ __forceinline__ void prism_state_prepare(const PrismSource& in, const PrismTile<D>& sm, int bg, int t0, int n, int tid, Sync together) {
   const int b = bg / in.G, g = bg % in.G, warp = tid >> 5, lane = tid & 31, L = in.L, items = n * L;
   const long long ldz = in.ldz, first = (long long)b * in.T + t0;
@@ -93,7 +93,7 @@ __device__ __forceinline__ void prism_state_prepare(const PrismSource& in, const
       const long long at = (row[y] * in.G + g) * D + c;
       r[y] = __bfloat162float(in.v[at]) - __bfloat162float(in.u[at]);
     }
-#pragma unroll 1
+#pragma unroll LU
     for (int l = 0; l < L; ++l) {
       __nv_bfloat16 z[U];
 #pragma unroll

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from elfa_b200 import native, ops
-from elfa_b200.native import lib
+from elfa_b200.native import lib, stream_ptr
 from elfa_b200.ops import efla as eops
 
 pytestmark = pytest.mark.gpu
@@ -48,6 +48,29 @@ def test_state_of_any_stride(cuda_device, order):
     want = eops.prism_stream(u, v, wp, wb, wk, s0, 0.97, d)
     got = eops.prism_stream(u, v, wp, wb, wk, view, 0.97, d)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def _state_us(dev, B, G, d, L, T):
+    u, v, z = (torch.randn(B, T, n, device=dev).bfloat16() for n in (G * d, G * d, 3 * L * d))
+    s0, best = torch.randn(B, G, d, d, device=dev), []
+    s1 = torch.empty_like(s0)
+    for _ in range(5):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        torch.cuda._sleep(4_000_000)
+        e[0].record()
+        for _ in range(40):
+            lib.call("elfa_prism_state", u, v, z, 3 * L * d, L * d, 2 * L * d, s0, s1, B, T, G, d, L, 0.9, stream_ptr(u))
+        e[1].record()
+        torch.cuda.synchronize()
+        best.append(25 * e[0].elapsed_time(e[1]))
+    return min(best)
+
+
+def test_many_states_and_one_token(cuda_device):
+    """2048 states of 32, eight iterations, against 128, which are one for each SM: measured 3.0 times as long, 7.1 with tiles that leave two CTAs to an SM. One token:
+    eight iterations against two, 1.0 and, with their loads one behind the other, 1.6."""
+    assert _state_us(cuda_device, 128, 16, 32, 8, 64) < 4.5 * _state_us(cuda_device, 8, 16, 32, 8, 64)
+    assert _state_us(cuda_device, 2, 16, 64, 8, 1) < 1.35 * _state_us(cuda_device, 2, 16, 64, 2, 1)
 
 
 def test_lengths_of_several_threads(cuda_device):
