@@ -362,7 +362,9 @@ ELFA_API int elfa_xent_row_max(void) { return XENT_ROW_MAX; }
 // Threads per row: what a thread does once (the joints, the logarithm, two barriers) should be little beside its share of the row, and rows in different phases
 // should share an SM. 16384 rows, us, 32 / 64 / 128 / 256 / 512 threads: V 256 17 / 20 / 27 / 45 / 89; 1000 27 / 29 / 35 / 51 / 94; 2048 36 / 34 / 45 / 61 /
 // 101; 4096 55 / 51 / 60 / 78 / 123; 8000 119 / 94 / 95 / 108 / 160; 12000 198 / 143 / 135 / 136 / 183; 16384 305 / 216 / 192 / 167 / 218. 4096 rows: 8192
-// 42 / 34 / 34 / 35 / 47; 24000 160 / 114 / 90 / 74 / 80; 32000 266 / 162 / 125 / 98 / 94. 64 and 300 rows: the numbers taken are the best there, or within 1 us.
+// 42 / 34 / 34 / 35 / 47; 24000 160 / 114 / 90 / 74 / 80; 32000 266 / 162 / 125 / 98 / 94. Few rows leave the SMs room, and a call
+// takes what one row takes: up to two rows to an SM as for a row four times as wide, up to eight twice (16 rows: 1000 5.4 / 4.1 / 4.1 / 4.1 / 4.1, 4096 6.2 /
+// 6.2 / 4.1 / 4.1 / 4.1, 8192 10.2 / 6.2 / 6.2 / 5.1 / 5.0; 600 rows: 1000 6.2 / 5.3 / 4.1 / 4.2 / 6.2, 4096 8.2 / 6.2 / 6.2 / 6.2 / 8.2, 8192 12.3 / 8.2 / 8.2 / 8.2 / 10.2).
 ELFA_API int elfa_xent_row(void* logits, long long ld, const long long* targets, float* loss_out, int rows, int V, float smoothing,
                            float grad_scale, void* stream) {
   ELFA_REQUIRE(logits && targets && loss_out && rows > 0 && V > 0, "xent_row: bad arguments");
@@ -371,9 +373,10 @@ ELFA_API int elfa_xent_row(void* logits, long long ld, const long long* targets,
   unsigned int* st = status_word();
   ELFA_REQUIRE(st != nullptr, "xent: no status word");
   auto* s = static_cast<cudaStream_t>(stream);
-  if (V <= 1024) return launch_xent_row<32>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
-  if (V <= 4096) return launch_xent_row<64>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
-  if (V <= 8192) return launch_xent_row<128>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
+  const int w = rows <= 300 ? 4 * V : (rows <= 1200 ? 2 * V : V);
+  if (w <= 1024) return launch_xent_row<32>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
+  if (w <= 4096) return launch_xent_row<64>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
+  if (w <= 8192) return launch_xent_row<128>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
   if (V <= 24576) return launch_xent_row<256>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
   return launch_xent_row<512>(logits, ld, targets, loss_out, rows, V, smoothing, grad_scale, st, s);
 }
