@@ -8,9 +8,16 @@
 // Scan and state belong to the CTAs that have no tile of their phase's product, where those are enough for them. A phase's weights do not depend on the
 // phases before it: the blocks that fit are copied to shared memory between the arrival at the barrier and the wait, and each CTA asks for its part of the
 // next layer's into L2 there. The phases go through one copy of the code, in loops rather than unrolled: a warp that meets straight-line code for the first
-// time takes about eight cycles
-// per instruction. Two layers, 1024 wide, B 2: a step 67 us (and 17 for the logits); prompt of 64 tokens and
-// four steps 1131 us with the chain, 788 with this.
+// time takes about eight cycles per instruction. Two layers, 1024 wide, B 2: a step 67 us (and 17 for the logits); prompt of 64 tokens and four steps 1131 us
+// with the chain, 740 to 770 with this. Wide products and many rows are the chain's (efla_decode_better).
+//
+// The launch is cooperative, and its CTAs start together: it waits until all of them have room, two to an SM, whatever else runs, where the chain's small
+// launches go into what is free. Steps of 4 layers, 1024 wide, B 2, microseconds with chain / this, alone 498 / 334, and beside another stream of the same
+// priority, with that stream's passes per second: products of 4096^3 (8900 alone) 1826 / 576, 8732 / 7093; of 8192^3 (1280) 4638 / 1509, 1285 / 755; one
+// elementwise pass after the other over 0.5 GB (6170) 6846 / 486, 6128 / 3978; prompts of 4 x 2048 tokens (133 / 170), whose states' kernel holds 64 SMs for
+// a millisecond, 556 / 1209, 116 / 142. A kernel that holds 20 SMs for 200 ms keeps a step waiting for 200 ms. Four threads that decode on a stream each:
+// 3084 / 2949 steps a second. What a step waits for must not itself wait for the step (a kernel that spins for a peer which needs this step's result). On a
+// stream with a part of the SMs the chain is taken.
 //
 // The softmax family has no such kernel: cached attention and the joint of its slices are two more phases, each about as long as the launch it would
 // replace (a layer of the same width, B 4, 512 positions: 35 us in one kernel, 42 as eight launches whose starts overlap, whole calls 3 to 7 % slower).
@@ -321,9 +328,9 @@ __device__ __forceinline__ void product(const Team& c, const Cut& u, const Weigh
     }
   }
 }
-// Other work beside a product, `items` equal pieces: it belongs to the CTAs of the clusters that have no tile, where those take no more rounds than all
-// CTAs would, and otherwise to all of them, ahead of the product, those without a tile first. Two layers, eight rows, us, all on the CTAs without a tile / so: 2048 wide,
-// 16 heads of 128, w_down leaves eight CTAs for 128 states, 450 / 245; 1024 wide, 8 heads of 128, no PRISM, no product beside the scan, 147 / 95.
+// Other work beside a product, `items` equal pieces: it belongs to the CTAs of the clusters that have no tile, where those take no more rounds than all CTAs
+// would, and otherwise to all of them, ahead of the product, those without a tile first. Two layers, eight rows, us, all on the CTAs without a tile / so:
+// 2048 wide, 16 heads of 128, w_down leaves eight CTAs for 128 states, 450 / 245; 1024 wide, 8 heads of 128, no PRISM, no product beside the scan, 147 / 95.
 // (-> the CTA has a part; its number and how many there are)
 __device__ __forceinline__ bool side_work(const Team& c, const Cut& u, int items, int& at, int& n) {
   const int free = c.ctas - u.used * CL;
@@ -724,8 +731,8 @@ void efla_cuts(const EflaDims& m, Cut* cut) {
 // Whether a layer takes less time here than as a chain: what the launches cost, against what every CTA does again on the rows (M D values) and the half
 // blocks of further rounds of tiles, where the chain's own grids take one. Microseconds, from 328 shapes (256 to 4096 wide, 1, 2, 4 and 8 rows, MLPs 2, 8 / 3
 // and 4 times as wide, heads of 64 and 128, with PRISM and without): the slower form is taken at 17 of them, by up to 9 %. Two layers, chain / kernel: 1024 wide,
-// MLP 4096, PRISM, B 1 155 / 70, B 8 151 / 102, without PRISM, B 8 90 / 79; 2048 wide, MLP 8192, PRISM, B 1 180 / 127, B 8 197 / 202, without, B 1 122 / 109, B 8
-// 138 / 155; 2560 wide, MLP 10240, PRISM, B 4 209 / 238, without, B 8 157 / 260; 4096 wide, MLP 8192, PRISM, B 1 252 / 196, B 4 252 / 286.
+// MLP 4096, PRISM, B 1 136 / 70, B 8 148 / 102, without PRISM, B 8 90 / 79; 2048 wide, MLP 8192, PRISM, B 1 180 / 127, B 8 197 / 202, without, B 1 122 / 109, B 8
+// 138 / 155; 2560 wide, MLP 10240, PRISM, B 4 209 / 238, without, B 8 157 / 260; 4096 wide, MLP 8192, PRISM, B 1 239 / 196, B 4 252 / 286.
 bool efla_decode_better(const EflaDims& m, const Cut* cut) {
   int again = 0;
   for (int i = 0; i < 5; ++i)

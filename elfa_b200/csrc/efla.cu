@@ -561,8 +561,9 @@ int launch_shortconv_tile(const __nv_bfloat16* in, const __nv_bfloat16* w, const
   return ELFA_OK;
 }
 
-// The slices of shortconv_dw_kernel: no sum longer than SC_CHAIN steps (its error grows with its length: in one wave of warps, up to 2048 steps, it was
-// twice that of sums of 512), in whole waves of its warps (12 of them per SM).
+// The slices of shortconv_dw_kernel: no sum longer than SC_CHAIN steps (its error grows with its length: in one wave of warps, up to 2048 steps, it was twice
+// that of sums of 512), in whole waves of its warps (12 of them per SM). The scratch that this takes: a slice per 256 steps or more, (W + 1) C floats each:
+// 21 MB at B 8, T 2048, C 1024, W 64, 34 MB at W 128; of long inputs as many bytes as x has at W 127, half of them at W 63.
 constexpr int SC_CHAIN = 256;
 struct ShortConvSlices {
   int span, spans, seqs, slices;

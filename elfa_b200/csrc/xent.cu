@@ -359,12 +359,12 @@ ELFA_API int elfa_xent_row_max(void) { return XENT_ROW_MAX; }
 
 // Both passes in one for whole rows (no vocabulary split): the logits become d loss / d logits * grad_scale in place, loss_out gets the
 // per-token loss. V a multiple of 8 and at most elfa_xent_row_max(), rows on 16-byte boundaries.
-// Threads per row: what a thread does once (the joints, the logarithm, two barriers) should be little beside its share of the row, and rows in different phases
-// should share an SM. 16384 rows, us, 32 / 64 / 128 / 256 / 512 threads: V 256 17 / 20 / 27 / 45 / 89; 1000 27 / 29 / 35 / 51 / 94; 2048 36 / 34 / 45 / 61 /
-// 101; 4096 55 / 51 / 60 / 78 / 123; 8000 119 / 94 / 95 / 108 / 160; 12000 198 / 143 / 135 / 136 / 183; 16384 305 / 216 / 192 / 167 / 218. 4096 rows: 8192
-// 42 / 34 / 34 / 35 / 47; 24000 160 / 114 / 90 / 74 / 80; 32000 266 / 162 / 125 / 98 / 94. Few rows leave the SMs room, and a call
-// takes what one row takes: up to two rows to an SM as for a row four times as wide, up to eight twice (16 rows: 1000 5.4 / 4.1 / 4.1 / 4.1 / 4.1, 4096 6.2 /
-// 6.2 / 4.1 / 4.1 / 4.1, 8192 10.2 / 6.2 / 6.2 / 5.1 / 5.0; 600 rows: 1000 6.2 / 5.3 / 4.1 / 4.2 / 6.2, 4096 8.2 / 6.2 / 6.2 / 6.2 / 8.2, 8192 12.3 / 8.2 / 8.2 / 8.2 / 10.2).
+// Threads per row: what a thread does once (the joints, the logarithm, two barriers) should be little beside its share of the row, and rows in different
+// phases should share an SM. 16384 rows, us, 32 / 64 / 128 / 256 / 512 threads: V 256 17 / 20 / 27 / 45 / 89; 1000 27 / 29 / 35 / 51 / 94; 2048 36 / 34 / 45
+// / 61 / 101; 4096 55 / 51 / 60 / 78 / 123; 8000 119 / 94 / 95 / 108 / 160; 12000 198 / 143 / 135 / 136 / 183; 16384 305 / 216 / 192 / 167 / 218. 4096 rows:
+// 8192 42 / 34 / 34 / 35 / 47; 24000 160 / 114 / 90 / 74 / 80; 32000 266 / 162 / 125 / 98 / 94. Few rows leave the SMs room, and a call takes what one row
+// takes: up to two rows to an SM as for a row four times as wide, up to eight twice (16 rows: 1000 5.4 / 4.1 / 4.1 / 4.1 / 4.1, 4096 6.2 / 6.2 / 4.1 / 4.1 /
+// 4.1, 8192 10.2 / 6.2 / 6.2 / 5.1 / 5.0; 600 rows: 1000 6.2 / 5.3 / 4.1 / 4.2 / 6.2, 4096 8.2 / 6.2 / 6.2 / 6.2 / 8.2, 8192 12.3 / 8.2 / 8.2 / 8.2 / 10.2).
 ELFA_API int elfa_xent_row(void* logits, long long ld, const long long* targets, float* loss_out, int rows, int V, float smoothing,
                            float grad_scale, void* stream) {
   ELFA_REQUIRE(logits && targets && loss_out && rows > 0 && V > 0, "xent_row: bad arguments");
