@@ -729,15 +729,15 @@ void efla_cuts(const EflaDims& m, Cut* cut) {
 }
 
 // Whether a layer takes less time here than as a chain: what the launches cost, against what every CTA does again on the rows (M D values) and the half
-// blocks of further rounds of tiles, where the chain's own grids take one. Microseconds, from 328 shapes (256 to 4096 wide, 1, 2, 4 and 8 rows, MLPs 2, 8 / 3
-// and 4 times as wide, heads of 64 and 128, with PRISM and without): the slower form is taken at 17 of them, by up to 9 %. Two layers, chain / kernel: 1024 wide,
+// blocks of further rounds of tiles, where the chain's own grids take one. Microseconds, from 736 shapes (256 to 4096 wide, 1 to 8 rows, MLPs 2, 8 / 3
+// and 4 times as wide, heads of 64 and 128, with PRISM and without): the slower form is taken at 41 of them, by up to 10 %. Two layers, chain / kernel: 1024 wide,
 // MLP 4096, PRISM, B 1 136 / 70, B 8 148 / 102, without PRISM, B 8 90 / 79; 2048 wide, MLP 8192, PRISM, B 1 180 / 127, B 8 197 / 202, without, B 1 122 / 109, B 8
 // 138 / 155; 2560 wide, MLP 10240, PRISM, B 4 209 / 238, without, B 8 157 / 260; 4096 wide, MLP 8192, PRISM, B 1 239 / 196, B 4 252 / 286.
 bool efla_decode_better(const EflaDims& m, const Cut* cut) {
   int again = 0;
   for (int i = 0; i < 5; ++i)
     if (cut[i].rounds > 1) again += (cut[i].rounds - 1) * ((cut[i].ks + BLOCK_ROWS - 1) / BLOCK_ROWS) * (cut[i].narrow ? 1 : 2);
-  return (m.prism ? 28 : 17) > 1.4 * (double)(m.B * m.T * m.D) / 1024 + again;
+  return (m.prism ? 28 : 17) > 1.6 * (double)(m.B * m.T * m.D) / 1024 + again;
 }
 
 }  // namespace
