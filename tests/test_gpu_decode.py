@@ -100,7 +100,7 @@ def _us(model, ids, states):
     return min(best)
 
 
-@pytest.mark.parametrize("H,hd,prism,most", [(16, 128, True, 2.1), (8, 128, False, 1.55)])
+@pytest.mark.parametrize("H,hd,prism,most", [(16, 128, True, 2.1), (8, 128, False, 1.7)])
 def test_scan_and_state_are_spread(cuda_device, H, hd, prism, most):
     """Eight sequences against one. 2048 wide the product beside the states leaves eight CTAs without a tile, 128 states are too many for those; without PRISM no
     product goes beside the scan. Measured 1.6 and 1.3; with everything on those few CTAs 3.0 and 2.0."""

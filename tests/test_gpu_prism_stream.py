@@ -70,7 +70,7 @@ def test_many_states_and_one_token(cuda_device):
     """2048 states of 32, eight iterations, against 128, which are one for each SM: measured 3.0 times as long, 7.1 with tiles that leave two CTAs to an SM. One token:
     eight iterations against two, 1.0 and, with their loads one behind the other, 1.6."""
     assert _state_us(cuda_device, 128, 16, 32, 8, 64) < 4.5 * _state_us(cuda_device, 8, 16, 32, 8, 64)
-    assert _state_us(cuda_device, 2, 16, 64, 8, 1) < 1.35 * _state_us(cuda_device, 2, 16, 64, 2, 1)
+    assert _state_us(cuda_device, 2, 16, 64, 8, 1) < 1.45 * _state_us(cuda_device, 2, 16, 64, 2, 1)
 
 
 def test_lengths_of_several_threads(cuda_device):

@@ -120,4 +120,4 @@ def test_few_wide_rows_take_no_longer_than_few_narrow_ones(cuda_device):
             torch.cuda.synchronize()
             best.append(e[0].elapsed_time(e[1]))
         us.append(min(best))
-    assert us[1] < 1.25 * us[0]
+    assert us[1] < 1.4 * us[0]
